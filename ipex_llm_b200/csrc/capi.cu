@@ -181,7 +181,7 @@ static bool use_skinny(int qtype, int64_t n_rows, int64_t k, int64_t m, int x_dt
 
 size_t lowbit_matmul_workspace_size(int64_t n_rows, int64_t k, int64_t m, int x_dtype) {
     if (use_skinny(B200_QT_SYM_INT4, n_rows, k, m, x_dtype)) return gemm_skinny_workspace_size(n_rows, k, m);
-    if (use_gemm(B200_QT_SYM_INT4, n_rows, k, m, x_dtype)) return gemm_tc_workspace_size(n_rows, k, m, x_dtype);
+    if (use_gemm(B200_QT_SYM_INT4, n_rows, k, m, x_dtype)) return gemm_tc_workspace_size(n_rows, k, m);
     return gemv_workspace_size(n_rows, k, m, x_dtype);
 }
 
@@ -191,11 +191,8 @@ static int matmul_dispatch(const void* d_w, int qtype, int64_t n_rows, int64_t k
     if (use_skinny(qtype, n_rows, k, m, x_dtype))
         return gemm_skinny_launch(d_w, qtype, n_rows, k, d_x, x_dtype, m, d_y, y_dtype, d_bias, accumulate, workspace,
                                   workspace_bytes, st, gemv_get_pdl());
-    if (use_gemm(qtype, n_rows, k, m, x_dtype)) {
-        int64_t done = 0;
-        return gemm_tc_launch(d_w, qtype, n_rows, k, d_x, x_dtype, m, d_y, y_dtype, d_bias, accumulate, workspace,
-                              workspace_bytes, st, &done);
-    }
+    if (use_gemm(qtype, n_rows, k, m, x_dtype))
+        return gemm_tc_launch(d_w, qtype, n_rows, k, d_x, x_dtype, m, d_y, y_dtype, d_bias, accumulate, workspace, workspace_bytes, st);
     return gemv_launch(d_w, qtype, n_rows, k, d_x, x_dtype, m, d_y, y_dtype, d_bias, accumulate, workspace, workspace_bytes, st);
 }
 
@@ -226,10 +223,10 @@ int lowbit_matmul_cuda(const void* d_w, int qtype, int64_t n_rows, int64_t k, co
 }
 
 size_t lowbit_mlp_workspace_size(int64_t n_rows, int64_t k, int64_t m, int x_dtype) {
+    if (use_skinny(B200_QT_SYM_INT4, n_rows, k, m, x_dtype)) return gemm_skinny_mlp_workspace_size(n_rows, k, m);
+    if (use_gemm(B200_QT_SYM_INT4, n_rows, k, m, x_dtype)) return 256;                 // one launch, no intermediates
     const size_t base = (lowbit_matmul_workspace_size(n_rows, k, m, x_dtype) + 255) / 256 * 256;
-    const size_t two = base + 2 * (size_t)m * n_rows * sizeof(float);
-    const size_t sk = use_skinny(B200_QT_SYM_INT4, n_rows, k, m, x_dtype) ? gemm_skinny_mlp_workspace_size(n_rows, k, m) : 0;
-    return two > sk ? two : sk;
+    return base + 2 * (size_t)m * n_rows * sizeof(float);
 }
 
 int lowbit_mlp_cuda(const void* d_w_gate, const void* d_w_up, int qtype, int64_t n_rows, int64_t k, const void* d_x,
@@ -262,25 +259,19 @@ int lowbit_mlp_cuda(const void* d_w_gate, const void* d_w_up, int qtype, int64_t
     if (fused) {
         rc = gemv_launch_ex(d_w_gate, d_w_up, act + 1, qtype, n_rows, k, d_x, x_dtype, m, d_y, y_dtype, nullptr, 0, workspace,
                             workspace_bytes, st);
-    } else if (use_skinny(qtype, n_rows, k, m, x_dtype) && workspace_bytes >= gemm_skinny_mlp_workspace_size(n_rows, k, m)) {
+    } else if (use_skinny(qtype, n_rows, k, m, x_dtype)) {
         // 17..64 half-precision rows: both matrices in one pass of the skinny tensor-core kernel, act * up in its reduction launch
         rc = gemm_skinny_mlp_launch(d_w_gate, d_w_up, act + 1, qtype, n_rows, k, d_x, x_dtype, m, d_y, y_dtype, workspace, workspace_bytes,
                                     st, gemv_get_pdl());
+    } else if (use_gemm(qtype, n_rows, k, m, x_dtype)) {
+        rc = gemm_tc_mlp_launch(d_w_gate, d_w_up, act + 1, qtype, n_rows, k, d_x, x_dtype, m, d_y, y_dtype, st);
     } else {
-        // the two intermediates: fp32 behind the exact GEMV; behind the tensor-core kernels (whose contract rounds the weights to
-        // the activation dtype anyway) in y's half-precision dtype -- half the bytes through the GEMM epilogue and the activation
-        const bool tc = use_skinny(qtype, n_rows, k, m, x_dtype) || use_gemm(qtype, n_rows, k, m, x_dtype);
-        const int t_dtype = (tc && y_dtype != DT_F32) ? y_dtype : DT_F32;
-        char* tg = (char*)workspace + base;
-        char* tu = tg + (size_t)m * n_rows * (t_dtype == DT_F32 ? 4 : 2);
-        if (m > 128 && (n_rows % 128) == 0 && use_gemm(qtype, n_rows, k, m, x_dtype)) {
-            // prefill sizes: gate and up from one grid of the tensor-core kernel (one set of rounds over the SMs instead of two)
-            rc = gemm_tc_pair_launch(d_w_gate, d_w_up, qtype, n_rows, k, d_x, x_dtype, m, tg, tu, t_dtype, workspace, base, st);
-        } else {
-            rc = matmul_dispatch(d_w_gate, qtype, n_rows, k, d_x, x_dtype, m, tg, t_dtype, nullptr, 0, workspace, base, st);
-            if (!rc) rc = matmul_dispatch(d_w_up, qtype, n_rows, k, d_x, x_dtype, m, tu, t_dtype, nullptr, 0, workspace, base, st);
-        }
-        if (!rc) rc = act_mul_launch(tg, tu, t_dtype, d_y, y_dtype, m * n_rows, act + 1, st);
+        // behind the exact GEMV: the two intermediates in fp32
+        float* tg = (float*)((char*)workspace + base);
+        float* tu = tg + (size_t)m * n_rows;
+        rc = matmul_dispatch(d_w_gate, qtype, n_rows, k, d_x, x_dtype, m, tg, DT_F32, nullptr, 0, workspace, base, st);
+        if (!rc) rc = matmul_dispatch(d_w_up, qtype, n_rows, k, d_x, x_dtype, m, tu, DT_F32, nullptr, 0, workspace, base, st);
+        if (!rc) rc = act_mul_launch(tg, tu, d_y, y_dtype, m * n_rows, act + 1, st);
     }
     if (rc == LB_ERR_ARG) set_error(rc, "lowbit_mlp_cuda: bad argument (qtype %d, N %lld, K %lld, M %lld)", qtype, (long long)n_rows, (long long)k, (long long)m);
     if (rc == LB_ERR_WORKSPACE) set_error(rc, "lowbit_mlp_cuda: workspace too small (%zu bytes)", workspace_bytes);
@@ -334,6 +325,44 @@ int lowbit_moe_cuda(const void* d_x, int x_dtype, const void* d_topk_ids, int id
     if (rc == LB_ERR_WORKSPACE) set_error(rc, "lowbit_moe_cuda: workspace too small (%zu < %zu bytes)", workspace_bytes, need);
     return rc;
 }
+
+int lowbit_moe_tokens_supported(int qtype, int64_t hidden, int64_t inter, int n_experts, int top_k) {
+    return experts_supported(qtype, hidden, inter, n_experts, top_k) ? 1 : 0;
+}
+
+size_t lowbit_moe_tokens_workspace_size(int64_t hidden, int64_t inter, int n_experts, int64_t n_tokens, int top_k) {
+    return experts_workspace_size(hidden, inter, n_experts, n_tokens, top_k);
+}
+
+int lowbit_moe_tokens_cuda(const void* d_x, int x_dtype, int64_t n_tokens, const void* d_topk_ids, int ids_dtype, const void* d_topk_weight,
+                           int weight_dtype, int top_k, const uint64_t* d_gates, const uint64_t* d_ups, const uint64_t* d_downs,
+                           int n_experts, int64_t hidden, int64_t inter, int qtype, int act, void* d_y, void* workspace,
+                           size_t workspace_bytes, void* stream) {
+    t_launches = 0;
+    if (n_tokens == 0) return LB_OK;
+    if (!d_x || !d_topk_ids || !d_topk_weight || !d_gates || !d_ups || !d_downs || !d_y || n_experts <= 0 || n_tokens < 0 ||
+        (ids_dtype != 0 && ids_dtype != 1) || (act != 0 && act != 1) || weight_dtype < 0 || weight_dtype > 2) {
+        set_error(LB_ERR_ARG, "lowbit_moe_tokens_cuda: null pointer, bad ids_dtype / weight_dtype / act, n_tokens < 0 or n_experts <= 0");
+        return LB_ERR_ARG;
+    }
+    if (!experts_supported(qtype, hidden, inter, n_experts, top_k)) {
+        set_error(LB_ERR_ARG, "lowbit_moe_tokens_cuda: unsupported problem (qtype %d, hidden %lld, inter %lld, %d experts, top_k %d)", qtype,
+                  (long long)hidden, (long long)inter, n_experts, top_k);
+        return LB_ERR_ARG;
+    }
+    MoeParams P = {};
+    P.x = d_x; P.x_dtype = x_dtype; P.ids = d_topk_ids; P.ids_i64 = ids_dtype; P.weights = d_topk_weight; P.w_dtype = weight_dtype;
+    P.top_k = top_k; P.gates = (const unsigned long long*)d_gates; P.ups = (const unsigned long long*)d_ups;
+    P.downs = (const unsigned long long*)d_downs; P.n_experts = n_experts; P.hidden = hidden; P.inter = inter;
+    P.qtype = qtype; P.act = act + 1; P.y = d_y; P.y_dtype = x_dtype;
+    P.workspace = workspace; P.workspace_bytes = workspace_bytes;
+    const int rc = experts_launch(P, n_tokens, (cudaStream_t)stream);
+    if (rc == LB_ERR_ARG) set_error(rc, "lowbit_moe_tokens_cuda: bad argument (dtype codes or alignment)");
+    if (rc == LB_ERR_WORKSPACE) set_error(rc, "lowbit_moe_tokens_cuda: workspace too small (%zu bytes)", workspace_bytes);
+    return rc;
+}
+
+int lowbit_gemm_wait_expired(void) { return gemm_tc_wait_expired(); }
 
 // ------------------------------------------------------------------ family (1)
 size_t ggml_quantize_tensor(const float* src, void* dst, int qtype, size_t n, int k, int64_t* hist,

@@ -1,0 +1,668 @@
+// gemm_pair.cu -- kernel (c): prompt-sized dequant-GEMM on the 5th-generation tensor cores, two SMs per tile.
+//
+// y[M][N] (+)= x[M][K] . dequant(W[N][K])^T for M > 64 activation rows: what LowBitLinear.forward asks of xe_linear.forward_new
+// during prefill (reference low_bit_linear.py:700-708).  The same kernel serves an MLP's first half (act(gate) * up in the
+// epilogue) and the routed feed-forwards of a mixture of experts (one launch over every expert's rows).
+//
+// A cluster of two CTAs computes a tile of 256 features x N tokens (N = 16 .. 256) with tcgen05.mma.cta_group::2: the EXPANDED
+// WEIGHTS are the A operand (128 features per CTA), the tokens are B, and each CTA stages HALF of the tokens.  What bounds the
+// one-CTA tile of 256 tokens x 128 features it replaced was the L2: 32 KB of activations + 4.4 KB of packed weights per CTA and
+// k-block of 0.46 us are 12 TB/s over the chip, and four 53 KB stages left no depth to hide it; a pair moves 16 + 4.4 KB per CTA
+// for the same arithmetic.  At 128-token tiles the bound was the chain load -> expand -> MMA through one ring (0.33 us per
+// k-block, the MMAs 0.14): here activations, packed weights and expanded tiles have rings of their own, so the expansion runs
+// ahead of the activations and four groups of warps have four k-blocks in flight.  Measured per k-block: 0.25 us up to 192 tokens
+// (the expansion's pace), 0.335 at 256; 14336 x 4096 at 4000 tokens 1357 -> 1468 TFLOP/s, 4096 x 11008 at 512 tokens 59.7 -> 50.6 us.
+//   warp 0       TMA: this CTA's half of the tokens, boxes of 32 rows x 64 elements (128-byte swizzle), ring of kX slots;
+//   warp 1       CTA 0: issues the MMAs (M = 256, N, K = 16; four per k-block) in warp-uniform control flow, one commit per ring
+//                (multicast to both CTAs); CTA 1: relays "my half has landed" to CTA 0's barrier;
+//   warp 2       bulk copies of the PACKED weights of two 64-row groups (codes, scales, minima), ring of kP slots;
+//   warp 3       allocates TMEM (2 x 256 columns: the epilogue of a tile overlaps the next tile's main loop);
+//   warps 4-19   four groups of four: group (k-block mod 4) expands the codes to fp16 / bf16 (scale applied with one multiply per
+//                pair, one rounding) into the K-major 128B-swizzled A slot it owns;
+//   warps 20-23  epilogue: TMEM lane = feature, column = token.  The two 64-row groups are interleaved by 16 rows, so that with a
+//                gate group and an up group in one tile the lanes l and l + 16 of a warp hold gate and up of one feature.
+// The signals between the two CTAs are plain arrivals: with cluster-scope release / acquire on them (a full memory fence per
+// arrival) a k-block took 0.75 us instead of 0.25; what they order is shared memory, written behind a proxy fence and read by the
+// tensor cores of the SM that wrote it.
+// Every wait is bounded: one that runs out raises g_wait_expired (lowbit_gemm_wait_expired) and the kernel winds down.
+#include "tc_common.cuh"
+
+namespace lowbit {
+namespace gemmtc {
+
+constexpr int kPairThreads = 32 * 24;
+constexpr int kPairTok = 256;                 // most tokens of a tile
+constexpr int kPairDeq0 = 4, kPairEpi0 = 20;  // first dequant / epilogue warp
+constexpr int kMaxExperts = 256;
+constexpr long long kPairWaitCycles = 4000000000ll;       // about two seconds
+__device__ unsigned int g_wait_expired;
+
+template <int QT> struct PairSmem {
+    static constexpr int kGroup = PackedBlock<QT>::kGroup;
+    static constexpr int kPacked = 2 * kGroup;                         // two 64-row groups, one k-block
+    static constexpr int kLut = Expand<QT>::kLutBytes;
+    static constexpr int kTab = 2 * (kMaxExperts + 4) * 4;             // tile prefix and row offsets of the experts
+    static constexpr int kOut = 2 * 32 * 256;                          // epilogue: two chunks of 32 tokens x 128 features, 16 bits
+    static constexpr int kA = 4;                                       // slots of 16 KB, one per dequant group
+    static constexpr int kP = 8;                                       // see the dequant loop: at least twice the groups
+    static constexpr int kFixed = 1024 + 512 + kTab + kLut + kOut + kA * kTileBytesAB + kP * kPacked;
+    static constexpr int kX = (232448 - kFixed) / kTileBytesAB < 8 ? (232448 - kFixed) / kTileBytesAB : 8;      // slots of 128 rows x 128 bytes
+    static constexpr int kTotal = kFixed + kX * kTileBytesAB;
+    static_assert(kX >= 3 && kP >= 2 * kA, "ring depths");
+    static_assert((3 * kX + 2 * kP + 2 * kA + 4) * 8 + 8 <= 512, "barrier region");
+};
+
+struct PairArgs {
+    const uint8_t* w;
+    const uint8_t* w2;                 // MLP: the up projection (w = gate); the tile's second 64-row group
+    const unsigned long long* tab;     // experts: device addresses of w / w2 per expert, row offsets [n_experts + 1]
+    const unsigned long long* tab2;
+    const int* offs;
+    int n_experts;
+    TiledGeom G;
+    int M;
+    int tt;                            // tokens per tile (multiple of 16); experts: chosen per expert
+    int n_fp;                          // pairs of feature tiles
+    int ksplit;
+    int act;                           // 0: y = x W^T; 1 / 2: y = act(x W^T) * (x W2^T)
+    void* y; int y_dtype;
+    const void* bias; int accumulate;
+    float* part;                       // ksplit > 1: [ksplit][M][N]
+};
+
+__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok != 0;
+}
+// whole warp; the same answer in every lane.  false: the limit ran out
+__device__ __forceinline__ bool mbar_wait_lim(uint32_t bar, uint32_t parity) {
+    if (__all_sync(0xffffffffu, mbar_test(bar, parity))) return true;
+    const long long t0 = clock64();
+    while (!__all_sync(0xffffffffu, mbar_test(bar, parity))) {
+        if (__any_sync(0xffffffffu, clock64() - t0 > kPairWaitCycles)) {
+            if ((threadIdx.x & 31) == 0) atomicExch(&g_wait_expired, 1u);
+            return false;
+        }
+    }
+    return true;
+}
+// one arrival at the barrier at this shared-memory offset of CTA `rank` of the cluster
+__device__ __forceinline__ void mbar_arrive_at(uint32_t bar, uint32_t rank) {
+    asm volatile("{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %0, %1;\n\t"
+                 "mbarrier.arrive.shared::cluster.b64 _, [ra];\n\t}" ::"r"(bar), "r"(rank) : "memory");
+}
+__device__ __forceinline__ void umma2_f16_w(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate, uint32_t leader) {
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "setp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(leader) : "memory");
+}
+// arrives at the barrier at this offset in BOTH CTAs when the MMAs issued so far are done
+__device__ __forceinline__ void umma2_commit_w(uint32_t bar, uint32_t leader) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t"
+        "setp.ne.b32 q, %1, 0;\n\t"
+        "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %2;\n\t}"
+        ::"r"(bar), "r"(leader), "h"((uint16_t)3) : "memory");
+}
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
+    uint32_t r[16];
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
+}
+__device__ __forceinline__ void cluster_sync_all() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// one feature's values of up to 16 consecutive tokens, straight to memory: 32-bit results and partial sums, whose two runs of 16
+// features per token are 64 bytes each
+__device__ __forceinline__ void store_feature(float* p, int64_t stride, const float (&v)[16], int cnt, float bias, bool accumulate) {
+#pragma unroll
+    for (int j = 0; j < 16; j++) if (j < cnt) p[j * stride] = accumulate ? v[j] + bias + p[j * stride] : v[j] + bias;
+}
+// gate (lanes 0-15) and up (lanes 16-31) of 16 features and 16 tokens -> act(gate) * up: the halves exchange one token of every two,
+// so that all lanes work; out[i] is token 2 i + half
+__device__ __forceinline__ void gate_up(const float (&v)[16], int act, int half, float (&out)[8]) {
+#pragma unroll
+    for (int j = 0; j < 16; j += 2) {
+        const float got = __shfl_xor_sync(0xffffffffu, half ? v[j] : v[j + 1], 16);
+        out[j >> 1] = apply_act(half ? got : v[j], act) * (half ? v[j + 1] : got);
+    }
+}
+
+template <int QT, bool BF>
+__global__ void __launch_bounds__(kPairThreads, 1)
+pair_kernel(const __grid_constant__ CUtensorMap xmap, const PairArgs A) {
+    using E = Expand<QT>;
+    using SM = PairSmem<QT>;
+    constexpr int KX = SM::kX, KP = SM::kP, KA = SM::kA;
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;       // 128B swizzle wants 1024-byte alignment
+    const uint32_t xring = base, aring = base + KX * kTileBytesAB, pring = aring + KA * kTileBytesAB;
+    const uint32_t bars = pring + KP * SM::kPacked;                    // a multiple of 16 bytes behind the packed ring
+    const uint32_t lut0 = bars + 512, obuf = lut0 + SM::kLut;
+    auto x_full = [&](int s) { return bars + s * 8; };
+    auto x_empty = [&](int s) { return bars + (KX + s) * 8; };
+    auto xp_full = [&](int s) { return bars + (2 * KX + s) * 8; };                     // CTA 0: the other half has landed
+    auto p_full = [&](int s) { return bars + (3 * KX + s) * 8; };
+    auto p_empty = [&](int s) { return bars + (3 * KX + KP + s) * 8; };
+    auto a_full = [&](int s) { return bars + (3 * KX + 2 * KP + s) * 8; };             // CTA 0: both CTAs' tiles are expanded
+    auto a_empty = [&](int s) { return bars + (3 * KX + 2 * KP + KA + s) * 8; };
+    auto tmem_full = [&](int b) { return bars + (3 * KX + 2 * KP + 2 * KA + b) * 8; };
+    auto tmem_empty = [&](int b) { return bars + (3 * KX + 2 * KP + 2 * KA + 2 + b) * 8; };   // CTA 0: both epilogues have drained it
+    const uint32_t tmem_slot = bars + (3 * KX + 2 * KP + 2 * KA + 4) * 8;
+    int* const cum = reinterpret_cast<int*>(smem_raw + (obuf + SM::kOut - smem_u32(smem_raw)));    // experts: tiles before expert e
+    int* const off = cum + kMaxExperts + 4;                                                        //          rows before expert e
+
+    // the warp index through a shuffle: the compiler then treats everything derived from it as warp-uniform
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+    const int rank = (int)(blockIdx.x & 1);
+    const uint32_t lut = lut0 + 4 * lane;
+    if constexpr (E::kLutBytes > 0) E::fill_lut(smem_raw + (lut0 - smem_u32(smem_raw)), threadIdx.x, kPairThreads);
+    const int nb = (int)A.G.nb;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < KX; s++) { mbar_init(x_full(s), 1); mbar_init(x_empty(s), 1); mbar_init(xp_full(s), 1); }
+        for (int s = 0; s < KP; s++) { mbar_init(p_full(s), 1); mbar_init(p_empty(s), 4); }
+        for (int s = 0; s < KA; s++) { mbar_init(a_full(s), 8); mbar_init(a_empty(s), 1); }
+        for (int b = 0; b < 2; b++) { mbar_init(tmem_full(b), 1); mbar_init(tmem_empty(b), 8); }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    // an expert's rows in tiles of at most 256 tokens, evenly cut
+    auto tiles_of = [](int rows) { return (rows + kPairTok - 1) / kPairTok; };
+    if (warp == 2 && A.offs) {
+        int before = 0;
+        for (int e0 = 0; e0 < A.n_experts; e0 += 32) {
+            const int e = e0 + lane, lo = A.offs[min(e, A.n_experts)], hi = A.offs[min(e + 1, A.n_experts)];
+            int t = tiles_of(hi - lo);
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) { const int o = __shfl_up_sync(0xffffffffu, t, d); if (lane >= d) t += o; }
+            if (e < A.n_experts) { cum[e + 1] = before + t; off[e + 1] = hi; }
+            before += __shfl_sync(0xffffffffu, t, 31);
+        }
+        if (lane == 0) { cum[0] = 0; off[0] = 0; }
+    }
+    if (warp == 3) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tmem_slot), "r"(512u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    cluster_sync_all();                                    // both CTAs' barriers exist before anybody signals them
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    uint32_t tmem_base;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem_base) : "r"(tmem_slot));
+
+    // ---- work units: (feature pair, token tile, K split), feature pairs fastest: the clusters running at one moment share a token
+    // tile's activations in L2 and stream different weights
+    const int n_tiles = A.offs ? cum[A.n_experts] : (A.M + A.tt - 1) / A.tt;
+    const int n_units = n_tiles * A.n_fp * A.ksplit, stride = (int)(gridDim.x >> 1);
+    struct Unit { int m0, m_end, n_tok, ft, e, ks, kb0, kb1; };
+    auto decode = [&](int unit, Unit& U) {                 // units of one role come in rising order: U.e only moves forward
+        const int fp = unit % A.n_fp, rest = unit / A.n_fp;
+        int t = rest;
+        if (A.offs) {
+            while (cum[U.e + 1] <= t) U.e++;
+            const int lo = off[U.e], rows = off[U.e + 1] - lo, n = tiles_of(rows);
+            const int tt = ((rows + n - 1) / n + 15) & ~15;
+            U.m0 = lo + (t - cum[U.e]) * tt;
+            U.m_end = min(off[U.e + 1], U.m0 + tt);
+            U.ks = 0;
+        } else {
+            t = rest % n_tiles;
+            U.ks = rest / n_tiles;
+            U.m0 = t * A.tt;
+            U.m_end = min(A.M, U.m0 + A.tt);
+        }
+        U.n_tok = max(16, (U.m_end - U.m0 + 15) & ~15);
+        U.ft = 2 * fp + rank;
+        U.kb0 = A.ksplit == 1 ? 0 : (U.ks * nb) / A.ksplit;
+        U.kb1 = A.ksplit == 1 ? nb : ((U.ks + 1) * nb) / A.ksplit;
+    };
+    Unit U;
+    U.e = 0;
+
+    if (warp == 0) {
+        // ================= activations: this CTA's half of the tile's tokens =================
+        const uint32_t leader = elect_leader();
+        int s = 0, round = 0;
+        for (int unit = blockIdx.x >> 1; unit < n_units; unit += stride) {
+            decode(unit, U);
+            const int half = U.n_tok >> 1, boxes = (half + 31) >> 5, row0 = U.m0 + rank * half;
+            for (int kb = U.kb0; kb < U.kb1; kb++) {
+                if (!mbar_wait_lim(x_empty(s), (uint32_t)((round & 1) ^ 1))) goto done;
+                mbar_expect_tx_w(x_full(s), boxes * 4096, leader);
+                for (int i = 0; i < boxes; i++)
+                    tma_load_2d_w(xring + s * kTileBytesAB + i * 4096, &xmap, kb * 64, row0 + i * 32, x_full(s), leader);
+                if (++s == KX) { s = 0; round++; }
+            }
+        }
+    } else if (warp == 1) {
+        if (rank == 0) {
+            // ================= MMA issuer =================
+            const uint32_t leader = elect_leader();
+            int sx = 0, rx = 0, it = 0, ti = 0;
+            for (int unit = blockIdx.x >> 1; unit < n_units; unit += stride, ti++) {
+                decode(unit, U);
+                // c F32 (1<<4), a/b format (0 f16, 1 bf16), both K-major, N (>>3 at bit 17), M = 256 (>>4 at bit 24)
+                const uint32_t idesc = (1u << 4) | ((BF ? 1u : 0u) << 7) | ((BF ? 1u : 0u) << 10) | (((uint32_t)U.n_tok >> 3) << 17) | ((256u >> 4) << 24);
+                const int buf = ti & 1;
+                if (!mbar_wait_lim(tmem_empty(buf), (uint32_t)(((ti >> 1) & 1) ^ 1))) goto done;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t acc = tmem_base + buf * kPairTok;
+                for (int kb = U.kb0; kb < U.kb1; kb++, it++) {
+                    const int sa = it & 3;
+                    if (!mbar_wait_lim(x_full(sx), (uint32_t)(rx & 1))) goto done;
+                    if (!mbar_wait_lim(xp_full(sx), (uint32_t)(rx & 1))) goto done;
+                    if (!mbar_wait_lim(a_full(sa), (uint32_t)((it >> 2) & 1))) goto done;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    const uint64_t ad = make_desc(aring + sa * kTileBytesAB), xd = make_desc(xring + sx * kTileBytesAB);
+#pragma unroll
+                    for (int k4 = 0; k4 < 4; k4++)           // the address field counts 16-byte units
+                        umma2_f16_w(acc, ad + (uint64_t)((k4 * 32) >> 4), xd + (uint64_t)((k4 * 32) >> 4), idesc, (kb > U.kb0 || k4 > 0) ? 1u : 0u, leader);
+                    umma2_commit_w(a_empty(sa), leader);
+                    umma2_commit_w(x_empty(sx), leader);
+                    if (++sx == KX) { sx = 0; rx++; }
+                }
+                umma2_commit_w(tmem_full(buf), leader);
+            }
+        } else {
+            // ================= relay: CTA 1's half has landed =================
+            int sx = 0, rx = 0;
+            for (int unit = blockIdx.x >> 1; unit < n_units; unit += stride) {
+                decode(unit, U);
+                for (int kb = U.kb0; kb < U.kb1; kb++) {
+                    if (!mbar_wait_lim(x_full(sx), (uint32_t)(rx & 1))) goto done;
+                    if (lane == 0) mbar_arrive_at(xp_full(sx), 0);
+                    if (++sx == KX) { sx = 0; rx++; }
+                }
+            }
+        }
+    } else if (warp == 2) {
+        // ================= packed weights of this CTA's two 64-row groups =================
+        const uint32_t leader = elect_leader();
+        const int n_rg = (int)(A.G.rows >> 6);
+        int s = 0, round = 0;
+        for (int unit = blockIdx.x >> 1; unit < n_units; unit += stride) {
+            decode(unit, U);
+            const uint8_t* w0 = A.offs ? reinterpret_cast<const uint8_t*>(A.tab[U.e]) : A.w;
+            const uint8_t* w1 = A.act ? (A.offs ? reinterpret_cast<const uint8_t*>(A.tab2[U.e]) : A.w2) : w0;
+            // the last pair's second tile may not exist: it repeats the last group and stores nothing
+            const int64_t rg0 = min(A.act ? U.ft : 2 * U.ft, n_rg - 1), rg1 = min(A.act ? U.ft : 2 * U.ft + 1, n_rg - 1);
+            for (int kb = U.kb0; kb < U.kb1; kb++) {
+                if (!mbar_wait_lim(p_empty(s), (uint32_t)((round & 1) ^ 1))) goto done;
+                mbar_expect_tx_w(p_full(s), SM::kPacked, leader);
+#pragma unroll
+                for (int gi = 0; gi < 2; gi++) {
+                    const uint8_t* wb = gi ? w1 : w0;
+                    const int64_t u = (gi ? rg1 : rg0) * nb + kb;
+                    const uint32_t dst = pring + s * SM::kPacked + gi * SM::kGroup;
+                    bulk_g2s_w(dst, wb + u * PackedBlock<QT>::kSuper, PackedBlock<QT>::kSuper, p_full(s), leader);
+                    bulk_g2s_w(dst + PackedBlock<QT>::kSuper, wb + A.G.off_s + u * 128, 128, p_full(s), leader);
+                    if (E::kHasMin) bulk_g2s_w(dst + PackedBlock<QT>::kSuper + 128, wb + A.G.off_m + u * 128, 128, p_full(s), leader);
+                }
+                if (++s == KP) { s = 0; round++; }
+            }
+        }
+    } else if (warp >= kPairDeq0 && warp < kPairEpi0) {
+        // ================= dequant: group (warp - 4) / 4 takes every fourth k-block; a warp expands 16 rows of either row group =================
+        const int grp = (warp - kPairDeq0) >> 2, dw = (warp - kPairDeq0) & 3;
+        const int g = lane >> 2, t = lane & 3;
+        const uint32_t row0 = aring + grp * kTileBytesAB + 4 * dw * 1024 + g * 128;        // rows 32 dw + g, + 8; + 16, + 24 for the second group
+        int it = 0, sp = 0, rp = 0;
+        for (int unit = blockIdx.x >> 1; unit < n_units; unit += stride) {
+            decode(unit, U);
+            for (int kb = U.kb0; kb < U.kb1; kb++, it++, (++sp == KP ? (sp = 0, rp++) : 0)) {
+                if ((it & 3) != grp) continue;
+                // this group has waited for the MMAs of k-block it - 8 (below, at its last k-block): all before it were expanded, so the
+                // packed slot's earlier trips are over (it - KP <= it - 8) and its parity is unambiguous
+                if (!mbar_wait_lim(p_full(sp), (uint32_t)(rp & 1))) goto done;
+                const uint32_t pk = pring + sp * SM::kPacked;
+                typename E::Codes cw[2];
+                uint32_t dq[2], mq[2] = {0u, 0u};
+#pragma unroll
+                for (int gi = 0; gi < 2; gi++) {
+                    const uint32_t gb = pk + gi * SM::kGroup;
+                    E::load(gb + dw * E::kTileBytes, lane, cw[gi]);
+                    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(dq[gi]) : "r"(gb + PackedBlock<QT>::kSuper + g * 16 + dw * 4));
+                    if (E::kHasMin) asm volatile("ld.shared.u32 %0, [%1];" : "=r"(mq[gi]) : "r"(gb + PackedBlock<QT>::kSuper + 128 + g * 16 + dw * 4));
+                }
+                // expanded into registers while the MMAs still read the slot's last tile
+                uint32_t lo[2][8], hi[2][8];
+#pragma unroll
+                for (int gi = 0; gi < 2; gi++) {
+                    const __half2 d2 = u2h(dq[gi]), m2 = u2h(mq[gi]);
+                    const __half2 dlo = __low2half2(d2), dhi = __high2half2(d2);
+                    const __half2 mlo = __low2half2(m2), mhi = __high2half2(m2);
+#pragma unroll
+                    for (int k4 = 0; k4 < 4; k4++) {
+                        uint32_t a[4];
+                        E::run(cw[gi], k4, dlo, dhi, mlo, mhi, lut, a);
+                        if (BF) {
+#pragma unroll
+                            for (int i = 0; i < 4; i++) a[i] = h2_to_bf2(a[i]);
+                        }
+                        lo[gi][2 * k4] = a[0]; lo[gi][2 * k4 + 1] = a[2];
+                        hi[gi][2 * k4] = a[1]; hi[gi][2 * k4 + 1] = a[3];
+                    }
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(p_empty(sp));
+                if (!mbar_wait_lim(a_empty(grp), (uint32_t)(((it >> 2) & 1) ^ 1))) goto done;
+#pragma unroll
+                for (int gi = 0; gi < 2; gi++)
+#pragma unroll
+                    for (int q = 0; q < 2; q++) {               // k-steps 2q, 2q+1 -> one 16-byte chunk per row; 128B swizzle: chunk ^ (row & 7)
+                        const uint32_t at = row0 + gi * 2048 + (uint32_t)((2 * t + q) ^ g) * 16;
+                        asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(lo[gi][4 * q]), "r"(lo[gi][4 * q + 1]), "r"(lo[gi][4 * q + 2]), "r"(lo[gi][4 * q + 3]) : "memory");
+                        asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(at + 1024), "r"(hi[gi][4 * q]), "r"(hi[gi][4 * q + 1]), "r"(hi[gi][4 * q + 2]), "r"(hi[gi][4 * q + 3]) : "memory");
+                    }
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // generic-proxy writes -> async-proxy (MMA) reads
+                __syncwarp();
+                if (lane == 0) mbar_arrive_at(a_full(grp), 0);
+            }
+        }
+    } else if (warp >= kPairEpi0) {
+        // ================= epilogue: TMEM lanes 32 * (warp % 4) .. + 31 =================
+        const int quarter = warp & 3, half = lane >> 4, e_tid = threadIdx.x - 32 * kPairEpi0;
+        const int64_t N = A.G.rows;
+        const bool wide = A.ksplit > 1 || A.y_dtype == DT_F32;        // 32-bit results go straight to memory
+        uint32_t chunk = 0;
+        int ti = 0;
+        for (int unit = blockIdx.x >> 1; unit < n_units; unit += stride, ti++) {
+            decode(unit, U);
+            const int buf = ti & 1, rows = U.m_end - U.m0;
+            const int64_t f0 = (int64_t)U.ft * (A.act ? 64 : 128);
+            const int64_t n = f0 + (A.act ? 0 : 64 * half) + 16 * quarter + (lane & 15);
+            const bool valid = f0 < N;                                // the last pair's second tile may not exist
+            float b = 0.0f;
+            if (A.bias && valid && A.ksplit == 1)
+                b = A.y_dtype == DT_F32 ? ((const float*)A.bias)[n] : A.y_dtype == DT_F16 ? __half2float(((const __half*)A.bias)[n])
+                                                                                          : __bfloat162float(((const __nv_bfloat16*)A.bias)[n]);
+            // the four warps go on together or not at all: they meet at named barriers below
+            uint32_t go = mbar_wait_lim(tmem_full(buf), (uint32_t)((ti >> 1) & 1)) ? 1u : 0u;
+            asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %0, 0;\n\tbarrier.cta.red.and.pred q, 1, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "+r"(go)::"memory");
+            if (!go) goto done;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const uint32_t acc = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * kPairTok);
+            if (wide) {
+#pragma unroll 1
+                for (int c = 0; c < rows; c += 16) {
+                    float v[16];
+                    tmem_ld16(acc + c, v);
+                    const int64_t at = (int64_t)(U.m0 + c) * N + n;
+                    if (A.act) {
+                        float o[8];
+                        gate_up(v, A.act, half, o);
+#pragma unroll
+                        for (int i = 0; i < 8; i++)
+                            if (valid && c + 2 * i + half < rows) ((float*)A.y)[at + (2 * i + half) * N] = o[i];
+                    } else if (valid) {
+                        if (A.ksplit > 1) store_feature(A.part + (int64_t)U.ks * A.M * N + at, N, v, rows - c, 0.0f, false);
+                        else store_feature((float*)A.y + at, N, v, rows - c, b, A.accumulate != 0);
+                    }
+                    __syncwarp();
+                }
+            } else {
+                // 16-bit results: 32 tokens at a time through shared memory, so that a token's 128 (64 behind the activation)
+                // features leave as one run of 16-byte stores.  Straight from the lanes (2-byte stores, runs of 32 bytes) a tile of
+                // 256 tokens took 8 us, 60 clocks per token and warp.  The two runs of 16 features that a warp holds sit in different
+                // halves of the banks (the chunk's pieces are permuted, and put back by the copy).
+                const bool f16 = A.y_dtype == DT_F16, y_vec = (reinterpret_cast<uintptr_t>(A.y) & 15) == 0;
+                auto put = [&](uint16_t* dst, const uint4& q) {
+                    if (y_vec) { *reinterpret_cast<uint4*>(dst) = q; return; }
+                    const uint32_t w[4] = {q.x, q.y, q.z, q.w};          // a result that does not start on 16 bytes
+#pragma unroll
+                    for (int i = 0; i < 8; i++) dst[i] = (uint16_t)(w[i >> 1] >> (16 * (i & 1)));
+                };
+                uint16_t* const yb = (uint16_t*)A.y + (int64_t)U.m0 * N + f0;
+#pragma unroll 1
+                for (int c = 0; c < rows; c += 32, chunk ^= 1u) {
+                    const uint32_t ob = obuf + chunk * 8192;
+#pragma unroll
+                    for (int h = 0; h < 2; h++) {
+                        float v[16];
+                        tmem_ld16(acc + c + 16 * h, v);
+                        if (A.act) {
+                            float o[8];
+                            gate_up(v, A.act, half, o);
+                            const uint32_t at = ob + (uint32_t)((16 * h + half) * 128 + (((16 * quarter + (lane & 15)) * 2) ^ (half << 6)));
+#pragma unroll
+                            for (int i = 0; i < 8; i++) {
+                                const uint16_t bits = f16 ? __half_as_ushort(__float2half_rn(o[i])) : __bfloat16_as_ushort(__float2bfloat16_rn(o[i]));
+                                asm volatile("st.shared.u16 [%0], %1;" ::"r"(at + i * 256), "h"(bits) : "memory");
+                            }
+                        } else {
+                            if (A.accumulate) {
+                                const uint16_t* yp = (const uint16_t*)A.y + (int64_t)(U.m0 + c + 16 * h) * N + n;
+#pragma unroll
+                                for (int j = 0; j < 16; j++)
+                                    if (valid && c + 16 * h + j < rows)
+                                        v[j] += f16 ? __half2float(__ushort_as_half(yp[j * N])) : __bfloat162float(__ushort_as_bfloat16(yp[j * N]));
+                            }
+                            const uint32_t at = ob + (uint32_t)(16 * h * 256 + quarter * 64 + half * 32 + (lane & 15) * 2);
+#pragma unroll
+                            for (int j = 0; j < 16; j++) {
+                                const uint16_t bits = f16 ? __half_as_ushort(__float2half_rn(v[j] + b)) : __bfloat16_as_ushort(__float2bfloat16_rn(v[j] + b));
+                                asm volatile("st.shared.u16 [%0], %1;" ::"r"(at + j * 256), "h"(bits) : "memory");
+                            }
+                        }
+                    }
+                    asm volatile("barrier.cta.sync 1, 128;" ::: "memory");
+                    // the other buffer is written next: everybody passes the next barrier only after this copy
+                    const int n_rows = min(32, rows - c);
+                    if (valid) {
+                        if (A.act) {
+                            for (int i = e_tid; i < n_rows * 8; i += 128) {
+                                const int r = i >> 3, p = i & 7;
+                                put(yb + (int64_t)(c + r) * N + p * 8, lds128(ob + r * 128 + (uint32_t)((p ^ ((r & 1) << 2)) * 16)));
+                            }
+                        } else {
+                            for (int i = e_tid; i < n_rows * 16; i += 128) {
+                                const int r = i >> 4, p = i & 15;              // piece p: 8 features from 8 p
+                                put(yb + (int64_t)(c + r) * N + p * 8, lds128(ob + r * 256 + (uint32_t)((((p >> 1) & 3) * 4 + (p >> 3) * 2 + (p & 1)) * 16)));
+                            }
+                        }
+                    }
+                }
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive_at(tmem_empty(buf), 0);
+        }
+    }
+done:
+    __syncwarp();
+    __syncthreads();
+    cluster_sync_all();                                    // nobody signals a CTA that has left, no MMA reads its memory
+    if (warp == 3) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512u) : "memory");
+    }
+}
+
+// K split: y[token][n] = sum over splits (in split order) of the fp32 partials, + bias, + y when accumulating
+__global__ void __launch_bounds__(256) reduce_partials_kernel(const float* __restrict__ part, int ksplit, int64_t mn, int64_t n_cols,
+                                                              void* y, int y_dtype, const void* bias, int accumulate) {
+    for (int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) * 4; i < mn; i += (int64_t)gridDim.x * blockDim.x * 4) {
+        float4 a = *reinterpret_cast<const float4*>(part + i);
+        for (int ks = 1; ks < ksplit; ks++) {
+            const float4 b = *reinterpret_cast<const float4*>(part + ks * mn + i);
+            a.x += b.x; a.y += b.y; a.z += b.z; a.w += b.w;
+        }
+        float v[4] = {a.x, a.y, a.z, a.w};
+        const int64_t col = i % n_cols;                           // n_cols % 128 == 0: the four values share a row
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            if (bias) v[j] += y_dtype == DT_F32 ? ((const float*)bias)[col + j]
+                            : (y_dtype == DT_F16 ? __half2float(((const __half*)bias)[col + j]) : __bfloat162float(((const __nv_bfloat16*)bias)[col + j]));
+            if (y_dtype == DT_F32) { float* p = (float*)y + i + j; *p = accumulate ? *p + v[j] : v[j]; }
+            else if (y_dtype == DT_F16) { __half* p = (__half*)y + i + j; *p = __float2half_rn(accumulate ? __half2float(*p) + v[j] : v[j]); }
+            else { __nv_bfloat16* p = (__nv_bfloat16*)y + i + j; *p = __float2bfloat16_rn(accumulate ? __bfloat162float(*p) + v[j] : v[j]); }
+        }
+    }
+}
+
+// clusters of two that can be resident at once (one CTA per SM; an SM without a partner in its group stays idle)
+template <int QT, bool BF>
+static int pair_clusters() {
+    static int cached[64] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    int& n = cached[dev & 63];
+    if (n) return n;
+    constexpr int SMEM = PairSmem<QT>::kTotal;
+    if (cudaFuncSetAttribute(pair_kernel<QT, BF>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess) { cudaGetLastError(); return 0; }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(sm_count() & ~1)); cfg.blockDim = dim3(kPairThreads); cfg.dynamicSmemBytes = SMEM;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    cfg.attrs = at; cfg.numAttrs = 1;
+    int c = 0;
+    if (cudaOccupancyMaxActiveClusters(&c, pair_kernel<QT, BF>, &cfg) != cudaSuccess || c <= 0) { cudaGetLastError(); c = sm_count() / 2; }
+    n = c;
+    return n;
+}
+
+template <int QT, bool BF>
+static int pair_launch_one(const CUtensorMap& map, const PairArgs& A, int64_t units, cudaStream_t st) {
+    const int clusters = pair_clusters<QT, BF>();
+    if (clusters <= 0) { set_error(LB_ERR_CUDA, "the two-SM matmul kernel cannot be configured on this device"); return LB_ERR_CUDA; }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2u * (unsigned)(units < clusters ? units : clusters)); cfg.blockDim = dim3(kPairThreads);
+    cfg.dynamicSmemBytes = PairSmem<QT>::kTotal; cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    cfg.attrs = at; cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, pair_kernel<QT, BF>, map, A);
+    note_launch();
+    return LB_OK;
+}
+static int pair_launch(int qt, bool bf, const CUtensorMap& map, const PairArgs& A, int64_t units, cudaStream_t st) {
+#define PAIR_CASE(Q) case Q: return bf ? pair_launch_one<Q, true>(map, A, units, st) : pair_launch_one<Q, false>(map, A, units, st);
+    switch (qt) { PAIR_CASE(QT_SYM_INT4) PAIR_CASE(QT_ASYM_INT4) PAIR_CASE(QT_NF4) PAIR_CASE(QT_FP8_E4M3) PAIR_CASE(QT_FP8_E5M2) PAIR_CASE(QT_FP6) }
+#undef PAIR_CASE
+    return LB_ERR_ARG;
+}
+
+// Token tile and K splits of a matmul: the pair that minimises rounds of the resident clusters x k-blocks per unit x time per
+// k-block (measured, sym_int4: 0.25 us up to 192 tokens, where the expansion of 128 x 64 weights per CTA sets the pace, 0.335 at
+// 256) + the start and end of a unit and, when K is split, the partial sums' round trip through memory at ~4 TB/s and the second
+// launch.
+struct PairPlan { int tt, ks; };
+static PairPlan pair_plan(int64_t n_fp, int64_t nb, int64_t m, int64_t n_out, bool may_split) {
+    const int64_t clusters = sm_count() / 2, nt0 = (m + kPairTok - 1) / kPairTok;
+    PairPlan best = {256, 1};
+    double best_cost = 1e30;
+    for (int64_t nt = nt0; nt <= nt0 + 8 && nt <= (m + 31) / 32; nt++) {
+        const int64_t tt = ((m + nt - 1) / nt + 15) & ~int64_t(15);
+        const double per_kb = tt <= 192 ? 0.25 : 0.25 + 0.00133 * (double)(tt - 192);
+        const int64_t max_ks = may_split ? (nb / 8 < 8 ? nb / 8 : 8) : 1;
+        for (int64_t ks = 1; ks == 1 || ks <= max_ks; ks++) {
+            const int64_t rounds = (n_fp * nt * ks + clusters - 1) / clusters;
+            double cost = (double)rounds * ((double)((nb + ks - 1) / ks) * per_kb + 1.0);
+            if (ks > 1) cost += (double)ks * (double)m * (double)n_out * 8.0 / 4.0e6 + 2.0;
+            if (cost < best_cost - 1e-9) { best_cost = cost; best = {(int)tt, (int)ks}; }
+        }
+    }
+    return best;
+}
+}  // namespace gemmtc
+
+bool gemm_tc_supported(int qt, int64_t n_rows, int64_t k) {
+    qt = canon_qtype(qt);
+    const bool q = qt == QT_SYM_INT4 || qt == QT_ASYM_INT4 || qt == QT_NF4 || qt == QT_FP8_E4M3 || qt == QT_FP8_E5M2 || qt == QT_FP6;
+    return q && n_rows >= 128 && (n_rows % 128) == 0 && k >= 64 && (k % 64) == 0;
+}
+
+size_t gemm_tc_workspace_size(int64_t n_rows, int64_t k, int64_t m) {
+    using namespace gemmtc;
+    const PairPlan p = pair_plan((n_rows / 128 + 1) / 2, k / 64, m, n_rows, true);
+    return p.ks > 1 ? (size_t)p.ks * m * n_rows * sizeof(float) : 0;
+}
+
+int gemm_tc_launch(const void* w, int qt, int64_t n_rows, int64_t k, const void* x, int x_dtype, int64_t m, void* y,
+                   int y_dtype, const void* bias, int accumulate, void* workspace, size_t workspace_bytes, cudaStream_t st) {
+    using namespace gemmtc;
+    qt = canon_qtype(qt);
+    if (!gemm_tc_supported(qt, n_rows, k) || (x_dtype != DT_F16 && x_dtype != DT_BF16)) return LB_ERR_ARG;
+    if (((uintptr_t)x & 15) || ((uintptr_t)w & 15)) return LB_ERR_ARG;
+    const bool bf = x_dtype == DT_BF16;
+    CUtensorMap map;
+    if (const int rc = encode_rows(&map, x, bf, m, k, 32)) return rc;
+    PairArgs A = {};
+    A.w = (const uint8_t*)w; A.G = make_geom(n_rows, k, qt); A.M = (int)m; A.y = y; A.y_dtype = y_dtype; A.bias = bias; A.accumulate = accumulate;
+    A.n_fp = (int)((n_rows / 128 + 1) / 2);
+    PairPlan p = pair_plan(A.n_fp, k / 64, m, n_rows, true);
+    // a caller's workspace without room for partial sums: the whole K range per unit
+    if (p.ks > 1 && (!workspace || workspace_bytes < (size_t)p.ks * m * n_rows * sizeof(float))) p = pair_plan(A.n_fp, k / 64, m, n_rows, false);
+    A.tt = p.tt; A.ksplit = p.ks; A.part = (float*)workspace;
+    const int64_t units = (int64_t)A.n_fp * ((m + p.tt - 1) / p.tt) * p.ks;
+    if (const int rc = pair_launch(qt, bf, map, A, units, st)) return rc;
+    if (p.ks > 1) {
+        const int64_t mn = m * n_rows;
+        int rg = (int)((mn / 4 + 255) / 256); if (rg > sm_count() * 8) rg = sm_count() * 8;
+        reduce_partials_kernel<<<rg, 256, 0, st>>>(A.part, p.ks, mn, n_rows, y, y_dtype, bias, accumulate);
+        note_launch();
+    }
+    return check_launch();
+}
+
+// first half of an MLP at prompt sizes: y = act(x . Wgate^T) * (x . Wup^T), both products in one tile's accumulators (a gate and an
+// up row group per CTA), the activation in the epilogue: the two [M][N] intermediates and their kernel do not exist
+int gemm_tc_mlp_launch(const void* w_gate, const void* w_up, int act, int qt, int64_t n_rows, int64_t k, const void* x, int x_dtype,
+                       int64_t m, void* y, int y_dtype, cudaStream_t st) {
+    using namespace gemmtc;
+    qt = canon_qtype(qt);
+    if (!gemm_tc_supported(qt, n_rows, k) || (x_dtype != DT_F16 && x_dtype != DT_BF16) || act < 1 || act > 2) return LB_ERR_ARG;
+    if (((uintptr_t)x & 15) || ((uintptr_t)w_gate & 15) || ((uintptr_t)w_up & 15)) return LB_ERR_ARG;
+    const bool bf = x_dtype == DT_BF16;
+    CUtensorMap map;
+    if (const int rc = encode_rows(&map, x, bf, m, k, 32)) return rc;
+    PairArgs A = {};
+    A.w = (const uint8_t*)w_gate; A.w2 = (const uint8_t*)w_up; A.act = act; A.G = make_geom(n_rows, k, qt); A.M = (int)m; A.y = y; A.y_dtype = y_dtype;
+    A.n_fp = (int)((n_rows / 64 + 1) / 2); A.ksplit = 1;
+    A.tt = pair_plan(A.n_fp, k / 64, m, n_rows, false).tt;
+    if (const int rc = pair_launch(qt, bf, map, A, (int64_t)A.n_fp * ((m + A.tt - 1) / A.tt), st)) return rc;
+    return check_launch();
+}
+
+// the same kernel over every expert's rows: x [rows][k] sorted by expert, offs [n_experts + 1] row offsets on the device, tab /
+// tab2 device addresses of the experts' weights (tab2: the up projections, act in the epilogue; or NULL)
+int gemm_tc_experts_launch(const unsigned long long* tab, const unsigned long long* tab2, int act, const int* offs, int n_experts, int qt,
+                           int64_t n_rows, int64_t k, const void* x, int x_dtype, int64_t rows, void* y, int y_dtype, cudaStream_t st) {
+    using namespace gemmtc;
+    qt = canon_qtype(qt);
+    if (!gemm_tc_supported(qt, n_rows, k) || (x_dtype != DT_F16 && x_dtype != DT_BF16) || n_experts > kMaxExperts || ((uintptr_t)x & 15)) return LB_ERR_ARG;
+    const bool bf = x_dtype == DT_BF16;
+    CUtensorMap map;
+    if (const int rc = encode_rows(&map, x, bf, rows, k, 32)) return rc;
+    PairArgs A = {};
+    A.tab = tab; A.tab2 = tab2; A.act = tab2 ? act : 0; A.offs = offs; A.n_experts = n_experts;
+    A.G = make_geom(n_rows, k, qt); A.M = (int)rows; A.y = y; A.y_dtype = y_dtype; A.ksplit = 1; A.tt = kPairTok;
+    A.n_fp = (int)((n_rows / (tab2 ? 64 : 128) + 1) / 2);
+    const int64_t most = (rows < n_experts ? rows : n_experts) + rows / kPairTok;        // tiles: one per used expert and one per 256 rows
+    if (const int rc = pair_launch(qt, bf, map, A, most * A.n_fp, st)) return rc;
+    return check_launch();
+}
+
+int gemm_tc_wait_expired() {
+    unsigned int v = 0;
+    if (cudaMemcpyFromSymbol(&v, gemmtc::g_wait_expired, sizeof(v)) != cudaSuccess) { cudaGetLastError(); return -1; }
+    return (int)v;
+}
+
+}  // namespace lowbit

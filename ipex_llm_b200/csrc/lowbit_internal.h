@@ -52,7 +52,7 @@ int gemv_launch_ex(const void* w, const void* w2, int act, int qt, int64_t n_row
                    int64_t m, void* y, int y_dtype, const void* bias, int accumulate, void* workspace,
                    size_t workspace_bytes, cudaStream_t st);
 bool gemv_mlp_fused_supported(int qt, int64_t n_rows, int64_t k, int64_t m, int x_dtype);
-int act_mul_launch(const void* gate, const void* up, int in_dtype, void* y, int y_dtype, int64_t n, int act, cudaStream_t st);
+int act_mul_launch(const float* gate, const float* up, void* y, int y_dtype, int64_t n, int act, cudaStream_t st);
 
 // one-token mixture-of-experts (reference xe_linear.moe_forward_vec)
 struct MoeParams {
@@ -73,15 +73,21 @@ bool moe_supported(int qt, int64_t hidden, int64_t inter, int top_k);
 size_t moe_workspace_size(int64_t hidden, int64_t inter, int top_k, int x_dtype);
 int moe_launch(const MoeParams& P, cudaStream_t st);
 
-// gemm_tc.cu (tcgen05 prefill GEMM)
+// many-token mixture-of-experts (experts.cu): MoeParams with x / y [n_tokens][hidden], ids / weights [n_tokens][top_k]
+bool experts_supported(int qt, int64_t hidden, int64_t inter, int n_experts, int top_k);
+size_t experts_workspace_size(int64_t hidden, int64_t inter, int n_experts, int64_t n_tokens, int top_k);
+int experts_launch(const MoeParams& P, int64_t n_tokens, cudaStream_t st);
+
+// gemm_pair.cu (tcgen05 prompt matmul, two SMs per tile)
 bool gemm_tc_supported(int qt, int64_t n_rows, int64_t k);
-size_t gemm_tc_workspace_size(int64_t n_rows, int64_t k, int64_t m, int x_dtype);
+size_t gemm_tc_workspace_size(int64_t n_rows, int64_t k, int64_t m);
 int gemm_tc_launch(const void* w, int qt, int64_t n_rows, int64_t k, const void* x, int x_dtype, int64_t m, void* y,
-                   int y_dtype, const void* bias, int accumulate, void* workspace, size_t workspace_bytes, cudaStream_t st,
-                   int64_t* n_done);
-// gate and up of an MLP in one grid (m > 128, n_rows % 128 == 0)
-int gemm_tc_pair_launch(const void* w, const void* w2, int qt, int64_t n_rows, int64_t k, const void* x, int x_dtype, int64_t m,
-                        void* y, void* y2, int y_dtype, void* workspace, size_t workspace_bytes, cudaStream_t st);
+                   int y_dtype, const void* bias, int accumulate, void* workspace, size_t workspace_bytes, cudaStream_t st);
+int gemm_tc_mlp_launch(const void* w_gate, const void* w_up, int act, int qt, int64_t n_rows, int64_t k, const void* x, int x_dtype,
+                       int64_t m, void* y, int y_dtype, cudaStream_t st);
+int gemm_tc_experts_launch(const unsigned long long* tab, const unsigned long long* tab2, int act, const int* offs, int n_experts, int qt,
+                           int64_t n_rows, int64_t k, const void* x, int x_dtype, int64_t rows, void* y, int y_dtype, cudaStream_t st);
+int gemm_tc_wait_expired();       // 1 after a wait of the two-SM kernel ran out on the current device (its results are then undefined)
 
 // M above this goes to the tensor-core GEMM when the shape allows, else to chunks of the GEMV
 constexpr int64_t kGemvMaxM = 32;

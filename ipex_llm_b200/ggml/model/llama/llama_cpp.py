@@ -316,6 +316,37 @@ def lowbit_moe_cuda(d_x, x_dtype, d_ids, ids_dtype, d_weight, weight_dtype, top_
                                 workspace_bytes, stream), "lowbit_moe_cuda")
 
 
+_lib.lowbit_moe_tokens_supported.argtypes = [ctypes.c_int, ctypes.c_int64, ctypes.c_int64, ctypes.c_int, ctypes.c_int]
+_lib.lowbit_moe_tokens_supported.restype = ctypes.c_int
+_lib.lowbit_moe_tokens_workspace_size.argtypes = [ctypes.c_int64, ctypes.c_int64, ctypes.c_int, ctypes.c_int64, ctypes.c_int]
+_lib.lowbit_moe_tokens_workspace_size.restype = ctypes.c_size_t
+_lib.lowbit_moe_tokens_cuda.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_int64, ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p, ctypes.c_int,
+                                        ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int, ctypes.c_int64,
+                                        ctypes.c_int64, ctypes.c_int, ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_size_t, ctypes.c_void_p]
+_lib.lowbit_moe_tokens_cuda.restype = ctypes.c_int
+_lib.lowbit_gemm_wait_expired.argtypes = []
+_lib.lowbit_gemm_wait_expired.restype = ctypes.c_int
+
+
+def lowbit_moe_tokens_supported(qtype, hidden, inter, n_experts, top_k):
+    return bool(_lib.lowbit_moe_tokens_supported(qtype, hidden, inter, n_experts, top_k))
+
+
+def lowbit_moe_tokens_workspace_size(hidden, inter, n_experts, n_tokens, top_k):
+    return _lib.lowbit_moe_tokens_workspace_size(hidden, inter, n_experts, n_tokens, top_k)
+
+
+def lowbit_moe_tokens_cuda(d_x, x_dtype, n_tokens, d_ids, ids_dtype, d_weight, weight_dtype, top_k, d_gates, d_ups, d_downs, n_experts,
+                           hidden, inter, qtype, act, d_y, workspace, workspace_bytes, stream):
+    _check(_lib.lowbit_moe_tokens_cuda(d_x, x_dtype, n_tokens, d_ids, ids_dtype, d_weight, weight_dtype, top_k, d_gates, d_ups, d_downs,
+                                       n_experts, hidden, inter, qtype, act, d_y, workspace, workspace_bytes, stream), "lowbit_moe_tokens_cuda")
+
+
+def lowbit_gemm_wait_expired():
+    """whether a bounded wait inside the two-SM matmul kernel has run out on the current device (synchronises)"""
+    return _lib.lowbit_gemm_wait_expired() == 1
+
+
 _lib.lowbit_set_programmatic_dependent_launch.argtypes = [ctypes.c_int]
 _lib.lowbit_set_programmatic_dependent_launch.restype = None
 _lib.lowbit_get_programmatic_dependent_launch.argtypes = []

@@ -367,6 +367,41 @@ def moe_forward_vec(x: torch.Tensor, topk_ids: torch.Tensor, topk_weight: torch.
     return out
 
 
+def moe_tokens_supported(x: torch.Tensor, n_experts: int, hidden: int, inter: int, top_k: int, qtype: int) -> bool:
+    """shape / dtype test of the many-token experts kernel sequence (``moe_forward_tokens``)"""
+    return (x.device.type == "cuda" and x.dtype in (torch.float16, torch.bfloat16)
+            and ggml.lowbit_moe_tokens_supported(qtype, hidden, inter, n_experts, top_k))
+
+
+def moe_forward_tokens(x: torch.Tensor, topk_ids: torch.Tensor, topk_weight: torch.Tensor, gates: torch.Tensor, ups: torch.Tensor,
+                       downs: torch.Tensor, hidden: int, inter: int, qtype: int, act: int = SILU):
+    """The routed experts' MLPs of many tokens (the expert loop of models/qwen3_moe.py:106-132): x [T, hidden] fp16 / bf16,
+    ``topk_ids`` / ``topk_weight`` [T, top_k] and the address tables as in ``moe_forward_vec``; the pairs are sorted by expert on
+    the device, every expert's rows run in one launch per projection.  Returns [T, hidden] in x's dtype."""
+    T, top_k = topk_ids.shape
+    invalidInputError(x.dim() == 2 and tuple(x.shape) == (T, hidden), f"activation shape {tuple(x.shape)} != ({T}, {hidden})")
+    invalidInputError(x.dtype in (torch.float16, torch.bfloat16), f"unsupported activation dtype {x.dtype}")
+    invalidInputError(topk_ids.dtype in (torch.int32, torch.int64), "topk_ids must be int32 or int64")
+    invalidInputError(topk_weight.dtype in _TORCH_TO_DT and topk_weight.shape == topk_ids.shape, "topk_weight must match topk_ids")
+    invalidInputError(gates.numel() == ups.numel() == downs.numel() and gates.element_size() == 8,
+                      "gates / ups / downs must be equally long tensors of 64-bit addresses")
+    x = x.contiguous()
+    if x.data_ptr() % 16:
+        x = x.clone()                                        # rows cut out of a wider buffer: the kernels load 16 bytes at a time
+    topk_ids, topk_weight = topk_ids.contiguous(), topk_weight.contiguous()
+    out = torch.empty((T, hidden), dtype=x.dtype, device=x.device)
+    if T == 0:
+        return out
+    dev = x.device
+    need = ggml.lowbit_moe_tokens_workspace_size(hidden, inter, gates.numel(), T, top_k)
+    ws = torch.empty(need, dtype=torch.uint8, device=dev)     # rows of activations: from the allocator, not kept
+    with _on_device(dev):
+        ggml.lowbit_moe_tokens_cuda(x.data_ptr(), _TORCH_TO_DT[x.dtype], T, topk_ids.data_ptr(), 1 if topk_ids.dtype == torch.int64 else 0,
+                                    topk_weight.data_ptr(), _TORCH_TO_DT[topk_weight.dtype], top_k, gates.data_ptr(), ups.data_ptr(),
+                                    downs.data_ptr(), gates.numel(), hidden, inter, qtype, act, out.data_ptr(), ws.data_ptr(), need, _raw_stream(dev))
+    return out
+
+
 def ggml_matmul_src1_x_src0_t(src0: torch.Tensor, src1: torch.Tensor, src0_shape: torch.Size, src0_qtype: int):
     """LBL:494-529: result[M,N] = src1[M,K] . W[N,K]^T with W = canonical packed blocks on the
     CPU; fp32 in, fp32 out, one call across the reference C ABI (which runs on the GPU here)."""

@@ -1,0 +1,135 @@
+"""The two-SM prompt matmul (csrc/gemm_pair.cu): edges of its tiles against float64 on the dequantised weights, plain, with the fused
+MLP's activation, and over the experts of a mixture (csrc/experts.cu).
+
+Bounds.  Weights are rounded once to the activation dtype and the sum is taken in 32 bits, so a product's error is at most
+u * sum|x w| with u = 2^-11 (fp16) / 2^-9 + 2^-11 (bf16, whose expansion goes through fp16), plus 2^-20 * sum|x w| for the
+accumulation, plus u * |y| for a 16-bit result's own rounding."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+U = {torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -9 + 2.0 ** -11}
+
+
+@pytest.fixture(scope="module")
+def lbl(native_lib, cuda_device):
+    from ipex_llm_b200.transformers import low_bit_linear
+    yield low_bit_linear
+    assert not native_lib.lowbit_gemm_wait_expired()
+
+
+def weights(lbl, dev, seed, n, k, qtype, count=1):
+    g = torch.Generator(device=dev).manual_seed(seed)
+    out = []
+    for _ in range(count):
+        w = torch.empty(n, k, device=dev).normal_(0.0, 0.02, generator=g)
+        qt = lbl.ggml_tensor_qtype[qtype]
+        tiled = lbl.FP4Params(w, qtype=qt).to(dev).data
+        out.append((tiled, lbl.dequantize_device_layout(tiled, (n, k), qt).double()))
+    return out, qt
+
+
+def acts(dev, seed, m, k, dtype):
+    return torch.empty(m, k, device=dev).normal_(generator=torch.Generator(device=dev).manual_seed(seed)).to(dtype)
+
+
+def product(x, w, u):
+    """x w^T in 64 bits and the bound of a 32-bit sum over weights rounded to u"""
+    return x @ w.T, (u + 2.0 ** -20) * (x.abs() @ w.abs().T)
+
+
+# one row over a 16- / 128- / 256-token tile, a lone feature pair and an odd one, one k-block, K splits and several rounds of tiles
+@pytest.mark.parametrize("m,n,k", [(65, 128, 64), (96, 384, 128), (129, 256, 4096), (256, 640, 192), (257, 128, 2048), (513, 2176, 320),
+                                   (100, 4096, 1024), (1037, 19072, 64)])
+@pytest.mark.parametrize("qtype,dtype", [("sym_int4", torch.float16), ("asym_int4", torch.bfloat16), ("nf4", torch.float16), ("fp8_e4m3", torch.bfloat16),
+                                         ("fp8_e5m2", torch.float16), ("fp6", torch.bfloat16)])
+def test_prompt_matmul_edges(lbl, cuda_device, qtype, dtype, m, n, k):
+    [(w, wd)], qt = weights(lbl, cuda_device, m + n, n, k, qtype)
+    x = acts(cuda_device, k, m, k, dtype)
+    want, bound = product(x.double(), wd, U[dtype])
+    y32 = lbl.lowbit_matmul(x, w, (n, k), qt, out_dtype=torch.float32)
+    assert bool(((y32.double() - want).abs() <= bound + 1e-30).all())
+    y = lbl.lowbit_matmul(x, w, (n, k), qt)
+    assert torch.equal(y, y32.to(dtype))
+    # bias and accumulation are added in 32 bits; a result that starts off a 16-byte boundary is written all the same
+    bias = acts(cuda_device, 5, 1, n, dtype)[0]
+    out = torch.empty(m * n + 1, dtype=dtype, device=cuda_device)[1:].view(m, n)
+    out.copy_(acts(cuda_device, 6, m, n, dtype))
+    old = out.double()
+    lbl.lowbit_matmul(x, w, (n, k), qt, out=out, bias=bias, accumulate=True)
+    # two 32-bit additions (2^-24 of each partial result), then one rounding to 16 bits: half a unit in the last place, at least half
+    # of the format's smallest step
+    base, terms = y32.double() + bias.double() + old, y32.double().abs() + bias.double().abs() + old.abs()
+    u16, tiny = (2.0 ** -11, 2.0 ** -25) if dtype == torch.float16 else (2.0 ** -8, 0.0)
+    assert bool(((out.double() - base).abs() <= 2.0 ** -22 * terms + u16 * base.abs() + tiny).all())
+
+
+def test_prompt_matmul_without_scratch_for_partial_sums(lbl, native_lib, cuda_device):
+    """a workspace too small for the K split the shape would take: the same product from whole K ranges"""
+    m, n, k = 100, 256, 4096
+    [(w, wd)], qt = weights(lbl, cuda_device, 3, n, k, "sym_int4")
+    x = acts(cuda_device, 4, m, k, torch.float16)
+    assert native_lib.lowbit_matmul_workspace_size(n, k, m, native_lib.DT_F16) > 256
+    y, ws = torch.empty(m, n, dtype=torch.float32, device=cuda_device), torch.empty(256, dtype=torch.uint8, device=cuda_device)
+    native_lib.lowbit_matmul_cuda(w.data_ptr(), qt, n, k, x.data_ptr(), native_lib.DT_F16, m, y.data_ptr(), native_lib.DT_F32, None, False,
+                                  ws.data_ptr(), ws.numel(), torch.cuda.current_stream().cuda_stream)
+    want, bound = product(x.double(), wd, U[torch.float16])
+    assert bool(((y.double() - want).abs() <= bound).all())
+
+
+def gated(x, wg, wu, u, act):
+    """act(x wg^T) * (x wu^T) and its bound: both activations' slopes are below 1.13"""
+    f = torch.nn.functional.silu if act == 0 else torch.nn.functional.gelu
+    g, bg = product(x, wg, u)
+    p, bp = product(x, wu, u)
+    a = f(g)
+    return a * p, 1.13 * bg * (p.abs() + bp) + a.abs() * bp + 1e-6 * (a * p).abs() + 1e-6 * p.abs()
+
+
+@pytest.mark.parametrize("m,n,k", [(65, 128, 128), (257, 384, 64), (600, 1408, 512)])
+@pytest.mark.parametrize("qtype,dtype,act", [("sym_int4", torch.bfloat16, 0), ("asym_int4", torch.float16, 1), ("nf4", torch.bfloat16, 0), ("fp6", torch.float16, 0),
+                                             ("fp8_e4m3", torch.float16, 1)])
+def test_prompt_mlp_edges(lbl, cuda_device, qtype, dtype, act, m, n, k):
+    ((wg, g), (wu, p)), qt = weights(lbl, cuda_device, m, n, k, qtype, 2)
+    x = acts(cuda_device, n, m, k, dtype)
+    want, bound = gated(x.double(), g, p, U[dtype], act)
+    y32 = lbl.mlp_forward(x, wg, wu, m, k, n, act, qt, out=torch.empty(m, n, dtype=torch.float32, device=cuda_device))
+    assert bool(((y32.double() - want).abs() <= bound).all())
+    assert torch.equal(lbl.mlp_forward(x, wg, wu, m, k, n, act, qt), y32.to(dtype))
+    odd = torch.empty(m * n + 1, dtype=dtype, device=cuda_device)[1:].view(m, n)                  # not on a 16-byte boundary
+    assert torch.equal(lbl.mlp_forward(x, wg, wu, m, k, n, act, qt, out=odd), y32.to(dtype))
+
+
+@pytest.mark.parametrize("rows,experts,top_k,skew", [(1, 4, 2, False), (2, 3, 1, False), (40, 16, 4, False), (300, 4, 2, True), (700, 40, 2, False), (600, 2, 2, False)])
+@pytest.mark.parametrize("qtype,dtype", [("sym_int4", torch.bfloat16), ("fp8_e4m3", torch.float16)])
+def test_experts_of_many_tokens(lbl, cuda_device, qtype, dtype, rows, experts, top_k, skew):
+    """unused experts, experts of one row, of more rows than a tile, every token on one expert; ids outside the table add nothing"""
+    H, I = 256, 384
+    ws, qt = weights(lbl, cuda_device, rows, I, H, qtype, 2 * experts)
+    downs, _ = weights(lbl, cuda_device, rows + 1, H, I, qtype, experts)
+    table = lambda ts: torch.tensor([t.data_ptr() for t, _ in ts], dtype=torch.int64, device=cuda_device)         # noqa: E731
+    gen = torch.Generator(device=cuda_device).manual_seed(rows)
+    ids = torch.randint(0, experts, (rows, top_k), generator=gen, device=cuda_device)
+    if skew:
+        ids[:, 0] = experts - 1
+        ids[5, 1] = experts + 7
+        ids[6, 0] = -1
+    wgt = torch.rand(rows, top_k, generator=gen, device=cuda_device)
+    x = acts(cuda_device, 1, rows, H, dtype)
+    got = lbl.moe_forward_tokens(x, ids if skew else ids.int(), wgt, table(ws[:experts]), table(ws[experts:]), table(downs), H, I, qt)
+    want = torch.zeros(rows, H, dtype=torch.float64, device=cuda_device)
+    bound, u = torch.zeros_like(want), U[dtype]
+    for e in range(experts):
+        r, s = torch.where(ids == e)
+        if not len(r):
+            continue
+        h, bh = gated(x[r].double(), ws[e][1], ws[experts + e][1], u, 0)
+        bh = bh + u * (h.abs() + bh)                                          # the hidden rows are rounded to the activation dtype
+        y, by = product(h, downs[e][1], u)
+        by = by + (1 + u) * bh @ downs[e][1].abs().T
+        by = by + u * (y.abs() + by)
+        want.index_add_(0, r, y * wgt[r, s, None].double())
+        bound.index_add_(0, r, by * wgt[r, s, None].double())
+    bound = bound + u * want.abs() + 1e-7                                     # fp16's smallest step
+    assert bool(((got.double() - want).abs() <= bound).all())
