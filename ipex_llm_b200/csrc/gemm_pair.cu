@@ -34,8 +34,6 @@ constexpr int kPairThreads = 32 * 24;
 constexpr int kPairTok = 256;                 // most tokens of a tile
 constexpr int kPairDeq0 = 4, kPairEpi0 = 20;  // first dequant / epilogue warp
 constexpr int kMaxExperts = 256;
-constexpr long long kPairWaitCycles = 4000000000ll;       // about two seconds
-__device__ unsigned int g_wait_expired;
 
 template <int QT> struct PairSmem {
     static constexpr int kGroup = PackedBlock<QT>::kGroup;
@@ -70,24 +68,6 @@ struct PairArgs {
     float* part;                       // ksplit > 1: [ksplit][M][N]
 };
 
-__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    return ok != 0;
-}
-// whole warp; the same answer in every lane.  false: the limit ran out
-__device__ __forceinline__ bool mbar_wait_lim(uint32_t bar, uint32_t parity) {
-    if (__all_sync(0xffffffffu, mbar_test(bar, parity))) return true;
-    const long long t0 = clock64();
-    while (!__all_sync(0xffffffffu, mbar_test(bar, parity))) {
-        if (__any_sync(0xffffffffu, clock64() - t0 > kPairWaitCycles)) {
-            if ((threadIdx.x & 31) == 0) atomicExch(&g_wait_expired, 1u);
-            return false;
-        }
-    }
-    return true;
-}
 // one arrival at the barrier at this shared-memory offset of CTA `rank` of the cluster
 __device__ __forceinline__ void mbar_arrive_at(uint32_t bar, uint32_t rank) {
     asm volatile("{\n\t.reg .b32 ra;\n\tmapa.shared::cluster.u32 ra, %0, %1;\n\t"
@@ -357,8 +337,6 @@ pair_kernel(const __grid_constant__ CUtensorMap xmap, const PairArgs A) {
                         hi[gi][2 * k4] = a[1]; hi[gi][2 * k4 + 1] = a[3];
                     }
                 }
-                __syncwarp();
-                if (lane == 0) mbar_arrive(p_empty(sp));
                 if (!mbar_wait_lim(a_empty(grp), (uint32_t)(((it >> 2) & 1) ^ 1))) goto done;
 #pragma unroll
                 for (int gi = 0; gi < 2; gi++)
@@ -370,7 +348,9 @@ pair_kernel(const __grid_constant__ CUtensorMap xmap, const PairArgs A) {
                     }
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");      // generic-proxy writes -> async-proxy (MMA) reads
                 __syncwarp();
-                if (lane == 0) mbar_arrive_at(a_full(grp), 0);
+                // the packed slot goes back only here: the stores above used every loaded code.  An arrival right behind the expansion could
+                // be issued while the second row group's loads were still under way, and the next copy then overtook them
+                if (lane == 0) { mbar_arrive(p_empty(sp)); mbar_arrive_at(a_full(grp), 0); }
             }
         }
     } else if (warp >= kPairEpi0) {
@@ -659,10 +639,6 @@ int gemm_tc_experts_launch(const unsigned long long* tab, const unsigned long lo
     return check_launch();
 }
 
-int gemm_tc_wait_expired() {
-    unsigned int v = 0;
-    if (cudaMemcpyFromSymbol(&v, gemmtc::g_wait_expired, sizeof(v)) != cudaSuccess) { cudaGetLastError(); return -1; }
-    return (int)v;
-}
+int gemm_tc_wait_expired() { return gemmtc::wait_expired_here(); }
 
 }  // namespace lowbit

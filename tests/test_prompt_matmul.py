@@ -133,3 +133,17 @@ def test_experts_of_many_tokens(lbl, cuda_device, qtype, dtype, rows, experts, t
         bound.index_add_(0, r, by * wgt[r, s, None].double())
     bound = bound + u * want.abs() + 1e-7                                     # fp16's smallest step
     assert bool(((got.double() - want).abs() <= bound).all())
+
+
+@pytest.mark.parametrize("qtype,dtype", [("asym_int4", torch.float16), ("sym_int4", torch.bfloat16), ("nf4", torch.float16), ("fp8_e4m3", torch.bfloat16)])
+def test_prompt_matmul_rings_over_many_rounds(lbl, cuda_device, qtype, dtype):
+    """several tiles per cluster and 32-bit results, whose slow epilogue stalls the MMAs until every ring is full: each slot is refilled
+    only after its readers have used what they loaded"""
+    m, n, k = 2048, 14336, 1024
+    [(w, wd)], qt = weights(lbl, cuda_device, 8, n, k, qtype)
+    x = acts(cuda_device, 9, m, k, dtype)
+    want, bound = product(x.double(), wd, U[dtype])
+    first = lbl.lowbit_matmul(x, w, (n, k), qt, out_dtype=torch.float32)
+    assert bool(((first.double() - want).abs() <= bound).all())
+    for _ in range(8):
+        assert torch.equal(lbl.lowbit_matmul(x, w, (n, k), qt, out_dtype=torch.float32), first)
