@@ -345,7 +345,7 @@ int lowbit_moe_tokens_cuda(const void* d_x, int x_dtype, int64_t n_tokens, const
                            int64_t hidden, int64_t inter, int qtype, int act, void* d_y,
                            void* workspace, size_t workspace_bytes, void* stream);
 
-/* 1 when a bounded wait inside the two-SM matmul kernel has run out on the current device since the library was loaded (the
+/* 1 when a bounded wait inside the prompt matmul or the prompt attention has run out on the current device since the library was loaded (the
  * launch's results are then undefined), 0 otherwise, -1 without a device.  Synchronises. */
 int lowbit_gemm_wait_expired(void);
 

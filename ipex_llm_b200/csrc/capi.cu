@@ -362,7 +362,10 @@ int lowbit_moe_tokens_cuda(const void* d_x, int x_dtype, int64_t n_tokens, const
     return rc;
 }
 
-int lowbit_gemm_wait_expired(void) { return gemm_tc_wait_expired(); }
+int lowbit_gemm_wait_expired(void) {
+    const int a = gemm_tc_wait_expired(), b = sdp_prompt_wait_expired();
+    return a < 0 || b < 0 ? -1 : a | b;
+}
 
 // ------------------------------------------------------------------ family (1)
 size_t ggml_quantize_tensor(const float* src, void* dst, int qtype, size_t n, int k, int64_t* hist,

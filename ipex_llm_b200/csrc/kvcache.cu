@@ -19,6 +19,7 @@
 #include "../../include/b200_lowbit.h"
 #include "lowbit_common.cuh"
 #include "lowbit_internal.h"
+#include "tc_common.cuh"
 
 namespace lowbit {
 namespace {
@@ -437,6 +438,7 @@ size_t sdp_workspace(int B, int Hq, int Hkv, int S, int L, int D, bool mma) {
     return (size_t)B * Hkv * sdp_tiles(Hq, Hkv, S, mma) * sdp_splits(B, Hq, Hkv, S, L, D, mma) * sdp_rt(Hq, Hkv, S, mma) * (D + 2) * sizeof(float);
 }
 }  // namespace
+int sdp_prompt_wait_expired() { return gemmtc::wait_expired_here(); }
 }  // namespace lowbit
 
 // ------------------------------------------------------------------ C ABI (declared in include/b200_lowbit.h)
@@ -666,10 +668,7 @@ extern "C" int lowbit_sdp_fp8_prefill_strided_cuda(const void* d_q, int q_dtype,
     A.causal = causal; A.scale_log2e = scale * 1.4426950408889634f;
     A.B = B; A.Hq = Hq; A.Hkv = Hkv; A.S = S; A.L = L; A.D = D;
     A.out = d_out; A.out_dtype = out_dtype; A.o_sb = out_strides[0]; A.o_sh = out_strides[1]; A.o_ss = out_strides[2];
-    const dim3 grid((unsigned)((S + PF_ROWS - 1) / PF_ROWS), (unsigned)(B * Hq), 1);
-    sdp_fp8_prefill_kernel<<<grid, PF_WARPS * 32, 0, (cudaStream_t)stream>>>(A);
-    note_launch();
-    return check_launch();
+    return sdp_prompt_launch(A, (cudaStream_t)stream);
 }
 
 // ------------------------------------------------------------------ the attention of one decode step, one call

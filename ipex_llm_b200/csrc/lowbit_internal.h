@@ -88,6 +88,7 @@ int gemm_tc_mlp_launch(const void* w_gate, const void* w_up, int act, int qt, in
 int gemm_tc_experts_launch(const unsigned long long* tab, const unsigned long long* tab2, int act, const int* offs, int n_experts, int qt,
                            int64_t n_rows, int64_t k, const void* x, int x_dtype, int64_t rows, void* y, int y_dtype, cudaStream_t st);
 int gemm_tc_wait_expired();       // 1 after a wait of the two-SM kernel ran out on the current device (its results are then undefined)
+int sdp_prompt_wait_expired();    // the same of the prompt attention (kvcache.cu)
 
 // M above this goes to the tensor-core GEMM when the shape allows, else to chunks of the GEMV
 constexpr int64_t kGemvMaxM = 32;

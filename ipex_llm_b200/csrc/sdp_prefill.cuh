@@ -2,217 +2,355 @@
 // Attention of MANY query tokens over the e5m2 cache -- xe_addons.sdp_fp8_causal / sdp_fp8_non_causal of the reference
 // (models/common.py:264-286: the prefill, where key.dtype == uint8 because DynamicFp8Cache.update returned the cache).
 //
-// fp16 / bf16 queries, head_dim 128.  One CTA = 64 query rows of one (sequence, query head): 4 warps x one full m16 tile
-// (rows g and g + 8 per lane -- the decode kernel in sdp_mma.cuh uses the same fragments with rows 8..15 zero).  All four
-// warps walk the same keys, so the 32-key chunks (4 KB of K + 4 KB of V) are staged ONCE per CTA through a 3-stage
-// cp.async ring with the decode kernel's XOR swizzles, and read by every warp:
-//   S = Q . K^T : mma.m16n8k16, e5m2 -> fp16 by byte permute, head dimension in the permuted order of sdp_mma.cuh;
-//   online softmax per row in the accumulator layout (a row's 32 scores of a chunk sit in the 4 lanes of a quad);
-//   O += P . V  : the score accumulators are the A fragments of P; a tile of ones accumulates the denominator from the
-//                 same rounded P.
-// Causal: query token s (0-based among the S new ones) sees keys <= L - S + s; chunks beyond a tile's last row are
-// never loaded, chunks beyond a warp's last row are skipped by that warp.  An additive mask [B][1|Hq][S][L] is honoured.
-// Softmax and accumulation in fp32, P and Q enter the MMAs as fp16: the decode kernel's tolerance statement applies.
+// fp16 / bf16 queries, head_dim 128, both products on the 5th-generation tensor cores.  One CTA = NT tiles of 128 query rows of one
+// (sequence, query head), walking the keys in tiles of 128:
+//   S_t = Q_t . K^T   tcgen05.mma M = 128, N = 128, K = 16, both operands in shared memory, S in TMEM (lane = query row);
+//   softmax           four warps per tile, one thread per row: the row's 128 scores in registers, P (fp16) back into TMEM over S;
+//   O_t += P_t . V    A operand = P in TMEM, B operand = V as it lies in the cache (rows = keys: the MN-major descriptor).
+// Warps 0 .. 4 NT - 1: softmax; the next four read the cache (16 bytes a thread, coalesced), expand e5m2 -> fp16 (one byte permute
+// per pair) and write K and V into a ring of four 32 KB swizzled tiles; the last warp issues the MMAs and owns TMEM.
+// With two tiles a CTA their softmax and MMAs alternate: P_t . V, then Q_t . K of the next keys, of one tile run while the other is in
+// its softmax, and every key tile is expanded once for 256 rows.  P lies over S, so a tile's next Q . K waits for its P . V (a commit,
+// not the issue order).  What bounds it: per 128 keys and 256 rows 2048 clocks of MMAs, 2048 of ex2 (16 a clock), and the chain
+// Q.K -> softmax -> P.V of one tile.  The kernel it replaces (64 rows a CTA, mma.sync) was bound by the legacy tensor path:
+// 4000 causal tokens, 32 heads: 601 us, 218 TFLOP/s.
+// Causal: query token s (0-based among the S new ones) sees keys <= L - S + s; key tiles beyond a tile's last row are skipped.  An
+// additive mask [B][1|Hq][S][L] is honoured.  Softmax and accumulation in 32 bits; Q and P enter the MMAs as fp16.  P is kept relative
+// to a reference 2^8 below fp16's comfortable range (values up to 2^14, nothing above 2^-32 of the row's maximum is flushed), and the
+// reference follows the row's maximum only when that grew by more than 2^6: O is then rescaled in TMEM, which is rarely.
 
-__device__ __forceinline__ void mma16816_f16_full(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-        : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+constexpr int SP_ROWS = 128, SP_KEYS = 128, SP_SLOTS = 4;
+constexpr int SP_TILE = 128 * 256;                                    // 128 rows x 128 fp16, as two swizzled halves of 64 columns
+constexpr int SP_BARS = 256;
+__host__ __device__ constexpr int sp_smem(int nt) { return 1024 + (nt + SP_SLOTS) * SP_TILE + SP_BARS; }
+constexpr int sp_threads(int nt) { return 32 * (4 * nt + 5); }
+
+__device__ __forceinline__ void sp_tmem_ld32(uint32_t taddr, float* v) {
+    uint32_t* r = reinterpret_cast<uint32_t*>(v);
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+          "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
+          "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        : "r"(taddr));
+}
+__device__ __forceinline__ void sp_tmem_st32(uint32_t taddr, const uint32_t* r) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
+        "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
+        ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+          "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]),
+          "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]),
+          "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31]) : "memory");
+}
+__device__ __forceinline__ void sp_umma_ts_w(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate, uint32_t leader) {
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "setp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+        ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(leader) : "memory");
+}
+__device__ __forceinline__ void sp_sts128(uint32_t a, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
+    asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
 }
 
-constexpr int PF_WARPS = 4;
-constexpr int PF_ROWS = 16 * PF_WARPS;           // query rows per CTA
-constexpr int PF_STAGES = 3;
-
-__global__ void __launch_bounds__(PF_WARPS * 32, 1)
-sdp_fp8_prefill_kernel(const SdpArgs A) {
-    constexpr int D = 128, NC = 2, BPL = 16, VW = 4;
-    __shared__ __align__(128) uint8_t ring[PF_STAGES * 8192];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int g = lane >> 2, t = lane & 3;
-    const int hq = blockIdx.y % A.Hq, b = blockIdx.y / A.Hq;
-    const int hkv = hq / (A.Hq / A.Hkv);
-    const int q0 = blockIdx.x * PF_ROWS;                              // first query token of the CTA
-    const int row_a = q0 + 16 * warp + g, row_b = row_a + 8;          // this lane's two query tokens
+template <int NT>
+__global__ void __launch_bounds__(sp_threads(NT), 1)
+sdp_fp8_prompt_kernel(const SdpArgs A, int n_qt) {
+    using namespace gemmtc;
+    extern __shared__ uint8_t sp_raw[];
+    const uint32_t base = (smem_u32(sp_raw) + 1023u) & ~1023u;
+    const uint32_t qs = base, ring = base + NT * SP_TILE, bars = ring + SP_SLOTS * SP_TILE;
+    auto kv_full = [&](int s) { return bars + s * 8; };
+    auto kv_empty = [&](int s) { return bars + 32 + s * 8; };
+    auto q_ready = [&](int t) { return bars + 64 + t * 8; };
+    auto s_full = [&](int t) { return bars + 80 + t * 8; };
+    auto p_full = [&](int t) { return bars + 96 + t * 8; };
+    auto pv_done = [&](int t) { return bars + 112 + t * 8; };
+    const uint32_t tmem_slot = bars + 128;
+    constexpr uint32_t TMEM_COLS = NT * 256;                           // S_t at 128 t, O_t behind all S
+    const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+    const int hq = blockIdx.x % A.Hq, b = blockIdx.x / A.Hq, hkv = hq / (A.Hq / A.Hkv);
+    const int q0 = (n_qt - 1 - (int)blockIdx.y) * NT * SP_ROWS;        // the longest tiles of a causal prompt start first
     const int L = A.L, S = A.S;
+    // key tiles that the rows of tile t need (0: no rows)
+    auto tiles_of = [&](int t) {
+        const int first = q0 + t * SP_ROWS;
+        if (first >= S) return 0;
+        const int last = min(first + SP_ROWS, S) - 1;
+        const int end = A.causal ? min(L, L - S + last + 1) : L;
+        return (end + SP_KEYS - 1) / SP_KEYS;
+    };
+    int nk = tiles_of(0);
+    if (NT == 2) nk = max(nk, tiles_of(1));
 
-    // A fragments of Q (fp16): rows g (qa) and g + 8 (qb), elements 64c + 16t .. +15 as 8 pairs each
-    uint32_t qa[NC][8], qb[NC][8];
-    auto load_q = [&](int row, uint32_t (&dst)[NC][8]) {
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < SP_SLOTS; s++) { mbar_init(kv_full(s), 4); mbar_init(kv_empty(s), 1); }
+        for (int t = 0; t < 2; t++) { mbar_init(q_ready(t), 4); mbar_init(s_full(t), 1); mbar_init(p_full(t), 4); mbar_init(pv_done(t), 1); }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 4 * NT + 4) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tmem_slot), "r"(TMEM_COLS) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    uint32_t tmem;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem) : "r"(tmem_slot));
+
+    if (warp < 4 * NT) {
+        // ================= softmax: thread = query row =================
+        const int t = warp >> 2, quarter = warp & 3, r = 32 * quarter + lane, row = q0 + t * SP_ROWS + r;
+        const int nkt = tiles_of(t);
+        if (nkt > 0) {
+            // the row as fp16 into the swizzled operand tile (rows beyond S: zeros)
+            const uint4* qrow = reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(A.q) + b * A.q_sb + hq * A.q_sh + (int64_t)row * A.q_ss);
+            const uint32_t qd = qs + t * SP_TILE + r * 128;
+#pragma unroll 4
+            for (int c = 0; c < 16; c++) {
+                uint4 w = make_uint4(0u, 0u, 0u, 0u);
+                if (row < S) {
+                    w = qrow[c];
+                    if (A.q_dtype != DT_F16) {
+                        uint32_t u[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
-        for (int c = 0; c < NC; c++)
-#pragma unroll
-            for (int i = 0; i < 8; i++) dst[c][i] = 0u;
-        if (row < S) {
-            const uint16_t* qrow = reinterpret_cast<const uint16_t*>(A.q) + b * A.q_sb + hq * A.q_sh + (int64_t)row * A.q_ss + 16 * t;
-#pragma unroll
-            for (int c = 0; c < NC; c++) {
-                const uint4 w0 = *reinterpret_cast<const uint4*>(qrow + 64 * c), w1 = *reinterpret_cast<const uint4*>(qrow + 64 * c + 8);
-                const uint32_t ws[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
-#pragma unroll
-                for (int i = 0; i < 8; i++) {
-                    if (A.q_dtype == DT_F16) dst[c][i] = ws[i];
-                    else {
-                        const __half2 h = __floats2half2_rn(__uint_as_float(ws[i] << 16), __uint_as_float(ws[i] & 0xffff0000u));
-                        dst[c][i] = *reinterpret_cast<const uint32_t*>(&h);
+                        for (int i = 0; i < 4; i++) {
+                            const __half2 h = __floats2half2_rn(__uint_as_float(u[i] << 16), __uint_as_float(u[i] & 0xffff0000u));
+                            u[i] = *reinterpret_cast<const uint32_t*>(&h);
+                        }
+                        w = make_uint4(u[0], u[1], u[2], u[3]);
                     }
                 }
+                sp_sts128(qd + (c >> 3) * (SP_TILE / 2) + (((c & 7) ^ (r & 7)) << 4), w.x, w.y, w.z, w.w);
             }
-        }
-    };
-    load_q(row_a, qa);
-    load_q(row_b, qb);
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(q_ready(t));
 
-    // keys this CTA / this warp / each row needs
-    const int last_row_cta = min(q0 + PF_ROWS, S) - 1, last_row_warp = min(q0 + 16 * warp + 15, S - 1);
-    const int key_end = A.causal ? min(L, L - S + last_row_cta + 1) : L;           // exclusive
-    const int key_end_warp = A.causal ? min(L, L - S + last_row_warp + 1) : L;
-    const int lim_a = A.causal ? L - S + row_a : L - 1, lim_b = A.causal ? L - S + row_b : L - 1;   // last visible key
-    const int first_full = A.causal ? L - S + q0 + 16 * warp : L;                  // keys below are visible to every row of the warp
-    const int64_t mbase_a = b * A.m_sb + hq * A.m_sh + (int64_t)row_a * A.m_ss, mbase_b = b * A.m_sb + hq * A.m_sh + (int64_t)row_b * A.m_ss;
-
-    const uint8_t* const kb0 = A.k + b * A.k_sb + hkv * A.k_sh;
-    const uint8_t* const vb0 = A.v + b * A.v_sb + hkv * A.v_sh;
-    const uint32_t ring_s = (uint32_t)__cvta_generic_to_shared(ring);
-    const int cr = threadIdx.x >> 3, unit = threadIdx.x & 7;         // thread copies piece `unit` of rows cr and cr + 16
-    auto stage_chunk = [&](int c0, int slot) {
-        if (c0 < key_end) {
-            const uint32_t dst = ring_s + slot * 8192;
+            const uint32_t lanes = (uint32_t)(32 * quarter) << 16;
+            const uint32_t st = tmem + lanes + t * 128, ot = tmem + lanes + (NT + t) * 128;
+            const int lim = A.causal ? L - S + row : L - 1;                       // last visible key
+            const int plain_end = A.mask ? -1 : A.causal ? min(L, L - S + q0 + t * SP_ROWS + 32 * quarter + 1) : L;   // keys below: visible to the whole warp
+            const int64_t mbase = b * A.m_sb + hq * A.m_sh + (int64_t)row * A.m_ss;
+            float m_ref = -CUDART_INF_F, sum = 0.0f;
+            for (int j = 0; j < nkt; j++) {
+                if (!mbar_wait_lim(s_full(t), (uint32_t)(j & 1))) goto done;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                float s[128];
 #pragma unroll
-            for (int i = 0; i < 2; i++) {
-                const int r = cr + 16 * i;
-                const int64_t key = min(c0 + r, key_end - 1);        // rows beyond the range repeat the last key (p = 0)
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst + r * 128 + ((unit ^ ((r & 1) << 2)) << 4)),
-                             "l"(kb0 + key * A.k_ss + 16 * unit) : "memory");
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst + 4096 + r * 128 + ((unit ^ (((r >> 1) & 3) << 1)) << 4)),
-                             "l"(vb0 + key * A.v_ss + 16 * unit) : "memory");
-            }
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-
-    float m_a = -CUDART_INF_F, m_b = -CUDART_INF_F;
-    float o[BPL][4], ol[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                for (int c = 0; c < 4; c++) sp_tmem_ld32(st + 32 * c, s + 32 * c);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                float mul = A.scale_log2e;
+                const int k0 = j * SP_KEYS;
+                if (k0 + SP_KEYS > plain_end) {
+                    mul = 1.0f;
 #pragma unroll
-    for (int u = 0; u < BPL; u++) o[u][0] = o[u][1] = o[u][2] = o[u][3] = 0.0f;
-
-    stage_chunk(0, 0);
-    stage_chunk(32, 1);
-    int slot = 0;
-    for (int c0 = 0; c0 < key_end; c0 += 32) {
-        asm volatile("cp.async.wait_group 1;" ::: "memory");
-        __syncthreads();                              // chunk c0 has landed for everybody; everybody is done with chunk c0 - 32
-        {
-            int ahead = slot + 2; if (ahead >= PF_STAGES) ahead -= PF_STAGES;
-            stage_chunk(c0 + 64, ahead);
-        }
-        const uint8_t* stage = ring + slot * 8192;
-        if (++slot == PF_STAGES) slot = 0;
-        if (c0 >= key_end_warp) continue;             // nothing in this chunk is visible to this warp's rows
-        // ---- scores of 4 tiles x 8 keys, rows g and g + 8
-        float sc[4][4];
-#pragma unroll
-        for (int n = 0; n < 4; n++) {
-            sc[n][0] = sc[n][1] = sc[n][2] = sc[n][3] = 0.0f;
-#pragma unroll
-            for (int c = 0; c < NC; c++) {
-                const uint4 kw = *reinterpret_cast<const uint4*>(stage + (8 * n + g) * 128 + (((4 * c + t) ^ ((g & 1) << 2)) << 4));
-                const uint32_t ws[4] = {kw.x, kw.y, kw.z, kw.w};
-#pragma unroll
-                for (int s = 0; s < 4; s++)
-                    mma16816_f16_full(sc[n], qa[c][2 * s], qb[c][2 * s], qa[c][2 * s + 1], qb[c][2 * s + 1],
-                                      __byte_perm(ws[s], 0u, 0x1404u), __byte_perm(ws[s], 0u, 0x3424u));
-            }
-        }
-        // ---- scale, mask, online softmax of the two rows; this lane's values are keys c0 + 8n + 2t + i
-        const bool plain = c0 + 32 <= key_end && c0 + 31 <= first_full && !A.mask;     // every key visible to every row
-        float mx_a = -CUDART_INF_F, mx_b = -CUDART_INF_F;
-#pragma unroll
-        for (int n = 0; n < 4; n++)
-#pragma unroll
-            for (int i = 0; i < 2; i++) {
-                float sa = sc[n][i] * A.scale_log2e, sb = sc[n][2 + i] * A.scale_log2e;
-                if (!plain) {
-                    const int key = c0 + 8 * n + 2 * t + i;
-                    const bool oka = key <= lim_a && key < key_end && row_a < S, okb = key <= lim_b && key < key_end && row_b < S;
-                    if (A.mask) {
-                        if (oka) sa += load_as_float(A.mask, A.mask_dtype, mbase_a + key) * 1.4426950408889634f;
-                        if (okb) sb += load_as_float(A.mask, A.mask_dtype, mbase_b + key) * 1.4426950408889634f;
+                    for (int i = 0; i < 128; i++) {
+                        float v = s[i] * A.scale_log2e;
+                        const bool ok = k0 + i <= lim && k0 + i < L && row < S;
+                        if (A.mask && ok) v += load_as_float(A.mask, A.mask_dtype, mbase + k0 + i) * 1.4426950408889634f;
+                        s[i] = ok ? v : -CUDART_INF_F;
                     }
-                    if (!oka) sa = -CUDART_INF_F;
-                    if (!okb) sb = -CUDART_INF_F;
                 }
-                sc[n][i] = sa; sc[n][2 + i] = sb;
-                mx_a = fmaxf(mx_a, sa); mx_b = fmaxf(mx_b, sb);
-            }
-        mx_a = fmaxf(mx_a, __shfl_xor_sync(0xffffffffu, mx_a, 1)); mx_a = fmaxf(mx_a, __shfl_xor_sync(0xffffffffu, mx_a, 2));
-        mx_b = fmaxf(mx_b, __shfl_xor_sync(0xffffffffu, mx_b, 1)); mx_b = fmaxf(mx_b, __shfl_xor_sync(0xffffffffu, mx_b, 2));
-        const float mn_a = fmaxf(m_a, mx_a), mn_b = fmaxf(m_b, mx_b);
-        const float ref_a = (mn_a == -CUDART_INF_F) ? 0.0f : mn_a, ref_b = (mn_b == -CUDART_INF_F) ? 0.0f : mn_b;   // all masked so far: p = 0
-        const float corr_a = ex2_approx(m_a - ref_a), corr_b = ex2_approx(m_b - ref_b);
-        m_a = mn_a; m_b = mn_b;
-        uint32_t pa[4], pb[4];                        // A fragments of P (fp16 pairs), rows g and g + 8
+                float mx0 = s[0], mx1 = s[1], mx2 = s[2], mx3 = s[3];
 #pragma unroll
-        for (int n = 0; n < 4; n++) {
-            const __half2 ha = __floats2half2_rn(ex2_approx(sc[n][0] - ref_a), ex2_approx(sc[n][1] - ref_a));
-            const __half2 hb = __floats2half2_rn(ex2_approx(sc[n][2] - ref_b), ex2_approx(sc[n][3] - ref_b));
-            pa[n] = *reinterpret_cast<const uint32_t*>(&ha);
-            pb[n] = *reinterpret_cast<const uint32_t*>(&hb);
+                for (int i = 4; i < 128; i += 4) { mx0 = fmaxf(mx0, s[i]); mx1 = fmaxf(mx1, s[i + 1]); mx2 = fmaxf(mx2, s[i + 2]); mx3 = fmaxf(mx3, s[i + 3]); }
+                const float mx = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3)) * mul;
+                const bool grow = mx > m_ref + 6.0f;                                // -inf: any visible key
+                if (__any_sync(0xffffffffu, grow)) {
+                    const float m_new = grow ? mx : m_ref;
+                    if (j > 0) {
+                        // the P . V before this Q . K is done: O is at rest
+                        const float corr = grow ? ex2_approx(m_ref - m_new) : 1.0f;
+                        sum *= corr;
+#pragma unroll 1
+                        for (int c = 0; c < 128; c += 32) {
+                            float o[32];
+                            sp_tmem_ld32(ot + c, o);
+                            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+                            for (int i = 0; i < 32; i++) o[i] *= corr;
+                            sp_tmem_st32(ot + c, reinterpret_cast<const uint32_t*>(o));
+                        }
+                    }
+                    m_ref = m_new;
+                }
+                const float shift = 8.0f - (m_ref == -CUDART_INF_F ? 0.0f : m_ref);
+                float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f, a3 = 0.0f;
+#pragma unroll
+                for (int h = 0; h < 2; h++) {
+                    uint32_t pk[32];
+#pragma unroll
+                    for (int i = 0; i < 32; i += 2) {
+                        const float* x = s + 64 * h + 2 * i;
+                        const float p0 = ex2_approx(fmaf(x[0], mul, shift)), p1 = ex2_approx(fmaf(x[1], mul, shift));
+                        const float p2 = ex2_approx(fmaf(x[2], mul, shift)), p3 = ex2_approx(fmaf(x[3], mul, shift));
+                        a0 += p0; a1 += p1; a2 += p2; a3 += p3;
+                        const __half2 h0 = __floats2half2_rn(p0, p1), h1 = __floats2half2_rn(p2, p3);
+                        pk[i] = *reinterpret_cast<const uint32_t*>(&h0);
+                        pk[i + 1] = *reinterpret_cast<const uint32_t*>(&h1);
+                    }
+                    sp_tmem_st32(st + 32 * h, pk);
+                }
+                sum += (a0 + a1) + (a2 + a3);
+                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                __syncwarp();
+                if (lane == 0) mbar_arrive(p_full(t));
+            }
+            if (!mbar_wait_lim(pv_done(t), (uint32_t)((nkt - 1) & 1))) goto done;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const float inv = sum > 0.0f ? 1.0f / sum : 0.0f;                       // a row with every key masked gives zeros
+            const int64_t oi = (int64_t)b * A.o_sb + (int64_t)hq * A.o_sh + (int64_t)row * A.o_ss;
+#pragma unroll 1
+            for (int c = 0; c < 128; c += 32) {
+                float o[32];
+                sp_tmem_ld32(ot + c, o);
+                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                if (row < S) {
+                    if (A.out_dtype == DT_F32) {
+                        float4* p = reinterpret_cast<float4*>((float*)A.out + oi + c);
+#pragma unroll
+                        for (int i = 0; i < 8; i++) p[i] = make_float4(o[4 * i] * inv, o[4 * i + 1] * inv, o[4 * i + 2] * inv, o[4 * i + 3] * inv);
+                    } else {
+                        uint4* p = reinterpret_cast<uint4*>((uint16_t*)A.out + oi + c);
+#pragma unroll
+                        for (int i = 0; i < 4; i++) {
+                            uint32_t w[4];
+#pragma unroll
+                            for (int k = 0; k < 4; k++) {
+                                const float x = o[8 * i + 2 * k] * inv, y = o[8 * i + 2 * k + 1] * inv;
+                                if (A.out_dtype == DT_F16) { const __half2 v = __floats2half2_rn(x, y); w[k] = *reinterpret_cast<const uint32_t*>(&v); }
+                                else { const __nv_bfloat162 v = __floats2bfloat162_rn(x, y); w[k] = *reinterpret_cast<const uint32_t*>(&v); }
+                            }
+                            p[i] = make_uint4(w[0], w[1], w[2], w[3]);
+                        }
+                    }
+                }
+                __syncwarp();
+            }
         }
-        ol[0] *= corr_a; ol[1] *= corr_a; ol[2] *= corr_b; ol[3] *= corr_b;
+    } else if (warp < 4 * NT + 4) {
+        // ================= the cache: item 2 j = keys of tile j, 2 j + 1 = its values =================
+        const int tid = threadIdx.x - 128 * NT, piece = tid & 7, r0 = tid >> 3;       // rows r0, r0 + 16, ...
+        const uint8_t* const kb = A.k + b * A.k_sb + hkv * A.k_sh + 16 * piece;
+        const uint8_t* const vb = A.v + b * A.v_sb + hkv * A.v_sh + 16 * piece;
+        uint4 w[8];
+        auto fetch = [&](int item) {
+            const uint8_t* p = (item & 1) ? vb : kb;
+            const int64_t ss = (item & 1) ? A.v_ss : A.k_ss;
+            const int k0 = (item >> 1) * SP_KEYS + r0;
 #pragma unroll
-        for (int u = 0; u < BPL; u++) { o[u][0] *= corr_a; o[u][1] *= corr_a; o[u][2] *= corr_b; o[u][3] *= corr_b; }
-        // ---- O += P . V (and the denominators through a tile of ones)
+            for (int i = 0; i < 8; i++) w[i] = k0 + 16 * i < L ? *reinterpret_cast<const uint4*>(p + (k0 + 16 * i) * ss) : make_uint4(0u, 0u, 0u, 0u);
+        };
+        // a thread's 16 elements are two chunks of one row's half; lanes of the second half write them in the other order, so that a
+        // quarter warp (one row) meets every bank once
+        const int half = piece >> 2, c0 = 2 * (piece & 3) + half;
+        if (nk > 0) fetch(0);
+        for (int item = 0; item < 2 * nk; item++) {
+            const int s = item % SP_SLOTS, round = item / SP_SLOTS;
+            if (!mbar_wait_lim(kv_empty(s), (uint32_t)((round & 1) ^ 1))) goto done;
+            const uint32_t dst = ring + s * SP_TILE + half * (SP_TILE / 2);
 #pragma unroll
-        for (int j = 0; j < 2; j++) {
-            uint32_t vw[4][VW];
-#pragma unroll
-            for (int h = 0; h < 4; h++) {
-                const uint4 w = *reinterpret_cast<const uint4*>(stage + 4096 + (16 * j + 2 * t + (h & 1) + 8 * (h >> 1)) * 128 + ((g ^ (2 * t)) << 4));
-                vw[h][0] = w.x; vw[h][1] = w.y; vw[h][2] = w.z; vw[h][3] = w.w;
+            for (int i = 0; i < 8; i++) {
+                const int r = r0 + 16 * i;
+                const uint32_t lo0 = __byte_perm(w[i].x, 0u, 0x1404u), lo1 = __byte_perm(w[i].x, 0u, 0x3424u), lo2 = __byte_perm(w[i].y, 0u, 0x1404u),
+                               lo3 = __byte_perm(w[i].y, 0u, 0x3424u), hi0 = __byte_perm(w[i].z, 0u, 0x1404u), hi1 = __byte_perm(w[i].z, 0u, 0x3424u),
+                               hi2 = __byte_perm(w[i].w, 0u, 0x1404u), hi3 = __byte_perm(w[i].w, 0u, 0x3424u);
+                const uint32_t a = dst + r * 128 + ((c0 ^ (r & 7)) << 4), z = dst + r * 128 + (((c0 ^ 1) ^ (r & 7)) << 4);
+                if (half) { sp_sts128(a, hi0, hi1, hi2, hi3); sp_sts128(z, lo0, lo1, lo2, lo3); }
+                else { sp_sts128(a, lo0, lo1, lo2, lo3); sp_sts128(z, hi0, hi1, hi2, hi3); }
             }
-            mma16816_f16_full(ol, pa[2 * j], pb[2 * j], pa[2 * j + 1], pb[2 * j + 1], 0x3c003c00u, 0x3c003c00u);
+            if (item + 1 < 2 * nk) fetch(item + 1);
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(kv_full(s));
+        }
+    } else {
+        // ================= MMA issuer: the whole warp runs the loop, one elected lane issues =================
+        const uint32_t leader = elect_leader();
+        // c F32, a / b fp16, N = 128, M = 128; S: both operands K-major; O: A in TMEM, B (values) MN-major (bit 16)
+        const uint32_t id_s = (1u << 4) | ((128u >> 3) << 17) | ((128u >> 4) << 24), id_o = id_s | (1u << 16);
+        const int nk0 = tiles_of(0), nk1 = NT == 2 ? tiles_of(1) : 0;
+        auto scores = [&](int t, int j) {
+            const uint64_t qd = make_desc(qs + t * SP_TILE), kd = make_desc(ring + ((2 * j) % SP_SLOTS) * SP_TILE);
 #pragma unroll
-            for (int q = 0; q < VW; q++) {
-                // bytes of keys (2t, 2t+1) and (2t+8, 2t+9) interleaved: [a0 b0 a1 b1], [a2 b2 a3 b3]
-                const uint32_t lo01 = __byte_perm(vw[0][q], vw[1][q], 0x5140u), lo23 = __byte_perm(vw[0][q], vw[1][q], 0x7362u);
-                const uint32_t hi01 = __byte_perm(vw[2][q], vw[3][q], 0x5140u), hi23 = __byte_perm(vw[2][q], vw[3][q], 0x7362u);
+            for (int k = 0; k < 8; k++) {
+                const uint64_t step = (uint64_t)(((k >> 2) * (SP_TILE / 2) + (k & 3) * 32) >> 4);
+                umma_f16_w(tmem + t * 128, qd + step, kd + step, id_s, k > 0 ? 1u : 0u, leader);
+            }
+            umma_commit_w(s_full(t), leader);
+        };
+        auto values = [&](int t, int j) {
+            // V tile: element (d, key) at half(d / 64), row key: LBO = the next 64 d, SBO = the next 8 keys; 16 keys a step
+            const uint64_t vd = (make_desc(ring + ((2 * j + 1) % SP_SLOTS) * SP_TILE) & ~((uint64_t)0x3fff << 16)) | ((uint64_t)((SP_TILE / 2) >> 4) << 16);
 #pragma unroll
-                for (int e = 0; e < 4; e++) {
-                    const uint32_t sel = (e & 1) ? 0x3424u : 0x1404u;
-                    mma16816_f16_full(o[4 * q + e], pa[2 * j], pb[2 * j], pa[2 * j + 1], pb[2 * j + 1],
-                                      __byte_perm(e < 2 ? lo01 : lo23, 0u, sel), __byte_perm(e < 2 ? hi01 : hi23, 0u, sel));
+            for (int k = 0; k < 8; k++)
+                sp_umma_ts_w(tmem + (NT + t) * 128, tmem + t * 128 + k * 8, vd + (uint64_t)((k * 2048) >> 4), id_o, (j > 0 || k > 0) ? 1u : 0u, leader);
+            umma_commit_w(pv_done(t), leader);
+        };
+        if (nk > 0) {
+            if (!mbar_wait_lim(kv_full(0), 0u)) goto done;
+            for (int t = 0; t < NT; t++) {
+                if ((t == 0 ? nk0 : nk1) == 0) continue;
+                if (!mbar_wait_lim(q_ready(t), 0u)) goto done;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                scores(t, 0);
+            }
+            umma_commit_w(kv_empty(0), leader);
+        }
+        for (int j = 0; j < nk; j++) {
+            const int vi = 2 * j + 1, ki = 2 * j + 2;
+            if (!mbar_wait_lim(kv_full(vi % SP_SLOTS), (uint32_t)((vi / SP_SLOTS) & 1))) goto done;
+            if (j + 1 < nk && !mbar_wait_lim(kv_full(ki % SP_SLOTS), (uint32_t)((ki / SP_SLOTS) & 1))) goto done;
+            const int last = NT == 2 && j < nk1 ? 1 : 0;
+            for (int t = 0; t < NT; t++) {
+                const int nkt = t == 0 ? nk0 : nk1;
+                if (j >= nkt) continue;
+                if (!mbar_wait_lim(p_full(t), (uint32_t)(j & 1))) goto done;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                values(t, j);
+                if (t == last) umma_commit_w(kv_empty(vi % SP_SLOTS), leader);
+                if (j + 1 < nkt) {
+                    if (!mbar_wait_lim(pv_done(t), (uint32_t)(j & 1))) goto done;         // S and P share their columns
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    scores(t, j + 1);
                 }
             }
+            if (j + 1 < nk) umma_commit_w(kv_empty(ki % SP_SLOTS), leader);
         }
     }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    // ---- normalise and store: row g holds columns 32t .. 32t + 31 (o[u][i] = column 16 (2t + i) + u), row g + 8 likewise
-    auto store_row = [&](int row, int base, float denom) {
-        if (row >= S) return;
-        const float inv = denom > 0.0f ? 1.0f / denom : 0.0f;         // a row with every key masked gives zeros
-        const int64_t oi = (int64_t)b * A.o_sb + (int64_t)hq * A.o_sh + (int64_t)row * A.o_ss + 32 * t;
-#pragma unroll
-        for (int i = 0; i < 2; i++) {
-            if (A.out_dtype == DT_F32) {
-                float* p = (float*)A.out + oi + 16 * i;
-#pragma unroll
-                for (int u = 0; u < BPL; u += 4)
-                    *reinterpret_cast<float4*>(p + u) = make_float4(o[u][base + i] * inv, o[u + 1][base + i] * inv, o[u + 2][base + i] * inv, o[u + 3][base + i] * inv);
-            } else {
-                uint32_t w[8];
-#pragma unroll
-                for (int u = 0; u < BPL; u += 2) {
-                    const float x = o[u][base + i] * inv, y = o[u + 1][base + i] * inv;
-                    if (A.out_dtype == DT_F16) { const __half2 h = __floats2half2_rn(x, y); w[u / 2] = *reinterpret_cast<const uint32_t*>(&h); }
-                    else { const __nv_bfloat162 h = __floats2bfloat162_rn(x, y); w[u / 2] = *reinterpret_cast<const uint32_t*>(&h); }
-                }
-                uint16_t* p = (uint16_t*)A.out + oi + 16 * i;
-                *reinterpret_cast<uint4*>(p) = make_uint4(w[0], w[1], w[2], w[3]);
-                *reinterpret_cast<uint4*>(p + 8) = make_uint4(w[4], w[5], w[6], w[7]);
-            }
-        }
-    };
-    store_row(row_a, 0, ol[0]);
-    store_row(row_b, 2, ol[2]);
+done:
+    __syncwarp();
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 4 * NT + 4) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
+    }
+}
+
+template <int NT> int sdp_prompt_launch_nt(const SdpArgs& A, cudaStream_t st) {
+    static bool configured_dev[64] = {};                                  // the attribute is per device context
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (!configured_dev[dev & 63]) {
+        cudaFuncSetAttribute(sdp_fp8_prompt_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, sp_smem(NT));
+        configured_dev[dev & 63] = true;
+    }
+    const int n_qt = (A.S + NT * SP_ROWS - 1) / (NT * SP_ROWS);
+    sdp_fp8_prompt_kernel<NT><<<dim3((unsigned)(A.B * A.Hq), (unsigned)n_qt), sp_threads(NT), sp_smem(NT), st>>>(A, n_qt);
+    note_launch();
+    return check_launch();
+}
+// 256 rows a CTA share every key tile's expansion, 128 spread a short prompt over twice the SMs: two tiles once they fill the chip
+int sdp_prompt_launch(const SdpArgs& A, cudaStream_t st) {
+    const int64_t two = (int64_t)A.B * A.Hq * ((A.S + 2 * SP_ROWS - 1) / (2 * SP_ROWS));
+    return two >= sm_count() ? sdp_prompt_launch_nt<2>(A, st) : sdp_prompt_launch_nt<1>(A, st);
 }

@@ -67,6 +67,32 @@ __device__ __forceinline__ void tma_load_2d_w(uint32_t dst, const CUtensorMap* m
                  "@q cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n\t}"
                  ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(bar), "r"(leader) : "memory");
 }
+// ---- bounded waits: one that runs out raises this translation unit's flag, and the kernel winds down
+constexpr long long kWaitCycles = 4000000000ll;           // about two seconds
+static __device__ unsigned int g_wait_expired;
+__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok != 0;
+}
+// whole warp; the same answer in every lane.  false: the limit ran out
+__device__ __forceinline__ bool mbar_wait_lim(uint32_t bar, uint32_t parity) {
+    if (__all_sync(0xffffffffu, mbar_test(bar, parity))) return true;
+    const long long t0 = clock64();
+    while (!__all_sync(0xffffffffu, mbar_test(bar, parity))) {
+        if (__any_sync(0xffffffffu, clock64() - t0 > kWaitCycles)) {
+            if ((threadIdx.x & 31) == 0) atomicExch(&g_wait_expired, 1u);
+            return false;
+        }
+    }
+    return true;
+}
+static int wait_expired_here() {
+    unsigned int v = 0;
+    if (cudaMemcpyFromSymbol(&v, g_wait_expired, sizeof(v)) != cudaSuccess) { cudaGetLastError(); return -1; }
+    return (int)v;
+}
 __device__ __forceinline__ uint32_t elect_leader() {
     uint32_t pred;
     asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(pred));

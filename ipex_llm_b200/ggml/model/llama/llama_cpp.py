@@ -343,7 +343,7 @@ def lowbit_moe_tokens_cuda(d_x, x_dtype, n_tokens, d_ids, ids_dtype, d_weight, w
 
 
 def lowbit_gemm_wait_expired():
-    """whether a bounded wait inside the two-SM matmul kernel has run out on the current device (synchronises)"""
+    """whether a bounded wait inside the prompt matmul or the prompt attention has run out on the current device (synchronises)"""
     return _lib.lowbit_gemm_wait_expired() == 1
 
 

@@ -1,15 +1,17 @@
 """The two-SM prompt matmul (csrc/gemm_pair.cu): edges of its tiles against float64 on the dequantised weights, plain, with the fused
 MLP's activation, and over the experts of a mixture (csrc/experts.cu).
 
-Bounds.  Weights are rounded once to the activation dtype and the sum is taken in 32 bits, so a product's error is at most
-u * sum|x w| with u = 2^-11 (fp16) / 2^-9 + 2^-11 (bf16, whose expansion goes through fp16), plus 2^-20 * sum|x w| for the
-accumulation, plus u * |y| for a 16-bit result's own rounding."""
+Bounds.  Weights are rounded once to the activation dtype, so a product's error is at most u * sum|x w| with u = 2^-11 (fp16) or
+(1 + 2^-8)(1 + 2^-11) - 1 (bf16 has eight significant bits; its expansion goes through fp16).  The 32-bit sum: a step of the tensor cores aligns its 16 products
+and the accumulator to the largest of them and drops what falls below 2^-23 of it, 17 terms a step, so ACC = 2^-18 * sum|x w| covers
+two steps' worth at full size (the later ones' drops are relative to sums that rarely reach sum|x w|).  A 16-bit result adds u * |y|."""
 import pytest
 import torch
 
 pytestmark = pytest.mark.gpu
 
-U = {torch.float16: 2.0 ** -11, torch.bfloat16: 2.0 ** -9 + 2.0 ** -11}
+U = {torch.float16: 2.0 ** -11, torch.bfloat16: (1 + 2.0 ** -8) * (1 + 2.0 ** -11) - 1}
+ACC = 2.0 ** -18
 
 
 @pytest.fixture(scope="module")
@@ -36,7 +38,7 @@ def acts(dev, seed, m, k, dtype):
 
 def product(x, w, u):
     """x w^T in 64 bits and the bound of a 32-bit sum over weights rounded to u"""
-    return x @ w.T, (u + 2.0 ** -20) * (x.abs() @ w.abs().T)
+    return x @ w.T, (u + ACC) * (x.abs() @ w.abs().T)
 
 
 # one row over a 16- / 128- / 256-token tile, a lone feature pair and an odd one, one k-block, K splits and several rounds of tiles
