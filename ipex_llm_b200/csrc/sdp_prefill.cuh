@@ -5,7 +5,7 @@
 // fp16 / bf16 queries, head_dim 128, both products on the 5th-generation tensor cores.  One CTA = NT tiles of 128 query rows of one
 // (sequence, query head), walking the keys in tiles of 128:
 //   S_t = Q_t . K^T   tcgen05.mma M = 128, N = 128, K = 16, both operands in shared memory, S in TMEM (lane = query row);
-//   softmax           four warps per tile, one thread per row: the row's 128 scores in registers, P (fp16) back into TMEM over S;
+//   softmax           four warps per tile, one thread per row, P (fp16) back into TMEM over S;
 //   O_t += P_t . V    A operand = P in TMEM, B operand = V as it lies in the cache (rows = keys: the MN-major descriptor).
 // Warps 0 .. 4 NT - 1: softmax; the next four read the cache (16 bytes a thread, coalesced), expand e5m2 -> fp16 (one byte permute
 // per pair) and write K and V into a ring of four 32 KB swizzled tiles; the last warp issues the MMAs and owns TMEM.
@@ -13,7 +13,7 @@
 // its softmax, and every key tile is expanded once for 256 rows.  P lies over S, so a tile's next Q . K waits for its P . V (a commit,
 // not the issue order).  What bounds it: per 128 keys and 256 rows 2048 clocks of MMAs, 2048 of ex2 (16 a clock), and the chain
 // Q.K -> softmax -> P.V of one tile.  The kernel it replaces (64 rows a CTA, mma.sync) was bound by the legacy tensor path:
-// 4000 causal tokens, 32 heads: 601 us, 218 TFLOP/s.
+// 4000 causal tokens, 32 heads over 8: 596 us, 220 TFLOP/s; this one 154 us, 849 (6000 tokens of two sequences: 2402 -> 606 us, 974).
 // Causal: query token s (0-based among the S new ones) sees keys <= L - S + s; key tiles beyond a tile's last row are skipped.  An
 // additive mask [B][1|Hq][S][L] is honoured.  Softmax and accumulation in 32 bits; Q and P enter the MMAs as fp16.  P is kept relative
 // to a reference 2^8 below fp16's comfortable range (values up to 2^14, nothing above 2^-32 of the row's maximum is flushed), and the
@@ -59,7 +59,7 @@ __device__ __forceinline__ void sp_sts128(uint32_t a, uint32_t x, uint32_t y, ui
     asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
 }
 
-template <int NT>
+template <int NT, bool MASK>
 __global__ void __launch_bounds__(sp_threads(NT), 1)
 sdp_fp8_prompt_kernel(const SdpArgs A, int n_qt) {
     using namespace gemmtc;
@@ -68,11 +68,10 @@ sdp_fp8_prompt_kernel(const SdpArgs A, int n_qt) {
     const uint32_t qs = base, ring = base + NT * SP_TILE, bars = ring + SP_SLOTS * SP_TILE;
     auto kv_full = [&](int s) { return bars + s * 8; };
     auto kv_empty = [&](int s) { return bars + 32 + s * 8; };
-    auto q_ready = [&](int t) { return bars + 64 + t * 8; };
-    auto s_full = [&](int t) { return bars + 80 + t * 8; };
-    auto p_full = [&](int t) { return bars + 96 + t * 8; };
-    auto pv_done = [&](int t) { return bars + 112 + t * 8; };
-    const uint32_t tmem_slot = bars + 128;
+    auto s_full = [&](int t) { return bars + 64 + t * 8; };
+    auto p_full = [&](int t) { return bars + 80 + t * 8; };
+    auto pv_done = [&](int t) { return bars + 96 + t * 8; };
+    const uint32_t tmem_slot = bars + 112;
     constexpr uint32_t TMEM_COLS = NT * 256;                           // S_t at 128 t, O_t behind all S
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const int hq = blockIdx.x % A.Hq, b = blockIdx.x / A.Hq, hkv = hq / (A.Hq / A.Hkv);
@@ -89,30 +88,14 @@ sdp_fp8_prompt_kernel(const SdpArgs A, int n_qt) {
     int nk = tiles_of(0);
     if (NT == 2) nk = max(nk, tiles_of(1));
 
-    if (threadIdx.x == 0) {
-        for (int s = 0; s < SP_SLOTS; s++) { mbar_init(kv_full(s), 4); mbar_init(kv_empty(s), 1); }
-        for (int t = 0; t < 2; t++) { mbar_init(q_ready(t), 4); mbar_init(s_full(t), 1); mbar_init(p_full(t), 4); mbar_init(pv_done(t), 1); }
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    if (warp == 4 * NT + 4) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tmem_slot), "r"(TMEM_COLS) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    uint32_t tmem;
-    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem) : "r"(tmem_slot));
-
+    // ---- before the barriers exist: the queries into their tiles, the first keys on their way
     if (warp < 4 * NT) {
-        // ================= softmax: thread = query row =================
-        const int t = warp >> 2, quarter = warp & 3, r = 32 * quarter + lane, row = q0 + t * SP_ROWS + r;
-        const int nkt = tiles_of(t);
-        if (nkt > 0) {
-            // the row as fp16 into the swizzled operand tile (rows beyond S: zeros)
+        const int t = warp >> 2, r = 32 * (warp & 3) + lane, row = q0 + t * SP_ROWS + r;
+        if (tiles_of(t) > 0) {
+            // the row as fp16 into the swizzled operand tile (rows beyond S: zeros), in front of the block's first barrier
             const uint4* qrow = reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(A.q) + b * A.q_sb + hq * A.q_sh + (int64_t)row * A.q_ss);
             const uint32_t qd = qs + t * SP_TILE + r * 128;
-#pragma unroll 4
+#pragma unroll 8
             for (int c = 0; c < 16; c++) {
                 uint4 w = make_uint4(0u, 0u, 0u, 0u);
                 if (row < S) {
@@ -130,38 +113,79 @@ sdp_fp8_prompt_kernel(const SdpArgs A, int n_qt) {
                 sp_sts128(qd + (c >> 3) * (SP_TILE / 2) + (((c & 7) ^ (r & 7)) << 4), w.x, w.y, w.z, w.w);
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) mbar_arrive(q_ready(t));
+        }
+    }
+    const int tid = threadIdx.x - 128 * NT, piece = tid & 7, r0 = tid >> 3;       // loader warps: rows r0, r0 + 16, ... of a tile, piece of 16 columns
+    uint4 w[8];
+    auto fetch = [&](int item) {                                                  // item 2 j = keys of tile j, 2 j + 1 = its values
+        const uint8_t* p = (item & 1) ? A.v + b * A.v_sb + hkv * A.v_sh + 16 * piece : A.k + b * A.k_sb + hkv * A.k_sh + 16 * piece;
+        const int64_t ss = (item & 1) ? A.v_ss : A.k_ss;
+        const int k0 = (item >> 1) * SP_KEYS + r0;
+#pragma unroll
+        for (int i = 0; i < 8; i++) w[i] = k0 + 16 * i < L ? *reinterpret_cast<const uint4*>(p + (k0 + 16 * i) * ss) : make_uint4(0u, 0u, 0u, 0u);
+    };
+    if (warp >= 4 * NT && warp < 4 * NT + 4 && nk > 0) fetch(0);
 
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < SP_SLOTS; s++) { mbar_init(kv_full(s), 4); mbar_init(kv_empty(s), 1); }
+        for (int t = 0; t < 2; t++) { mbar_init(s_full(t), 1); mbar_init(p_full(t), 4); mbar_init(pv_done(t), 1); }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 4 * NT + 4) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tmem_slot), "r"(TMEM_COLS) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    uint32_t tmem;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem) : "r"(tmem_slot));
+
+    if (warp < 4 * NT) {
+        // ================= softmax: thread = query row =================
+        const int t = warp >> 2, quarter = warp & 3, r = 32 * quarter + lane, row = q0 + t * SP_ROWS + r;
+        const int nkt = tiles_of(t);
+        if (nkt > 0) {
             const uint32_t lanes = (uint32_t)(32 * quarter) << 16;
             const uint32_t st = tmem + lanes + t * 128, ot = tmem + lanes + (NT + t) * 128;
-            const int lim = A.causal ? L - S + row : L - 1;                       // last visible key
-            const int plain_end = A.mask ? -1 : A.causal ? min(L, L - S + q0 + t * SP_ROWS + 32 * quarter + 1) : L;   // keys below: visible to the whole warp
+            const int n_vis = row >= S ? 0 : A.causal ? min(L, L - S + row + 1) : L;                    // keys the row sees
+            const int plain_end = MASK ? -1 : A.causal ? min(L, L - S + q0 + t * SP_ROWS + 32 * quarter + 1) : L;   // keys below: visible to the whole warp
             const int64_t mbase = b * A.m_sb + hq * A.m_sh + (int64_t)row * A.m_ss;
             float m_ref = -CUDART_INF_F, sum = 0.0f;
             for (int j = 0; j < nkt; j++) {
                 if (!mbar_wait_lim(s_full(t), (uint32_t)(j & 1))) goto done;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                float s[128];
-#pragma unroll
-                for (int c = 0; c < 4; c++) sp_tmem_ld32(st + 32 * c, s + 32 * c);
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                float mul = A.scale_log2e;
                 const int k0 = j * SP_KEYS;
-                if (k0 + SP_KEYS > plain_end) {
-                    mul = 1.0f;
+                const bool plain = k0 + SP_KEYS <= plain_end;
+                const float mul = MASK ? 1.0f : A.scale_log2e;
+                // the row's scores pass through the registers twice, 64 at a time (maximum, then exponentials): holding all 128 spilled
+                auto load = [&](int c, float (&x)[64]) {
+                    sp_tmem_ld32(st + 64 * c, x);
+                    sp_tmem_ld32(st + 64 * c + 32, x + 32);
+                    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                    if (MASK) {
 #pragma unroll
-                    for (int i = 0; i < 128; i++) {
-                        float v = s[i] * A.scale_log2e;
-                        const bool ok = k0 + i <= lim && k0 + i < L && row < S;
-                        if (A.mask && ok) v += load_as_float(A.mask, A.mask_dtype, mbase + k0 + i) * 1.4426950408889634f;
-                        s[i] = ok ? v : -CUDART_INF_F;
+                        for (int i = 0; i < 64; i++) {
+                            const int key = k0 + 64 * c + i;
+                            x[i] = key < n_vis ? x[i] * A.scale_log2e + load_as_float(A.mask, A.mask_dtype, mbase + key) * 1.4426950408889634f : -CUDART_INF_F;
+                        }
+                    } else if (!plain) {
+                        const int left = n_vis - k0 - 64 * c;
+#pragma unroll
+                        for (int i = 0; i < 64; i++) x[i] = i < left ? x[i] : -CUDART_INF_F;
                     }
-                }
-                float mx0 = s[0], mx1 = s[1], mx2 = s[2], mx3 = s[3];
+                };
+                float mx = -CUDART_INF_F;
+#pragma unroll 1
+                for (int c = 0; c < 2; c++) {
+                    float x[64];
+                    load(c, x);
+                    float m0 = x[0], m1 = x[1], m2 = x[2], m3 = x[3];
 #pragma unroll
-                for (int i = 4; i < 128; i += 4) { mx0 = fmaxf(mx0, s[i]); mx1 = fmaxf(mx1, s[i + 1]); mx2 = fmaxf(mx2, s[i + 2]); mx3 = fmaxf(mx3, s[i + 3]); }
-                const float mx = fmaxf(fmaxf(mx0, mx1), fmaxf(mx2, mx3)) * mul;
+                    for (int i = 4; i < 64; i += 4) { m0 = fmaxf(m0, x[i]); m1 = fmaxf(m1, x[i + 1]); m2 = fmaxf(m2, x[i + 2]); m3 = fmaxf(m3, x[i + 3]); }
+                    mx = fmaxf(mx, fmaxf(fmaxf(m0, m1), fmaxf(m2, m3)));
+                }
+                mx *= mul;
                 const bool grow = mx > m_ref + 6.0f;                                // -inf: any visible key
                 if (__any_sync(0xffffffffu, grow)) {
                     const float m_new = grow ? mx : m_ref;
@@ -183,20 +207,22 @@ sdp_fp8_prompt_kernel(const SdpArgs A, int n_qt) {
                 }
                 const float shift = 8.0f - (m_ref == -CUDART_INF_F ? 0.0f : m_ref);
                 float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f, a3 = 0.0f;
-#pragma unroll
-                for (int h = 0; h < 2; h++) {
+                // P of keys 64 c .. 64 c + 63 goes to columns 32 c .. 32 c + 31, whose scores have been read
+#pragma unroll 1
+                for (int c = 0; c < 2; c++) {
+                    float x[64];
+                    load(c, x);
                     uint32_t pk[32];
 #pragma unroll
                     for (int i = 0; i < 32; i += 2) {
-                        const float* x = s + 64 * h + 2 * i;
-                        const float p0 = ex2_approx(fmaf(x[0], mul, shift)), p1 = ex2_approx(fmaf(x[1], mul, shift));
-                        const float p2 = ex2_approx(fmaf(x[2], mul, shift)), p3 = ex2_approx(fmaf(x[3], mul, shift));
+                        const float p0 = ex2_approx(fmaf(x[2 * i], mul, shift)), p1 = ex2_approx(fmaf(x[2 * i + 1], mul, shift));
+                        const float p2 = ex2_approx(fmaf(x[2 * i + 2], mul, shift)), p3 = ex2_approx(fmaf(x[2 * i + 3], mul, shift));
                         a0 += p0; a1 += p1; a2 += p2; a3 += p3;
                         const __half2 h0 = __floats2half2_rn(p0, p1), h1 = __floats2half2_rn(p2, p3);
                         pk[i] = *reinterpret_cast<const uint32_t*>(&h0);
                         pk[i + 1] = *reinterpret_cast<const uint32_t*>(&h1);
                     }
-                    sp_tmem_st32(st + 32 * h, pk);
+                    sp_tmem_st32(st + 32 * c, pk);
                 }
                 sum += (a0 + a1) + (a2 + a3);
                 asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
@@ -237,22 +263,10 @@ sdp_fp8_prompt_kernel(const SdpArgs A, int n_qt) {
             }
         }
     } else if (warp < 4 * NT + 4) {
-        // ================= the cache: item 2 j = keys of tile j, 2 j + 1 = its values =================
-        const int tid = threadIdx.x - 128 * NT, piece = tid & 7, r0 = tid >> 3;       // rows r0, r0 + 16, ...
-        const uint8_t* const kb = A.k + b * A.k_sb + hkv * A.k_sh + 16 * piece;
-        const uint8_t* const vb = A.v + b * A.v_sb + hkv * A.v_sh + 16 * piece;
-        uint4 w[8];
-        auto fetch = [&](int item) {
-            const uint8_t* p = (item & 1) ? vb : kb;
-            const int64_t ss = (item & 1) ? A.v_ss : A.k_ss;
-            const int k0 = (item >> 1) * SP_KEYS + r0;
-#pragma unroll
-            for (int i = 0; i < 8; i++) w[i] = k0 + 16 * i < L ? *reinterpret_cast<const uint4*>(p + (k0 + 16 * i) * ss) : make_uint4(0u, 0u, 0u, 0u);
-        };
+        // ================= the cache: expanded into the ring, item by item =================
         // a thread's 16 elements are two chunks of one row's half; lanes of the second half write them in the other order, so that a
         // quarter warp (one row) meets every bank once
         const int half = piece >> 2, c0 = 2 * (piece & 3) + half;
-        if (nk > 0) fetch(0);
         for (int item = 0; item < 2 * nk; item++) {
             const int s = item % SP_SLOTS, round = item / SP_SLOTS;
             if (!mbar_wait_lim(kv_empty(s), (uint32_t)((round & 1) ^ 1))) goto done;
@@ -297,10 +311,9 @@ sdp_fp8_prompt_kernel(const SdpArgs A, int n_qt) {
         };
         if (nk > 0) {
             if (!mbar_wait_lim(kv_full(0), 0u)) goto done;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             for (int t = 0; t < NT; t++) {
                 if ((t == 0 ? nk0 : nk1) == 0) continue;
-                if (!mbar_wait_lim(q_ready(t), 0u)) goto done;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 scores(t, 0);
             }
             umma_commit_w(kv_empty(0), leader);
@@ -336,21 +349,22 @@ done:
     }
 }
 
-template <int NT> int sdp_prompt_launch_nt(const SdpArgs& A, cudaStream_t st) {
+template <int NT, bool MASK> int sdp_prompt_launch_nt(const SdpArgs& A, cudaStream_t st) {
     static bool configured_dev[64] = {};                                  // the attribute is per device context
     int dev = 0;
     cudaGetDevice(&dev);
     if (!configured_dev[dev & 63]) {
-        cudaFuncSetAttribute(sdp_fp8_prompt_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, sp_smem(NT));
+        cudaFuncSetAttribute(sdp_fp8_prompt_kernel<NT, MASK>, cudaFuncAttributeMaxDynamicSharedMemorySize, sp_smem(NT));
         configured_dev[dev & 63] = true;
     }
     const int n_qt = (A.S + NT * SP_ROWS - 1) / (NT * SP_ROWS);
-    sdp_fp8_prompt_kernel<NT><<<dim3((unsigned)(A.B * A.Hq), (unsigned)n_qt), sp_threads(NT), sp_smem(NT), st>>>(A, n_qt);
+    sdp_fp8_prompt_kernel<NT, MASK><<<dim3((unsigned)(A.B * A.Hq), (unsigned)n_qt), sp_threads(NT), sp_smem(NT), st>>>(A, n_qt);
     note_launch();
     return check_launch();
 }
 // 256 rows a CTA share every key tile's expansion, 128 spread a short prompt over twice the SMs: two tiles once they fill the chip
 int sdp_prompt_launch(const SdpArgs& A, cudaStream_t st) {
     const int64_t two = (int64_t)A.B * A.Hq * ((A.S + 2 * SP_ROWS - 1) / (2 * SP_ROWS));
-    return two >= sm_count() ? sdp_prompt_launch_nt<2>(A, st) : sdp_prompt_launch_nt<1>(A, st);
+    if (A.mask) return two >= sm_count() ? sdp_prompt_launch_nt<2, true>(A, st) : sdp_prompt_launch_nt<1, true>(A, st);
+    return two >= sm_count() ? sdp_prompt_launch_nt<2, false>(A, st) : sdp_prompt_launch_nt<1, false>(A, st);
 }
