@@ -1,8 +1,9 @@
 """Build the package's shared libraries in-tree with nvcc for sm_100a.
 
-    python -m ipex_llm_b200.build_native [--force] [--verbose] [--only lowbit|mixers]
+    python -m ipex_llm_b200.build_native [--force] [--verbose] [--only lowbit|mixers|host]
 
-Two libraries, each from its own folder of sources, so that a model that needs one of them does not wait for the other:
+Two kernel libraries, each from its own folder of sources, so that a model that needs one of them does not wait for the other, and
+a small CPython module (``b200_host.so``, csrc/host: the host side of one linear):
 ``libb200lowbit.so`` (csrc/*.cu: the low-bit linears and what surrounds them in llama-family decoders) and
 ``libb200mixers.so`` (csrc/mixers/*.cu: windowed sigmoid attention, linear recurrences, the normalisations of models built
 from them).  They land in ipex_llm_b200/libs/ (git-ignored).  nvcc cross-compiles without a GPU.  Objects are cached in
@@ -133,6 +134,34 @@ def build(force=False, verbose=False, ptxas_info=False):
     return LIB
 
 
+HOST_SRC = os.path.join(CSRC, "host", "linear_host.cpp")
+HOST_LIB = os.path.join(LIBDIR, "b200_host.so")
+
+
+def build_host(force=False, verbose=False):
+    """libs/b200_host.so: the CPython module behind LowBitLinear.forward (csrc/host).  Safe to call from several processes at once."""
+    import sysconfig
+    if not force and os.path.exists(HOST_LIB) and os.path.getmtime(HOST_LIB) >= os.path.getmtime(HOST_SRC):
+        return HOST_LIB
+    import torch
+    from torch.utils import cpp_extension
+    os.makedirs(LIBDIR, exist_ok=True)
+    lib_dir = os.path.join(os.path.dirname(torch.__file__), "lib")
+    cuda = os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include")
+    includes = [d for d in cpp_extension.include_paths() if os.path.isdir(d)] + [cuda, sysconfig.get_paths()["include"]]
+    tmp = f"{HOST_LIB}.{os.getpid()}"
+    cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+    cmd += [f for d in includes for f in ("-isystem", d)]
+    cmd += [HOST_SRC, "-o", tmp, "-L", lib_dir, "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda", f"-Wl,-rpath,{lib_dir}"]
+    if verbose:
+        print(" ".join(cmd), flush=True)
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed on {HOST_SRC}:\n{r.stdout}\n{r.stderr}")
+    os.replace(tmp, HOST_LIB)
+    return HOST_LIB
+
+
 if __name__ == "__main__":
     only = sys.argv[sys.argv.index("--only") + 1] if "--only" in sys.argv else None
     kw = dict(force="--force" in sys.argv, verbose="--verbose" in sys.argv, ptxas_info="--ptxas-info" in sys.argv)
@@ -140,3 +169,5 @@ if __name__ == "__main__":
         print(build(**kw))
     if only in (None, "mixers"):
         print(build_mixers(**kw))
+    if only in (None, "host"):
+        print(build_host(force=kw["force"], verbose=kw["verbose"]))

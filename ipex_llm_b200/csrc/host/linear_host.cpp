@@ -1,0 +1,90 @@
+// linear_host.cpp -- the host side of one LowBitLinear.forward (reference low_bit_linear.py:638-725) in one native call:
+// checks, output, scratch, stream and launch.  In Python (tensor views, a ctypes call of fourteen arguments, the scratch lookup) the
+// same took 20 us around a 4 us kernel.  A CPython module (b200_host); the kernels are reached through the addresses of
+// libb200lowbit.so's entry points, which the package hands over once.
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/python_variable.h>
+#include <ATen/ops/empty.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+
+namespace {
+
+using MatmulFn = int (*)(const void*, int, int64_t, int64_t, const void*, int, int64_t, void*, int, const void*, int, void*, size_t, void*);
+using WorkspaceFn = size_t (*)(int64_t, int64_t, int64_t, int);
+using HintFn = void (*)(const void*, size_t);
+MatmulFn g_matmul = nullptr;
+WorkspaceFn g_workspace = nullptr;
+HintFn g_hint = nullptr;
+
+int dtype_code(c10::ScalarType t) {
+    return t == at::kFloat ? 0 : t == at::kHalf ? 1 : t == at::kBFloat16 ? 2 : -1;
+}
+
+PyObject* attach(PyObject*, PyObject* args) {
+    unsigned long long m, w, h;
+    if (!PyArg_ParseTuple(args, "KKK", &m, &w, &h)) return nullptr;
+    g_matmul = reinterpret_cast<MatmulFn>(m);
+    g_workspace = reinterpret_cast<WorkspaceFn>(w);
+    g_hint = reinterpret_cast<HintFn>(h);
+    Py_RETURN_NONE;
+}
+
+// linear(x, weight, bias | None, out_features, in_features, qtype, max_rows_f32, next_weight | None)
+//   -> the result; None when this call is not the plain case (the caller's general path then serves or refuses it); an int: the
+//      native error code.  max_rows_f32: 32-bit activations of more rows are left to the caller (it casts them).
+PyObject* linear(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
+    HANDLE_TH_ERRORS
+    if (n_args != 8 || !g_matmul) {
+        PyErr_SetString(PyExc_TypeError, "b200_host.linear takes eight arguments, after attach()");
+        return nullptr;
+    }
+    // exact tensors with storage only: subclasses, traced and batched tensors keep to the general path
+    if (!THPVariable_CheckExact(a[0]) || !THPVariable_Check(a[1])) Py_RETURN_NONE;
+    const at::Tensor& x = THPVariable_Unpack(a[0]);
+    const at::Tensor& w = THPVariable_Unpack(a[1]);
+    if (!x.is_cuda() || !w.is_cuda() || !x.has_storage() || !w.has_storage() || x.dim() < 1 || x.device() != w.device() || !x.is_contiguous()) Py_RETURN_NONE;
+    const int dt = dtype_code(x.scalar_type());
+    const int64_t n = PyLong_AsLongLong(a[3]), k = PyLong_AsLongLong(a[4]);
+    const int qtype = (int)PyLong_AsLong(a[5]);
+    const int64_t max_f32 = PyLong_AsLongLong(a[6]);
+    if (PyErr_Occurred()) return nullptr;
+    if (dt < 0 || x.size(-1) != k || x.numel() == 0) Py_RETURN_NONE;
+    const int64_t rows = x.numel() / k;
+    if (dt == 0 && rows > max_f32) Py_RETURN_NONE;
+    const void* xp = x.const_data_ptr();
+    if (reinterpret_cast<uintptr_t>(xp) & 15) Py_RETURN_NONE;
+    const void* bias = nullptr;
+    if (a[2] != Py_None) {
+        if (!THPVariable_Check(a[2])) Py_RETURN_NONE;
+        const at::Tensor& b = THPVariable_Unpack(a[2]);
+        if (b.scalar_type() != x.scalar_type() || b.device() != x.device() || !b.is_contiguous() || b.numel() != n) Py_RETURN_NONE;
+        bias = b.const_data_ptr();
+    }
+    const c10::cuda::CUDAGuard guard(x.device());
+    auto sizes = x.sizes().vec();
+    sizes.back() = n;
+    const auto options = x.options().requires_grad(false);
+    at::Tensor y = at::empty(sizes, options), scratch;
+    const size_t need = g_workspace(n, k, rows, dt);
+    if (need) scratch = at::empty({(int64_t)need}, options.dtype(at::kByte));
+    if (a[7] != Py_None && rows <= 32 && THPVariable_Check(a[7])) {
+        const at::Tensor& nx = THPVariable_Unpack(a[7]);
+        if (nx.is_cuda() && nx.has_storage()) g_hint(nx.const_data_ptr(), nx.nbytes());
+    }
+    // a scratch of no bytes: any non-null pointer (NULL would ask the library for its own, under its lock)
+    const int rc = g_matmul(w.const_data_ptr(), qtype, n, k, xp, dt, rows, y.mutable_data_ptr(), dt, bias, 0,
+                            need ? scratch.mutable_data_ptr() : y.mutable_data_ptr(), need, c10::cuda::getCurrentCUDAStream(x.device().index()).stream());
+    if (rc) return PyLong_FromLong(rc);
+    return THPVariable_Wrap(std::move(y));
+    END_HANDLE_TH_ERRORS
+}
+
+PyMethodDef methods[] = {{"attach", attach, METH_VARARGS, nullptr},
+                         {"linear", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(linear)), METH_FASTCALL, nullptr},
+                         {nullptr, nullptr, 0, nullptr}};
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "b200_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit_b200_host() { return PyModule_Create(&module); }
