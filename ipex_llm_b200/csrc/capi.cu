@@ -224,7 +224,7 @@ int lowbit_matmul_cuda(const void* d_w, int qtype, int64_t n_rows, int64_t k, co
 
 size_t lowbit_mlp_workspace_size(int64_t n_rows, int64_t k, int64_t m, int x_dtype) {
     if (use_skinny(B200_QT_SYM_INT4, n_rows, k, m, x_dtype)) return gemm_skinny_mlp_workspace_size(n_rows, k, m);
-    if (use_gemm(B200_QT_SYM_INT4, n_rows, k, m, x_dtype)) return 256;                 // one launch, no intermediates
+    if (use_gemm(B200_QT_SYM_INT4, n_rows, k, m, x_dtype)) return gemm_tc_mlp_workspace_size(n_rows, k, m);
     const size_t base = (lowbit_matmul_workspace_size(n_rows, k, m, x_dtype) + 255) / 256 * 256;
     return base + 2 * (size_t)m * n_rows * sizeof(float);
 }
@@ -264,7 +264,7 @@ int lowbit_mlp_cuda(const void* d_w_gate, const void* d_w_up, int qtype, int64_t
         rc = gemm_skinny_mlp_launch(d_w_gate, d_w_up, act + 1, qtype, n_rows, k, d_x, x_dtype, m, d_y, y_dtype, workspace, workspace_bytes,
                                     st, gemv_get_pdl());
     } else if (use_gemm(qtype, n_rows, k, m, x_dtype)) {
-        rc = gemm_tc_mlp_launch(d_w_gate, d_w_up, act + 1, qtype, n_rows, k, d_x, x_dtype, m, d_y, y_dtype, st);
+        rc = gemm_tc_mlp_launch(d_w_gate, d_w_up, act + 1, qtype, n_rows, k, d_x, x_dtype, m, d_y, y_dtype, workspace, workspace_bytes, st);
     } else {
         // behind the exact GEMV: the two intermediates in fp32
         float* tg = (float*)((char*)workspace + base);

@@ -382,7 +382,9 @@ pair_kernel(const __grid_constant__ CUtensorMap xmap, const PairArgs A) {
                     float v[16];
                     tmem_ld16(acc + c, v);
                     const int64_t at = (int64_t)(U.m0 + c) * N + n;
-                    if (A.act) {
+                    if (A.act && A.ksplit > 1) {                     // [K split][token][gate features | up features]
+                        if (valid) store_feature(A.part + ((int64_t)U.ks * A.M + U.m0 + c) * 2 * N + half * N + n, 2 * N, v, rows - c, 0.0f, false);
+                    } else if (A.act) {
                         float o[8];
                         gate_up(v, A.act, half, o);
 #pragma unroll
@@ -491,6 +493,24 @@ __global__ void __launch_bounds__(256) reduce_partials_kernel(const float* __res
             else if (y_dtype == DT_F16) { __half* p = (__half*)y + i + j; *p = __float2half_rn(accumulate ? __half2float(*p) + v[j] : v[j]); }
             else { __nv_bfloat16* p = (__nv_bfloat16*)y + i + j; *p = __float2bfloat16_rn(accumulate ? __bfloat162float(*p) + v[j] : v[j]); }
         }
+    }
+}
+
+// the same behind a split MLP: y[token][n] = act(sum of the gate partials) * (sum of the up partials)
+__global__ void __launch_bounds__(256) reduce_gated_kernel(const float* __restrict__ part, int ksplit, int64_t m, int64_t n, void* y, int y_dtype, int act) {
+    const int64_t mn = m * n, n4 = n / 4;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < mn / 4; i += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t token = i / n4, col = (i - token * n4) * 4;
+        const float* p = part + token * 2 * n + col;
+        float4 g = make_float4(0.0f, 0.0f, 0.0f, 0.0f), u = g;
+        for (int ks = 0; ks < ksplit; ks++, p += 2 * mn) {
+            const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + n);
+            g.x += a.x; g.y += a.y; g.z += a.z; g.w += a.w;
+            u.x += b.x; u.y += b.y; u.z += b.z; u.w += b.w;
+        }
+        const float r[4] = {apply_act(g.x, act) * u.x, apply_act(g.y, act) * u.y, apply_act(g.z, act) * u.z, apply_act(g.w, act) * u.w};
+#pragma unroll
+        for (int j = 0; j < 4; j++) store_out(y, y_dtype, token * n + col + j, r[j], nullptr, 0, 0);
     }
 }
 
@@ -604,7 +624,7 @@ int gemm_tc_launch(const void* w, int qt, int64_t n_rows, int64_t k, const void*
 // first half of an MLP at prompt sizes: y = act(x . Wgate^T) * (x . Wup^T), both products in one tile's accumulators (a gate and an
 // up row group per CTA), the activation in the epilogue: the two [M][N] intermediates and their kernel do not exist
 int gemm_tc_mlp_launch(const void* w_gate, const void* w_up, int act, int qt, int64_t n_rows, int64_t k, const void* x, int x_dtype,
-                       int64_t m, void* y, int y_dtype, cudaStream_t st) {
+                       int64_t m, void* y, int y_dtype, void* workspace, size_t workspace_bytes, cudaStream_t st) {
     using namespace gemmtc;
     qt = canon_qtype(qt);
     if (!gemm_tc_supported(qt, n_rows, k) || (x_dtype != DT_F16 && x_dtype != DT_BF16) || act < 1 || act > 2) return LB_ERR_ARG;
@@ -614,10 +634,22 @@ int gemm_tc_mlp_launch(const void* w_gate, const void* w_up, int act, int qt, in
     if (const int rc = encode_rows(&map, x, bf, m, k, 32)) return rc;
     PairArgs A = {};
     A.w = (const uint8_t*)w_gate; A.w2 = (const uint8_t*)w_up; A.act = act; A.G = make_geom(n_rows, k, qt); A.M = (int)m; A.y = y; A.y_dtype = y_dtype;
-    A.n_fp = (int)((n_rows / 64 + 1) / 2); A.ksplit = 1;
-    A.tt = pair_plan(A.n_fp, k / 64, m, n_rows, false).tt;
-    if (const int rc = pair_launch(qt, bf, map, A, (int64_t)A.n_fp * ((m + A.tt - 1) / A.tt), st)) return rc;
+    A.n_fp = (int)((n_rows / 64 + 1) / 2);
+    PairPlan p = pair_plan(A.n_fp, k / 64, m, 2 * n_rows, true);
+    if (p.ks > 1 && (!workspace || workspace_bytes < (size_t)p.ks * m * 2 * n_rows * sizeof(float))) p = pair_plan(A.n_fp, k / 64, m, 2 * n_rows, false);
+    A.tt = p.tt; A.ksplit = p.ks; A.part = (float*)workspace;
+    if (const int rc = pair_launch(qt, bf, map, A, (int64_t)A.n_fp * ((m + A.tt - 1) / A.tt) * p.ks, st)) return rc;
+    if (p.ks > 1) {
+        int rg = (int)((m * n_rows / 4 + 255) / 256); if (rg > sm_count() * 8) rg = sm_count() * 8;
+        reduce_gated_kernel<<<rg, 256, 0, st>>>(A.part, p.ks, m, n_rows, y, y_dtype, act);
+        note_launch();
+    }
     return check_launch();
+}
+size_t gemm_tc_mlp_workspace_size(int64_t n_rows, int64_t k, int64_t m) {
+    using namespace gemmtc;
+    const PairPlan p = pair_plan((n_rows / 64 + 1) / 2, k / 64, m, 2 * n_rows, true);
+    return p.ks > 1 ? (size_t)p.ks * m * 2 * n_rows * sizeof(float) : 256;
 }
 
 // the same kernel over every expert's rows: x [rows][k] sorted by expert, offs [n_experts + 1] row offsets on the device, tab /

@@ -84,7 +84,8 @@ size_t gemm_tc_workspace_size(int64_t n_rows, int64_t k, int64_t m);
 int gemm_tc_launch(const void* w, int qt, int64_t n_rows, int64_t k, const void* x, int x_dtype, int64_t m, void* y,
                    int y_dtype, const void* bias, int accumulate, void* workspace, size_t workspace_bytes, cudaStream_t st);
 int gemm_tc_mlp_launch(const void* w_gate, const void* w_up, int act, int qt, int64_t n_rows, int64_t k, const void* x, int x_dtype,
-                       int64_t m, void* y, int y_dtype, cudaStream_t st);
+                       int64_t m, void* y, int y_dtype, void* workspace, size_t workspace_bytes, cudaStream_t st);
+size_t gemm_tc_mlp_workspace_size(int64_t n_rows, int64_t k, int64_t m);
 int gemm_tc_experts_launch(const unsigned long long* tab, const unsigned long long* tab2, int act, const int* offs, int n_experts, int qt,
                            int64_t n_rows, int64_t k, const void* x, int x_dtype, int64_t rows, void* y, int y_dtype, cudaStream_t st);
 int gemm_tc_wait_expired();       // 1 after a wait of the two-SM kernel ran out on the current device (its results are then undefined)
