@@ -64,6 +64,13 @@ int mixers_gated_delta_rule(int dtype, const void* conv, int B, int S, int kv_he
                             const void* proj, int ld, int off_b, int off_a, const void* A_log, const void* dt_bias, float* state,
                             int slot0, const int32_t* pad, float* o, mixers_stream_t stream);
 
+/* The same over a prompt, 32 tokens at a time (dim <= 128): the part of every chunk that needs no earlier state in one launch, the serial
+ * part as small matrix products in a second.  workspace: mixers_gated_delta_chunks_workspace() bytes, 16-byte aligned. */
+long mixers_gated_delta_chunks_workspace(int B, int S, int kv_heads, int heads, int dim);      /* -1: not served */
+int mixers_gated_delta_chunks(int dtype, const void* conv, int B, int S, int kv_heads, int heads, int dim, int vdim, const void* proj, int ld,
+                              int off_b, int off_a, const void* A_log, const void* dt_bias, float* state, int slot0, const int32_t* pad,
+                              float* o, float* workspace, mixers_stream_t stream);
+
 /* Delta rule whose state decays per key channel.  conv as above; beta = sigmoid(proj[.., off_b + h]); z [B, S, heads * dim]: decay
  * logits, a = exp(-exp(A_log[h]) * softplus(z + dt_bias)) with dt_bias [heads * dim].  Per head:  M <- diag(a) M;
  * u = beta (v - M^T k);  M <- M + k u^T;  o = M^T q (q, k unit vectors, q times dim^-1/2). */

@@ -30,6 +30,8 @@ _SIGNATURES = {
     "mixers_short_conv_silu": [_c_int, _c_ptr] + [_c_int] * 6 + [_c_ptr, _c_ptr, _c_ptr, _c_int, _c_ptr, _c_ptr, _c_ptr],
     "mixers_gated_delta_rule": [_c_int, _c_ptr] + [_c_int] * 6 + [_c_ptr, _c_int, _c_int, _c_int, _c_ptr, _c_ptr, _c_ptr, _c_int, _c_ptr,
                                                                  _c_ptr, _c_ptr],
+    "mixers_gated_delta_chunks": [_c_int, _c_ptr] + [_c_int] * 6 + [_c_ptr, _c_int, _c_int, _c_int, _c_ptr, _c_ptr, _c_ptr, _c_int, _c_ptr,
+                                                                   _c_ptr, _c_ptr, _c_ptr],
     "mixers_gated_linear_attention": [_c_int, _c_ptr] + [_c_int] * 6 + [_c_ptr, _c_float, _c_ptr, _c_int, _c_ptr, _c_ptr, _c_ptr],
     "mixers_gated_rms_norm": [_c_int, _c_ptr, _c_long, _c_int, _c_int, _c_ptr, _c_int, _c_int, _c_ptr, _c_int, _c_float, _c_ptr, _c_int, _c_int,
                               _c_float, _c_int, _c_ptr, _c_ptr],
@@ -95,6 +97,8 @@ def lib():
         for name, argtypes in _SIGNATURES.items():
             fn = getattr(loaded, name)
             fn.argtypes, fn.restype = argtypes, _c_int
+        loaded.mixers_gated_delta_chunks_workspace.argtypes = [_c_int] * 5
+        loaded.mixers_gated_delta_chunks_workspace.restype = _c_long
         loaded.mixers_softmax_attention_workspace.argtypes = [_c_int] * 7
         loaded.mixers_softmax_attention_workspace.restype = _c_long
         _lib, LIB_PATH = loaded, path

@@ -131,6 +131,9 @@ def state_space_scan(conv, groups, heads, n_state, vdim, proj, off_dt, A_log, dt
     return o
 
 
+DELTA_CHUNK_TOKENS = 64       # from this many new tokens on the delta rule runs chunk by chunk instead of token by token
+
+
 def gated_delta_rule(conv, kv_heads, heads, dim, vdim, proj, off_b, off_a, A_log, dt_bias, state, slot0, pad):
     """the delta-rule recurrence over the new tokens; state fp32 [B, heads, dim, vdim] in place; returns o fp32 [B, S, heads, vdim]"""
     B, S, C = conv.shape
@@ -138,9 +141,14 @@ def gated_delta_rule(conv, kv_heads, heads, dim, vdim, proj, off_b, off_a, A_log
                       and state.dtype == torch.float32 and state.is_contiguous() and state.shape == (B, heads, dim, vdim),
                       "gated_delta_rule: unexpected layout")
     o = torch.empty(B, S, heads, vdim, dtype=torch.float32, device=conv.device)
-    native.call("mixers_gated_delta_rule", native.dtype_code(conv.dtype), native.ptr(conv), B, S, kv_heads, heads, dim, vdim, native.ptr(proj),
-                proj.shape[-1], off_b, off_a, native.ptr(A_log), native.ptr(dt_bias), native.ptr(state), slot0, native.ptr(pad), native.ptr(o),
-                native.stream(conv.device))
+    args = (native.dtype_code(conv.dtype), native.ptr(conv), B, S, kv_heads, heads, dim, vdim, native.ptr(proj), proj.shape[-1], off_b, off_a,
+            native.ptr(A_log), native.ptr(dt_bias), native.ptr(state), slot0, native.ptr(pad), native.ptr(o))
+    need = native.lib().mixers_gated_delta_chunks_workspace(B, S, kv_heads, heads, dim) if S >= DELTA_CHUNK_TOKENS else -1
+    if need > 0:
+        ws = torch.empty(need, dtype=torch.uint8, device=conv.device)
+        native.call("mixers_gated_delta_chunks", *args, native.ptr(ws), native.stream(conv.device))
+    else:
+        native.call("mixers_gated_delta_rule", *args, native.stream(conv.device))
     return o
 
 

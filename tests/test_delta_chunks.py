@@ -1,0 +1,91 @@
+"""The gated delta rule 32 tokens at a time (csrc/mixers/delta_chunks.cu) against float64 and against the token-by-token kernel.
+
+Bound: all arithmetic is 32-bit; a token's value passes through a handful of dot products of up to 128 terms and its chunk's
+triangular system, whose entries are at most 1 for unit keys, so 2e-6 of the largest |value| leaves a factor of about ten over what
+sums of that length show."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from ipex_llm_b200.transformers.models import mixer_ops
+    return mixer_ops
+
+
+def inputs(dev, B, S, G, H, D, V, dtype, seed=0, gate_std=1.0):
+    g = torch.Generator(device=dev).manual_seed(seed + S)
+    conv = torch.randn(B, S, 2 * G * D + H * V, generator=g, device=dev).to(dtype)
+    proj = (torch.randn(B, S, 2 * H + 3, generator=g, device=dev) * gate_std).to(dtype)
+    a_log, bias = (torch.randn(H, generator=g, device=dev) * 0.5 - 1).to(dtype), (torch.randn(H, generator=g, device=dev) * 0.5).to(dtype)
+    state = torch.randn(B, H, D, V, generator=g, device=dev)
+    return conv, proj, a_log, bias, state
+
+
+def statement(conv, proj, a_log, bias, state, G, H, D, V, slot0, pad):
+    B, S, _ = conv.shape
+    c, p = conv.double(), proj.double()
+    unit = lambda t: t / torch.sqrt((t * t).sum(-1, keepdim=True) + 1e-6)                                       # noqa: E731
+    q = (unit(c[..., :G * D].view(B, S, G, D)) * D ** -0.5).repeat_interleave(H // G, 2)
+    k = unit(c[..., G * D:2 * G * D].view(B, S, G, D)).repeat_interleave(H // G, 2)
+    v = c[..., 2 * G * D:].view(B, S, H, V)
+    beta = torch.sigmoid(p[..., 1:1 + H])
+    decay = torch.exp(-torch.exp(a_log.double()) * torch.nn.functional.softplus(p[..., 1 + H:1 + 2 * H] + bias.double()))
+    M, o = state.double().clone(), torch.zeros(B, S, H, V, dtype=torch.float64, device=conv.device)
+    for t in range(S):
+        real = (slot0 + t >= pad).view(B, 1, 1, 1)
+        N = M * decay[:, t, :, None, None]
+        u = beta[:, t, :, None] * (v[:, t] - torch.einsum("bhdv,bhd->bhv", N, k[:, t]))
+        N = N + k[:, t, :, :, None] * u[:, :, None, :]
+        M = torch.where(real, N, M)
+        o[:, t] = torch.where(real[..., 0], torch.einsum("bhdv,bhd->bhv", N, q[:, t]), 0.0)
+    return o, M
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("B,S,G,H,D,V,pads", [(1, 64, 1, 1, 128, 16, (0,)), (2, 65, 1, 2, 64, 17, (0, 40)), (1, 95, 2, 2, 5, 9, (3,)), (3, 127, 1, 3, 70, 33, (0, 127, 64)),
+                                              (1, 200, 2, 32, 128, 128, (0,)), (2, 96, 1, 1, 65, 256, (31, 33)), (1, 333, 4, 16, 128, 128, (0,))])
+def test_against_float64_and_the_token_walk(ops, cuda_device, monkeypatch, dtype, B, S, G, H, D, V, pads):
+    conv, proj, a_log, bias, state = inputs(cuda_device, B, S, G, H, D, V, dtype)
+    pad = torch.tensor(pads, dtype=torch.int32, device=cuda_device)
+    want_o, want_s = statement(conv, proj, a_log, bias, state, G, H, D, V, 0, pad)
+    err = {}
+    for route, least in (("chunks", 1), ("tokens", 1 << 30)):
+        monkeypatch.setattr(ops, "DELTA_CHUNK_TOKENS", least)
+        s = state.clone()
+        o = ops.gated_delta_rule(conv, G, H, D, V, proj, 1, 1 + H, a_log, bias, s, 0, pad)
+        assert float((o.double() - want_o).abs().max()) <= 2e-6 * max(1.0, float(want_o.abs().max()))
+        assert float((s.double() - want_s).abs().max()) <= 2e-6 * max(1.0, float(want_s.abs().max()))
+        err[route] = float((o.double() - want_o).norm() / want_o.norm())
+    assert err["chunks"] <= 1.2 * err["tokens"] + 2.0 ** -24                       # as exact as the walk it replaces
+
+
+def test_portions_and_hard_gates(ops, cuda_device):
+    """a prompt in portions that end inside chunks; gates from 'forget all' to 'keep all' (decays that underflow, betas at 0 and 1)"""
+    B, S, G, H, D, V = 2, 300, 1, 2, 128, 40
+    conv, proj, a_log, bias, state = inputs(cuda_device, B, S, G, H, D, V, torch.float32, gate_std=40.0)
+    a_log = a_log + 3.0                                                              # exp(-20 softplus): zero in 32 bits for half of the tokens
+    proj[0, 70:75, 1 + H:1 + 2 * H] = 1e30
+    pad = torch.tensor([0, 7], dtype=torch.int32, device=cuda_device)
+    want_o, want_s = statement(conv, proj, a_log, bias, state, G, H, D, V, 0, pad)
+    s, got, at = state.clone(), [], 0
+    for n in (65, 100, 1, 134):
+        got.append(ops.gated_delta_rule(conv[:, at:at + n].contiguous(), G, H, D, V, proj[:, at:at + n].contiguous(), 1, 1 + H, a_log, bias, s, at, pad))
+        at += n
+    assert float((torch.cat(got, 1).double() - want_o).abs().max()) <= 2e-6 * float(want_o.abs().max())
+    assert float((s.double() - want_s).abs().max()) <= 2e-6 * float(want_s.abs().max())
+
+
+def test_equal_keys(ops, cuda_device):
+    """every key the same: the triangular system at its worst"""
+    B, S, G, H, D, V = 1, 160, 1, 1, 64, 16
+    conv, proj, a_log, bias, state = inputs(cuda_device, B, S, G, H, D, V, torch.float32)
+    conv[..., D:2 * D] = conv[:, :1, D:2 * D]
+    a_log = a_log - 9.0                                                              # hardly any decay
+    pad = torch.zeros(B, dtype=torch.int32, device=cuda_device)
+    want_o, want_s = statement(conv, proj, a_log, bias, state, G, H, D, V, 0, pad)
+    o = ops.gated_delta_rule(conv, G, H, D, V, proj, 1, 1 + H, a_log, bias, state, 0, pad)
+    assert float((o.double() - want_o).abs().max()) <= 2e-6 * float(want_o.abs().max())
+    assert float((state.double() - want_s).abs().max()) <= 2e-6 * float(want_s.abs().max())
