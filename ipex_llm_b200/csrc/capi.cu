@@ -168,6 +168,12 @@ static bool use_gemm(int qtype, int64_t n_rows, int64_t k, int64_t m, int x_dtyp
     return x_dtype != DT_F32 && m > max_m && gemm_tc_supported(qtype, n_rows, k);
 }
 
+// fp32 rows beyond one pass of the GEMV, fp32 results: the same arithmetic on pairs of SMs (gemm_exact.cu), where code x scale is the value.
+// The line lies at the GEMV's 32 rows: at 33 rows, two passes against one launch, 33.8 -> 17.4 us at 4096 x 4096, 18.2 -> 12.4 at 1024 x 1024
+static bool use_exact(int qtype, int64_t n_rows, int64_t k, int64_t m, int x_dtype, int y_dtype) {
+    return x_dtype == DT_F32 && y_dtype == DT_F32 && m > kGemvMaxM && gemm_exact_supported(qtype, n_rows, k, m);
+}
+
 // Batches between the GEMV's best range and a full 128-token tile take the tensor-core kernel with the operands swapped
 // (gemm_skinny_launch): weights rounded once to the activation dtype, the prefill kernel's precision contract.
 // Measured on 11008x4096 sym_int4: GEMV 12 us at M = 16 and 22 us at M = 32, this kernel 15.5 us for 9 <= M <= 32, 17-20 us
@@ -182,7 +188,10 @@ static bool use_skinny(int qtype, int64_t n_rows, int64_t k, int64_t m, int x_dt
 size_t lowbit_matmul_workspace_size(int64_t n_rows, int64_t k, int64_t m, int x_dtype) {
     if (use_skinny(B200_QT_SYM_INT4, n_rows, k, m, x_dtype)) return gemm_skinny_workspace_size(n_rows, k, m);
     if (use_gemm(B200_QT_SYM_INT4, n_rows, k, m, x_dtype)) return gemm_tc_workspace_size(n_rows, k, m);
-    return gemv_workspace_size(n_rows, k, m, x_dtype);
+    const size_t gemv = gemv_workspace_size(n_rows, k, m, x_dtype);
+    if (!use_exact(B200_QT_SYM_INT4, n_rows, k, m, x_dtype, DT_F32)) return gemv;
+    const size_t exact = gemm_exact_workspace_size(n_rows, k, m);          // the size is asked without the format: enough for either
+    return exact > gemv ? exact : gemv;
 }
 
 static int matmul_dispatch(const void* d_w, int qtype, int64_t n_rows, int64_t k, const void* d_x, int x_dtype, int64_t m,
@@ -193,6 +202,10 @@ static int matmul_dispatch(const void* d_w, int qtype, int64_t n_rows, int64_t k
                                   workspace_bytes, st, gemv_get_pdl());
     if (use_gemm(qtype, n_rows, k, m, x_dtype))
         return gemm_tc_launch(d_w, qtype, n_rows, k, d_x, x_dtype, m, d_y, y_dtype, d_bias, accumulate, workspace, workspace_bytes, st);
+    // a caller's scratch of the GEMV's size still runs its chunks of 32 rows
+    if (use_exact(qtype, n_rows, k, m, x_dtype, y_dtype) && workspace && workspace_bytes >= gemm_exact_workspace_size(n_rows, k, m) &&
+        !(((uintptr_t)d_x | (uintptr_t)d_w | (uintptr_t)workspace) & 15))
+        return gemm_exact_launch(d_w, qtype, n_rows, k, d_x, m, d_y, d_bias, accumulate, workspace, workspace_bytes, st);
     return gemv_launch(d_w, qtype, n_rows, k, d_x, x_dtype, m, d_y, y_dtype, d_bias, accumulate, workspace, workspace_bytes, st);
 }
 
@@ -363,8 +376,8 @@ int lowbit_moe_tokens_cuda(const void* d_x, int x_dtype, int64_t n_tokens, const
 }
 
 int lowbit_gemm_wait_expired(void) {
-    const int a = gemm_tc_wait_expired(), b = sdp_prompt_wait_expired();
-    return a < 0 || b < 0 ? -1 : a | b;
+    const int a = gemm_tc_wait_expired(), b = sdp_prompt_wait_expired(), c = gemm_exact_wait_expired();
+    return a < 0 || b < 0 || c < 0 ? -1 : a | b | c;
 }
 
 // ------------------------------------------------------------------ family (1)

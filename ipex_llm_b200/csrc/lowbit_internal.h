@@ -91,6 +91,13 @@ int gemm_tc_experts_launch(const unsigned long long* tab, const unsigned long lo
 int gemm_tc_wait_expired();       // 1 after a wait of the two-SM kernel ran out on the current device (its results are then undefined)
 int sdp_prompt_wait_expired();    // the same of the prompt attention (kvcache.cu)
 
+// gemm_exact.cu (the fp32 prompt matmul: codes and activation planes exact on the tensor cores)
+bool gemm_exact_supported(int qt, int64_t n_rows, int64_t k, int64_t m);
+size_t gemm_exact_workspace_size(int64_t n_rows, int64_t k, int64_t m);
+int gemm_exact_launch(const void* w, int qt, int64_t n_rows, int64_t k, const void* x, int64_t m, void* y, const void* bias, int accumulate,
+                      void* workspace, size_t workspace_bytes, cudaStream_t st);
+int gemm_exact_wait_expired();
+
 // M above this goes to the tensor-core GEMM when the shape allows, else to chunks of the GEMV
 constexpr int64_t kGemvMaxM = 32;
 // the tensor-core GEMM with the operands swapped (weights = the 128-row operand, tokens = N): 9 <= m <= 128

@@ -149,3 +149,32 @@ def test_prompt_matmul_rings_over_many_rounds(lbl, cuda_device, qtype, dtype):
     assert bool(((first.double() - want).abs() <= bound).all())
     for _ in range(8):
         assert torch.equal(lbl.lowbit_matmul(x, w, (n, k), qt, out_dtype=torch.float32), first)
+
+
+@pytest.mark.parametrize("m,n,k", [(33, 128, 64), (64, 384, 128), (65, 256, 4096), (127, 640, 192), (200, 4096, 1024), (300, 2176, 320), (513, 19072, 64)])
+@pytest.mark.parametrize("qtype", ["sym_int4", "fp8_e4m3", "fp8_e5m2", "fp6", "asym_int4", "nf4"])
+def test_prompt_matmul_fp32_keeps_its_contract(lbl, native_lib, cuda_device, qtype, m, n, k):
+    """32-bit activations to 2^-24 of sum|x w| (the bound of the GEMV's tests: 2e-6; nf4's table is held to 2^-17), no further off than the
+    GEMV's passes of 32 rows, which a workspace of their size still gets"""
+    [(w, wd)], qt = weights(lbl, cuda_device, m + n, n, k, qtype)
+    x = acts(cuda_device, k, m, k, torch.float32)
+    mag = x.double().abs() @ wd.abs().T
+    want, tol = x.double() @ wd.T, (2e-6 if qtype != "nf4" else 2.0 ** -17 + 2e-6)
+    y = lbl.lowbit_matmul(x, w, (n, k), qt)
+    assert y.dtype == torch.float32 and bool(((y.double() - want).abs() <= tol * mag).all())
+    small = native_lib.lowbit_matmul_workspace_size(n, k, 32, native_lib.DT_F32)
+    ws, passes = torch.empty(small, dtype=torch.uint8, device=cuda_device), torch.empty_like(y)
+    native_lib.lowbit_matmul_cuda(w.data_ptr(), qt, n, k, x.data_ptr(), native_lib.DT_F32, m, passes.data_ptr(), native_lib.DT_F32, None, False,
+                                  ws.data_ptr(), ws.numel(), torch.cuda.current_stream().cuda_stream)
+    assert bool(((passes.double() - want).abs() <= tol * mag).all())
+    assert float((y.double() - want).norm()) <= 1.05 * float((passes.double() - want).norm())
+    bias, out = acts(cuda_device, 5, 1, n, torch.float32)[0], torch.empty(m * n + 1, device=cuda_device)[1:].view(m, n)
+    out.copy_(acts(cuda_device, 6, m, n, torch.float32))
+    base = y.double() + bias.double() + out.double()
+    terms = y.abs() + bias.abs() + out.abs()
+    lbl.lowbit_matmul(x, w, (n, k), qt, out=out, bias=bias, accumulate=True)
+    assert bool(((out.double() - base).abs() <= 2.0 ** -22 * terms.double() + 2e-6 * mag).all())
+    # a strided or misaligned view of the activations, and 16-bit results, which keep to the GEMV
+    assert torch.equal(lbl.lowbit_matmul(torch.cat([x, x], 1)[:, :k], w, (n, k), qt), y)
+    half = lbl.lowbit_matmul(x, w, (n, k), qt, out_dtype=torch.float16)
+    assert bool(((half.double() - want).abs() <= tol * mag + 2.0 ** -11 * want.abs() + 2.0 ** -25).all())
