@@ -10,8 +10,10 @@
 // k-block of 0.46 us are 12 TB/s over the chip, and four 53 KB stages left no depth to hide it; a pair moves 16 + 4.4 KB per CTA
 // for the same arithmetic.  At 128-token tiles the bound was the chain load -> expand -> MMA through one ring (0.33 us per
 // k-block, the MMAs 0.14): here activations, packed weights and expanded tiles have rings of their own, so the expansion runs
-// ahead of the activations and four groups of warps have four k-blocks in flight.  Measured per k-block: 0.25 us up to 192 tokens
-// (the expansion's pace), 0.335 at 256; 14336 x 4096 at 4000 tokens 1357 -> 1468 TFLOP/s, 4096 x 11008 at 512 tokens 59.7 -> 50.6 us.
+// ahead of the activations and four groups of warps have four k-blocks in flight.  Measured per k-block: 0.19 us up to 170 tokens
+// (fp16; see pair_plan for the other paces), 0.282 at 256, where the tensor pipe is busy 512 of 525 clocks; 14336 x 4096 at 4000
+// tokens 1357 -> 1494 TFLOP/s, 4096 x 11008 at 512 tokens 59.7 -> 43.4 us.  At 128 tokens the MMAs need 256 of 360 clocks: A and B
+// both come from shared memory, beside the expansion's stores.
 //   warp 0       TMA: this CTA's half of the tokens, boxes of 32 rows x 64 elements (128-byte swizzle), ring of kX slots;
 //   warp 1       CTA 0: issues the MMAs (M = 256, N, K = 16; four per k-block) in warp-uniform control flow, one commit per ring
 //                (multicast to both CTAs); CTA 1: relays "my half has landed" to CTA 0's barrier;
@@ -42,11 +44,11 @@ template <int QT> struct PairSmem {
     static constexpr int kTab = 2 * (kMaxExperts + 4) * 4;             // tile prefix and row offsets of the experts
     static constexpr int kOut = 2 * 32 * 256;                          // epilogue: two chunks of 32 tokens x 128 features, 16 bits
     static constexpr int kA = 4;                                       // slots of 16 KB, one per dequant group
-    static constexpr int kP = 8;                                       // see the dequant loop: at least twice the groups
+    static constexpr int kP = 8;                                       // see the dequant loop: twice the groups
     static constexpr int kFixed = 1024 + 512 + kTab + kLut + kOut + kA * kTileBytesAB + kP * kPacked;
     static constexpr int kX = (232448 - kFixed) / kTileBytesAB < 8 ? (232448 - kFixed) / kTileBytesAB : 8;      // slots of 128 rows x 128 bytes
     static constexpr int kTotal = kFixed + kX * kTileBytesAB;
-    static_assert(kX >= 3 && kP >= 2 * kA, "ring depths");
+    static_assert(kX >= 3 && kP == 2 * kA && kTotal <= 232448, "ring depths");
     static_assert((3 * kX + 2 * kP + 2 * kA + 4) * 8 + 8 <= 512, "barrier region");
 };
 
@@ -190,6 +192,7 @@ pair_kernel(const __grid_constant__ CUtensorMap xmap, const PairArgs A) {
             // ================= MMA issuer =================
             const uint32_t leader = elect_leader();
             int sx = 0, rx = 0, it = 0, ti = 0;
+            bool ready = false;
             for (int unit = blockIdx.x >> 1; unit < n_units; unit += stride, ti++) {
                 decode(unit, U);
                 // c F32 (1<<4), a/b format (0 f16, 1 bf16), both K-major, N (>>3 at bit 17), M = 256 (>>4 at bit 24)
@@ -198,11 +201,9 @@ pair_kernel(const __grid_constant__ CUtensorMap xmap, const PairArgs A) {
                 if (!mbar_wait_lim(tmem_empty(buf), (uint32_t)(((ti >> 1) & 1) ^ 1))) goto done;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t acc = tmem_base + buf * kPairTok;
-                for (int kb = U.kb0; kb < U.kb1; kb++, it++) {
+                for (int kb = U.kb0; kb < U.kb1; kb++) {
                     const int sa = it & 3;
-                    if (!mbar_wait_lim(x_full(sx), (uint32_t)(rx & 1))) goto done;
-                    if (!mbar_wait_lim(xp_full(sx), (uint32_t)(rx & 1))) goto done;
-                    if (!mbar_wait_lim(a_full(sa), (uint32_t)((it >> 2) & 1))) goto done;
+                    if (!mbar_wait3_lim(ready, x_full(sx), (uint32_t)(rx & 1), xp_full(sx), (uint32_t)(rx & 1), a_full(sa), (uint32_t)((it >> 2) & 1))) goto done;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint64_t ad = make_desc(aring + sa * kTileBytesAB), xd = make_desc(xring + sx * kTileBytesAB);
 #pragma unroll
@@ -211,6 +212,9 @@ pair_kernel(const __grid_constant__ CUtensorMap xmap, const PairArgs A) {
                     umma2_commit_w(a_empty(sa), leader);
                     umma2_commit_w(x_empty(sx), leader);
                     if (++sx == KX) { sx = 0; rx++; }
+                    it++;
+                    // asked here, answered while the MMAs above are being issued
+                    ready = mbar_test3(x_full(sx), (uint32_t)(rx & 1), xp_full(sx), (uint32_t)(rx & 1), a_full(it & 3), (uint32_t)((it >> 2) & 1));
                 }
                 umma2_commit_w(tmem_full(buf), leader);
             }
@@ -257,13 +261,14 @@ pair_kernel(const __grid_constant__ CUtensorMap xmap, const PairArgs A) {
         const int grp = (warp - kPairDeq0) >> 2, dw = (warp - kPairDeq0) & 3;
         const int g = lane >> 2, t = lane & 3;
         const uint32_t row0 = aring + grp * kTileBytesAB + 4 * dw * 1024 + g * 128;        // rows 32 dw + g, + 8; + 16, + 24 for the second group
-        int it = 0, sp = 0, rp = 0;
+        // k-blocks are numbered over all units of the cluster: `end` behind the unit's last, `it` this group's next
+        int end = 0, it = grp;
         for (int unit = blockIdx.x >> 1; unit < n_units; unit += stride) {
             decode(unit, U);
-            for (int kb = U.kb0; kb < U.kb1; kb++, it++, (++sp == KP ? (sp = 0, rp++) : 0)) {
-                if ((it & 3) != grp) continue;
-                // this group has waited for the MMAs of k-block it - 8 (below, at its last k-block): all before it were expanded, so the
-                // packed slot's earlier trips are over (it - KP <= it - 8) and its parity is unambiguous
+            end += U.kb1 - U.kb0;
+            for (; it < end; it += 4) {
+                const int sp = it & (KP - 1), rp = it / KP;
+                // the slot's last trip (k-block it - 8) was this group's own, so the parity is unambiguous
                 if (!mbar_wait_lim(p_full(sp), (uint32_t)(rp & 1))) goto done;
                 const uint32_t pk = pring + sp * SM::kPacked;
                 typename E::Codes cw[2];
@@ -494,26 +499,39 @@ static int pair_launch(int qt, bool bf, const CUtensorMap& map, const PairArgs& 
 }
 
 // Token tile and K splits of a matmul: the pair that minimises rounds of the resident clusters x k-blocks per unit x time per
-// k-block (measured, sym_int4: 0.25 us up to 192 tokens, where the expansion of 128 x 64 weights per CTA sets the pace, 0.335 at
-// 256) + the start and end of a unit and, when K is split, the partial sums' round trip through memory at ~4 TB/s and the second
-// launch.
+// k-block + the start and end of a unit and, when K is split, the partial sums' round trip through memory at ~4 TB/s and the second
+// launch.  Time per k-block, measured at 4096 x 11008 and 4096 x 4096: 0.0011 us per token once the MMAs set the pace (0.282 at 256),
+// below that the expansion and the chain around it, whose pace depends on the codec (0.19 us with fp16 activations, 0.24 with bf16,
+// 0.29 for nf4's table).  What the line between (128 tokens, K whole) and (256, two splits) is worth at 512 tokens, 4096 x 11008:
+// sym_int4 fp16 43.4 against 48.2 us, bf16 50.3 against 48.8, nf4 58.1 against 50.1.
+constexpr double kPaces[3] = {0.19, 0.24, 0.29};
+static double pair_pace(int qt, bool bf) { return kPaces[qt == QT_NF4 ? 2 : bf ? 1 : 0]; }
 struct PairPlan { int tt, ks; };
-static PairPlan pair_plan(int64_t n_fp, int64_t nb, int64_t m, int64_t n_out, bool may_split) {
+static PairPlan pair_plan(double pace, int64_t n_fp, int64_t nb, int64_t m, int64_t n_out, bool may_split) {
     const int64_t clusters = sm_count() / 2, nt0 = (m + kPairTok - 1) / kPairTok;
     PairPlan best = {256, 1};
     double best_cost = 1e30;
     for (int64_t nt = nt0; nt <= nt0 + 8 && nt <= (m + 31) / 32; nt++) {
         const int64_t tt = ((m + nt - 1) / nt + 15) & ~int64_t(15);
-        const double per_kb = tt <= 192 ? 0.25 : 0.25 + 0.00133 * (double)(tt - 192);
+        const double mma = 0.0011 * (double)tt, per_kb = mma > pace ? mma : pace;
         const int64_t max_ks = may_split ? (nb / 8 < 8 ? nb / 8 : 8) : 1;
         for (int64_t ks = 1; ks == 1 || ks <= max_ks; ks++) {
             const int64_t rounds = (n_fp * nt * ks + clusters - 1) / clusters;
             double cost = (double)rounds * ((double)((nb + ks - 1) / ks) * per_kb + 1.0);
-            if (ks > 1) cost += (double)ks * (double)m * (double)n_out * 8.0 / 4.0e6 + 2.0;
+            if (ks > 1) cost += (double)ks * (double)m * (double)n_out * 8.0 / 4.0e6 + 3.0;
             if (cost < best_cost - 1e-9) { best_cost = cost; best = {(int)tt, (int)ks}; }
         }
     }
     return best;
+}
+// splits that a workspace has to hold, whatever the format and type
+static int most_splits(int64_t n_fp, int64_t nb, int64_t m, int64_t n_out) {
+    int ks = 1;
+    for (const double pace : kPaces) {
+        const PairPlan p = pair_plan(pace, n_fp, nb, m, n_out, true);
+        if (p.ks > ks) ks = p.ks;
+    }
+    return ks;
 }
 }  // namespace gemmtc
 
@@ -525,8 +543,8 @@ bool gemm_tc_supported(int qt, int64_t n_rows, int64_t k) {
 
 size_t gemm_tc_workspace_size(int64_t n_rows, int64_t k, int64_t m) {
     using namespace gemmtc;
-    const PairPlan p = pair_plan((n_rows / 128 + 1) / 2, k / 64, m, n_rows, true);
-    return p.ks > 1 ? (size_t)p.ks * m * n_rows * sizeof(float) : 0;
+    const int ks = most_splits((n_rows / 128 + 1) / 2, k / 64, m, n_rows);
+    return ks > 1 ? (size_t)ks * m * n_rows * sizeof(float) : 0;
 }
 
 int gemm_tc_launch(const void* w, int qt, int64_t n_rows, int64_t k, const void* x, int x_dtype, int64_t m, void* y,
@@ -541,9 +559,9 @@ int gemm_tc_launch(const void* w, int qt, int64_t n_rows, int64_t k, const void*
     PairArgs A = {};
     A.w = (const uint8_t*)w; A.G = make_geom(n_rows, k, qt); A.M = (int)m; A.y = y; A.y_dtype = y_dtype; A.bias = bias; A.accumulate = accumulate;
     A.n_fp = (int)((n_rows / 128 + 1) / 2);
-    PairPlan p = pair_plan(A.n_fp, k / 64, m, n_rows, true);
+    PairPlan p = pair_plan(pair_pace(qt, bf), A.n_fp, k / 64, m, n_rows, true);
     // a caller's workspace without room for partial sums: the whole K range per unit
-    if (p.ks > 1 && (!workspace || workspace_bytes < (size_t)p.ks * m * n_rows * sizeof(float))) p = pair_plan(A.n_fp, k / 64, m, n_rows, false);
+    if (p.ks > 1 && (!workspace || workspace_bytes < (size_t)p.ks * m * n_rows * sizeof(float))) p = pair_plan(pair_pace(qt, bf), A.n_fp, k / 64, m, n_rows, false);
     A.tt = p.tt; A.ksplit = p.ks; A.part = (float*)workspace;
     const int64_t units = (int64_t)A.n_fp * ((m + p.tt - 1) / p.tt) * p.ks;
     if (const int rc = pair_launch(qt, bf, map, A, units, st)) return rc;
@@ -570,8 +588,8 @@ int gemm_tc_mlp_launch(const void* w_gate, const void* w_up, int act, int qt, in
     PairArgs A = {};
     A.w = (const uint8_t*)w_gate; A.w2 = (const uint8_t*)w_up; A.act = act; A.G = make_geom(n_rows, k, qt); A.M = (int)m; A.y = y; A.y_dtype = y_dtype;
     A.n_fp = (int)((n_rows / 64 + 1) / 2);
-    PairPlan p = pair_plan(A.n_fp, k / 64, m, 2 * n_rows, true);
-    if (p.ks > 1 && (!workspace || workspace_bytes < (size_t)p.ks * m * 2 * n_rows * sizeof(float))) p = pair_plan(A.n_fp, k / 64, m, 2 * n_rows, false);
+    PairPlan p = pair_plan(pair_pace(qt, bf), A.n_fp, k / 64, m, 2 * n_rows, true);
+    if (p.ks > 1 && (!workspace || workspace_bytes < (size_t)p.ks * m * 2 * n_rows * sizeof(float))) p = pair_plan(pair_pace(qt, bf), A.n_fp, k / 64, m, 2 * n_rows, false);
     A.tt = p.tt; A.ksplit = p.ks; A.part = (float*)workspace;
     if (const int rc = pair_launch(qt, bf, map, A, (int64_t)A.n_fp * ((m + A.tt - 1) / A.tt) * p.ks, st)) return rc;
     if (p.ks > 1) {
@@ -583,8 +601,8 @@ int gemm_tc_mlp_launch(const void* w_gate, const void* w_up, int act, int qt, in
 }
 size_t gemm_tc_mlp_workspace_size(int64_t n_rows, int64_t k, int64_t m) {
     using namespace gemmtc;
-    const PairPlan p = pair_plan((n_rows / 64 + 1) / 2, k / 64, m, 2 * n_rows, true);
-    return p.ks > 1 ? (size_t)p.ks * m * 2 * n_rows * sizeof(float) : 256;
+    const int ks = most_splits((n_rows / 64 + 1) / 2, k / 64, m, 2 * n_rows);
+    return ks > 1 ? (size_t)ks * m * 2 * n_rows * sizeof(float) : 256;
 }
 
 // the same kernel over every expert's rows: x [rows][k] sorted by expert, offs [n_experts + 1] row offsets on the device, tab /

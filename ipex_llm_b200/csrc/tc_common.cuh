@@ -88,6 +88,30 @@ __device__ __forceinline__ bool mbar_wait_lim(uint32_t bar, uint32_t parity) {
     }
     return true;
 }
+// three barriers at once: a test takes about 100 clocks to answer, and these overlap.  Tests that do not suspend the warp: the answer
+// may be wanted early, for a phase that is far off
+__device__ __forceinline__ bool mbar_test3(uint32_t b0, uint32_t p0, uint32_t b1, uint32_t p1, uint32_t b2, uint32_t p2) {
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p, q, r;\n\t"
+                 "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+                 "mbarrier.test_wait.parity.shared::cta.b64 q, [%3], %4;\n\t"
+                 "mbarrier.test_wait.parity.shared::cta.b64 r, [%5], %6;\n\t"
+                 "and.pred p, p, q;\n\tand.pred p, p, r;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok) : "r"(b0), "r"(p0), "r"(b1), "r"(p1), "r"(b2), "r"(p2) : "memory");
+    return ok != 0;
+}
+// `ready`: what mbar_test3 said earlier
+__device__ __forceinline__ bool mbar_wait3_lim(bool ready, uint32_t b0, uint32_t p0, uint32_t b1, uint32_t p1, uint32_t b2, uint32_t p2) {
+    if (__all_sync(0xffffffffu, ready)) return true;
+    const long long t0 = clock64();
+    while (!__all_sync(0xffffffffu, mbar_test3(b0, p0, b1, p1, b2, p2))) {
+        if (__any_sync(0xffffffffu, clock64() - t0 > kWaitCycles)) {
+            if ((threadIdx.x & 31) == 0) atomicExch(&g_wait_expired, 1u);
+            return false;
+        }
+    }
+    return true;
+}
 static int wait_expired_here() {
     unsigned int v = 0;
     if (cudaMemcpyFromSymbol(&v, g_wait_expired, sizeof(v)) != cudaSuccess) { cudaGetLastError(); return -1; }
