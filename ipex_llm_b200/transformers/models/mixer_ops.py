@@ -131,7 +131,9 @@ def state_space_scan(conv, groups, heads, n_state, vdim, proj, off_dt, A_log, dt
     return o
 
 
-DELTA_CHUNK_TOKENS = 64       # from this many new tokens on the delta rule runs chunk by chunk instead of token by token
+# From this many new tokens on the delta rule runs chunk by chunk instead of token by token (two launches and a workspace against one
+# launch): 64 tokens 24.9 against 26.8 us at 16 heads of 128 x 128, 123 against 335 at four sequences of 32 heads of 128 x 256
+DELTA_CHUNK_TOKENS = 64
 
 
 def gated_delta_rule(conv, kv_heads, heads, dim, vdim, proj, off_b, off_a, A_log, dt_bias, state, slot0, pad):

@@ -89,3 +89,16 @@ def test_equal_keys(ops, cuda_device):
     o = ops.gated_delta_rule(conv, G, H, D, V, proj, 1, 1 + H, a_log, bias, state, 0, pad)
     assert float((o.double() - want_o).abs().max()) <= 2e-6 * float(want_o.abs().max())
     assert float((state.double() - want_s).abs().max()) <= 2e-6 * float(want_s.abs().max())
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_a_token_that_is_not_finite_stays_behind_the_earlier_ones(ops, cuda_device, bad):
+    """values at token 77, in the middle of a chunk: the tokens before it come out as without it"""
+    B, S, G, H, D, V = 1, 130, 1, 1, 128, 32
+    conv, proj, a_log, bias, state = inputs(cuda_device, B, S, G, H, D, V, torch.float32)
+    pad = torch.zeros(B, dtype=torch.int32, device=cuda_device)
+    o = ops.gated_delta_rule(conv, G, H, D, V, proj, 1, 1 + H, a_log, bias, state.clone(), 0, pad)
+    conv[0, 77, 2 * G * D + 3] = bad                                                 # one value column
+    got = ops.gated_delta_rule(conv, G, H, D, V, proj, 1, 1 + H, a_log, bias, state.clone(), 0, pad)
+    assert torch.equal(got[:, :77], o[:, :77]) and not bool(got[:, 77:, :, 3].isfinite().any())
+    assert torch.equal(got[..., :3], o[..., :3]) and torch.equal(got[..., 4:], o[..., 4:])
