@@ -293,8 +293,8 @@ def prefill_numbers(model, dev, peaks):
                 lbl.lowbit_matmul(xs[lin.in_len], lin.weight.data, lin.weight_shape, lin.qtype, out=ys[lin.out_len])
 
         def run_model_path():
-            # the linears as the model's forward issues them: qkv, o, gate + up through mlp_forward (ONE grid of the
-            # tensor-core kernel for both matrices, then the activation kernel -- its time is inside the figure), down
+            # the linears as the model's forward issues them: qkv, o, gate + up through mlp_forward (ONE launch of the
+            # tensor-core kernel for both matrices and the activation), down
             for qkv, o, gate, up, down in mlps:
                 lbl.lowbit_matmul(xs[HIDDEN], qkv.weight.data, qkv.weight_shape, qkv.qtype, out=ys[qkv.out_len])
                 lbl.lowbit_matmul(xs[HIDDEN], o.weight.data, o.weight_shape, o.qtype, out=ys[o.out_len])
@@ -321,7 +321,7 @@ def prefill_numbers(model, dev, peaks):
         out[f"M{M}"] = {"ms_per_layer": ms / 8, "tflops": tf, "frac_of_peak": tf / burst,
                         "tok_per_s_linears_only": M / (ms / 8 * LAYERS * 1e-3),
                         "model_path_ms_per_layer": ms_model / 8,
-                        "model_path_note": "qkv, o, mlp_forward (gate + up in one grid + the activation kernel), down"}
+                        "model_path_note": "qkv, o, mlp_forward (gate, up and the activation in one launch), down"}
         if peaks.get("bf16_tflops_sustained"):          # the loop is 120 GEMMs back to back: also against the sustained figure
             out[f"M{M}"]["frac_of_sustained_peak"] = tf / float(peaks["bf16_tflops_sustained"])
     ids = torch.randint(0, VOCAB, (1, PROMPT_LEN), device=dev)

@@ -269,7 +269,7 @@ int lowbit_relayout_cuda(const void* d_src, void* d_dst, int64_t rows, int64_t k
                          int to_device, void* stream);
 
 /* bytes of workspace lowbit_matmul_cuda needs for this problem: the three bf16 planes an fp32 activation
- * chunk is split into (GEMV), or the fp32 partial sums of the K-split small-batch GEMM; 0 for fp16 / bf16
+ * chunk is split into (GEMV; all rows' planes and partial sums beyond 32 rows), or the fp32 partial sums of a K-split GEMM; 0 for fp16 / bf16
  * activations on the GEMV.  Nothing in it has to be initialised; it may be reused by any number of calls
  * that do not overlap in time. */
 size_t lowbit_matmul_workspace_size(int64_t n_rows, int64_t k, int64_t m, int x_dtype);
@@ -287,8 +287,9 @@ size_t lowbit_matmul_workspace_size(int64_t n_rows, int64_t k, int64_t m, int x_
  * not a multiple of 128 or k not of 128), larger M the tensor-core kernels -- 17..64 rows the "skinny" one with the
  * weights as the 128-row operand, beyond that the prefill GEMM (activations and expanded weights enter the MMA as
  * fp16 / bf16, fp32 accumulation: about 1e-3 * sum|x w|); both may use a second, reduction launch.
- * fp32 activations: always the GEMV (chunks of 32 rows), which keeps them to 2^-24 -- the fp32-in / fp32-out
- * contract of ggml_compute_forward_mul_mat_q_fp32; cast to fp16 first to trade that precision for the GEMM,
+ * fp32 activations: kept to 2^-24 -- the fp32-in / fp32-out contract of ggml_compute_forward_mul_mat_q_fp32 -- by the
+ * GEMV, and beyond 32 rows with fp32 results by the tensor cores on three bf16 planes (formats whose value is code x scale;
+ * the others, other result types and a workspace of 32 rows' size keep to the GEMV, 32 rows at a time); cast to fp16 first to trade that precision for the GEMM,
  * as the reference's XPU path does (LBL:700-705). */
 int lowbit_matmul_cuda(const void* d_w, int qtype, int64_t n_rows, int64_t k,
                        const void* d_x, int x_dtype, int64_t m,
