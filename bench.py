@@ -62,7 +62,7 @@ def workload_config(k_steps):
 
 
 class ClockSampler:
-    """nvidia-smi clocks / throttle reasons during the timed region (B200_PROFILING.md recipe)."""
+    """nvidia-smi clocks / throttle reasons during the timed region."""
 
     def __init__(self, index=0):
         self.samples, self.stop_flag, self.index = [], False, index
