@@ -13,11 +13,13 @@
 // its softmax, and every key tile is expanded once for 256 rows.  P lies over S, so a tile's next Q . K waits for its P . V (a commit,
 // not the issue order).  What bounds it: per 128 keys and 256 rows 2048 clocks of MMAs, 2048 of ex2 (16 a clock), and the chain
 // Q.K -> softmax -> P.V of one tile.  The kernel it replaces (64 rows a CTA, mma.sync) was bound by the legacy tensor path:
-// 4000 causal tokens, 32 heads over 8: 596 us, 220 TFLOP/s; this one 154 us, 849 (6000 tokens of two sequences: 2402 -> 606 us, 974).
+// 4000 causal tokens, 32 heads over 8, the call: 609 us, 215 TFLOP/s; this one 164 us, 800.
 // Causal: query token s (0-based among the S new ones) sees keys <= L - S + s; key tiles beyond a tile's last row are skipped.  An
 // additive mask [B][1|Hq][S][L] is honoured.  Softmax and accumulation in 32 bits; Q and P enter the MMAs as fp16.  P is kept relative
 // to a reference 2^8 below fp16's comfortable range (values up to 2^14, nothing above 2^-32 of the row's maximum is flushed), and the
 // reference follows the row's maximum only when that grew by more than 2^6: O is then rescaled in TMEM, which is rarely.
+// The denominator sums the same rounded P (2.5 us of the 164): summed from the unrounded values it left up to 10 % more error, most
+// where a row's softmax is peaked.
 
 constexpr int SP_ROWS = 128, SP_KEYS = 128, SP_SLOTS = 4;
 constexpr int SP_TILE = 128 * 256;                                    // 128 rows x 128 fp16, as two swizzled halves of 64 columns
@@ -54,6 +56,10 @@ __device__ __forceinline__ void sp_umma_ts_w(uint32_t tmem_d, uint32_t tmem_a, u
         "setp.ne.b32 q, %5, 0;\n\t"
         "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
         ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(leader) : "memory");
+}
+// a += the first, b += the second of a pair of fp16 values, in 32 bits
+__device__ __forceinline__ void sp_add2(float& a, float& b, uint32_t pair) {
+    asm("{\n\t.reg .b16 lo, hi;\n\tmov.b32 {lo, hi}, %2;\n\tadd.rn.f32.f16 %0, lo, %0;\n\tadd.rn.f32.f16 %1, hi, %1;\n\t}" : "+f"(a), "+f"(b) : "r"(pair));
 }
 __device__ __forceinline__ void sp_sts128(uint32_t a, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
     asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
@@ -217,10 +223,12 @@ sdp_fp8_prompt_kernel(const SdpArgs A, int n_qt) {
                     for (int i = 0; i < 32; i += 2) {
                         const float p0 = ex2_approx(fmaf(x[2 * i], mul, shift)), p1 = ex2_approx(fmaf(x[2 * i + 1], mul, shift));
                         const float p2 = ex2_approx(fmaf(x[2 * i + 2], mul, shift)), p3 = ex2_approx(fmaf(x[2 * i + 3], mul, shift));
-                        a0 += p0; a1 += p1; a2 += p2; a3 += p3;
                         const __half2 h0 = __floats2half2_rn(p0, p1), h1 = __floats2half2_rn(p2, p3);
                         pk[i] = *reinterpret_cast<const uint32_t*>(&h0);
                         pk[i + 1] = *reinterpret_cast<const uint32_t*>(&h1);
+                        // the denominator from the same rounded values that P . V takes: their rounding then cancels in the quotient
+                        sp_add2(a0, a1, pk[i]);
+                        sp_add2(a2, a3, pk[i + 1]);
                     }
                     sp_tmem_st32(st + 32 * c, pk);
                 }

@@ -82,3 +82,17 @@ def test_masks(kv, cuda_device, S, L, Hq, kind):
     else:
         m = torch.randn(2, 1, S, L, generator=g, device=cuda_device)
     check(kv, q, k, v, m.expand(2, Hq, S, L), False)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("S,L,Hq", [(70, 300, 2), (300, 512, 80)])
+def test_the_rounding_of_the_probabilities_cancels(kv, native_lib, cuda_device, dtype, S, L, Hq):
+    """Values of one everywhere: an output is the sum of the rounded probabilities over the denominator, and one again when the
+    denominator sums the same rounded values.  What is left are 32-bit sums: L / 16 steps of the tensor cores, each dropping up to
+    2^-22 of the sum, and L / 4 additions of 2^-24.  Summed before their rounding, a few large probabilities leave 1e-4."""
+    q, k, v = inputs(cuda_device, 1, Hq, Hq, S, L, dtype)
+    v = torch.ones(v.shape, device=cuda_device).to(torch.float8_e5m2).view(torch.uint8)
+    out = torch.empty(1, Hq, S, 128, device=cuda_device)
+    for scale in (128 ** -0.5, 0.3):
+        native_lib.lowbit_sdp_fp8_prefill(q, k, v, None, True, scale, out, torch.cuda.current_stream().cuda_stream)
+        assert float((out - 1).abs().max()) <= L / 16 * 2.0 ** -22 + L / 4 * 2.0 ** -24
