@@ -73,12 +73,10 @@ class LowBitExperts(nn.Module):
         return new
 
     def _address_tables(self, device):
-        """u64 device arrays of the experts' weight addresses (qwen3_moe.py:88-99), rebuilt when the weights moved"""
-        key = (device, self.gate_proj[0].weight.data.data_ptr(), self.down_proj[-1].weight.data.data_ptr())
-        if self._tables is None or self._tables[0] != key:
-            def table(mods):
-                return torch.tensor([m.weight.data.data_ptr() for m in mods], dtype=torch.int64, device=device)
-            self._tables = (key, table(self.gate_proj), table(self.up_proj), table(self.down_proj))
+        """u64 device arrays of the experts' weight addresses (qwen3_moe.py:88-99), rebuilt when any of the weights moved"""
+        addresses = [[m.weight.data_ptr() for m in mods] for mods in (self.gate_proj, self.up_proj, self.down_proj)]
+        if self._tables is None or self._tables[0] != (device, addresses):
+            self._tables = ((device, addresses), *(torch.tensor(a, dtype=torch.int64, device=device) for a in addresses))
         return self._tables[1:]
 
     def fused_one_token(self, x, top_k_index, top_k_weights, out=None, accumulate=False):

@@ -1,0 +1,93 @@
+"""``LowBitExperts`` (transformers/models/mixtral.py): which route a call takes, and that each gives what the loop over the experts'
+modules gives."""
+import pytest
+import torch
+
+E, H, I = 4, 256, 384
+
+
+class Fused(torch.nn.Module):
+    """the layout a checkpoint's experts have before conversion"""
+
+    def __init__(self, dev, seed=0, experts=E):
+        super().__init__()
+        g = torch.Generator(device=dev).manual_seed(seed)
+        draw = lambda *s: torch.nn.Parameter(torch.empty(*s, device=dev).normal_(0.0, 0.05, generator=g), requires_grad=False)      # noqa: E731
+        self.gate_up_proj, self.down_proj, self.act_fn = draw(experts, 2 * I, H), draw(experts, H, I), torch.nn.SiLU()
+
+
+def layer(dev, qtype="sym_int4", seed=0, experts=E):
+    from ipex_llm_b200.transformers.low_bit_linear import ggml_tensor_qtype
+    from ipex_llm_b200.transformers.models.mixtral import LowBitExperts
+    return LowBitExperts.from_fused(Fused(dev, seed, experts).eval(), ggml_tensor_qtype[qtype])
+
+
+def plain_layer(seed=0, experts=E):
+    """on the CPU, where the packed bytes are not needed: weights with addresses of their own"""
+    from ipex_llm_b200.transformers.low_bit_linear import FP4Params, ggml_tensor_qtype
+    from ipex_llm_b200.transformers.models.mixtral import LowBitExperts
+    with torch.device("meta"):
+        m = LowBitExperts(experts, H, I, ggml_tensor_qtype["sym_int4"], torch.nn.SiLU())
+    for mods, (n, k) in ((m.gate_proj, (I, H)), (m.up_proj, (I, H)), (m.down_proj, (H, I))):
+        for lin in mods:
+            lin._parameters["weight"] = FP4Params(torch.zeros(n * k // 64 * 34, dtype=torch.uint8), quantized=True, _shape=(n, k), qtype=lin.qtype)
+    return m.eval()
+
+
+def replace(mods, e):
+    """a re-quantised expert: other bytes at another address"""
+    from ipex_llm_b200.transformers.low_bit_linear import FP4Params
+    old = mods[e].weight
+    mods[e]._parameters["weight"] = FP4Params(old.data.flip(0).contiguous() if old.data.device.type == "cpu" else old.data.clone(), quantized=True,
+                                              _shape=old._shape, qtype=old.qtype)
+
+
+@pytest.mark.parametrize("name", ["gate_proj", "up_proj", "down_proj"])
+@pytest.mark.parametrize("e", range(E))
+def test_the_address_tables_follow_every_expert(name, e):
+    m = plain_layer()
+    m._address_tables(torch.device("cpu"))
+    replace(getattr(m, name), e)
+    for table, mods in zip(m._address_tables(torch.device("cpu")), (m.gate_proj, m.up_proj, m.down_proj)):
+        assert table.tolist() == [lin.weight.data_ptr() for lin in mods]
+
+
+def routing(dev, rows, top_k=2, seed=1, experts=E):
+    g = torch.Generator(device=dev).manual_seed(seed)
+    w, idx = torch.softmax(torch.randn(rows, experts, generator=g, device=dev), -1).topk(top_k, dim=-1)
+    return idx, w / w.sum(-1, keepdim=True)
+
+
+def loop(m, x, idx, w):
+    """the statement: every expert's modules over its rows, in 32 bits around them"""
+    out = torch.zeros(x.shape, dtype=torch.float32, device=x.device)
+    for e in range(m.num_experts):
+        r, s = torch.where(idx == e)
+        if len(r):
+            a = torch.nn.functional.silu(m.gate_proj[e](x[r]).float()) * m.up_proj[e](x[r]).float()
+            out.index_add_(0, r, m.down_proj[e](a.to(x.dtype)).float() * w[r, s, None].float())
+    return out
+
+
+# the loop rounds gate and up to the activation dtype (u each, the activation's slope below 1.13), the hidden row and the expert's
+# output on both sides: fewer than eight roundings of u = 2^-11 / 2^-8 each, taken relative to the largest |output|
+TOL = {torch.float16: 8 * 2.0 ** -11, torch.bfloat16: 8 * 2.0 ** -8}
+
+
+def same(m, x, idx, w):
+    got, want = m(x, idx, w).float(), loop(m, x, idx, w)
+    assert float((got - want).abs().max()) <= TOL[x.dtype] * float(want.abs().max())
+    return got
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows", [1, 100])
+def test_a_replaced_expert_is_the_one_that_runs(native_lib, cuda_device, rows):
+    m, other = layer(cuda_device), layer(cuda_device, seed=5)
+    x = torch.randn(rows, H, device=cuda_device).half()
+    idx, w = routing(cuda_device, rows)
+    idx[0, 0], idx[0, 1] = 2, 1
+    before = same(m, x, idx, w)
+    old = m.up_proj[2].weight                                                       # kept: its memory is not handed out again
+    m.up_proj[2]._parameters["weight"] = other.up_proj[2].weight
+    assert float((same(m, x, idx, w) - before)[0].abs().max()) > 0 and old is not m.up_proj[2].weight
