@@ -3,7 +3,7 @@
     python -m ipex_llm_b200.build_native [--force] [--verbose] [--only lowbit|mixers|host]
 
 Two kernel libraries, each from its own folder of sources, so that a model that needs one of them does not wait for the other, and
-a small CPython module (``b200_host.so``, csrc/host: the host side of one linear):
+a small CPython module (``b200_host-*.so``, csrc/host: the host side of one linear):
 ``libb200lowbit.so`` (csrc/*.cu: the low-bit linears and what surrounds them in llama-family decoders) and
 ``libb200mixers.so`` (csrc/mixers/*.cu: windowed sigmoid attention, linear recurrences, the normalisations of models built
 from them).  They land in ipex_llm_b200/libs/ (git-ignored).  nvcc cross-compiles without a GPU.  Objects are cached in
@@ -135,21 +135,28 @@ def build(force=False, verbose=False, ptxas_info=False):
 
 
 HOST_SRC = os.path.join(CSRC, "host", "linear_host.cpp")
-HOST_LIB = os.path.join(LIBDIR, "b200_host.so")
+
+
+def host_lib():
+    """the module's file: its name carries what it is bound to, so that another Python or torch builds its own"""
+    import sysconfig
+    import torch
+    return os.path.join(LIBDIR, f"b200_host-{sysconfig.get_config_var('SOABI')}-torch{torch.__version__}.so")
 
 
 def build_host(force=False, verbose=False):
-    """libs/b200_host.so: the CPython module behind LowBitLinear.forward (csrc/host).  Safe to call from several processes at once."""
+    """the CPython module behind LowBitLinear.forward (csrc/host).  Safe to call from several processes at once."""
     import sysconfig
-    if not force and os.path.exists(HOST_LIB) and os.path.getmtime(HOST_LIB) >= os.path.getmtime(HOST_SRC):
-        return HOST_LIB
+    path = host_lib()
+    if not force and os.path.exists(path) and os.path.getmtime(path) >= os.path.getmtime(HOST_SRC):
+        return path
     import torch
     from torch.utils import cpp_extension
     os.makedirs(LIBDIR, exist_ok=True)
     lib_dir = os.path.join(os.path.dirname(torch.__file__), "lib")
     cuda = os.path.join(os.path.dirname(os.path.dirname(_nvcc())), "include")
     includes = [d for d in cpp_extension.include_paths() if os.path.isdir(d)] + [cuda, sysconfig.get_paths()["include"]]
-    tmp = f"{HOST_LIB}.{os.getpid()}"
+    tmp = f"{path}.{os.getpid()}"
     cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
     cmd += [f for d in includes for f in ("-isystem", d)]
     cmd += [HOST_SRC, "-o", tmp, "-L", lib_dir, "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda", f"-Wl,-rpath,{lib_dir}"]
@@ -158,8 +165,8 @@ def build_host(force=False, verbose=False):
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError(f"g++ failed on {HOST_SRC}:\n{r.stdout}\n{r.stderr}")
-    os.replace(tmp, HOST_LIB)
-    return HOST_LIB
+    os.replace(tmp, path)
+    return path
 
 
 if __name__ == "__main__":

@@ -15,7 +15,11 @@ Differences that are the point of this build:
 """
 import ctypes
 import functools
+import importlib.machinery
+import importlib.util
 import os
+import threading
+import warnings
 from functools import reduce
 from operator import mul
 
@@ -36,21 +40,29 @@ FP8E5 = ggml_tensor_qtype["fp8_e5m2"]
 FP6 = ggml_tensor_qtype["fp6"]
 WOQ_INT4 = ggml_tensor_qtype["woq_int4"]
 
+_host = None                # the native host side of one linear; False where it cannot be had
+_host_lock = threading.Lock()
+
+
 def _load_host():
-    """the native host side of one linear (csrc/host), built on first use where it is missing, bound to the kernel library"""
-    import importlib.machinery
-    import importlib.util
-    from ipex_llm_b200 import build_native
-    path = build_native.build_host()
-    loader = importlib.machinery.ExtensionFileLoader("b200_host", path)
-    module = importlib.util.module_from_spec(importlib.util.spec_from_loader("b200_host", loader))
-    loader.exec_module(module)
-    module.attach(*(ctypes.cast(getattr(ggml._lib, f), ctypes.c_void_p).value
-                    for f in ("lowbit_matmul_cuda", "lowbit_matmul_workspace_size", "lowbit_hint_next_weights")))
-    return module.linear
+    """csrc/host, built where it is missing, bound to the kernel library.  Asked for by the first call that can use it; where it can be
+    neither built nor loaded, the Python statements behind it serve every call."""
+    global _host
+    with _host_lock:
+        if _host is None:
+            try:
+                from ipex_llm_b200 import build_native
+                loader = importlib.machinery.ExtensionFileLoader("b200_host", build_native.build_host())
+                module = importlib.util.module_from_spec(importlib.util.spec_from_loader("b200_host", loader))
+                loader.exec_module(module)
+                module.attach(*(ctypes.cast(getattr(ggml._lib, f), ctypes.c_void_p).value
+                                for f in ("lowbit_matmul_cuda", "lowbit_matmul_workspace_size", "lowbit_hint_next_weights")))
+                _host = module
+            except Exception as e:
+                warnings.warn(f"the native host side of LowBitLinear is not available, its Python statements run instead: {e}")
+                _host = False
+    return _host
 
-
-_host_linear = _load_host()
 
 _TORCH_TO_DT = {torch.float32: ggml.DT_F32, torch.float16: ggml.DT_F16, torch.bfloat16: ggml.DT_BF16}
 
@@ -600,13 +612,14 @@ class LowBitLinear(nn.Linear):
         return result
 
     def forward(self, x: torch.Tensor):
-        if not (self.training or self.optimize_lm_head or self.act_order) and self.mp_group is None:
+        if x.is_cuda and not (self.training or self.optimize_lm_head or self.act_order) and self.mp_group is None:
             # the plain case on the GPU: one native call does what the statements below do, and returns None where they are needed
+            host = _host if _host is not None else _load_host()
             params, nxt = self._parameters, self.next_linear
             weight = params["weight"]
-            if weight.quantized:
-                result = _host_linear(x, weight, params["bias"], self.out_len, self.in_len, self.qtype,
-                                      GEMV_MAX_M if self.conver_to_half else 1 << 62, None if nxt is None else nxt.weight)
+            if host and weight.quantized:
+                result = host.linear(x, weight, params["bias"], self.out_len, self.in_len, self.qtype,
+                                     GEMV_MAX_M if self.conver_to_half else 1 << 62, None if nxt is None else nxt.weight)
                 if result is not None:
                     return result if type(result) is not int else ggml._check(result, "lowbit_matmul_cuda")
         invalidInputError(not (self.training and x.requires_grad),
