@@ -17,6 +17,12 @@ MatmulFn g_matmul = nullptr;
 WorkspaceFn g_workspace = nullptr;
 HintFn g_hint = nullptr;
 
+// other threads run Python meanwhile: an allocation or a launch may have to wait for the device
+struct WithoutGil {
+    PyThreadState* const state = PyEval_SaveThread();
+    ~WithoutGil() { PyEval_RestoreThread(state); }
+};
+
 int dtype_code(c10::ScalarType t) {
     return t == at::kFloat ? 0 : t == at::kHalf ? 1 : t == at::kBFloat16 ? 2 : -1;
 }
@@ -61,20 +67,29 @@ PyObject* linear(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
         if (b.scalar_type() != x.scalar_type() || b.device() != x.device() || !b.is_contiguous() || b.numel() != n) Py_RETURN_NONE;
         bias = b.const_data_ptr();
     }
-    const c10::cuda::CUDAGuard guard(x.device());
-    auto sizes = x.sizes().vec();
-    sizes.back() = n;
-    const auto options = x.options().requires_grad(false);
-    at::Tensor y = at::empty(sizes, options), scratch;
-    const size_t need = g_workspace(n, k, rows, dt);
-    if (need) scratch = at::empty({(int64_t)need}, options.dtype(at::kByte));
+    const void* next = nullptr;
+    size_t next_bytes = 0;
     if (a[7] != Py_None && rows <= 32 && THPVariable_Check(a[7])) {
         const at::Tensor& nx = THPVariable_Unpack(a[7]);
-        if (nx.is_cuda() && nx.has_storage()) g_hint(nx.const_data_ptr(), nx.nbytes());
+        if (nx.is_cuda() && nx.has_storage()) { next = nx.const_data_ptr(); next_bytes = nx.nbytes(); }
     }
-    // a scratch of no bytes: any non-null pointer (NULL would ask the library for its own, under its lock)
-    const int rc = g_matmul(w.const_data_ptr(), qtype, n, k, xp, dt, rows, y.mutable_data_ptr(), dt, bias, 0,
-                            need ? scratch.mutable_data_ptr() : y.mutable_data_ptr(), need, c10::cuda::getCurrentCUDAStream(x.device().index()).stream());
+    at::Tensor y;
+    int rc;
+    {
+        const WithoutGil released;
+        const c10::cuda::CUDAGuard guard(x.device());
+        auto sizes = x.sizes().vec();
+        sizes.back() = n;
+        const auto options = x.options().requires_grad(false);
+        y = at::empty(sizes, options);
+        at::Tensor scratch;
+        const size_t need = g_workspace(n, k, rows, dt);
+        if (need) scratch = at::empty({(int64_t)need}, options.dtype(at::kByte));
+        if (next) g_hint(next, next_bytes);
+        // a scratch of no bytes: any non-null pointer (NULL would ask the library for its own, under its lock)
+        rc = g_matmul(w.const_data_ptr(), qtype, n, k, xp, dt, rows, y.mutable_data_ptr(), dt, bias, 0,
+                      need ? scratch.mutable_data_ptr() : y.mutable_data_ptr(), need, c10::cuda::getCurrentCUDAStream(x.device().index()).stream());
+    }
     if (rc) return PyLong_FromLong(rc);
     return THPVariable_Wrap(std::move(y));
     END_HANDLE_TH_ERRORS

@@ -3,6 +3,8 @@ import os
 import subprocess
 import sys
 import sysconfig
+import threading
+import time
 
 import pytest
 import torch
@@ -55,3 +57,32 @@ def test_both_give_the_same_bits(lbl, cuda_device, monkeypatch, rows, dtype):
         assert lbl._host
         monkeypatch.setattr(lbl, "_host", False)
         assert torch.equal(lin(x), native)
+
+
+@pytest.mark.gpu
+def test_other_threads_run_while_a_launch_waits(lbl, cuda_device):
+    """more launches than the device's queue holds, behind half a second of a busy stream: the calls wait, other threads do not"""
+    lin = lbl.LowBitLinear(128, 128, lbl.SYM_INT4, bias=False).to(cuda_device).eval()
+    x = torch.randn(1, 128, device=cuda_device).half()
+    longest, stop = [0.0], threading.Event()
+
+    def clock():
+        last = time.monotonic()
+        while not stop.is_set():
+            time.sleep(0.001)
+            now = time.monotonic()
+            longest[0], last = max(longest[0], now - last), now
+    with torch.no_grad():
+        lin(x)
+        torch.cuda.synchronize()
+        torch.cuda._sleep(1000000000)                                               # cycles
+        ticking = threading.Thread(target=clock)
+        ticking.start()
+        try:
+            for _ in range(4000):
+                lin(x)
+            torch.cuda.synchronize()
+        finally:
+            stop.set()
+            ticking.join()
+    assert longest[0] < 0.2
