@@ -1,7 +1,9 @@
 // linear_host.cpp -- the host side of one LowBitLinear.forward (reference low_bit_linear.py:638-725) in one native call:
 // checks, output, scratch, stream and launch.  In Python (tensor views, a ctypes call of fourteen arguments, the scratch lookup) the
 // same took 20 us around a 4 us kernel.  A CPython module (b200_host); the kernels are reached through the addresses of
-// libb200lowbit.so's entry points, which the package hands over once.
+// libb200lowbit.so's entry points, which the package hands over once.  Beside it, the look at a mixture's experts that every call of
+// theirs begins with (expert_addresses).
+#include <vector>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <ATen/ops/empty.h>
@@ -95,7 +97,73 @@ PyObject* linear(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     END_HANDLE_TH_ERRORS
 }
 
+// ---- the experts of a mixture: one walk over their modules for a call, however many there are
+struct Name {                                       // an interned attribute name
+    PyObject* const o;
+    explicit Name(const char* s) : o(PyUnicode_InternFromString(s)) {}
+};
+// an attribute in the instance's own dictionary, borrowed; NULL when it is not there
+PyObject* own(PyObject* dict, const Name& name) { return PyDict_GetItemWithError(dict, name.o); }
+bool is_number(PyObject* v, long want) { return v && PyLong_Check(v) && PyLong_AsLong(v) == want; }
+
+// whether nothing about `module` asks for its own forward: class, hooks, format, sizes; *address: its weight
+bool plain_linear(PyObject* module, PyObject* cls, long qtype, long in_features, long out_features, long device, int64_t* address) {
+    static const Name forward("forward"), hooks("_forward_hooks"), pre("_forward_pre_hooks"), mp("mp_group"), order("act_order"), head("optimize_lm_head"),
+        training("training"), type("qtype"), in("in_len"), out("out_len"), params("_parameters"), weight("weight"), bias("bias"), quantized("quantized");
+    if ((PyObject*)Py_TYPE(module) != cls) return false;
+    PyObject* const d = PyObject_GenericGetDict(module, nullptr);
+    if (!d) return false;
+    bool ok = false;
+    do {
+        if (own(d, forward) || own(d, mp) != Py_None || own(d, order) != Py_False || own(d, head) != Py_False || own(d, training) != Py_False) break;
+        PyObject *const fh = own(d, hooks), *const ph = own(d, pre);
+        if (!fh || !ph || PyObject_Size(fh) != 0 || PyObject_Size(ph) != 0) break;
+        if (!is_number(own(d, type), qtype) || !is_number(own(d, in), in_features) || !is_number(own(d, out), out_features)) break;
+        PyObject* const p = own(d, params);
+        if (!p || !PyDict_Check(p)) break;
+        PyObject *const w = PyDict_GetItemWithError(p, weight.o), *const b = PyDict_GetItemWithError(p, bias.o);
+        if (!w || b != Py_None || !THPVariable_Check(w)) break;
+        const at::Tensor& t = THPVariable_Unpack(w);
+        if (!t.has_storage() || !t.is_contiguous() || (device < 0 ? !t.is_cpu() : !t.is_cuda() || t.device().index() != device)) break;
+        PyObject* const q = PyObject_GetAttr(w, quantized.o);
+        Py_XDECREF(q);
+        if (q != Py_True) break;
+        *address = reinterpret_cast<int64_t>(t.const_data_ptr());
+        ok = (*address & 15) == 0;
+    } while (false);
+    Py_DECREF(d);
+    return ok;
+}
+
+// expert_addresses(class, qtype, hidden, inter, device index | -1 (CPU), gates, ups, downs: the module lists' dictionaries)
+//   -> the weights' addresses, gates first, as bytes of 64-bit numbers; None when any of the modules has to run itself
+PyObject* expert_addresses(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
+    HANDLE_TH_ERRORS
+    if (n_args != 8 || !PyDict_Check(a[5]) || !PyDict_Check(a[6]) || !PyDict_Check(a[7])) {
+        PyErr_SetString(PyExc_TypeError, "b200_host.expert_addresses takes a class, four numbers and three dictionaries");
+        return nullptr;
+    }
+    const long qtype = PyLong_AsLong(a[1]), hidden = PyLong_AsLong(a[2]), inter = PyLong_AsLong(a[3]), device = PyLong_AsLong(a[4]);
+    if (PyErr_Occurred()) return nullptr;
+    std::vector<int64_t> out;
+    for (int i = 0; i < 3; i++) {
+        PyObject *key, *module;
+        Py_ssize_t pos = 0;
+        while (PyDict_Next(a[5 + i], &pos, &key, &module)) {
+            int64_t address = 0;
+            if (!plain_linear(module, a[0], qtype, i < 2 ? hidden : inter, i < 2 ? inter : hidden, device, &address)) {
+                PyErr_Clear();
+                Py_RETURN_NONE;
+            }
+            out.push_back(address);
+        }
+    }
+    return PyBytes_FromStringAndSize(reinterpret_cast<const char*>(out.data()), (Py_ssize_t)(out.size() * sizeof(int64_t)));
+    END_HANDLE_TH_ERRORS
+}
+
 PyMethodDef methods[] = {{"attach", attach, METH_VARARGS, nullptr},
+                         {"expert_addresses", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(expert_addresses)), METH_FASTCALL, nullptr},
                          {"linear", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(linear)), METH_FASTCALL, nullptr},
                          {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "b200_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};

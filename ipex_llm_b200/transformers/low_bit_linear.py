@@ -13,6 +13,7 @@ Differences that are the point of this build:
   * a quantised ``FP4Params`` ignores dtype casts (LBL only guards torch_fp8, :443-444): the
     nf4 buffer is bf16-typed (LBL:139-145) and ``model.to(torch.float16)`` must not touch it.
 """
+import array
 import ctypes
 import functools
 import importlib.machinery
@@ -393,6 +394,35 @@ def moe_forward_vec(x: torch.Tensor, topk_ids: torch.Tensor, topk_weight: torch.
                              hidden, inter, qtype, act, ctypes.c_void_p(out.data_ptr()), _TORCH_TO_DT[out.dtype],
                              accumulate, ctypes.c_void_p(ws.data_ptr()), ws.numel(), _stream_ptr(dev))
     return out
+
+
+def _expert_addresses(cls, qtype, hidden, inter, device, gates, ups, downs):
+    """what csrc/host's expert_addresses does, where that cannot be had"""
+    out = array.array("q")
+    for mods, k, n in ((gates, hidden, inter), (ups, hidden, inter), (downs, inter, hidden)):
+        for m in mods.values():
+            d = m.__dict__
+            if (type(m) is not cls or "forward" in d or d["_forward_hooks"] or d["_forward_pre_hooks"] or d["mp_group"] is not None or d["act_order"]
+                    or d["optimize_lm_head"] or d["training"] or (d["qtype"], d["in_len"], d["out_len"]) != (qtype, k, n)):
+                return None
+            w, bias = (d["_parameters"].get(name, False) for name in ("weight", "bias"))
+            if (bias is not None or getattr(w, "quantized", None) is not True or not w.is_contiguous()
+                    or (-1 if w.device.type == "cpu" else w.device.index) != device or w.data_ptr() % 16):
+                return None
+            out.append(w.data_ptr())
+    return out.tobytes()
+
+
+def expert_addresses(qtype: int, hidden: int, inter: int, device: torch.device, gates, ups, downs):
+    """The weight addresses of a mixture's experts (three ModuleLists), gates first, as the bytes of 64-bit numbers; None when any of
+    them is not a plain LowBitLinear of this format and these sizes on ``device`` -- another class, a hook, a bias, a tensor-parallel
+    group -- and so has to run itself.  Looked at anew for every call: 24 modules 7 us, 384 modules 78 us
+    (in Python 40 and 585)."""
+    if nn.modules.module._has_any_global_hook():
+        return None
+    host = _host if _host is not None else _load_host()
+    look = host.expert_addresses if host else _expert_addresses
+    return look(LowBitLinear, qtype, hidden, inter, -1 if device.type == "cpu" else device.index, gates._modules, ups._modules, downs._modules)
 
 
 def moe_tokens_supported(x: torch.Tensor, n_experts: int, hidden: int, inter: int, top_k: int, qtype: int) -> bool:

@@ -10,10 +10,12 @@ the experts' weight addresses behind the ``use_fuse_moe`` gate; more tokens in h
 same tables (sorted on the device, one launch per projection over all experts); anything else -> per-expert ``LowBitLinear``
 calls over the tokens routed to each expert.  Attention, RMSNorm and the model forward are the Mistral ones.
 """
+import array
+
 import torch
 from torch import nn
 
-from ipex_llm_b200.transformers.low_bit_linear import moe_forward_tokens, moe_tokens_supported
+from ipex_llm_b200.transformers.low_bit_linear import expert_addresses, moe_forward_tokens, moe_tokens_supported
 from ipex_llm_b200.transformers.models.common import merge_qkv_base
 from ipex_llm_b200.transformers.models.llama import decoder_model_forward, decoder_attention_forward
 from ipex_llm_b200.transformers.models.utils import use_fuse_moe
@@ -72,36 +74,43 @@ class LowBitExperts(nn.Module):
             new.eval()
         return new
 
-    def _address_tables(self, device):
-        """u64 device arrays of the experts' weight addresses (qwen3_moe.py:88-99), rebuilt when any of the weights moved"""
-        addresses = [[m.weight.data_ptr() for m in mods] for mods in (self.gate_proj, self.up_proj, self.down_proj)]
-        if self._tables is None or self._tables[0] != (device, addresses):
-            self._tables = ((device, addresses), *(torch.tensor(a, dtype=torch.int64, device=device) for a in addresses))
-        return self._tables[1:]
+    def _address_tables(self, device, addresses=None):
+        """u64 device arrays of the experts' weight addresses (qwen3_moe.py:88-99), rebuilt when any of the weights moved.  ``addresses``:
+        what expert_addresses has just said of them"""
+        if addresses is None:
+            addresses = array.array("q", [m.weight.data_ptr() for mods in (self.gate_proj, self.up_proj, self.down_proj) for m in mods]).tobytes()
+        tables = self._tables
+        if tables is None or tables[0] != (device, addresses):
+            tables = self._tables = ((device, addresses), *torch.frombuffer(bytearray(addresses), dtype=torch.int64).to(device).chunk(3))
+        return tables[1:]
 
     def fused_one_token(self, x, top_k_index, top_k_weights, out=None, accumulate=False):
         from ipex_llm_b200.transformers.low_bit_linear import moe_forward_vec
-        gates, ups, downs = self._address_tables(x.device)
+        gates, ups, downs = self._address_tables(x.device, self._plain_addresses(x.device))
         return moe_forward_vec(x, top_k_index, top_k_weights, gates, ups, downs, self.hidden_dim, self.intermediate_dim,
                                self.qtype, out=out, accumulate=accumulate)
 
+    def _plain_addresses(self, device):
+        if not len(self.gate_proj) == len(self.up_proj) == len(self.down_proj) == self.num_experts:
+            return None
+        return expert_addresses(self.qtype, self.hidden_dim, self.intermediate_dim, device, self.gate_proj, self.up_proj, self.down_proj)
+
     def _many_tokens_ok(self, x, top_k_index, top_k_weights):
-        mods = [m for ms in (self.gate_proj, self.up_proj, self.down_proj) for m in ms]
         return (x.dim() == 2 and x.shape[0] > 0 and type(self.act_fn).__name__ in ("SiLU", "SiLUActivation") and not self.training
                 and not (torch.is_grad_enabled() and (x.requires_grad or top_k_weights.requires_grad))
                 and top_k_index.dim() == 2 and top_k_index.shape == top_k_weights.shape and top_k_index.dtype in (torch.int32, torch.int64)
                 and top_k_weights.dtype in (torch.float32, torch.float16, torch.bfloat16)
-                and moe_tokens_supported(x, self.num_experts, self.hidden_dim, self.intermediate_dim, top_k_index.shape[1], self.qtype)
-                and all(m.weight.data.device == x.device and m.weight.data.data_ptr() % 16 == 0 and m.bias is None and m.mp_group is None
-                        and not m.act_order and m.weight.quantized for m in mods))
+                and moe_tokens_supported(x, self.num_experts, self.hidden_dim, self.intermediate_dim, top_k_index.shape[1], self.qtype))
 
     def forward(self, hidden_states, top_k_index, top_k_weights):
         if hidden_states.shape[0] == 1 and use_fuse_moe(hidden_states, self.qtype) and \
                 self.gate_proj[0].weight.data.device.type == "cuda" and not self.training:
             return self.fused_one_token(hidden_states, top_k_index, top_k_weights)
         if self._many_tokens_ok(hidden_states, top_k_index, top_k_weights):
-            return moe_forward_tokens(hidden_states, top_k_index, top_k_weights, *self._address_tables(hidden_states.device), self.hidden_dim,
-                                      self.intermediate_dim, self.qtype)
+            addresses = self._plain_addresses(hidden_states.device)         # None: an expert that has to run itself
+            if addresses is not None:
+                return moe_forward_tokens(hidden_states, top_k_index, top_k_weights, *self._address_tables(hidden_states.device, addresses),
+                                          self.hidden_dim, self.intermediate_dim, self.qtype)
         final = torch.zeros_like(hidden_states)
         expert_mask = torch.nn.functional.one_hot(top_k_index, num_classes=self.num_experts).permute(2, 1, 0)
         for e in torch.greater(expert_mask.sum(dim=(-1, -2)), 0).nonzero()[:, 0].tolist():

@@ -91,3 +91,104 @@ def test_a_replaced_expert_is_the_one_that_runs(native_lib, cuda_device, rows):
     old = m.up_proj[2].weight                                                       # kept: its memory is not handed out again
     m.up_proj[2]._parameters["weight"] = other.up_proj[2].weight
     assert float((same(m, x, idx, w) - before)[0].abs().max()) > 0 and old is not m.up_proj[2].weight
+
+
+class Wrapper(torch.nn.Module):
+    """an expert that scales what a linear gives, and passes its attributes through"""
+
+    def __init__(self, inner):
+        super().__init__()
+        self.inner = inner
+
+    def __getattr__(self, name):
+        try:
+            return super().__getattr__(name)
+        except AttributeError:
+            return getattr(super().__getattr__("inner"), name)
+
+    def forward(self, x):
+        return 2 * self.inner(x)
+
+
+def odd_linear(lin):
+    new = torch.nn.Linear(lin.in_len, lin.out_len, bias=False, dtype=torch.float16)
+    return new.requires_grad_(False)
+
+
+def hooked(lin):
+    lin.register_forward_hook(lambda mod, args, out: 3 * out)
+    return lin
+
+
+def pre_hooked(lin):
+    lin.register_forward_pre_hook(lambda mod, args: (0.5 * args[0],))
+    return lin
+
+
+def own_forward(lin):
+    plain = lin.forward
+    lin.forward = lambda x: -plain(x)
+    return lin
+
+
+def with_bias(lin):
+    lin._parameters["bias"] = torch.nn.Parameter(torch.ones(lin.out_len, dtype=torch.float16, device=lin.weight.device), requires_grad=False)
+    return lin
+
+
+def subclass(lin):
+    class Another(type(lin)):
+        def forward(self, x):
+            return 4 * super().forward(x)
+    lin.__class__ = Another
+    return lin
+
+
+ODD = [odd_linear, Wrapper, hooked, pre_hooked, own_forward, with_bias, subclass]
+
+
+@pytest.mark.parametrize("native", [True, False])
+def test_only_plain_experts_are_read_by_their_addresses(monkeypatch, native):
+    from ipex_llm_b200.transformers import low_bit_linear as lbl
+    if not native:
+        monkeypatch.setattr(lbl, "_host", False)
+    cpu = torch.device("cpu")
+    m = plain_layer()
+    want = [lin.weight.data_ptr() for mods in (m.gate_proj, m.up_proj, m.down_proj) for lin in mods]
+    assert torch.frombuffer(bytearray(m._plain_addresses(cpu)), dtype=torch.int64).tolist() == want and (not native or lbl._host)
+    odd = list(ODD) + [lambda lin: setattr(lin, "qtype", lbl.NF4) or lin, lambda lin: setattr(lin, "act_order", True) or lin, lambda lin: lin.train(),
+                       lambda lin: setattr(lin, "mp_group", object()) or lin, lambda lin: setattr(lin.weight, "quantized", False) or lin,
+                       lambda lin: setattr(lin, "in_len", lin.in_len + 64) or lin, lambda lin: lin._parameters.pop("weight") is None or lin]
+    for i, change in enumerate(odd):
+        m = plain_layer()
+        mods = (m.gate_proj, m.up_proj, m.down_proj)[i % 3]
+        mods[i % E] = change(mods[i % E])
+        assert m._plain_addresses(cpu) is None, i
+    m = plain_layer()
+    m.up_proj = m.up_proj[:3]
+    assert m._plain_addresses(cpu) is None
+    hook = torch.nn.modules.module.register_module_forward_hook(lambda *a: None)
+    try:
+        assert plain_layer()._plain_addresses(cpu) is None
+    finally:
+        hook.remove()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("change", ODD)
+@pytest.mark.parametrize("name,e", [("gate_proj", 0), ("up_proj", 2), ("down_proj", 3)])
+def test_an_expert_that_is_not_plain_runs_itself(native_lib, cuda_device, change, name, e):
+    m = layer(cuda_device)
+    mods = getattr(m, name)
+    mods[e] = change(mods[e]).to(cuda_device)
+    x = torch.randn(90, H, device=cuda_device).half()
+    idx, w = routing(cuda_device, 90)
+    idx[:, 0] = torch.where(idx[:, 1] == e, (e + 1) % E, e)
+    same(m, x, idx, w)
+
+
+@pytest.mark.gpu
+def test_an_expert_of_another_format_runs_itself(native_lib, cuda_device):
+    m = layer(cuda_device)
+    m.up_proj[1] = layer(cuda_device, "fp8_e4m3", seed=7).up_proj[1]
+    same(m, torch.randn(90, H, device=cuda_device).half(), *routing(cuda_device, 90))
