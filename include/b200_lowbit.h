@@ -332,12 +332,14 @@ int lowbit_moe_cuda(const void* d_x, int x_dtype, const void* d_topk_ids, int id
                     void* d_y, int y_dtype, int accumulate,
                     void* workspace, size_t workspace_bytes, void* stream);
 
-/* The same for many tokens -- the expert loop of transformers/models/qwen3_moe.py:106-132 and deepseek.py:313-330 as five launches
- * without a host synchronisation: y[t] = sum_z weight[t][z] * Wdown[e] . (act(Wgate[e] . x[t]) * (Wup[e] . x[t])), e = ids[t][z],
- * summed in 32 bits in choice order.  x, y [n_tokens][hidden] fp16 or bf16 (one dtype); ids, weights [n_tokens][top_k]; an id
- * outside [0, n_experts) contributes zero.  hidden and inter multiples of 128, at most 256 experts, weights 16-byte aligned.
- * Precision: the prompt matmul's (weights rounded once to the activation dtype); the hidden rows and the experts' outputs are
- * rounded to the activation dtype.  workspace: lowbit_moe_tokens_workspace_size() bytes, 256-byte aligned. */
+/* The same for many tokens -- the expert loop of transformers/models/qwen3_moe.py:106-132 and deepseek.py:313-330:
+ * y[t] = sum_z weight[t][z] * Wdown[e] . (act(Wgate[e] . x[t]) * (Wup[e] . x[t])), e = ids[t][z], summed in 32 bits in choice order.
+ * x, y [n_tokens][hidden] fp16 or bf16 (one dtype); ids, weights [n_tokens][top_k]; an id outside [0, n_experts) contributes zero.
+ * hidden and inter multiples of 128, at most 256 experts, weights 16-byte aligned.  Sorted on the device; the host waits for the row
+ * counts while the large products run, so a stream under capture is refused.
+ * Precision, expert by expert, that of lowbit_matmul_cuda at its number of rows: up to 16 the weights are exact, above they are rounded
+ * once to the activation dtype; the hidden rows and the experts' outputs are rounded to the activation dtype.
+ * workspace: lowbit_moe_tokens_workspace_size() bytes, 256-byte aligned. */
 int lowbit_moe_tokens_supported(int qtype, int64_t hidden, int64_t inter, int n_experts, int top_k);
 size_t lowbit_moe_tokens_workspace_size(int64_t hidden, int64_t inter, int n_experts, int64_t n_tokens, int top_k);
 int lowbit_moe_tokens_cuda(const void* d_x, int x_dtype, int64_t n_tokens, const void* d_topk_ids, int ids_dtype,

@@ -180,7 +180,7 @@ static bool use_exact(int qtype, int64_t n_rows, int64_t k, int64_t m, int x_dty
 // up to 64 (the split-K prefill kernel: 22-25 us), 29 us at 96-128 -- hence the window 17..64.
 // LOWBIT_SKINNY_MIN_M / LOWBIT_SKINNY_MAX_M (development) move the window; MIN_M above MAX_M switches the kernel off.
 static bool use_skinny(int qtype, int64_t n_rows, int64_t k, int64_t m, int x_dtype) {
-    static const int64_t min_m = [] { const char* e = getenv("LOWBIT_SKINNY_MIN_M"); return e ? (int64_t)atoi(e) : (int64_t)17; }();
+    static const int64_t min_m = [] { const char* e = getenv("LOWBIT_SKINNY_MIN_M"); return e ? (int64_t)atoi(e) : kExactRows + 1; }();
     static const int64_t max_m = [] { const char* e = getenv("LOWBIT_SKINNY_MAX_M"); return e ? (int64_t)atoi(e) : (int64_t)64; }();
     return m >= min_m && m <= max_m && gemm_skinny_supported(qtype, n_rows, k, m, x_dtype);
 }
@@ -370,7 +370,7 @@ int lowbit_moe_tokens_cuda(const void* d_x, int x_dtype, int64_t n_tokens, const
     P.qtype = qtype; P.act = act + 1; P.y = d_y; P.y_dtype = x_dtype;
     P.workspace = workspace; P.workspace_bytes = workspace_bytes;
     const int rc = experts_launch(P, n_tokens, (cudaStream_t)stream);
-    if (rc == LB_ERR_ARG) set_error(rc, "lowbit_moe_tokens_cuda: bad argument (dtype codes or alignment)");
+    if (rc == LB_ERR_ARG) set_error(rc, "lowbit_moe_tokens_cuda: bad argument (dtype codes or alignment), or the stream is being captured");
     if (rc == LB_ERR_WORKSPACE) set_error(rc, "lowbit_moe_tokens_cuda: workspace too small (%zu bytes)", workspace_bytes);
     return rc;
 }

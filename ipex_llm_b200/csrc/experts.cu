@@ -1,11 +1,13 @@
 // experts.cu -- the routed feed-forwards of many tokens (reference models/qwen3_moe.py:106-132, deepseek.py:313-330: a loop over the
-// experts, each a handful of operators on its tokens' rows).  Five launches, no host synchronisation:
+// experts, each a handful of operators on its tokens' rows):
 //   sort      the (token, choice) pairs by expert: counts, row offsets, a row per pair (one block, shared-memory counters);
 //   gather    the tokens' activations into sorted rows;
 //   act(gate) * up of every expert's rows, then down, both by the two-SM matmul kernel over all experts at once (gemm_pair.cu);
+//             experts of at most kExactRows rows by the GEMV, two launches each, whose weights stay code x scale in 32 bits;
 //   combine   y[token] = sum over its choices, in choice order, of weight * row, in 32 bits, rounded once.
+// The host learns the counts while the two large products run: it waits for the sort only.
 // The loop it replaces was bound by its launches, 30 per expert with two host synchronisations: 1.89 ms for 512 tokens, two of eight
-// experts of 4096 x 14336, of which the matmuls were 0.9; these five take 0.49 ms.
+// experts of 4096 x 14336, of which the matmuls were 0.9; so 0.49 ms.
 #include "lowbit_common.cuh"
 #include "lowbit_internal.h"
 
@@ -14,8 +16,18 @@ namespace lowbit {
 namespace {
 constexpr int kSortThreads = 1024, kSortExperts = 256;
 
+// what the host reads: row offsets, then the three address tables
+struct HostView {
+    int offs[kSortExperts + 2];
+    unsigned long long tab[3][kSortExperts];
+};
+
 __global__ void __launch_bounds__(kSortThreads) experts_sort_kernel(const void* __restrict__ ids, int ids_i64, int pairs, int top_k, int n_experts,
-                                                                    int* __restrict__ offs, int* __restrict__ row_of, int* __restrict__ token_of) {
+                                                                    const unsigned long long* __restrict__ gates, const unsigned long long* __restrict__ ups,
+                                                                    const unsigned long long* __restrict__ downs, HostView* __restrict__ view,
+                                                                    int* __restrict__ row_of, int* __restrict__ token_of) {
+    int* const offs = view->offs;
+    for (int e = threadIdx.x; e < n_experts; e += kSortThreads) { view->tab[0][e] = gates[e]; view->tab[1][e] = ups[e]; view->tab[2][e] = downs[e]; }
     __shared__ int count[kSortExperts], next[kSortExperts];
     for (int e = threadIdx.x; e < kSortExperts; e += kSortThreads) count[e] = 0;
     __syncthreads();
@@ -87,12 +99,12 @@ __global__ void __launch_bounds__(256) experts_combine_kernel(const uint4* __res
     }
 }
 
-struct ExpertsScratch { size_t offs, row_of, token_of, x, h, out, total; };
-ExpertsScratch experts_scratch(int64_t hidden, int64_t inter, int n_experts, int64_t pairs) {
+struct ExpertsScratch { size_t view, row_of, token_of, x, h, out, total; };
+ExpertsScratch experts_scratch(int64_t hidden, int64_t inter, int64_t pairs) {
     auto up = [](size_t b) { return (b + 255) / 256 * 256; };
     ExpertsScratch S;
     size_t at = 0;
-    S.offs = at; at += up((size_t)(n_experts + 1) * 4);
+    S.view = at; at += up(sizeof(HostView));
     S.row_of = at; at += up((size_t)pairs * 4);
     S.token_of = at; at += up((size_t)pairs * 4);
     S.x = at; at += up((size_t)pairs * hidden * 2);
@@ -101,32 +113,77 @@ ExpertsScratch experts_scratch(int64_t hidden, int64_t inter, int n_experts, int
     S.total = at;
     return S;
 }
+// page-locked memory for one call's view, the calling thread's own (a call waits for the copy before it returns)
+struct PinnedView {
+    HostView* p = nullptr;
+    HostView* get() {
+        if (!p && cudaHostAlloc(&p, sizeof(HostView), cudaHostAllocPortable) != cudaSuccess) { cudaGetLastError(); p = nullptr; }
+        return p;
+    }
+    ~PinnedView() { if (p) cudaFreeHost(p); }
+};
+thread_local PinnedView t_view;
+
+// the experts of few rows, whatever their number: weights exact
+int experts_of_few_rows(const MoeParams& P, const HostView& V, char* x, char* h, char* out, cudaStream_t st) {
+    for (int e = 0; e < P.n_experts; e++) {
+        const int64_t lo = V.offs[e], n = V.offs[e + 1] - lo;
+        if (n < 1 || n > kExactRows) continue;
+        int rc = gemv_launch_ex((const void*)V.tab[0][e], (const void*)V.tab[1][e], P.act, P.qtype, P.inter, P.hidden, x + lo * P.hidden * 2, P.x_dtype, n,
+                                h + lo * P.inter * 2, P.x_dtype, nullptr, 0, nullptr, 0, st);
+        if (!rc) rc = gemv_launch((const void*)V.tab[2][e], P.qtype, P.hidden, P.inter, h + lo * P.inter * 2, P.x_dtype, n, out + lo * P.hidden * 2, P.x_dtype,
+                                  nullptr, 0, nullptr, 0, st);
+        if (rc) return rc;
+    }
+    return LB_OK;
+}
 }  // namespace
 
 bool experts_supported(int qt, int64_t hidden, int64_t inter, int n_experts, int top_k) {
     return gemm_tc_supported(qt, inter, hidden) && gemm_tc_supported(qt, hidden, inter) && n_experts >= 1 && n_experts <= kSortExperts && top_k >= 1;
 }
 size_t experts_workspace_size(int64_t hidden, int64_t inter, int n_experts, int64_t n_tokens, int top_k) {
-    return experts_scratch(hidden, inter, n_experts, n_tokens * top_k).total;
+    (void)n_experts;
+    return experts_scratch(hidden, inter, n_tokens * top_k).total;
 }
 int experts_launch(const MoeParams& P, int64_t n_tokens, cudaStream_t st) {
     const int64_t pairs = n_tokens * P.top_k;
     if (!experts_supported(P.qtype, P.hidden, P.inter, P.n_experts, P.top_k) || pairs > 0x3fffffff || P.accumulate) return LB_ERR_ARG;
     if ((P.x_dtype != DT_F16 && P.x_dtype != DT_BF16) || P.y_dtype != P.x_dtype) return LB_ERR_ARG;
     if (((uintptr_t)P.x & 15) || ((uintptr_t)P.y & 15) || ((uintptr_t)P.workspace & 255)) return LB_ERR_ARG;
-    const ExpertsScratch S = experts_scratch(P.hidden, P.inter, P.n_experts, pairs);
+    const ExpertsScratch S = experts_scratch(P.hidden, P.inter, pairs);
     if (!P.workspace || P.workspace_bytes < S.total) return LB_ERR_WORKSPACE;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone) { cudaGetLastError(); return LB_ERR_ARG; }
+    HostView* const host = t_view.get();
+    cudaEvent_t sorted = nullptr;
+    if (!host || cudaEventCreateWithFlags(&sorted, cudaEventDisableTiming) != cudaSuccess) {
+        cudaGetLastError();
+        set_error(LB_ERR_CUDA, "lowbit_moe_tokens_cuda: no page-locked memory or event for the row counts");
+        return LB_ERR_CUDA;
+    }
     char* ws = (char*)P.workspace;
-    int *offs = (int*)(ws + S.offs), *row_of = (int*)(ws + S.row_of), *token_of = (int*)(ws + S.token_of);
+    HostView* const view = (HostView*)(ws + S.view);
+    int *row_of = (int*)(ws + S.row_of), *token_of = (int*)(ws + S.token_of);
+    char *x = ws + S.x, *h = ws + S.h, *out = ws + S.out;
     const int vec = (int)(P.hidden / 8);
-    experts_sort_kernel<<<1, kSortThreads, 0, st>>>(P.ids, P.ids_i64, (int)pairs, P.top_k, P.n_experts, offs, row_of, token_of);
-    experts_gather_kernel<<<(unsigned)pairs, 256, 0, st>>>((const uint4*)P.x, (uint4*)(ws + S.x), token_of, offs + P.n_experts, vec);
+    experts_sort_kernel<<<1, kSortThreads, 0, st>>>(P.ids, P.ids_i64, (int)pairs, P.top_k, P.n_experts, P.gates, P.ups, P.downs, view, row_of, token_of);
+    cudaMemcpyAsync(host, view, sizeof(HostView), cudaMemcpyDeviceToHost, st);
+    cudaEventRecord(sorted, st);
+    experts_gather_kernel<<<(unsigned)pairs, 256, 0, st>>>((const uint4*)P.x, (uint4*)x, token_of, view->offs + P.n_experts, vec);
     note_launch(); note_launch();
-    int rc = gemm_tc_experts_launch(P.gates, P.ups, P.act, offs, P.n_experts, P.qtype, P.inter, P.hidden, ws + S.x, P.x_dtype, pairs, ws + S.h, P.x_dtype, st);
-    if (!rc) rc = gemm_tc_experts_launch(P.downs, nullptr, 0, offs, P.n_experts, P.qtype, P.hidden, P.inter, ws + S.h, P.x_dtype, pairs, ws + S.out, P.x_dtype, st);
+    int rc = LB_OK;
+    if (pairs > kExactRows) {
+        rc = gemm_tc_experts_launch(P.gates, P.ups, P.act, view->offs, P.n_experts, P.qtype, P.inter, P.hidden, x, P.x_dtype, pairs, h, P.x_dtype, st);
+        if (!rc) rc = gemm_tc_experts_launch(P.downs, nullptr, 0, view->offs, P.n_experts, P.qtype, P.hidden, P.inter, h, P.x_dtype, pairs, out, P.x_dtype, st);
+    }
+    const cudaError_t waited = cudaEventSynchronize(sorted);
+    cudaEventDestroy(sorted);
     if (rc) return rc;
-    if (P.x_dtype == DT_BF16) experts_combine_kernel<true><<<(unsigned)n_tokens, 256, 0, st>>>((const uint4*)(ws + S.out), row_of, P.weights, P.w_dtype, P.top_k, (uint4*)P.y, vec);
-    else experts_combine_kernel<false><<<(unsigned)n_tokens, 256, 0, st>>>((const uint4*)(ws + S.out), row_of, P.weights, P.w_dtype, P.top_k, (uint4*)P.y, vec);
+    if (waited != cudaSuccess) { set_error(LB_ERR_CUDA, "CUDA error: %s", cudaGetErrorString(waited)); cudaGetLastError(); return LB_ERR_CUDA; }
+    if ((rc = experts_of_few_rows(P, *host, x, h, out, st))) return rc;
+    if (P.x_dtype == DT_BF16) experts_combine_kernel<true><<<(unsigned)n_tokens, 256, 0, st>>>((const uint4*)out, row_of, P.weights, P.w_dtype, P.top_k, (uint4*)P.y, vec);
+    else experts_combine_kernel<false><<<(unsigned)n_tokens, 256, 0, st>>>((const uint4*)out, row_of, P.weights, P.w_dtype, P.top_k, (uint4*)P.y, vec);
     note_launch();
     return check_launch();
 }

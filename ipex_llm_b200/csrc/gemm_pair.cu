@@ -118,8 +118,8 @@ pair_kernel(const __grid_constant__ CUtensorMap xmap, const PairArgs A) {
         for (int b = 0; b < 2; b++) { mbar_init(tmem_full(b), 1); mbar_init(tmem_empty(b), 8); }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    // an expert's rows in tiles of at most 256 tokens, evenly cut
-    auto tiles_of = [](int rows) { return (rows + kPairTok - 1) / kPairTok; };
+    // an expert's rows in tiles of at most 256 tokens, evenly cut; few rows are another kernel's
+    auto tiles_of = [](int rows) { return rows > (int)kExactRows ? (rows + kPairTok - 1) / kPairTok : 0; };
     if (warp == 2 && A.offs) {
         int before = 0;
         for (int e0 = 0; e0 < A.n_experts; e0 += 32) {
@@ -606,7 +606,8 @@ size_t gemm_tc_mlp_workspace_size(int64_t n_rows, int64_t k, int64_t m) {
 }
 
 // the same kernel over every expert's rows: x [rows][k] sorted by expert, offs [n_experts + 1] row offsets on the device, tab /
-// tab2 device addresses of the experts' weights (tab2: the up projections, act in the epilogue; or NULL)
+// tab2 device addresses of the experts' weights (tab2: the up projections, act in the epilogue; or NULL).  Experts of at most
+// kExactRows rows are left out
 int gemm_tc_experts_launch(const unsigned long long* tab, const unsigned long long* tab2, int act, const int* offs, int n_experts, int qt,
                            int64_t n_rows, int64_t k, const void* x, int x_dtype, int64_t rows, void* y, int y_dtype, cudaStream_t st) {
     using namespace gemmtc;

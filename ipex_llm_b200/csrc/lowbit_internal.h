@@ -73,6 +73,10 @@ bool moe_supported(int qt, int64_t hidden, int64_t inter, int top_k);
 size_t moe_workspace_size(int64_t hidden, int64_t inter, int top_k, int x_dtype);
 int moe_launch(const MoeParams& P, cudaStream_t st);
 
+// up to this many half-precision rows a product keeps the weights as code x scale in 32 bits (the GEMV); above, the tensor cores take them
+// rounded once to the activation dtype.  Measured line: see use_skinny in capi.cu
+constexpr int64_t kExactRows = 16;
+
 // many-token mixture-of-experts (experts.cu): MoeParams with x / y [n_tokens][hidden], ids / weights [n_tokens][top_k]
 bool experts_supported(int qt, int64_t hidden, int64_t inter, int n_experts, int top_k);
 size_t experts_workspace_size(int64_t hidden, int64_t inter, int n_experts, int64_t n_tokens, int top_k);

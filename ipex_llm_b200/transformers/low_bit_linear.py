@@ -435,7 +435,8 @@ def moe_forward_tokens(x: torch.Tensor, topk_ids: torch.Tensor, topk_weight: tor
                        downs: torch.Tensor, hidden: int, inter: int, qtype: int, act: int = SILU):
     """The routed experts' MLPs of many tokens (the expert loop of models/qwen3_moe.py:106-132): x [T, hidden] fp16 / bf16,
     ``topk_ids`` / ``topk_weight`` [T, top_k] and the address tables as in ``moe_forward_vec``; the pairs are sorted by expert on
-    the device, every expert's rows run in one launch per projection.  Returns [T, hidden] in x's dtype."""
+    the device, the experts' rows run in one launch per projection, those of experts with at most 16 rows on the GEMV (exact
+    weights).  Waits for the row counts: not under capture.  Returns [T, hidden] in x's dtype."""
     T, top_k = topk_ids.shape
     invalidInputError(x.dim() == 2 and tuple(x.shape) == (T, hidden), f"activation shape {tuple(x.shape)} != ({T}, {hidden})")
     invalidInputError(x.dtype in (torch.float16, torch.bfloat16), f"unsupported activation dtype {x.dtype}")

@@ -7,7 +7,7 @@ decode path takes the weight addresses from), quantised exactly like any other l
 reference's MoE block forwards (/root/reference/python/llm/src/ipex_llm/transformers/models/qwen3_moe.py:70-132,
 deepseek.py:280-330; the fork has no Mixtral forward of its own): one token -> ``moe_forward_vec`` over device tables of
 the experts' weight addresses behind the ``use_fuse_moe`` gate; more tokens in half precision -> ``moe_forward_tokens`` over the
-same tables (sorted on the device, one launch per projection over all experts); anything else -> per-expert ``LowBitLinear``
+same tables (sorted on the device, one launch per projection over the experts of many rows); anything else -> per-expert ``LowBitLinear``
 calls over the tokens routed to each expert.  Attention, RMSNorm and the model forward are the Mistral ones.
 """
 import array
@@ -100,7 +100,8 @@ class LowBitExperts(nn.Module):
                 and not (torch.is_grad_enabled() and (x.requires_grad or top_k_weights.requires_grad))
                 and top_k_index.dim() == 2 and top_k_index.shape == top_k_weights.shape and top_k_index.dtype in (torch.int32, torch.int64)
                 and top_k_weights.dtype in (torch.float32, torch.float16, torch.bfloat16)
-                and moe_tokens_supported(x, self.num_experts, self.hidden_dim, self.intermediate_dim, top_k_index.shape[1], self.qtype))
+                and moe_tokens_supported(x, self.num_experts, self.hidden_dim, self.intermediate_dim, top_k_index.shape[1], self.qtype)
+                and not torch.cuda.is_current_stream_capturing())
 
     def forward(self, hidden_states, top_k_index, top_k_weights):
         if hidden_states.shape[0] == 1 and use_fuse_moe(hidden_states, self.qtype) and \

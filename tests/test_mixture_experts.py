@@ -1,5 +1,7 @@
 """``LowBitExperts`` (transformers/models/mixtral.py): which route a call takes, and that each gives what the loop over the experts'
 modules gives."""
+import threading
+
 import pytest
 import torch
 
@@ -192,3 +194,44 @@ def test_an_expert_of_another_format_runs_itself(native_lib, cuda_device):
     m = layer(cuda_device)
     m.up_proj[1] = layer(cuda_device, "fp8_e4m3", seed=7).up_proj[1]
     same(m, torch.randn(90, H, device=cuda_device).half(), *routing(cuda_device, 90))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("qtype", ["sym_int4", "asym_int4", "nf4", "fp8_e4m3", "fp8_e5m2", "fp6"])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("rows", [(0, 1, 8, 9, 16, 17, 300, 2), (3, 16, 0, 0, 1, 5, 0, 7), (17, 33, 64, 65, 256, 257, 40, 18)])
+def test_few_rows_keep_exact_weights(native_lib, cuda_device, qtype, dtype, rows):
+    """up to 16 rows an expert's products are the GEMV's, bit for bit: weights as code x scale, not rounded to the activation dtype"""
+    from ipex_llm_b200.transformers import low_bit_linear as lbl
+    m = layer(cuda_device, qtype, experts=len(rows))
+    idx = torch.cat([torch.full((n, 1), e, device=cuda_device) for e, n in enumerate(rows)])
+    idx = idx[torch.randperm(len(idx), device=cuda_device)]
+    x = torch.randn(len(idx), H, device=cuda_device).to(dtype)
+    got = same(m, x, idx, torch.ones(len(idx), 1, device=cuda_device))
+    for e, n in enumerate(rows):
+        if 1 <= n <= 16:
+            r = torch.where(idx[:, 0] == e)[0]
+            h = lbl.mlp_forward(x[r], m.gate_proj[e].weight.data, m.up_proj[e].weight.data, n, H, I, lbl.SILU, m.qtype)
+            assert torch.equal(got[r].to(dtype), lbl.lowbit_matmul(h, m.down_proj[e].weight.data, (H, I), m.qtype))
+
+
+@pytest.mark.gpu
+def test_few_rows_from_several_threads_and_streams(native_lib, cuda_device):
+    """the row counts that the host waits for are each call's own"""
+    m = layer(cuda_device, experts=8)
+    calls = [(torch.randn(rows, H, device=cuda_device).half(), *routing(cuda_device, rows, seed=rows, experts=8)) for rows in (5, 40, 90, 200)]
+    want = [m(*c) for c in calls]
+    torch.cuda.synchronize()
+    wrong = []
+
+    def work(i):
+        with torch.no_grad(), torch.cuda.stream(torch.cuda.Stream()):
+            for _ in range(20):
+                if not torch.equal(m(*calls[i]), want[i]):
+                    wrong.append(i)
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not wrong
