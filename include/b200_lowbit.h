@@ -347,6 +347,8 @@ int lowbit_moe_tokens_cuda(const void* d_x, int x_dtype, int64_t n_tokens, const
                            const uint64_t* d_gates, const uint64_t* d_ups, const uint64_t* d_downs, int n_experts,
                            int64_t hidden, int64_t inter, int qtype, int act, void* d_y,
                            void* workspace, size_t workspace_bytes, void* stream);
+/* how many (token, choice) pairs of the calling thread's last lowbit_moe_tokens_cuda had an id outside [0, n_experts) */
+int64_t lowbit_moe_tokens_last_unrouted(void);
 
 /* 1 when a bounded wait inside the prompt matmul or the prompt attention has run out on the current device since the library was loaded (the
  * launch's results are then undefined), 0 otherwise, -1 without a device.  Synchronises. */

@@ -375,6 +375,8 @@ int lowbit_moe_tokens_cuda(const void* d_x, int x_dtype, int64_t n_tokens, const
     return rc;
 }
 
+int64_t lowbit_moe_tokens_last_unrouted(void) { return experts_unrouted(); }
+
 int lowbit_gemm_wait_expired(void) {
     const int a = gemm_tc_wait_expired(), b = sdp_prompt_wait_expired(), c = gemm_exact_wait_expired();
     return a < 0 || b < 0 || c < 0 ? -1 : a | b | c;

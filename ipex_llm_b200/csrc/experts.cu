@@ -123,6 +123,7 @@ struct PinnedView {
     ~PinnedView() { if (p) cudaFreeHost(p); }
 };
 thread_local PinnedView t_view;
+thread_local int64_t t_unrouted = 0;
 
 // the experts of few rows, whatever their number: weights exact
 int experts_of_few_rows(const MoeParams& P, const HostView& V, char* x, char* h, char* out, cudaStream_t st) {
@@ -146,8 +147,10 @@ size_t experts_workspace_size(int64_t hidden, int64_t inter, int n_experts, int6
     (void)n_experts;
     return experts_scratch(hidden, inter, n_tokens * top_k).total;
 }
+int64_t experts_unrouted() { return t_unrouted; }
 int experts_launch(const MoeParams& P, int64_t n_tokens, cudaStream_t st) {
     const int64_t pairs = n_tokens * P.top_k;
+    t_unrouted = 0;
     if (!experts_supported(P.qtype, P.hidden, P.inter, P.n_experts, P.top_k) || pairs > 0x3fffffff || P.accumulate) return LB_ERR_ARG;
     if ((P.x_dtype != DT_F16 && P.x_dtype != DT_BF16) || P.y_dtype != P.x_dtype) return LB_ERR_ARG;
     if (((uintptr_t)P.x & 15) || ((uintptr_t)P.y & 15) || ((uintptr_t)P.workspace & 255)) return LB_ERR_ARG;
@@ -181,6 +184,7 @@ int experts_launch(const MoeParams& P, int64_t n_tokens, cudaStream_t st) {
     cudaEventDestroy(sorted);
     if (rc) return rc;
     if (waited != cudaSuccess) { set_error(LB_ERR_CUDA, "CUDA error: %s", cudaGetErrorString(waited)); cudaGetLastError(); return LB_ERR_CUDA; }
+    t_unrouted = pairs - host->offs[P.n_experts];
     if ((rc = experts_of_few_rows(P, *host, x, h, out, st))) return rc;
     if (P.x_dtype == DT_BF16) experts_combine_kernel<true><<<(unsigned)n_tokens, 256, 0, st>>>((const uint4*)out, row_of, P.weights, P.w_dtype, P.top_k, (uint4*)P.y, vec);
     else experts_combine_kernel<false><<<(unsigned)n_tokens, 256, 0, st>>>((const uint4*)out, row_of, P.weights, P.w_dtype, P.top_k, (uint4*)P.y, vec);

@@ -81,6 +81,7 @@ constexpr int64_t kExactRows = 16;
 bool experts_supported(int qt, int64_t hidden, int64_t inter, int n_experts, int top_k);
 size_t experts_workspace_size(int64_t hidden, int64_t inter, int n_experts, int64_t n_tokens, int top_k);
 int experts_launch(const MoeParams& P, int64_t n_tokens, cudaStream_t st);
+int64_t experts_unrouted();       // pairs of the calling thread's last launch whose id was outside the table
 
 // gemm_pair.cu (tcgen05 prompt matmul, two SMs per tile)
 bool gemm_tc_supported(int qt, int64_t n_rows, int64_t k);

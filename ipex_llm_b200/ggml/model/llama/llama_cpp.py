@@ -324,6 +324,8 @@ _lib.lowbit_moe_tokens_cuda.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_
                                         ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int, ctypes.c_int64,
                                         ctypes.c_int64, ctypes.c_int, ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_size_t, ctypes.c_void_p]
 _lib.lowbit_moe_tokens_cuda.restype = ctypes.c_int
+_lib.lowbit_moe_tokens_last_unrouted.argtypes = []
+_lib.lowbit_moe_tokens_last_unrouted.restype = ctypes.c_int64
 _lib.lowbit_gemm_wait_expired.argtypes = []
 _lib.lowbit_gemm_wait_expired.restype = ctypes.c_int
 
@@ -340,6 +342,11 @@ def lowbit_moe_tokens_cuda(d_x, x_dtype, n_tokens, d_ids, ids_dtype, d_weight, w
                            hidden, inter, qtype, act, d_y, workspace, workspace_bytes, stream):
     _check(_lib.lowbit_moe_tokens_cuda(d_x, x_dtype, n_tokens, d_ids, ids_dtype, d_weight, weight_dtype, top_k, d_gates, d_ups, d_downs,
                                        n_experts, hidden, inter, qtype, act, d_y, workspace, workspace_bytes, stream), "lowbit_moe_tokens_cuda")
+
+
+def lowbit_moe_tokens_last_unrouted():
+    """how many (token, choice) pairs of this thread's last lowbit_moe_tokens_cuda had an id outside the table"""
+    return _lib.lowbit_moe_tokens_last_unrouted()
 
 
 def lowbit_gemm_wait_expired():

@@ -432,11 +432,12 @@ def moe_tokens_supported(x: torch.Tensor, n_experts: int, hidden: int, inter: in
 
 
 def moe_forward_tokens(x: torch.Tensor, topk_ids: torch.Tensor, topk_weight: torch.Tensor, gates: torch.Tensor, ups: torch.Tensor,
-                       downs: torch.Tensor, hidden: int, inter: int, qtype: int, act: int = SILU):
+                       downs: torch.Tensor, hidden: int, inter: int, qtype: int, act: int = SILU, strict: bool = False):
     """The routed experts' MLPs of many tokens (the expert loop of models/qwen3_moe.py:106-132): x [T, hidden] fp16 / bf16,
     ``topk_ids`` / ``topk_weight`` [T, top_k] and the address tables as in ``moe_forward_vec``; the pairs are sorted by expert on
     the device, the experts' rows run in one launch per projection, those of experts with at most 16 rows on the GEMV (exact
-    weights).  Waits for the row counts: not under capture.  Returns [T, hidden] in x's dtype."""
+    weights).  Waits for the row counts: not under capture.  An id outside the tables adds nothing, or with ``strict`` is an error.
+    Returns [T, hidden] in x's dtype."""
     T, top_k = topk_ids.shape
     invalidInputError(x.dim() == 2 and tuple(x.shape) == (T, hidden), f"activation shape {tuple(x.shape)} != ({T}, {hidden})")
     invalidInputError(x.dtype in (torch.float16, torch.bfloat16), f"unsupported activation dtype {x.dtype}")
@@ -458,6 +459,7 @@ def moe_forward_tokens(x: torch.Tensor, topk_ids: torch.Tensor, topk_weight: tor
         ggml.lowbit_moe_tokens_cuda(x.data_ptr(), _TORCH_TO_DT[x.dtype], T, topk_ids.data_ptr(), 1 if topk_ids.dtype == torch.int64 else 0,
                                     topk_weight.data_ptr(), _TORCH_TO_DT[topk_weight.dtype], top_k, gates.data_ptr(), ups.data_ptr(),
                                     downs.data_ptr(), gates.numel(), hidden, inter, qtype, act, out.data_ptr(), ws.data_ptr(), need, _raw_stream(dev))
+    invalidInputError(not strict or ggml.lowbit_moe_tokens_last_unrouted() == 0, f"a token is routed to an expert outside [0, {gates.numel()})")
     return out
 
 

@@ -111,7 +111,7 @@ class LowBitExperts(nn.Module):
             addresses = self._plain_addresses(hidden_states.device)         # None: an expert that has to run itself
             if addresses is not None:
                 return moe_forward_tokens(hidden_states, top_k_index, top_k_weights, *self._address_tables(hidden_states.device, addresses),
-                                          self.hidden_dim, self.intermediate_dim, self.qtype)
+                                          self.hidden_dim, self.intermediate_dim, self.qtype, strict=True)
         final = torch.zeros_like(hidden_states)
         expert_mask = torch.nn.functional.one_hot(top_k_index, num_classes=self.num_experts).permute(2, 1, 0)
         for e in torch.greater(expert_mask.sum(dim=(-1, -2)), 0).nonzero()[:, 0].tolist():

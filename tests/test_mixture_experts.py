@@ -235,3 +235,17 @@ def test_few_rows_from_several_threads_and_streams(native_lib, cuda_device):
     for t in threads:
         t.join()
     assert not wrong
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows", [5, 200])
+@pytest.mark.parametrize("bad", [-1, E, 1 << 40])
+def test_a_choice_outside_the_layer_is_an_error(native_lib, cuda_device, rows, bad):
+    m = layer(cuda_device)
+    x = torch.randn(rows, H, device=cuda_device).half()
+    idx, w = routing(cuda_device, rows)
+    wrong = idx.clone()
+    wrong[rows // 2, 1] = bad
+    with pytest.raises(RuntimeError, match="outside"):
+        m(x, wrong, w)
+    same(m, x, idx, w)                                                              # and the next call is none the worse
