@@ -431,6 +431,11 @@ def moe_tokens_supported(x: torch.Tensor, n_experts: int, hidden: int, inter: in
             and ggml.lowbit_moe_tokens_supported(qtype, hidden, inter, n_experts, top_k))
 
 
+# Bytes of sorted rows that the many-token experts may hold at a time (90 KB a token at 4096 x 14336, two choices): longer prompts run in
+# portions, each reading the weights again.  What the loop over the experts held for one expert of eight at 32k tokens is of this size
+MOE_MAX_SCRATCH = 512 << 20
+
+
 def moe_forward_tokens(x: torch.Tensor, topk_ids: torch.Tensor, topk_weight: torch.Tensor, gates: torch.Tensor, ups: torch.Tensor,
                        downs: torch.Tensor, hidden: int, inter: int, qtype: int, act: int = SILU, strict: bool = False):
     """The routed experts' MLPs of many tokens (the expert loop of models/qwen3_moe.py:106-132): x [T, hidden] fp16 / bf16,
@@ -453,13 +458,20 @@ def moe_forward_tokens(x: torch.Tensor, topk_ids: torch.Tensor, topk_weight: tor
     if T == 0:
         return out
     dev = x.device
-    need = ggml.lowbit_moe_tokens_workspace_size(hidden, inter, gates.numel(), T, top_k)
+    size = lambda n: ggml.lowbit_moe_tokens_workspace_size(hidden, inter, gates.numel(), n, top_k)           # noqa: E731
+    portions = min(T, -(-size(T) // MOE_MAX_SCRATCH))
+    step = -(-T // portions)
+    need = size(step)
     ws = torch.empty(need, dtype=torch.uint8, device=dev)     # rows of activations: from the allocator, not kept
+    unrouted = 0
     with _on_device(dev):
-        ggml.lowbit_moe_tokens_cuda(x.data_ptr(), _TORCH_TO_DT[x.dtype], T, topk_ids.data_ptr(), 1 if topk_ids.dtype == torch.int64 else 0,
-                                    topk_weight.data_ptr(), _TORCH_TO_DT[topk_weight.dtype], top_k, gates.data_ptr(), ups.data_ptr(),
-                                    downs.data_ptr(), gates.numel(), hidden, inter, qtype, act, out.data_ptr(), ws.data_ptr(), need, _raw_stream(dev))
-    invalidInputError(not strict or ggml.lowbit_moe_tokens_last_unrouted() == 0, f"a token is routed to an expert outside [0, {gates.numel()})")
+        for a in range(0, T, step):
+            xs, ids, weight = x[a:a + step], topk_ids[a:a + step], topk_weight[a:a + step]
+            ggml.lowbit_moe_tokens_cuda(xs.data_ptr(), _TORCH_TO_DT[x.dtype], xs.shape[0], ids.data_ptr(), 1 if ids.dtype == torch.int64 else 0,
+                                        weight.data_ptr(), _TORCH_TO_DT[weight.dtype], top_k, gates.data_ptr(), ups.data_ptr(), downs.data_ptr(),
+                                        gates.numel(), hidden, inter, qtype, act, out[a:a + step].data_ptr(), ws.data_ptr(), need, _raw_stream(dev))
+            unrouted += ggml.lowbit_moe_tokens_last_unrouted()
+    invalidInputError(not strict or unrouted == 0, f"a token is routed to an expert outside [0, {gates.numel()})")
     return out
 
 

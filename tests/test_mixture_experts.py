@@ -249,3 +249,25 @@ def test_a_choice_outside_the_layer_is_an_error(native_lib, cuda_device, rows, b
     with pytest.raises(RuntimeError, match="outside"):
         m(x, wrong, w)
     same(m, x, idx, w)                                                              # and the next call is none the worse
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows,limit", [(700, 1 << 20), (333, 100000), (3, 1), (4097, 4 << 20)])
+def test_long_prompts_run_in_portions(native_lib, cuda_device, monkeypatch, rows, limit):
+    """scratch stays below its bound (or at one token's), whatever the prompt's length"""
+    from ipex_llm_b200.transformers import low_bit_linear as lbl
+    m = layer(cuda_device)
+    x = torch.randn(rows, H, device=cuda_device).half()
+    idx, w = routing(cuda_device, rows)
+    monkeypatch.setattr(lbl, "MOE_MAX_SCRATCH", limit)
+    m(x, idx, w)
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    torch.cuda.reset_peak_memory_stats()
+    got = m(x, idx, w)
+    one = native_lib.lowbit_moe_tokens_workspace_size(H, I, E, 1, 2)
+    # a portion holds whole tokens, and every piece of it is rounded up to 256 bytes
+    assert torch.cuda.max_memory_allocated() - before <= got.numel() * 2 + max(limit, one) + one + 4096
+    same(m, x, idx, w)
+    with pytest.raises(RuntimeError, match="outside"):
+        m(x, torch.where(torch.arange(rows, device=cuda_device)[:, None] == 0, E, idx), w)
