@@ -65,7 +65,8 @@ int mixers_gated_delta_rule(int dtype, const void* conv, int B, int S, int kv_he
                             int slot0, const int32_t* pad, float* o, mixers_stream_t stream);
 
 /* The same over a prompt, 32 tokens at a time (dim <= 128): the part of every chunk that needs no earlier state in one launch, the serial
- * part as small matrix products in a second.  workspace: mixers_gated_delta_chunks_workspace() bytes, 16-byte aligned. */
+ * part as small matrix products in a second.  workspace: mixers_gated_delta_chunks_workspace() bytes, 16-byte aligned: at most 512 MB or
+ * what one chunk needs; longer prompts run in portions. */
 long mixers_gated_delta_chunks_workspace(int B, int S, int kv_heads, int heads, int dim);      /* -1: not served */
 int mixers_gated_delta_chunks(int dtype, const void* conv, int B, int S, int kv_heads, int heads, int dim, int vdim, const void* proj, int ld,
                               int off_b, int off_a, const void* A_log, const void* dt_bias, float* state, int slot0, const int32_t* pad,

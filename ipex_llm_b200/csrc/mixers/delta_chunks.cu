@@ -31,6 +31,7 @@ template <int D> __host__ __device__ constexpr int d_rows() { return 3 * 2 * DC 
 struct ChunkArgs {
     const void* conv; const void* proj; const void* A_log; const void* dt_bias;
     int B, S, kv_heads, heads, dim, vdim, ld_proj, off_b, off_a, slot0, n_chunks;
+    int seq;                                            // tokens from one sequence to the next: S, or more when S is a portion of them
     const int32_t* pad;
     float* rows;                                        // [B][kv_heads][n_chunks][3 planes][2][DC][D + 8] bf16
     float* side;                                        // [B][heads][n_chunks][D_SIDE]
@@ -70,7 +71,7 @@ __global__ void __launch_bounds__(DT) delta_gram_kernel(const ChunkArgs a) {
     const double q_scale = 1.0 / sqrt((double)a.dim);
     // unit vectors, a warp per token
     for (int t = warp; t < DC; t += DT / 32) {
-        const T* row = (const T*)a.conv + ((long)b * a.S + t0 + (t < nt ? t : 0)) * ld;
+        const T* row = (const T*)a.conv + ((long)b * a.seq + t0 + (t < nt ? t : 0)) * ld;
         float kv[D / 32], qv[D / 32], sk = 0.0f, sq = 0.0f;
 #pragma unroll
         for (int e = 0; e < D / 32; ++e) {
@@ -132,7 +133,7 @@ __global__ void __launch_bounds__(DT) delta_gram_kernel(const ChunkArgs a) {
     float* const L = tri + warp * DC * DC;
     for (int hi = warp; hi < n_rep; hi += DT / 32) {
         const int h = g * n_rep + hi;
-        const T* pr = (const T*)a.proj + ((long)b * a.S + t0 + (lane < nt ? lane : 0)) * a.ld_proj;
+        const T* pr = (const T*)a.proj + ((long)b * a.seq + t0 + (lane < nt ? lane : 0)) * a.ld_proj;
         // the gates in double: a decay's error counts as often as there are tokens behind it
         const double z = (double)to_f(pr[a.off_a + h]) + (double)to_f(((const T*)a.dt_bias)[h]);
         double lg = -exp((double)to_f(((const T*)a.A_log)[h])) * (z > 20.0 ? z : log1p(exp(z)));
@@ -254,7 +255,7 @@ __global__ void __launch_bounds__(DT + 32) delta_walk_kernel(const ChunkArgs a) 
     }
 
     const int ld = 2 * a.kv_heads * a.dim + a.heads * a.vdim, off_v = 2 * a.kv_heads * a.dim + h * a.vdim + col0;
-    float* const ob = a.o + (((long)b * a.S) * a.heads + h) * a.vdim + col0;
+    float* const ob = a.o + (((long)b * a.seq) * a.heads + h) * a.vdim + col0;
     const long o_ld = (long)a.heads * a.vdim;
     for (int i = tid; i < first * DV; i += DT) if (i % DV < cols) ob[(i / DV) * o_ld + i % DV] = 0.0f;
 
@@ -279,7 +280,7 @@ __global__ void __launch_bounds__(DT + 32) delta_walk_kernel(const ChunkArgs a) 
         const int t = first + c * DC + orow;
 #pragma unroll
         for (int e = 0; e < 2; ++e)
-            if (c < n && t < a.S && op + e < cols) v[e] = ((const T*)a.conv)[((long)b * a.S + t) * ld + off_v + op + e];
+            if (c < n && t < a.S && op + e < cols) v[e] = ((const T*)a.conv)[((long)b * a.seq + t) * ld + off_v + op + e];
     };
     v[0] = v[1] = from_f<T>(0.0f);
     values(0);
@@ -416,10 +417,39 @@ template <typename T, int D> int launch_chunks(const ChunkArgs& a, cudaStream_t 
 
 }  // namespace
 
+// Scratch of a call at most (or one chunk's, where that is more): 11 KB a token at 4 / 16 heads of 128, 22 KB at 8 / 32.  Longer prompts
+// run in portions of whole chunks, the state carried through memory as between two calls
+namespace {
+constexpr long kDeltaScratch = 512l << 20;
+long chunk_bytes(int B, int kv_heads, int heads, int dim) { return 4l * B * (kv_heads * (dim <= 64 ? d_rows<64>() : d_rows<128>()) + (long)heads * D_SIDE); }
+// chunks of one portion: portions of equal length
+long portion_chunks(int B, int S, int kv_heads, int heads, int dim) {
+    const long n = ((long)S + DC - 1) / DC, fit = kDeltaScratch / chunk_bytes(B, kv_heads, heads, dim), most = fit > 1 ? fit : 1;
+    const long portions = (n + most - 1) / most;
+    return (n + portions - 1) / portions;
+}
+}  // namespace
+
 extern "C" long mixers_gated_delta_chunks_workspace(int B, int S, int kv_heads, int heads, int dim) {
     if (B <= 0 || S <= 0 || dim <= 0 || dim > 128 || kv_heads <= 0 || kv_heads > 65535 || heads > 65535 || B > 65535) return -1;
-    const long n = (S + DC - 1) / DC, rows = dim <= 64 ? d_rows<64>() : d_rows<128>();
-    return 4 * n * B * (kv_heads * rows + (long)heads * D_SIDE);
+    return portion_chunks(B, S, kv_heads, heads, dim) * chunk_bytes(B, kv_heads, heads, dim);
+}
+
+template <typename T> static int run_portions(ChunkArgs a, cudaStream_t st) {
+    const int S = a.S, slot0 = a.slot0, step = DC * (int)portion_chunks(a.B, S, a.kv_heads, a.heads, a.dim);
+    const long ld = 2 * a.kv_heads * a.dim + a.heads * a.vdim;
+    const T *const conv = (const T*)a.conv, *const proj = (const T*)a.proj;
+    float* const o = a.o;
+    a.seq = S;
+    a.side = a.rows + (long)a.B * a.kv_heads * (step / DC) * (a.dim <= 64 ? d_rows<64>() : d_rows<128>());
+    for (long at = 0; at < S; at += step) {
+        a.S = (int)(S - at < step ? S - at : step);
+        a.n_chunks = (a.S + DC - 1) / DC;
+        a.slot0 = slot0 + (int)at;
+        a.conv = conv + at * ld; a.proj = proj + at * a.ld_proj; a.o = o + at * a.heads * a.vdim;
+        if (const int rc = a.dim <= 64 ? launch_chunks<T, 64>(a, st) : launch_chunks<T, 128>(a, st)) return rc;
+    }
+    return 0;
 }
 
 extern "C" int mixers_gated_delta_chunks(int dtype, const void* conv, int B, int S, int kv_heads, int heads, int dim, int vdim, const void* proj, int ld,
@@ -430,9 +460,7 @@ extern "C" int mixers_gated_delta_chunks(int dtype, const void* conv, int B, int
     ChunkArgs a = {};
     a.conv = conv; a.proj = proj; a.A_log = A_log; a.dt_bias = dt_bias;
     a.B = B; a.S = S; a.kv_heads = kv_heads; a.heads = heads; a.dim = dim; a.vdim = vdim; a.ld_proj = ld; a.off_b = off_b; a.off_a = off_a;
-    a.slot0 = slot0; a.n_chunks = (S + DC - 1) / DC; a.pad = pad; a.state = state; a.o = o;
-    a.rows = workspace;
-    a.side = workspace + (long)B * kv_heads * a.n_chunks * (dim <= 64 ? d_rows<64>() : d_rows<128>());
-    MIXERS_DISPATCH(dtype, return (dim <= 64 ? launch_chunks<T, 64>(a, (cudaStream_t)stream) : launch_chunks<T, 128>(a, (cudaStream_t)stream)));
+    a.slot0 = slot0; a.pad = pad; a.state = state; a.o = o; a.rows = workspace;
+    MIXERS_DISPATCH(dtype, return run_portions<T>(a, (cudaStream_t)stream));
     return 0;
 }

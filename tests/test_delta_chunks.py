@@ -102,3 +102,14 @@ def test_a_token_that_is_not_finite_stays_behind_the_earlier_ones(ops, cuda_devi
     got = ops.gated_delta_rule(conv, G, H, D, V, proj, 1, 1 + H, a_log, bias, state.clone(), 0, pad)
     assert torch.equal(got[:, :77], o[:, :77]) and not bool(got[:, 77:, :, 3].isfinite().any())
     assert torch.equal(got[..., :3], o[..., :3]) and torch.equal(got[..., 4:], o[..., 4:])
+
+
+def test_a_prompt_in_portions_of_its_scratch(ops, cuda_device):
+    """one chunk of these heads takes 304 MB, so that the four chunks run one by one; padding ends in each of them"""
+    B, S, G, H, D, V = 64, 100, 128, 128, 5, 9
+    conv, proj, a_log, bias, state = inputs(cuda_device, B, S, G, H, D, V, torch.float32)
+    pad = torch.arange(B, dtype=torch.int32, device=cuda_device) * 100 // 63
+    want_o, want_s = statement(conv, proj, a_log, bias, state, G, H, D, V, 0, pad)
+    o = ops.gated_delta_rule(conv, G, H, D, V, proj, 1, 1 + H, a_log, bias, state, 0, pad)
+    assert float((o.double() - want_o).abs().max()) <= 2e-6 * max(1.0, float(want_o.abs().max()))
+    assert float((state.double() - want_s).abs().max()) <= 2e-6 * max(1.0, float(want_s.abs().max()))
