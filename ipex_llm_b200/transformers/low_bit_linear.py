@@ -271,16 +271,10 @@ def use_batch_forward(x: torch.Tensor, qtype: int, output_len: int):
     return x.shape[0] <= GEMV_MAX_M and qtype in B200_SUPPORTED_QTYPE_IDS
 
 
-# ------------------------------------------------------------------ workspace (per device)
-_workspaces = {}
-
-
-def _get_workspace(device, need):
-    ws = _workspaces.get(device)
-    if ws is None or ws.numel() < need:
-        ws = torch.zeros(int(need * 1.25) + 256, dtype=torch.uint8, device=device)
-        _workspaces[device] = ws
-    return ws
+def _scratch(device, need, none=None):
+    """``need`` bytes of one call's own scratch, from the allocator on the current stream: two streams never meet in it.  ``none``: what
+    stands in for no bytes (NULL would ask the library for its own, under its lock)"""
+    return torch.empty(need, dtype=torch.uint8, device=device) if need or none is None else none
 
 
 def lowbit_matmul(x_2d: torch.Tensor, weight: torch.Tensor, weight_shape, qtype: int, out: torch.Tensor = None,
@@ -313,12 +307,13 @@ def lowbit_matmul(x_2d: torch.Tensor, weight: torch.Tensor, weight_shape, qtype:
         return out
     w = weight.view(torch.uint8) if weight.dtype != torch.uint8 else weight
     dev = x_2d.device
-    ws = _get_workspace(dev, _matmul_workspace_size(N, K, M, x_dt))
+    need = _matmul_workspace_size(N, K, M, x_dt)
+    ws = _scratch(dev, need, out)
     if next_weight is not None:      # L2 prefetch hint: the weights the following matmul on this stream reads
         ggml.lowbit_hint_next_weights(ctypes.c_void_p(next_weight.data_ptr()), next_weight.numel() * next_weight.element_size())
     with _on_device(dev):
         ggml.lowbit_matmul_cuda(w.data_ptr(), qtype, N, K, x_2d.data_ptr(), x_dt, M, out.data_ptr(), _TORCH_TO_DT[out_dtype],
-                                bias.data_ptr() if bias is not None else None, accumulate, ws.data_ptr(), ws.numel(), _raw_stream(dev))
+                                bias.data_ptr() if bias is not None else None, accumulate, ws.data_ptr(), need, _raw_stream(dev))
     return out
 
 
@@ -348,13 +343,14 @@ def mlp_forward(x_2d: torch.Tensor, gate_weight: torch.Tensor, up_weight: torch.
         return out
     dev = x_2d.device
     dt = _TORCH_TO_DT[x_2d.dtype]
-    ws = _get_workspace(dev, ggml.lowbit_mlp_workspace_size(N, K, M, dt))
+    need = ggml.lowbit_mlp_workspace_size(N, K, M, dt)
+    ws = _scratch(dev, need, out)
     g = gate_weight.view(torch.uint8) if gate_weight.dtype != torch.uint8 else gate_weight
     u = up_weight.view(torch.uint8) if up_weight.dtype != torch.uint8 else up_weight
     with torch.cuda.device(dev):
         ggml.lowbit_mlp_cuda(ctypes.c_void_p(g.data_ptr()), ctypes.c_void_p(u.data_ptr()), qtype, N, K,
                              ctypes.c_void_p(x_2d.data_ptr()), dt, M, ctypes.c_void_p(out.data_ptr()),
-                             _TORCH_TO_DT[out.dtype], act, ctypes.c_void_p(ws.data_ptr()), ws.numel(), _stream_ptr(dev))
+                             _TORCH_TO_DT[out.dtype], act, ctypes.c_void_p(ws.data_ptr()), need, _stream_ptr(dev))
     return out
 
 
@@ -385,7 +381,7 @@ def moe_forward_vec(x: torch.Tensor, topk_ids: torch.Tensor, topk_weight: torch.
         out = torch.empty((1, hidden), dtype=x.dtype, device=x.device)
     dev = x.device
     dt = _TORCH_TO_DT[x.dtype]
-    ws = _get_workspace(dev, ggml.lowbit_moe_workspace_size(hidden, inter, top_k, dt))
+    ws = _scratch(dev, ggml.lowbit_moe_workspace_size(hidden, inter, top_k, dt))
     with torch.cuda.device(dev):
         ggml.lowbit_moe_cuda(ctypes.c_void_p(x.data_ptr()), dt, ctypes.c_void_p(topk_ids.data_ptr()),
                              1 if topk_ids.dtype == torch.int64 else 0, ctypes.c_void_p(topk_weight.data_ptr()),
@@ -462,7 +458,7 @@ def moe_forward_tokens(x: torch.Tensor, topk_ids: torch.Tensor, topk_weight: tor
     portions = min(T, -(-size(T) // MOE_MAX_SCRATCH))
     step = -(-T // portions)
     need = size(step)
-    ws = torch.empty(need, dtype=torch.uint8, device=dev)     # rows of activations: from the allocator, not kept
+    ws = _scratch(dev, need)
     unrouted = 0
     with _on_device(dev):
         for a in range(0, T, step):

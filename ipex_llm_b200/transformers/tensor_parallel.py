@@ -165,7 +165,7 @@ class PeerAllReduce:
             bias = bias.to(out.dtype)
         own, peers = self._comm(m * n_rows * 4)
         dt = lbl._TORCH_TO_DT[x_2d.dtype]
-        ws = lbl._get_workspace(x_2d.device, ggml.lowbit_matmul_workspace_size(n_rows, k, m, dt))
+        ws = lbl._scratch(x_2d.device, max(16, ggml.lowbit_matmul_workspace_size(n_rows, k, m, dt)))
         w = weight.view(torch.uint8) if weight.dtype != torch.uint8 else weight
         with torch.cuda.device(x_2d.device):
             ggml.lowbit_matmul_allreduce(w, qtype, n_rows, k, x_2d, out, bias, accumulate, peers, self.rank, m * n_rows * 4, ws,
