@@ -282,7 +282,8 @@ size_t lowbit_matmul_workspace_size(int64_t n_rows, int64_t k, int64_t m, int x_
  * workspace: a buffer of at least lowbit_matmul_workspace_size() bytes, or NULL = one library-owned buffer per
  * device.  The NULL mode is for ONE stream per device and must not be used under stream capture: calls are
  * serialised on the host only (two streams would race on the buffer on the GPU), and growing the buffer
- * synchronises the device and reallocates.
+ * synchronises the device and reallocates.  16-byte aligned: one that is not is refused by fp32 activations, and costs prompts
+ * their K split.
  * Any M >= 1.  fp16 / bf16 activations: M <= 16 runs the HBM-bound GEMV kernel (so does 17 <= M <= 32 when n_rows is
  * not a multiple of 128 or k not of 128), larger M the tensor-core kernels -- 17..64 rows the "skinny" one with the
  * weights as the 128-row operand, beyond that the prefill GEMM (activations and expanded weights enter the MMA as
@@ -305,7 +306,7 @@ int lowbit_matmul_cuda(const void* d_w, int qtype, int64_t n_rows, int64_t k,
  * tensor-core kernel, act * up in its reduction launch.  M > 128 half-precision rows (prefill): gate and up as two outputs of
  * ONE grid of the tensor-core GEMM (half-precision scratch) + one elementwise kernel.  Otherwise two matmuls into scratch
  * (fp32 behind the exact GEMV) and the elementwise kernel.  Same result in every case up to the rounding of the intermediates.
- * workspace: NULL (library-owned) or lowbit_mlp_workspace_size() bytes. */
+ * workspace: NULL (library-owned) or lowbit_mlp_workspace_size() bytes, aligned as there. */
 size_t lowbit_mlp_workspace_size(int64_t n_rows, int64_t k, int64_t m, int x_dtype);
 int lowbit_mlp_cuda(const void* d_w_gate, const void* d_w_up, int qtype, int64_t n_rows, int64_t k,
                     const void* d_x, int x_dtype, int64_t m, void* d_y, int y_dtype, int act,

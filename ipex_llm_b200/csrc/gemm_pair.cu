@@ -524,6 +524,9 @@ static PairPlan pair_plan(double pace, int64_t n_fp, int64_t nb, int64_t m, int6
     }
     return best;
 }
+static bool holds_partials(const void* workspace, size_t bytes, size_t count) {
+    return workspace && ((uintptr_t)workspace & 15) == 0 && bytes >= count * sizeof(float);
+}
 // splits that a workspace has to hold, whatever the format and type
 static int most_splits(int64_t n_fp, int64_t nb, int64_t m, int64_t n_out) {
     int ks = 1;
@@ -560,8 +563,8 @@ int gemm_tc_launch(const void* w, int qt, int64_t n_rows, int64_t k, const void*
     A.w = (const uint8_t*)w; A.G = make_geom(n_rows, k, qt); A.M = (int)m; A.y = y; A.y_dtype = y_dtype; A.bias = bias; A.accumulate = accumulate;
     A.n_fp = (int)((n_rows / 128 + 1) / 2);
     PairPlan p = pair_plan(pair_pace(qt, bf), A.n_fp, k / 64, m, n_rows, true);
-    // a caller's workspace without room for partial sums: the whole K range per unit
-    if (p.ks > 1 && (!workspace || workspace_bytes < (size_t)p.ks * m * n_rows * sizeof(float))) p = pair_plan(pair_pace(qt, bf), A.n_fp, k / 64, m, n_rows, false);
+    // a caller's workspace without room for partial sums, or not aligned for their 16-byte loads: the whole K range per unit
+    if (p.ks > 1 && !holds_partials(workspace, workspace_bytes, (size_t)p.ks * m * n_rows)) p = pair_plan(pair_pace(qt, bf), A.n_fp, k / 64, m, n_rows, false);
     A.tt = p.tt; A.ksplit = p.ks; A.part = (float*)workspace;
     const int64_t units = (int64_t)A.n_fp * ((m + p.tt - 1) / p.tt) * p.ks;
     if (const int rc = pair_launch(qt, bf, map, A, units, st)) return rc;
@@ -589,7 +592,7 @@ int gemm_tc_mlp_launch(const void* w_gate, const void* w_up, int act, int qt, in
     A.w = (const uint8_t*)w_gate; A.w2 = (const uint8_t*)w_up; A.act = act; A.G = make_geom(n_rows, k, qt); A.M = (int)m; A.y = y; A.y_dtype = y_dtype;
     A.n_fp = (int)((n_rows / 64 + 1) / 2);
     PairPlan p = pair_plan(pair_pace(qt, bf), A.n_fp, k / 64, m, 2 * n_rows, true);
-    if (p.ks > 1 && (!workspace || workspace_bytes < (size_t)p.ks * m * 2 * n_rows * sizeof(float))) p = pair_plan(pair_pace(qt, bf), A.n_fp, k / 64, m, 2 * n_rows, false);
+    if (p.ks > 1 && !holds_partials(workspace, workspace_bytes, (size_t)p.ks * m * 2 * n_rows)) p = pair_plan(pair_pace(qt, bf), A.n_fp, k / 64, m, 2 * n_rows, false);
     A.tt = p.tt; A.ksplit = p.ks; A.part = (float*)workspace;
     if (const int rc = pair_launch(qt, bf, map, A, (int64_t)A.n_fp * ((m + A.tt - 1) / A.tt) * p.ks, st)) return rc;
     if (p.ks > 1) {

@@ -174,6 +174,7 @@ int gemv_launch_ex(const void* w, const void* w2, int act, int qt, int64_t n_row
             if (x_dtype == DT_F32) {
                 const size_t need = gemv_workspace_size(n_rows, k, mc, x_dtype);
                 if (!workspace || workspace_bytes < need) return LB_ERR_WORKSPACE;
+                if ((uintptr_t)workspace & 15) return LB_ERR_ARG;         // the planes are read 16 bytes at a time
                 __nv_bfloat16* planes = (__nv_bfloat16*)workspace;
                 const int64_t n = mc * k;
                 int sg = (int)((n + 255) / 256); if (sg > sm_count() * 8) sg = sm_count() * 8;

@@ -178,3 +178,33 @@ def test_prompt_matmul_fp32_keeps_its_contract(lbl, native_lib, cuda_device, qty
     assert torch.equal(lbl.lowbit_matmul(torch.cat([x, x], 1)[:, :k], w, (n, k), qt), y)
     half = lbl.lowbit_matmul(x, w, (n, k), qt, out_dtype=torch.float16)
     assert bool(((half.double() - want).abs() <= tol * mag + 2.0 ** -11 * want.abs() + 2.0 ** -25).all())
+
+
+@pytest.mark.parametrize("offset", [4, 8])
+def test_scratch_off_a_16_byte_boundary(lbl, native_lib, cuda_device, offset):
+    """shapes that would split K run it whole, within the same bounds; 32-bit activations, whose planes lie there, are refused"""
+    m, n, k = 100, 2048, 4096
+    ((wg, g), (wu, p)), qt = weights(lbl, cuda_device, 3, n, k, "sym_int4", 2)
+    x = acts(cuda_device, 4, m, k, torch.float16)
+    stream = torch.cuda.current_stream().cuda_stream
+    y = torch.empty(m, n, dtype=torch.float32, device=cuda_device)
+
+    def scratch(size):
+        return torch.empty(size + 16, dtype=torch.uint8, device=cuda_device)[offset:]
+    ws = scratch(native_lib.lowbit_matmul_workspace_size(n, k, m, native_lib.DT_F16))
+    assert ws.data_ptr() % 16 == offset and ws.numel() > m * n * 8
+    native_lib.lowbit_matmul_cuda(wg.data_ptr(), qt, n, k, x.data_ptr(), native_lib.DT_F16, m, y.data_ptr(), native_lib.DT_F32, None, False,
+                                  ws.data_ptr(), ws.numel(), stream)
+    want, bound = product(x.double(), g, U[torch.float16])
+    assert bool(((y.double() - want).abs() <= bound).all())
+    ws = scratch(native_lib.lowbit_mlp_workspace_size(n, k, m, native_lib.DT_F16))
+    native_lib.lowbit_mlp_cuda(wg.data_ptr(), wu.data_ptr(), qt, n, k, x.data_ptr(), native_lib.DT_F16, m, y.data_ptr(), native_lib.DT_F32, 0,
+                               ws.data_ptr(), ws.numel(), stream)
+    want, bound = gated(x.double(), g, p, U[torch.float16], 0)
+    assert bool(((y.double() - want).abs() <= bound).all())
+    x = acts(cuda_device, 4, m, k, torch.float32)
+    ws = scratch(native_lib.lowbit_matmul_workspace_size(n, k, m, native_lib.DT_F32))
+    for rows in (1, m):
+        with pytest.raises(RuntimeError):
+            native_lib.lowbit_matmul_cuda(wg.data_ptr(), qt, n, k, x.data_ptr(), native_lib.DT_F32, rows, y.data_ptr(), native_lib.DT_F32, None, False,
+                                          ws.data_ptr(), ws.numel(), stream)
