@@ -351,8 +351,10 @@ int lowbit_moe_tokens_cuda(const void* d_x, int x_dtype, int64_t n_tokens, const
 /* how many (token, choice) pairs of the calling thread's last lowbit_moe_tokens_cuda had an id outside [0, n_experts) */
 int64_t lowbit_moe_tokens_last_unrouted(void);
 
-/* 1 when a bounded wait inside the prompt matmul or the prompt attention has run out on the current device since the library was loaded (the
- * launch's results are then undefined), 0 otherwise, -1 without a device.  Synchronises. */
+/* The prompt matmul (fp32 activations included), the experts and the prompt attention bound their waits, at about two seconds each.  One
+ * that runs out ends the kernel, and the launch's results are undefined: the next call on the device that launches anything returns an
+ * error that says so.  1 when a wait has run out on the current device and no call has reported it yet, 0 otherwise, -1 without a
+ * device.  Synchronises. */
 int lowbit_gemm_wait_expired(void);
 
 /* No counterpart in the reference.  The fp32-activation matmul of lowbit_matmul_cuda, for hosts that

@@ -5,6 +5,7 @@
 // run the same CUDA kernels as family (2) and copy the result back.  No CPU arithmetic: if
 // CUDA is unusable the call records LB_ERR_NO_DEVICE and returns without writing.
 // Family (2): *_cuda symbols on device pointers + stream.
+#include <atomic>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -28,9 +29,45 @@ void set_error(int code, const char* fmt, ...) {
 }
 void note_launch() { t_launches++; }
 void reset_launch_count() { t_launches = 0; }
+// a word per device, each in a cache line of its own, in host memory that every device writes; never freed (recorded graphs hold it)
+constexpr int kWaitStride = 32;
+static std::atomic<unsigned int*> g_wait_words{nullptr};
+static thread_local long long t_wait_limit = 0;
+static unsigned int* wait_word() {
+    unsigned int* const w = g_wait_words.load(std::memory_order_acquire);
+    int dev = 0;
+    return w && cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64 ? w + dev * kWaitStride : nullptr;
+}
+int make_waits(Waits* out, long long limit) {
+    if (!g_wait_words.load(std::memory_order_acquire)) {
+        static std::mutex mu;
+        std::lock_guard<std::mutex> lk(mu);
+        if (!g_wait_words.load(std::memory_order_relaxed)) {
+            // the first launch may be one that is being captured: page-locking is no part of it
+            cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+            cudaThreadExchangeStreamCaptureMode(&mode);
+            void* p = nullptr;
+            const cudaError_t e = cudaHostAlloc(&p, 64 * kWaitStride * sizeof(unsigned int), cudaHostAllocPortable | cudaHostAllocMapped);
+            cudaThreadExchangeStreamCaptureMode(&mode);
+            if (e != cudaSuccess) { set_error(LB_ERR_CUDA, "cudaHostAlloc failed: %s", cudaGetErrorString(e)); cudaGetLastError(); return LB_ERR_CUDA; }
+            memset(p, 0, 64 * kWaitStride * sizeof(unsigned int));
+            g_wait_words.store((unsigned int*)p, std::memory_order_release);
+        }
+    }
+    out->word = wait_word();
+    out->limit = t_wait_limit ? t_wait_limit : limit;
+    if (!out->word) { set_error(LB_ERR_NO_DEVICE, "no current CUDA device"); return LB_ERR_NO_DEVICE; }
+    return LB_OK;
+}
 int check_launch() {
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) { set_error(LB_ERR_CUDA, "CUDA error: %s", cudaGetErrorString(e)); return LB_ERR_CUDA; }
+    unsigned int* const word = wait_word();
+    if (word && *(volatile unsigned int*)word) {
+        *(volatile unsigned int*)word = 0;
+        set_error(LB_ERR_CUDA, "a wait inside an earlier prompt matmul or prompt attention on this device ran out: the results since then are undefined");
+        return LB_ERR_CUDA;
+    }
     return LB_OK;
 }
 int sm_count() {
@@ -378,9 +415,13 @@ int lowbit_moe_tokens_cuda(const void* d_x, int x_dtype, int64_t n_tokens, const
 int64_t lowbit_moe_tokens_last_unrouted(void) { return experts_unrouted(); }
 
 int lowbit_gemm_wait_expired(void) {
-    const int a = gemm_tc_wait_expired(), b = sdp_prompt_wait_expired(), c = gemm_exact_wait_expired();
-    return a < 0 || b < 0 || c < 0 ? -1 : a | b | c;
+    if (cudaDeviceSynchronize() != cudaSuccess) { cudaGetLastError(); return -1; }
+    const unsigned int* const word = wait_word();
+    return word && *(const volatile unsigned int*)word ? 1 : 0;
 }
+/* development aid, not in the public header: the limit, in SM clocks, of the waits in this thread's launches (0: the usual one; below
+ * zero: the launches' copies stop half-way, and the waits for them run out after that many clocks) */
+void lowbit_debug_set_wait_limit(long long clocks) { t_wait_limit = clocks; }
 
 // ------------------------------------------------------------------ family (1)
 size_t ggml_quantize_tensor(const float* src, void* dst, int qtype, size_t n, int k, int64_t* hist,

@@ -31,7 +31,7 @@ template <int QT> struct ExSmem {
     static constexpr int kXSlot = 3 * 4096;                            // three planes x 32 rows x 128 bytes
     static constexpr int kTotal = 1024 + 512 + kA * kTileBytesAB + kP * kPacked + kX * kXSlot;
     static_assert(kTotal <= 232448, "shared memory");
-    static_assert((3 * kX + 2 * kP + 2 * kA + 2 * kExBufs) * 8 + 8 <= 512, "barrier region");
+    static_assert((3 * kX + 2 * kP + 2 * kA + 2 * kExBufs + 1) * 8 + 8 <= 512, "barrier region");
 };
 
 struct ExactArgs {
@@ -40,6 +40,7 @@ struct ExactArgs {
     int M, tt, n_fp, ksplit;
     float* y; const float* bias; int accumulate;
     float* part;
+    Waits waits;
 };
 
 template <int QT>
@@ -60,7 +61,8 @@ exact_kernel(const __grid_constant__ CUtensorMap xmap, const ExactArgs A) {
     auto a_empty = [&](int s) { return bars + (3 * KX + 2 * KP + KA + s) * 8; };
     auto t_full = [&](int b) { return bars + (3 * KX + 2 * KP + 2 * KA + b) * 8; };
     auto t_empty = [&](int b) { return bars + (3 * KX + 2 * KP + 2 * KA + kExBufs + b) * 8; };   // CTA 0: both epilogues have read it
-    const uint32_t tmem_slot = bars + (3 * KX + 2 * KP + 2 * KA + 2 * kExBufs) * 8;
+    const uint32_t drained = bars + (3 * KX + 2 * KP + 2 * KA + 2 * kExBufs) * 8;      // every MMA that was issued is done
+    const uint32_t tmem_slot = drained + 8;
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31, rank = (int)(blockIdx.x & 1);
     const int nb = (int)A.G.nb;
     if (threadIdx.x == 0) {
@@ -68,6 +70,7 @@ exact_kernel(const __grid_constant__ CUtensorMap xmap, const ExactArgs A) {
         for (int s = 0; s < KP; s++) { mbar_init(p_full(s), 1); mbar_init(p_empty(s), 4); }
         for (int s = 0; s < KA; s++) { mbar_init(a_full(s), 8); mbar_init(a_empty(s), 1); }
         for (int b = 0; b < kExBufs; b++) { mbar_init(t_full(b), 1); mbar_init(t_empty(b), 16); }
+        mbar_init(drained, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 3) {
@@ -94,16 +97,16 @@ exact_kernel(const __grid_constant__ CUtensorMap xmap, const ExactArgs A) {
         U.kb1 = ((U.ks + 1) * nb) / A.ksplit;
     };
     Unit U;
+    const uint32_t leader = elect_leader();
+    int s = 0, round = 0;                                  // the two copying warps' place in their ring
 
     if (warp == 0) {
         // ================= token planes: this CTA's half of the tile's tokens =================
-        const uint32_t leader = elect_leader();
-        int s = 0, round = 0;
         for (int unit = blockIdx.x >> 1; unit < n_units; unit += stride) {
             decode(unit, U);
             const int row0 = U.m0 + rank * (U.n_tok >> 1);
             for (int kb = U.kb0; kb < U.kb1; kb++) {
-                if (!mbar_wait_lim(x_empty(s), (uint32_t)((round & 1) ^ 1))) goto done;
+                if (!mbar_wait_lim(x_empty(s), (uint32_t)((round & 1) ^ 1), A.waits)) goto done;
                 mbar_expect_tx_w(x_full(s), SM::kXSlot, leader);
                 // rows of a plane beyond the last token belong to the next plane (or read zero): columns that nothing stores
                 for (int p = 0; p < 3; p++) tma_load_2d_w(xring + s * SM::kXSlot + p * 4096, &xmap, kb * 64, p * A.M + row0, x_full(s), leader);
@@ -113,16 +116,15 @@ exact_kernel(const __grid_constant__ CUtensorMap xmap, const ExactArgs A) {
     } else if (warp == 1) {
         if (rank == 0) {
             // ================= MMA issuer: 3 planes x 4 steps per k-block, into the k-block's own TMEM buffer =================
-            const uint32_t leader = elect_leader();
             int sx = 0, rx = 0, sa = 0, ra = 0, tb = 0, rt = 0;
             for (int unit = blockIdx.x >> 1; unit < n_units; unit += stride) {
                 decode(unit, U);
                 const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (((uint32_t)U.n_tok >> 3) << 17) | ((256u >> 4) << 24);
                 for (int kb = U.kb0; kb < U.kb1; kb++) {
-                    if (!mbar_wait_lim(t_empty(tb), (uint32_t)((rt & 1) ^ 1))) goto done;
-                    if (!mbar_wait_lim(x_full(sx), (uint32_t)(rx & 1))) goto done;
-                    if (!mbar_wait_lim(xp_full(sx), (uint32_t)(rx & 1))) goto done;
-                    if (!mbar_wait_lim(a_full(sa), (uint32_t)(ra & 1))) goto done;
+                    if (!mbar_wait_lim(t_empty(tb), (uint32_t)((rt & 1) ^ 1), A.waits)) goto done;
+                    if (!mbar_wait_lim(x_full(sx), (uint32_t)(rx & 1), A.waits)) goto done;
+                    if (!mbar_wait_lim(xp_full(sx), (uint32_t)(rx & 1), A.waits)) goto done;
+                    if (!mbar_wait_lim(a_full(sa), (uint32_t)(ra & 1), A.waits)) goto done;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint64_t ad = make_desc(aring + sa * kTileBytesAB), xd = make_desc(xring + sx * SM::kXSlot);
 #pragma unroll
@@ -145,7 +147,7 @@ exact_kernel(const __grid_constant__ CUtensorMap xmap, const ExactArgs A) {
             for (int unit = blockIdx.x >> 1; unit < n_units; unit += stride) {
                 decode(unit, U);
                 for (int kb = U.kb0; kb < U.kb1; kb++) {
-                    if (!mbar_wait_lim(x_full(sx), (uint32_t)(rx & 1))) goto done;
+                    if (!mbar_wait_lim(x_full(sx), (uint32_t)(rx & 1), A.waits)) goto done;
                     if (lane == 0) mbar_arrive_at(xp_full(sx), 0);
                     if (++sx == KX) { sx = 0; rx++; }
                 }
@@ -153,13 +155,12 @@ exact_kernel(const __grid_constant__ CUtensorMap xmap, const ExactArgs A) {
         }
     } else if (warp == 2) {
         // ================= packed weights of this CTA's two 64-row groups =================
-        const uint32_t leader = elect_leader();
         const int n_rg = (int)(A.G.rows >> 6);
-        int s = 0, round = 0;
         for (int unit = blockIdx.x >> 1; unit < n_units; unit += stride) {
             decode(unit, U);
-            for (int kb = U.kb0; kb < U.kb1; kb++) {
-                if (!mbar_wait_lim(p_empty(s), (uint32_t)((round & 1) ^ 1))) goto done;
+            const int kb_end = A.waits.limit < 0 ? (U.kb0 + U.kb1) / 2 : U.kb1;
+            for (int kb = U.kb0; kb < kb_end; kb++) {
+                if (!mbar_wait_lim(p_empty(s), (uint32_t)((round & 1) ^ 1), A.waits)) goto done;
                 mbar_expect_tx_w(p_full(s), 2 * PackedBlock<QT>::kSuper, leader);
 #pragma unroll
                 for (int gi = 0; gi < 2; gi++) {
@@ -168,6 +169,7 @@ exact_kernel(const __grid_constant__ CUtensorMap xmap, const ExactArgs A) {
                 }
                 if (++s == KP) { s = 0; round++; }
             }
+            if (kb_end < U.kb1) goto done;
         }
     } else if (warp >= kExDeq0 && warp < kExEpi0) {
         // ================= expansion: group (warp - 4) / 4 takes every third k-block =================
@@ -180,7 +182,7 @@ exact_kernel(const __grid_constant__ CUtensorMap xmap, const ExactArgs A) {
             for (int kb = U.kb0; kb < U.kb1; kb++, it++, (++turn == kExGroups ? turn = 0 : 0), (++sp == KP ? (sp = 0, rp++) : 0)) {
                 if (turn != grp) continue;
                 // at its last k-block this group waited for the MMAs of k-block it - 6 = it - KP: the packed slot's earlier trips are over
-                if (!mbar_wait_lim(p_full(sp), (uint32_t)(rp & 1))) goto done;
+                if (!mbar_wait_lim(p_full(sp), (uint32_t)(rp & 1), A.waits)) goto done;
                 typename E::Codes cw[2];
 #pragma unroll
                 for (int gi = 0; gi < 2; gi++) E::load(pring + sp * SM::kPacked + gi * SM::kGroup + dw * E::kTileBytes, lane, cw[gi]);
@@ -194,7 +196,7 @@ exact_kernel(const __grid_constant__ CUtensorMap xmap, const ExactArgs A) {
                         lo[gi][2 * k4] = h2_to_bf2(a[0]); lo[gi][2 * k4 + 1] = h2_to_bf2(a[2]);
                         hi[gi][2 * k4] = h2_to_bf2(a[1]); hi[gi][2 * k4 + 1] = h2_to_bf2(a[3]);
                     }
-                if (!mbar_wait_lim(a_empty(grp), (uint32_t)((ra & 1) ^ 1))) goto done;
+                if (!mbar_wait_lim(a_empty(grp), (uint32_t)((ra & 1) ^ 1), A.waits)) goto done;
                 ra++;
 #pragma unroll
                 for (int gi = 0; gi < 2; gi++)
@@ -237,7 +239,7 @@ exact_kernel(const __grid_constant__ CUtensorMap xmap, const ExactArgs A) {
 #pragma unroll
                 for (int i = 0; i < 4; i++) {
                     if (kb + i >= U.kb1) break;
-                    if (!mbar_wait_lim(t_full(tb), (uint32_t)(rt & 1))) goto done;
+                    if (!mbar_wait_lim(t_full(tb), (uint32_t)(rt & 1), A.waits)) goto done;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
                     for (int c = 0; c < 32; c += 16) {
@@ -270,6 +272,13 @@ exact_kernel(const __grid_constant__ CUtensorMap xmap, const ExactArgs A) {
     }
 done:
     __syncwarp();
+    // behind a wait that ran out copies and MMAs may still be under way: nobody leaves their memory
+    if (warp == 0) drain_ring(round * KX + s, KX, x_full, A.waits);
+    if (warp == 2) drain_ring(round * KP + s, KP, p_full, A.waits);
+    if (warp == 1) {
+        if (rank == 0) umma2_commit_w(drained, leader);    // arrives in both CTAs
+        mbar_wait_lim(drained, 0u, Waits{A.waits.word, kWaitCycles});
+    }
     __syncthreads();
     cluster_sync_all();
     if (warp == 3) {
@@ -365,6 +374,7 @@ int gemm_exact_launch(const void* w, int qt, int64_t n_rows, int64_t k, const vo
     if (const int rc = encode_rows(&map, workspace, true, 3 * m, k, 32)) return rc;
     const ExactPlan p = exact_plan(n_rows, k / 64, m);
     ExactArgs A = {};
+    if (const int rc = make_waits(&A.waits, kWaitCycles)) return rc;
     A.w = (const uint8_t*)w; A.G = make_geom(n_rows, k, qt); A.M = (int)m; A.tt = p.tt; A.n_fp = (int)((n_rows / 128 + 1) / 2); A.ksplit = p.ks;
     A.y = (float*)y; A.bias = (const float*)bias; A.accumulate = accumulate; A.part = (float*)((char*)workspace + exact_planes_bytes(k, m));
     const int64_t units = (int64_t)A.n_fp * ((m + p.tt - 1) / p.tt) * p.ks;
@@ -384,6 +394,5 @@ int gemm_exact_launch(const void* w, int qt, int64_t n_rows, int64_t k, const vo
     }
     return check_launch();
 }
-int gemm_exact_wait_expired() { return gemmtc::wait_expired_here(); }
 
 }  // namespace lowbit

@@ -26,7 +26,7 @@
 // The signals between the two CTAs are plain arrivals: with cluster-scope release / acquire on them (a full memory fence per
 // arrival) a k-block took 0.75 us instead of 0.25; what they order is shared memory, written behind a proxy fence and read by the
 // tensor cores of the SM that wrote it.
-// Every wait is bounded: one that runs out raises g_wait_expired (lowbit_gemm_wait_expired) and the kernel winds down.
+// Every wait is bounded: see tc_common.cuh.
 #include "tc_pair.cuh"
 
 namespace lowbit {
@@ -49,7 +49,7 @@ template <int QT> struct PairSmem {
     static constexpr int kX = (232448 - kFixed) / kTileBytesAB < 8 ? (232448 - kFixed) / kTileBytesAB : 8;      // slots of 128 rows x 128 bytes
     static constexpr int kTotal = kFixed + kX * kTileBytesAB;
     static_assert(kX >= 3 && kP == 2 * kA && kTotal <= 232448, "ring depths");
-    static_assert((3 * kX + 2 * kP + 2 * kA + 4) * 8 + 8 <= 512, "barrier region");
+    static_assert((3 * kX + 2 * kP + 2 * kA + 5) * 8 + 8 <= 512, "barrier region");
 };
 
 struct PairArgs {
@@ -68,6 +68,7 @@ struct PairArgs {
     void* y; int y_dtype;
     const void* bias; int accumulate;
     float* part;                       // ksplit > 1: [ksplit][M][N]
+    Waits waits;
 };
 
 // gate (lanes 0-15) and up (lanes 16-31) of 16 features and 16 tokens -> act(gate) * up: the halves exchange one token of every two,
@@ -100,7 +101,8 @@ pair_kernel(const __grid_constant__ CUtensorMap xmap, const PairArgs A) {
     auto a_empty = [&](int s) { return bars + (3 * KX + 2 * KP + KA + s) * 8; };
     auto tmem_full = [&](int b) { return bars + (3 * KX + 2 * KP + 2 * KA + b) * 8; };
     auto tmem_empty = [&](int b) { return bars + (3 * KX + 2 * KP + 2 * KA + 2 + b) * 8; };   // CTA 0: both epilogues have drained it
-    const uint32_t tmem_slot = bars + (3 * KX + 2 * KP + 2 * KA + 4) * 8;
+    const uint32_t drained = bars + (3 * KX + 2 * KP + 2 * KA + 4) * 8;               // every MMA that was issued is done
+    const uint32_t tmem_slot = drained + 8;
     int* const cum = reinterpret_cast<int*>(smem_raw + (obuf + SM::kOut - smem_u32(smem_raw)));    // experts: tiles before expert e
     int* const off = cum + kMaxExperts + 4;                                                        //          rows before expert e
 
@@ -116,6 +118,7 @@ pair_kernel(const __grid_constant__ CUtensorMap xmap, const PairArgs A) {
         for (int s = 0; s < KP; s++) { mbar_init(p_full(s), 1); mbar_init(p_empty(s), 4); }
         for (int s = 0; s < KA; s++) { mbar_init(a_full(s), 8); mbar_init(a_empty(s), 1); }
         for (int b = 0; b < 2; b++) { mbar_init(tmem_full(b), 1); mbar_init(tmem_empty(b), 8); }
+        mbar_init(drained, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     // an expert's rows in tiles of at most 256 tokens, evenly cut; few rows are another kernel's
@@ -171,16 +174,16 @@ pair_kernel(const __grid_constant__ CUtensorMap xmap, const PairArgs A) {
     };
     Unit U;
     U.e = 0;
+    const uint32_t leader = elect_leader();
+    int s = 0, round = 0;                                  // the two copying warps' place in their ring
 
     if (warp == 0) {
         // ================= activations: this CTA's half of the tile's tokens =================
-        const uint32_t leader = elect_leader();
-        int s = 0, round = 0;
         for (int unit = blockIdx.x >> 1; unit < n_units; unit += stride) {
             decode(unit, U);
             const int half = U.n_tok >> 1, boxes = (half + 31) >> 5, row0 = U.m0 + rank * half;
             for (int kb = U.kb0; kb < U.kb1; kb++) {
-                if (!mbar_wait_lim(x_empty(s), (uint32_t)((round & 1) ^ 1))) goto done;
+                if (!mbar_wait_lim(x_empty(s), (uint32_t)((round & 1) ^ 1), A.waits)) goto done;
                 mbar_expect_tx_w(x_full(s), boxes * 4096, leader);
                 for (int i = 0; i < boxes; i++)
                     tma_load_2d_w(xring + s * kTileBytesAB + i * 4096, &xmap, kb * 64, row0 + i * 32, x_full(s), leader);
@@ -190,7 +193,6 @@ pair_kernel(const __grid_constant__ CUtensorMap xmap, const PairArgs A) {
     } else if (warp == 1) {
         if (rank == 0) {
             // ================= MMA issuer =================
-            const uint32_t leader = elect_leader();
             int sx = 0, rx = 0, it = 0, ti = 0;
             bool ready = false;
             for (int unit = blockIdx.x >> 1; unit < n_units; unit += stride, ti++) {
@@ -198,12 +200,12 @@ pair_kernel(const __grid_constant__ CUtensorMap xmap, const PairArgs A) {
                 // c F32 (1<<4), a/b format (0 f16, 1 bf16), both K-major, N (>>3 at bit 17), M = 256 (>>4 at bit 24)
                 const uint32_t idesc = (1u << 4) | ((BF ? 1u : 0u) << 7) | ((BF ? 1u : 0u) << 10) | (((uint32_t)U.n_tok >> 3) << 17) | ((256u >> 4) << 24);
                 const int buf = ti & 1;
-                if (!mbar_wait_lim(tmem_empty(buf), (uint32_t)(((ti >> 1) & 1) ^ 1))) goto done;
+                if (!mbar_wait_lim(tmem_empty(buf), (uint32_t)(((ti >> 1) & 1) ^ 1), A.waits)) goto done;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t acc = tmem_base + buf * kPairTok;
                 for (int kb = U.kb0; kb < U.kb1; kb++) {
                     const int sa = it & 3;
-                    if (!mbar_wait3_lim(ready, x_full(sx), (uint32_t)(rx & 1), xp_full(sx), (uint32_t)(rx & 1), a_full(sa), (uint32_t)((it >> 2) & 1))) goto done;
+                    if (!mbar_wait3_lim(ready, x_full(sx), (uint32_t)(rx & 1), xp_full(sx), (uint32_t)(rx & 1), a_full(sa), (uint32_t)((it >> 2) & 1), A.waits)) goto done;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint64_t ad = make_desc(aring + sa * kTileBytesAB), xd = make_desc(xring + sx * kTileBytesAB);
 #pragma unroll
@@ -224,7 +226,7 @@ pair_kernel(const __grid_constant__ CUtensorMap xmap, const PairArgs A) {
             for (int unit = blockIdx.x >> 1; unit < n_units; unit += stride) {
                 decode(unit, U);
                 for (int kb = U.kb0; kb < U.kb1; kb++) {
-                    if (!mbar_wait_lim(x_full(sx), (uint32_t)(rx & 1))) goto done;
+                    if (!mbar_wait_lim(x_full(sx), (uint32_t)(rx & 1), A.waits)) goto done;
                     if (lane == 0) mbar_arrive_at(xp_full(sx), 0);
                     if (++sx == KX) { sx = 0; rx++; }
                 }
@@ -232,17 +234,16 @@ pair_kernel(const __grid_constant__ CUtensorMap xmap, const PairArgs A) {
         }
     } else if (warp == 2) {
         // ================= packed weights of this CTA's two 64-row groups =================
-        const uint32_t leader = elect_leader();
         const int n_rg = (int)(A.G.rows >> 6);
-        int s = 0, round = 0;
         for (int unit = blockIdx.x >> 1; unit < n_units; unit += stride) {
             decode(unit, U);
             const uint8_t* w0 = A.offs ? reinterpret_cast<const uint8_t*>(A.tab[U.e]) : A.w;
             const uint8_t* w1 = A.act ? (A.offs ? reinterpret_cast<const uint8_t*>(A.tab2[U.e]) : A.w2) : w0;
             // the last pair's second tile may not exist: it repeats the last group and stores nothing
             const int64_t rg0 = min(A.act ? U.ft : 2 * U.ft, n_rg - 1), rg1 = min(A.act ? U.ft : 2 * U.ft + 1, n_rg - 1);
-            for (int kb = U.kb0; kb < U.kb1; kb++) {
-                if (!mbar_wait_lim(p_empty(s), (uint32_t)((round & 1) ^ 1))) goto done;
+            const int kb_end = A.waits.limit < 0 ? (U.kb0 + U.kb1) / 2 : U.kb1;
+            for (int kb = U.kb0; kb < kb_end; kb++) {
+                if (!mbar_wait_lim(p_empty(s), (uint32_t)((round & 1) ^ 1), A.waits)) goto done;
                 mbar_expect_tx_w(p_full(s), SM::kPacked, leader);
 #pragma unroll
                 for (int gi = 0; gi < 2; gi++) {
@@ -255,6 +256,7 @@ pair_kernel(const __grid_constant__ CUtensorMap xmap, const PairArgs A) {
                 }
                 if (++s == KP) { s = 0; round++; }
             }
+            if (kb_end < U.kb1) goto done;
         }
     } else if (warp >= kPairDeq0 && warp < kPairEpi0) {
         // ================= dequant: group (warp - 4) / 4 takes every fourth k-block; a warp expands 16 rows of either row group =================
@@ -269,7 +271,7 @@ pair_kernel(const __grid_constant__ CUtensorMap xmap, const PairArgs A) {
             for (; it < end; it += 4) {
                 const int sp = it & (KP - 1), rp = it / KP;
                 // the slot's last trip (k-block it - 8) was this group's own, so the parity is unambiguous
-                if (!mbar_wait_lim(p_full(sp), (uint32_t)(rp & 1))) goto done;
+                if (!mbar_wait_lim(p_full(sp), (uint32_t)(rp & 1), A.waits)) goto done;
                 const uint32_t pk = pring + sp * SM::kPacked;
                 typename E::Codes cw[2];
                 uint32_t dq[2], mq[2] = {0u, 0u};
@@ -299,7 +301,7 @@ pair_kernel(const __grid_constant__ CUtensorMap xmap, const PairArgs A) {
                         hi[gi][2 * k4] = a[1]; hi[gi][2 * k4 + 1] = a[3];
                     }
                 }
-                if (!mbar_wait_lim(a_empty(grp), (uint32_t)(((it >> 2) & 1) ^ 1))) goto done;
+                if (!mbar_wait_lim(a_empty(grp), (uint32_t)(((it >> 2) & 1) ^ 1), A.waits)) goto done;
 #pragma unroll
                 for (int gi = 0; gi < 2; gi++)
 #pragma unroll
@@ -333,7 +335,7 @@ pair_kernel(const __grid_constant__ CUtensorMap xmap, const PairArgs A) {
                 b = A.y_dtype == DT_F32 ? ((const float*)A.bias)[n] : A.y_dtype == DT_F16 ? __half2float(((const __half*)A.bias)[n])
                                                                                           : __bfloat162float(((const __nv_bfloat16*)A.bias)[n]);
             // the four warps go on together or not at all: they meet at named barriers below
-            uint32_t go = mbar_wait_lim(tmem_full(buf), (uint32_t)((ti >> 1) & 1)) ? 1u : 0u;
+            uint32_t go = mbar_wait_lim(tmem_full(buf), (uint32_t)((ti >> 1) & 1), A.waits) ? 1u : 0u;
             asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %0, 0;\n\tbarrier.cta.red.and.pred q, 1, 128, p;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "+r"(go)::"memory");
             if (!go) goto done;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -428,6 +430,13 @@ pair_kernel(const __grid_constant__ CUtensorMap xmap, const PairArgs A) {
     }
 done:
     __syncwarp();
+    // behind a wait that ran out copies and MMAs may still be under way: nobody leaves their memory
+    if (warp == 0) drain_ring(round * KX + s, KX, x_full, A.waits);
+    if (warp == 2) drain_ring(round * KP + s, KP, p_full, A.waits);
+    if (warp == 1) {
+        if (rank == 0) umma2_commit_w(drained, leader);    // arrives in both CTAs
+        mbar_wait_lim(drained, 0u, Waits{A.waits.word, kWaitCycles});
+    }
     __syncthreads();
     cluster_sync_all();                                    // nobody signals a CTA that has left, no MMA reads its memory
     if (warp == 3) {
@@ -560,6 +569,7 @@ int gemm_tc_launch(const void* w, int qt, int64_t n_rows, int64_t k, const void*
     CUtensorMap map;
     if (const int rc = encode_rows(&map, x, bf, m, k, 32)) return rc;
     PairArgs A = {};
+    if (const int rc = make_waits(&A.waits, kWaitCycles)) return rc;
     A.w = (const uint8_t*)w; A.G = make_geom(n_rows, k, qt); A.M = (int)m; A.y = y; A.y_dtype = y_dtype; A.bias = bias; A.accumulate = accumulate;
     A.n_fp = (int)((n_rows / 128 + 1) / 2);
     PairPlan p = pair_plan(pair_pace(qt, bf), A.n_fp, k / 64, m, n_rows, true);
@@ -589,6 +599,7 @@ int gemm_tc_mlp_launch(const void* w_gate, const void* w_up, int act, int qt, in
     CUtensorMap map;
     if (const int rc = encode_rows(&map, x, bf, m, k, 32)) return rc;
     PairArgs A = {};
+    if (const int rc = make_waits(&A.waits, kWaitCycles)) return rc;
     A.w = (const uint8_t*)w_gate; A.w2 = (const uint8_t*)w_up; A.act = act; A.G = make_geom(n_rows, k, qt); A.M = (int)m; A.y = y; A.y_dtype = y_dtype;
     A.n_fp = (int)((n_rows / 64 + 1) / 2);
     PairPlan p = pair_plan(pair_pace(qt, bf), A.n_fp, k / 64, m, 2 * n_rows, true);
@@ -620,6 +631,7 @@ int gemm_tc_experts_launch(const unsigned long long* tab, const unsigned long lo
     CUtensorMap map;
     if (const int rc = encode_rows(&map, x, bf, rows, k, 32)) return rc;
     PairArgs A = {};
+    if (const int rc = make_waits(&A.waits, kWaitCycles)) return rc;
     A.tab = tab; A.tab2 = tab2; A.act = tab2 ? act : 0; A.offs = offs; A.n_experts = n_experts;
     A.G = make_geom(n_rows, k, qt); A.M = (int)rows; A.y = y; A.y_dtype = y_dtype; A.ksplit = 1; A.tt = kPairTok;
     A.n_fp = (int)((n_rows / (tab2 ? 64 : 128) + 1) / 2);
@@ -627,7 +639,5 @@ int gemm_tc_experts_launch(const unsigned long long* tab, const unsigned long lo
     if (const int rc = pair_launch(qt, bf, map, A, most * A.n_fp, st)) return rc;
     return check_launch();
 }
-
-int gemm_tc_wait_expired() { return gemmtc::wait_expired_here(); }
 
 }  // namespace lowbit

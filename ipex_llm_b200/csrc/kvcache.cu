@@ -131,6 +131,7 @@ struct SdpArgs {
     float* part;                                                   // [B][Hkv][row tiles][n_split][RT * (D + 2)]
     void* out; int out_dtype;                                      // [B][Hq][S][D] contiguous
     int64_t o_sb, o_sh, o_ss;                                      // prefill kernel only: element strides of out (rows of D contiguous)
+    Waits waits;                                                   // prefill kernel only
 };
 
 // key count and keys per split of this launch: the host's values, or -- when the cache length lives in device memory
@@ -438,7 +439,6 @@ size_t sdp_workspace(int B, int Hq, int Hkv, int S, int L, int D, bool mma) {
     return (size_t)B * Hkv * sdp_tiles(Hq, Hkv, S, mma) * sdp_splits(B, Hq, Hkv, S, L, D, mma) * sdp_rt(Hq, Hkv, S, mma) * (D + 2) * sizeof(float);
 }
 }  // namespace
-int sdp_prompt_wait_expired() { return gemmtc::wait_expired_here(); }
 }  // namespace lowbit
 
 // ------------------------------------------------------------------ C ABI (declared in include/b200_lowbit.h)

@@ -73,6 +73,11 @@ bool moe_supported(int qt, int64_t hidden, int64_t inter, int top_k);
 size_t moe_workspace_size(int64_t hidden, int64_t inter, int top_k, int x_dtype);
 int moe_launch(const MoeParams& P, cudaStream_t st);
 
+// bounded waits of the prompt kernels: a wait that runs out writes the device's word, which lies in host memory, and the launch's results
+// are undefined; the next check_launch() on the device reports and clears it
+struct Waits { unsigned int* word; long long limit; };       // limit: SM clocks
+int make_waits(Waits* w, long long limit);                   // the current device's, with this limit unless the calling thread has set one
+
 // up to this many half-precision rows a product keeps the weights as code x scale in 32 bits (the GEMV); above, the tensor cores take them
 // rounded once to the activation dtype.  Measured line: see use_skinny in capi.cu
 constexpr int64_t kExactRows = 16;
@@ -93,15 +98,12 @@ int gemm_tc_mlp_launch(const void* w_gate, const void* w_up, int act, int qt, in
 size_t gemm_tc_mlp_workspace_size(int64_t n_rows, int64_t k, int64_t m);
 int gemm_tc_experts_launch(const unsigned long long* tab, const unsigned long long* tab2, int act, const int* offs, int n_experts, int qt,
                            int64_t n_rows, int64_t k, const void* x, int x_dtype, int64_t rows, void* y, int y_dtype, cudaStream_t st);
-int gemm_tc_wait_expired();       // 1 after a wait of the two-SM kernel ran out on the current device (its results are then undefined)
-int sdp_prompt_wait_expired();    // the same of the prompt attention (kvcache.cu)
 
 // gemm_exact.cu (the fp32 prompt matmul: codes and activation planes exact on the tensor cores)
 bool gemm_exact_supported(int qt, int64_t n_rows, int64_t k, int64_t m);
 size_t gemm_exact_workspace_size(int64_t n_rows, int64_t k, int64_t m);
 int gemm_exact_launch(const void* w, int qt, int64_t n_rows, int64_t k, const void* x, int64_t m, void* y, const void* bias, int accumulate,
                       void* workspace, size_t workspace_bytes, cudaStream_t st);
-int gemm_exact_wait_expired();
 
 // M above this goes to the tensor-core GEMM when the shape allows, else to chunks of the GEMV
 constexpr int64_t kGemvMaxM = 32;

@@ -77,7 +77,8 @@ sdp_fp8_prompt_kernel(const SdpArgs A, int n_qt) {
     auto s_full = [&](int t) { return bars + 64 + t * 8; };
     auto p_full = [&](int t) { return bars + 80 + t * 8; };
     auto pv_done = [&](int t) { return bars + 96 + t * 8; };
-    const uint32_t tmem_slot = bars + 112;
+    const uint32_t drained = bars + 112;                               // every MMA that was issued is done
+    const uint32_t tmem_slot = bars + 120;
     constexpr uint32_t TMEM_COLS = NT * 256;                           // S_t at 128 t, O_t behind all S
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const int hq = blockIdx.x % A.Hq, b = blockIdx.x / A.Hq, hkv = hq / (A.Hq / A.Hkv);
@@ -135,6 +136,7 @@ sdp_fp8_prompt_kernel(const SdpArgs A, int n_qt) {
     if (threadIdx.x == 0) {
         for (int s = 0; s < SP_SLOTS; s++) { mbar_init(kv_full(s), 4); mbar_init(kv_empty(s), 1); }
         for (int t = 0; t < 2; t++) { mbar_init(s_full(t), 1); mbar_init(p_full(t), 4); mbar_init(pv_done(t), 1); }
+        mbar_init(drained, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 4 * NT + 4) {
@@ -147,6 +149,7 @@ sdp_fp8_prompt_kernel(const SdpArgs A, int n_qt) {
     uint32_t tmem;
     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem) : "r"(tmem_slot));
 
+    const uint32_t leader = elect_leader();
     if (warp < 4 * NT) {
         // ================= softmax: thread = query row =================
         const int t = warp >> 2, quarter = warp & 3, r = 32 * quarter + lane, row = q0 + t * SP_ROWS + r;
@@ -159,7 +162,7 @@ sdp_fp8_prompt_kernel(const SdpArgs A, int n_qt) {
             const int64_t mbase = b * A.m_sb + hq * A.m_sh + (int64_t)row * A.m_ss;
             float m_ref = -CUDART_INF_F, sum = 0.0f;
             for (int j = 0; j < nkt; j++) {
-                if (!mbar_wait_lim(s_full(t), (uint32_t)(j & 1))) goto done;
+                if (!mbar_wait_lim(s_full(t), (uint32_t)(j & 1), A.waits)) goto done;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const int k0 = j * SP_KEYS;
                 const bool plain = k0 + SP_KEYS <= plain_end;
@@ -238,7 +241,7 @@ sdp_fp8_prompt_kernel(const SdpArgs A, int n_qt) {
                 __syncwarp();
                 if (lane == 0) mbar_arrive(p_full(t));
             }
-            if (!mbar_wait_lim(pv_done(t), (uint32_t)((nkt - 1) & 1))) goto done;
+            if (!mbar_wait_lim(pv_done(t), (uint32_t)((nkt - 1) & 1), A.waits)) goto done;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const float inv = sum > 0.0f ? 1.0f / sum : 0.0f;                       // a row with every key masked gives zeros
             const int64_t oi = (int64_t)b * A.o_sb + (int64_t)hq * A.o_sh + (int64_t)row * A.o_ss;
@@ -275,9 +278,10 @@ sdp_fp8_prompt_kernel(const SdpArgs A, int n_qt) {
         // a thread's 16 elements are two chunks of one row's half; lanes of the second half write them in the other order, so that a
         // quarter warp (one row) meets every bank once
         const int half = piece >> 2, c0 = 2 * (piece & 3) + half;
-        for (int item = 0; item < 2 * nk; item++) {
+        const int items = A.waits.limit < 0 ? nk : 2 * nk;
+        for (int item = 0; item < items; item++) {
             const int s = item % SP_SLOTS, round = item / SP_SLOTS;
-            if (!mbar_wait_lim(kv_empty(s), (uint32_t)((round & 1) ^ 1))) goto done;
+            if (!mbar_wait_lim(kv_empty(s), (uint32_t)((round & 1) ^ 1), A.waits)) goto done;
             const uint32_t dst = ring + s * SP_TILE + half * (SP_TILE / 2);
 #pragma unroll
             for (int i = 0; i < 8; i++) {
@@ -296,7 +300,6 @@ sdp_fp8_prompt_kernel(const SdpArgs A, int n_qt) {
         }
     } else {
         // ================= MMA issuer: the whole warp runs the loop, one elected lane issues =================
-        const uint32_t leader = elect_leader();
         // c F32, a / b fp16, N = 128, M = 128; S: both operands K-major; O: A in TMEM, B (values) MN-major (bit 16)
         const uint32_t id_s = (1u << 4) | ((128u >> 3) << 17) | ((128u >> 4) << 24), id_o = id_s | (1u << 16);
         const int nk0 = tiles_of(0), nk1 = NT == 2 ? tiles_of(1) : 0;
@@ -318,7 +321,7 @@ sdp_fp8_prompt_kernel(const SdpArgs A, int n_qt) {
             umma_commit_w(pv_done(t), leader);
         };
         if (nk > 0) {
-            if (!mbar_wait_lim(kv_full(0), 0u)) goto done;
+            if (!mbar_wait_lim(kv_full(0), 0u, A.waits)) goto done;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             for (int t = 0; t < NT; t++) {
                 if ((t == 0 ? nk0 : nk1) == 0) continue;
@@ -328,18 +331,18 @@ sdp_fp8_prompt_kernel(const SdpArgs A, int n_qt) {
         }
         for (int j = 0; j < nk; j++) {
             const int vi = 2 * j + 1, ki = 2 * j + 2;
-            if (!mbar_wait_lim(kv_full(vi % SP_SLOTS), (uint32_t)((vi / SP_SLOTS) & 1))) goto done;
-            if (j + 1 < nk && !mbar_wait_lim(kv_full(ki % SP_SLOTS), (uint32_t)((ki / SP_SLOTS) & 1))) goto done;
+            if (!mbar_wait_lim(kv_full(vi % SP_SLOTS), (uint32_t)((vi / SP_SLOTS) & 1), A.waits)) goto done;
+            if (j + 1 < nk && !mbar_wait_lim(kv_full(ki % SP_SLOTS), (uint32_t)((ki / SP_SLOTS) & 1), A.waits)) goto done;
             const int last = NT == 2 && j < nk1 ? 1 : 0;
             for (int t = 0; t < NT; t++) {
                 const int nkt = t == 0 ? nk0 : nk1;
                 if (j >= nkt) continue;
-                if (!mbar_wait_lim(p_full(t), (uint32_t)(j & 1))) goto done;
+                if (!mbar_wait_lim(p_full(t), (uint32_t)(j & 1), A.waits)) goto done;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 values(t, j);
                 if (t == last) umma_commit_w(kv_empty(vi % SP_SLOTS), leader);
                 if (j + 1 < nkt) {
-                    if (!mbar_wait_lim(pv_done(t), (uint32_t)(j & 1))) goto done;         // S and P share their columns
+                    if (!mbar_wait_lim(pv_done(t), (uint32_t)(j & 1), A.waits)) goto done;         // S and P share their columns
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     scores(t, j + 1);
                 }
@@ -349,6 +352,11 @@ sdp_fp8_prompt_kernel(const SdpArgs A, int n_qt) {
     }
 done:
     __syncwarp();
+    if (warp == 4 * NT + 4) {
+        // behind a wait that ran out MMAs may still be under way: nobody leaves their memory
+        umma_commit_w(drained, leader);
+        mbar_wait_lim(drained, 0u, Waits{A.waits.word, kWaitCycles});
+    }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == 4 * NT + 4) {
@@ -371,7 +379,8 @@ template <int NT, bool MASK> int sdp_prompt_launch_nt(const SdpArgs& A, cudaStre
     return check_launch();
 }
 // 256 rows a CTA share every key tile's expansion, 128 spread a short prompt over twice the SMs: two tiles once they fill the chip
-int sdp_prompt_launch(const SdpArgs& A, cudaStream_t st) {
+int sdp_prompt_launch(SdpArgs A, cudaStream_t st) {
+    if (const int rc = make_waits(&A.waits, gemmtc::kWaitCycles)) return rc;
     const int64_t two = (int64_t)A.B * A.Hq * ((A.S + 2 * SP_ROWS - 1) / (2 * SP_ROWS));
     if (A.mask) return two >= sm_count() ? sdp_prompt_launch_nt<2, true>(A, st) : sdp_prompt_launch_nt<1, true>(A, st);
     return two >= sm_count() ? sdp_prompt_launch_nt<2, false>(A, st) : sdp_prompt_launch_nt<1, false>(A, st);

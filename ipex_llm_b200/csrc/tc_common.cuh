@@ -67,25 +67,27 @@ __device__ __forceinline__ void tma_load_2d_w(uint32_t dst, const CUtensorMap* m
                  "@q cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];\n\t}"
                  ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(bar), "r"(leader) : "memory");
 }
-// ---- bounded waits: one that runs out raises this translation unit's flag, and the kernel winds down
+// ---- bounded waits: one that runs out raises the device's word in host memory (lowbit_internal.h), and the kernel winds down: every
+// role leaves its loop, waits for the copies and MMAs of its own that are still under way, and the block frees its TMEM
 constexpr long long kWaitCycles = 4000000000ll;           // about two seconds
-static __device__ unsigned int g_wait_expired;
 __device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
     uint32_t ok;
     asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
                  : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     return ok != 0;
 }
+// whole warp.  A limit below zero (tests): copies of the kernel stop half-way, and the waits for them run out after that many clocks
+__device__ __forceinline__ bool wait_over(long long t0, const Waits& W) {
+    if (!__any_sync(0xffffffffu, clock64() - t0 > (W.limit < 0 ? -W.limit : W.limit))) return false;
+    if ((threadIdx.x & 31) == 0) { *(volatile unsigned int*)W.word = 1u; __threadfence_system(); }
+    return true;
+}
 // whole warp; the same answer in every lane.  false: the limit ran out
-__device__ __forceinline__ bool mbar_wait_lim(uint32_t bar, uint32_t parity) {
+__device__ __forceinline__ bool mbar_wait_lim(uint32_t bar, uint32_t parity, const Waits& W) {
     if (__all_sync(0xffffffffu, mbar_test(bar, parity))) return true;
     const long long t0 = clock64();
-    while (!__all_sync(0xffffffffu, mbar_test(bar, parity))) {
-        if (__any_sync(0xffffffffu, clock64() - t0 > kWaitCycles)) {
-            if ((threadIdx.x & 31) == 0) atomicExch(&g_wait_expired, 1u);
-            return false;
-        }
-    }
+    while (!__all_sync(0xffffffffu, mbar_test(bar, parity)))
+        if (wait_over(t0, W)) return false;
     return true;
 }
 // three barriers at once: a test takes about 100 clocks to answer, and these overlap.  Tests that do not suspend the warp: the answer
@@ -101,21 +103,18 @@ __device__ __forceinline__ bool mbar_test3(uint32_t b0, uint32_t p0, uint32_t b1
     return ok != 0;
 }
 // `ready`: what mbar_test3 said earlier
-__device__ __forceinline__ bool mbar_wait3_lim(bool ready, uint32_t b0, uint32_t p0, uint32_t b1, uint32_t p1, uint32_t b2, uint32_t p2) {
+__device__ __forceinline__ bool mbar_wait3_lim(bool ready, uint32_t b0, uint32_t p0, uint32_t b1, uint32_t p1, uint32_t b2, uint32_t p2, const Waits& W) {
     if (__all_sync(0xffffffffu, ready)) return true;
     const long long t0 = clock64();
-    while (!__all_sync(0xffffffffu, mbar_test3(b0, p0, b1, p1, b2, p2))) {
-        if (__any_sync(0xffffffffu, clock64() - t0 > kWaitCycles)) {
-            if ((threadIdx.x & 31) == 0) atomicExch(&g_wait_expired, 1u);
-            return false;
-        }
-    }
+    while (!__all_sync(0xffffffffu, mbar_test3(b0, p0, b1, p1, b2, p2)))
+        if (wait_over(t0, W)) return false;
     return true;
 }
-static int wait_expired_here() {
-    unsigned int v = 0;
-    if (cudaMemcpyFromSymbol(&v, g_wait_expired, sizeof(v)) != cudaSuccess) { cudaGetLastError(); return -1; }
-    return (int)v;
+// the phases of the last `n` of `issued` trips around a ring of n slots are complete: this warp's copies have landed
+template <typename Full> __device__ __forceinline__ void drain_ring(int issued, int n, Full full, const Waits& W) {
+    const Waits late = {W.word, kWaitCycles};
+    for (int i = issued > n ? issued - n : 0; i < issued; i++)
+        if (!mbar_wait_lim(full(i % n), (uint32_t)((i / n) & 1), late)) return;
 }
 __device__ __forceinline__ uint32_t elect_leader() {
     uint32_t pred;

@@ -326,6 +326,8 @@ _lib.lowbit_moe_tokens_cuda.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_
 _lib.lowbit_moe_tokens_cuda.restype = ctypes.c_int
 _lib.lowbit_moe_tokens_last_unrouted.argtypes = []
 _lib.lowbit_moe_tokens_last_unrouted.restype = ctypes.c_int64
+_lib.lowbit_debug_set_wait_limit.argtypes = [ctypes.c_longlong]
+_lib.lowbit_debug_set_wait_limit.restype = None
 _lib.lowbit_gemm_wait_expired.argtypes = []
 _lib.lowbit_gemm_wait_expired.restype = ctypes.c_int
 
@@ -350,7 +352,8 @@ def lowbit_moe_tokens_last_unrouted():
 
 
 def lowbit_gemm_wait_expired():
-    """whether a bounded wait inside the prompt matmul or the prompt attention has run out on the current device (synchronises)"""
+    """whether a bounded wait inside the prompt matmul or the prompt attention has run out on the current device and no call has
+    reported it yet (synchronises)"""
     return _lib.lowbit_gemm_wait_expired() == 1
 
 
