@@ -208,3 +208,18 @@ def test_scratch_off_a_16_byte_boundary(lbl, native_lib, cuda_device, offset):
         with pytest.raises(RuntimeError):
             native_lib.lowbit_matmul_cuda(wg.data_ptr(), qt, n, k, x.data_ptr(), native_lib.DT_F32, rows, y.data_ptr(), native_lib.DT_F32, None, False,
                                           ws.data_ptr(), ws.numel(), stream)
+
+
+@pytest.mark.parametrize("qtype,dtype", [("sym_int4", torch.float16), ("asym_int4", torch.bfloat16), ("nf4", torch.float16), ("fp8_e5m2", torch.bfloat16)])
+@pytest.mark.parametrize("act", [0, 1])
+@pytest.mark.parametrize("m,n,k", [(100, 2048, 4096), (65, 384, 2048), (150, 1024, 8192)])
+def test_prompt_mlp_with_a_split_k_range(lbl, native_lib, cuda_device, qtype, dtype, act, m, n, k):
+    """few tiles, long rows: gate and up partial sums in scratch, the activation in the second launch"""
+    ((wg, g), (wu, p)), qt = weights(lbl, cuda_device, m, n, k, qtype, 2)
+    x = acts(cuda_device, n, m, k, dtype)
+    # a size of at least two splits: 8 bytes of partial sums per split, token and feature
+    assert native_lib.lowbit_mlp_workspace_size(n, k, m, native_lib.DT_F16) >= 2 * 8 * m * n
+    want, bound = gated(x.double(), g, p, U[dtype], act)
+    y32 = lbl.mlp_forward(x, wg, wu, m, k, n, act, qt, out=torch.empty(m, n, dtype=torch.float32, device=cuda_device))
+    assert bool(((y32.double() - want).abs() <= bound).all())
+    assert torch.equal(lbl.mlp_forward(x, wg, wu, m, k, n, act, qt), y32.to(dtype))
