@@ -446,6 +446,8 @@ def moe_forward_tokens(x: torch.Tensor, topk_ids: torch.Tensor, topk_weight: tor
     invalidInputError(topk_weight.dtype in _TORCH_TO_DT and topk_weight.shape == topk_ids.shape, "topk_weight must match topk_ids")
     invalidInputError(gates.numel() == ups.numel() == downs.numel() and gates.element_size() == 8,
                       "gates / ups / downs must be equally long tensors of 64-bit addresses")
+    invalidInputError(x.is_cuda and all(t.device == x.device for t in (topk_ids, topk_weight, gates, ups, downs)),
+                      "activations, routing and address tables must be on one CUDA device")
     x = x.contiguous()
     if x.data_ptr() % 16:
         x = x.clone()                                        # rows cut out of a wider buffer: the kernels load 16 bytes at a time

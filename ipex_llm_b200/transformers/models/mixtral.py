@@ -98,14 +98,15 @@ class LowBitExperts(nn.Module):
     def _many_tokens_ok(self, x, top_k_index, top_k_weights):
         return (x.dim() == 2 and x.shape[0] > 0 and type(self.act_fn).__name__ in ("SiLU", "SiLUActivation") and not self.training
                 and not (torch.is_grad_enabled() and (x.requires_grad or top_k_weights.requires_grad))
-                and top_k_index.dim() == 2 and top_k_index.shape == top_k_weights.shape and top_k_index.dtype in (torch.int32, torch.int64)
+                and top_k_index.dim() == 2 and top_k_index.shape == top_k_weights.shape and top_k_index.shape[0] == x.shape[0]
+                and top_k_index.device == top_k_weights.device == x.device and top_k_index.dtype == torch.int64
                 and top_k_weights.dtype in (torch.float32, torch.float16, torch.bfloat16)
                 and moe_tokens_supported(x, self.num_experts, self.hidden_dim, self.intermediate_dim, top_k_index.shape[1], self.qtype)
                 and not torch.cuda.is_current_stream_capturing())
 
     def forward(self, hidden_states, top_k_index, top_k_weights):
         if hidden_states.shape[0] == 1 and use_fuse_moe(hidden_states, self.qtype) and \
-                self.gate_proj[0].weight.data.device.type == "cuda" and not self.training:
+                top_k_index.device == top_k_weights.device == hidden_states.device and self.gate_proj[0].weight.data.device.type == "cuda" and not self.training:
             return self.fused_one_token(hidden_states, top_k_index, top_k_weights)
         if self._many_tokens_ok(hidden_states, top_k_index, top_k_weights):
             addresses = self._plain_addresses(hidden_states.device)         # None: an expert that has to run itself

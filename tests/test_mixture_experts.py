@@ -271,3 +271,35 @@ def test_long_prompts_run_in_portions(native_lib, cuda_device, monkeypatch, rows
     same(m, x, idx, w)
     with pytest.raises(RuntimeError, match="outside"):
         m(x, torch.where(torch.arange(rows, device=cuda_device)[:, None] == 0, E, idx), w)
+
+
+def test_the_kernels_take_one_device_and_the_loops_types_only(native_lib, monkeypatch):
+    """an address of another device's memory would be read there; what the loop refuses, or serves in its own way, stays with it"""
+    from ipex_llm_b200.transformers import low_bit_linear as lbl
+    from ipex_llm_b200.transformers.models import mixtral
+    m = plain_layer()
+    monkeypatch.setattr(mixtral, "moe_tokens_supported", lambda *a: True)
+    monkeypatch.setattr(torch.cuda, "is_current_stream_capturing", lambda: False)
+    x, idx, w = torch.zeros(6, H, dtype=torch.float16), torch.zeros(6, 2, dtype=torch.int64), torch.zeros(6, 2)
+    with torch.no_grad():
+        assert m._many_tokens_ok(x, idx, w)
+        for args in ((x, idx.to("meta"), w), (x, idx, w.to("meta")), (x.to("meta"), idx, w), (x, idx.int(), w), (x, idx[:5], w[:5]), (x, idx, w[:, :1]),
+                     (x, idx, w.double())):
+            assert not m._many_tokens_ok(*args)
+    tables = [torch.zeros(E, dtype=torch.int64)] * 3
+    with pytest.raises(RuntimeError, match="device"):
+        lbl.moe_forward_tokens(x, idx, w, *tables, H, I, m.qtype)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("rows", [1, 70])
+def test_routing_on_the_host_is_refused(native_lib, cuda_device, rows):
+    m = layer(cuda_device)
+    x = torch.randn(rows, H, device=cuda_device).half()
+    idx, w = routing(cuda_device, rows)
+    for args in ((x, idx.cpu(), w), (x, idx, w.cpu()), (torch.cat([x, x]), torch.cat([idx, idx]).int(), torch.cat([w, w]))):
+        with pytest.raises(RuntimeError):
+            m(*args)
+    part = m(torch.cat([x, x]), idx, w)                                             # rows without a choice come out zero
+    assert not bool(part[rows:].any())
+    same(m, x, idx, w)
