@@ -235,17 +235,6 @@ class DynamicNormalCache(_LayeredCache):
     LAYER = NormalKVLayer
 
 
-_sdp_workspaces = {}
-
-
-def _workspace(device, need):
-    ws = _sdp_workspaces.get(device)
-    if ws is None or ws.numel() < need:
-        ws = torch.empty(int(need * 1.5) + 256, dtype=torch.uint8, device=device)
-        _sdp_workspaces[device] = ws
-    return ws
-
-
 def sdp_fp8(query, key, value, mask, scale, is_causal=False):
     """xe_addons.sdp_fp8(query, key, value, mask, scale): decode attention (new tokens <= 32) straight from the
     uint8 cache.  mask: None or additive [B, 1|H, S, L]."""
@@ -260,7 +249,8 @@ def sdp_fp8(query, key, value, mask, scale, is_causal=False):
             mask = mask.contiguous()
         mask = mask.expand(B, Hq, S, L)            # broadcast dimensions get stride 0: nothing is copied
     out = torch.empty((B, Hq, S, D), dtype=query.dtype, device=query.device)
-    ws = _workspace(query.device, ggml.lowbit_sdp_fp8_workspace_size(B, Hq, Hkv, S, L, D))
+    # this call's own, from the allocator on the current stream: two streams, or a recorded call and a later one, never meet in it
+    ws = torch.empty(ggml.lowbit_sdp_fp8_workspace_size(B, Hq, Hkv, S, L, D), dtype=torch.uint8, device=query.device)
     with torch.cuda.device(query.device):
         ggml.lowbit_sdp_fp8(query, key, value, mask, is_causal, scale, out, ws, _stream(query.device))
     return out

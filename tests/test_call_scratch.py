@@ -67,3 +67,42 @@ def test_streams_do_not_meet_in_scratch(lbl, cuda_device):
     torch.cuda.synchronize()
     for i, (a, b) in enumerate(got):
         assert torch.equal(a, want[i % 4][0]) and torch.equal(b, want[i % 4][1])
+
+
+def test_decode_attention_has_scratch_of_its_own(native_lib, monkeypatch):
+    from ipex_llm_b200.transformers import kv
+    ranges = []
+
+    def call(q, k, v, mask, causal, scale, out, ws, stream):
+        ranges.append((ws.data_ptr(), ws.data_ptr() + ws.numel()))
+        if len(ranges) == 1:
+            t = threading.Thread(target=run)
+            t.start()
+            t.join()
+    monkeypatch.setattr(kv.ggml, "lowbit_sdp_fp8", call)
+    monkeypatch.setattr(kv, "_stream", lambda d: 0)
+    monkeypatch.setattr(torch.cuda, "device", lambda d: contextlib.nullcontext())
+    cache = torch.zeros(2, 4, 1000, 128, dtype=torch.uint8)
+
+    def run():
+        kv.sdp_fp8(torch.zeros(2, 8, 1, 128), cache, cache, None, 0.1)
+    run()
+    (a, b), (c, d) = ranges
+    assert b > a and d > c and (b <= c or d <= a)
+
+
+@pytest.mark.gpu
+def test_decode_attention_on_several_streams(native_lib, cuda_device):
+    from ipex_llm_b200.transformers import kv
+    cache = [torch.randn(2, 4, 3000, 128, device=cuda_device).to(torch.float8_e5m2).view(torch.uint8) for _ in range(2)]
+    qs = [torch.randn(2, 16, 1, 128, device=cuda_device).half() for _ in range(4)]
+    want = [kv.sdp_fp8(q, *cache, None, 0.1) for q in qs]
+    streams = [torch.cuda.Stream() for _ in qs]
+    torch.cuda.synchronize()
+    got = []
+    for _ in range(50):
+        for q, s in zip(qs, streams):
+            with torch.cuda.stream(s):
+                got.append(kv.sdp_fp8(q, *cache, None, 0.1))
+    torch.cuda.synchronize()
+    assert all(torch.equal(o, want[i % 4]) for i, o in enumerate(got))
