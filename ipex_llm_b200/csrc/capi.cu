@@ -196,10 +196,9 @@ int lowbit_relayout_cuda(const void* d_src, void* d_dst, int64_t rows, int64_t k
     return rc;
 }
 
-// fp32 activations never take the tensor-core GEMM: it rounds them to one bf16 plane (2^-9), while the GEMV keeps
-// them to 2^-24 (three planes) -- the fp32-in / fp32-out contract of ggml_compute_forward_mul_mat_q_fp32
-// (LBL:494-529).  Larger fp32 batches run as chunks of the GEMV; a caller that accepts half precision casts first,
-// as the reference's XPU path does (LBL:700-705, conver_to_half).
+// fp32 activations never take this kernel: it rounds them to one 16-bit value, while their contract keeps them to 2^-24 (three bf16
+// planes) -- the fp32-in / fp32-out contract of ggml_compute_forward_mul_mat_q_fp32 (LBL:494-529), on the GEMV or in gemm_exact.cu.  A
+// caller that accepts half precision casts first, as the reference's XPU path does (LBL:700-705, conver_to_half).
 static bool use_gemm(int qtype, int64_t n_rows, int64_t k, int64_t m, int x_dtype) {
     static const int64_t max_m = [] { const char* e = getenv("LOWBIT_GEMV_MAX_M"); return e ? (int64_t)atoi(e) : kGemvMaxM; }();   // development
     return x_dtype != DT_F32 && m > max_m && gemm_tc_supported(qtype, n_rows, k);

@@ -12,7 +12,7 @@
 // k-block, the MMAs 0.14): here activations, packed weights and expanded tiles have rings of their own, so the expansion runs
 // ahead of the activations and four groups of warps have four k-blocks in flight.  Measured per k-block: 0.19 us up to 170 tokens
 // (fp16; see pair_plan for the other paces), 0.282 at 256, where the tensor pipe is busy 512 of 525 clocks; 14336 x 4096 at 4000
-// tokens 1357 -> 1494 TFLOP/s, 4096 x 11008 at 512 tokens 59.7 -> 43.4 us.  At 128 tokens the MMAs need 256 of 360 clocks: A and B
+// tokens 1357 -> 1494 TFLOP/s, 4096 x 11008 at 512 tokens 59.7 -> 43.4 us (the kernel in a recorded chain).  At 128 tokens the MMAs need 256 of 360 clocks: A and B
 // both come from shared memory, beside the expansion's stores.
 //   warp 0       TMA: this CTA's half of the tokens, boxes of 32 rows x 64 elements (128-byte swizzle), ring of kX slots;
 //   warp 1       CTA 0: issues the MMAs (M = 256, N, K = 16; four per k-block) in warp-uniform control flow, one commit per ring
@@ -510,8 +510,8 @@ static int pair_launch(int qt, bool bf, const CUtensorMap& map, const PairArgs& 
 // Token tile and K splits of a matmul: the pair that minimises rounds of the resident clusters x k-blocks per unit x time per
 // k-block + the start and end of a unit and, when K is split, the partial sums' round trip through memory at ~4 TB/s and the second
 // launch.  Time per k-block, measured at 4096 x 11008 and 4096 x 4096: 0.0011 us per token once the MMAs set the pace (0.282 at 256),
-// below that the expansion and the chain around it, whose pace depends on the codec (0.19 us with fp16 activations, 0.24 with bf16,
-// 0.29 for nf4's table).  What the line between (128 tokens, K whole) and (256, two splits) is worth at 512 tokens, 4096 x 11008:
+// below that the expansion and the chain around it: 0.19 us for sym_int4 with fp16 activations, 0.24 with bf16, 0.29 for nf4's table;
+// the other formats were not measured and take sym_int4's figures.  What the line between (128 tokens, K whole) and (256, two splits) is worth at 512 tokens, 4096 x 11008:
 // sym_int4 fp16 43.4 against 48.2 us, bf16 50.3 against 48.8, nf4 58.1 against 50.1.
 constexpr double kPaces[3] = {0.19, 0.24, 0.29};
 static double pair_pace(int qt, bool bf) { return kPaces[qt == QT_NF4 ? 2 : bf ? 1 : 0]; }
