@@ -5,21 +5,26 @@
 // fp16 / bf16 queries, head_dim 128, both products on the 5th-generation tensor cores.  One CTA = NT tiles of 128 query rows of one
 // (sequence, query head), walking the keys in tiles of 128:
 //   S_t = Q_t . K^T   tcgen05.mma M = 128, N = 128, K = 16, both operands in shared memory, S in TMEM (lane = query row);
-//   softmax           four warps per tile, one thread per row, P (fp16) back into TMEM over S;
+//   softmax           four warps per tile, one thread per row, P (two fp16 values each) back into TMEM over S;
 //   O_t += P_t . V    A operand = P in TMEM, B operand = V as it lies in the cache (rows = keys: the MN-major descriptor).
 // Warps 0 .. 4 NT - 1: softmax; the next four read the cache (16 bytes a thread, coalesced), expand e5m2 -> fp16 (one byte permute
 // per pair) and write K and V into a ring of four 32 KB swizzled tiles; the last warp issues the MMAs and owns TMEM.
 // With two tiles a CTA their softmax and MMAs alternate: P_t . V, then Q_t . K of the next keys, of one tile run while the other is in
 // its softmax, and every key tile is expanded once for 256 rows.  P lies over S, so a tile's next Q . K waits for its P . V (a commit,
-// not the issue order).  What bounds it: per 128 keys and 256 rows 2048 clocks of MMAs, 2048 of ex2 (16 a clock), and the chain
-// Q.K -> softmax -> P.V of one tile.  The kernel it replaces (64 rows a CTA, mma.sync) was bound by the legacy tensor path:
-// 4000 causal tokens, 32 heads over 8, the call: 609 us, 215 TFLOP/s; this one 164 us, 800.
+// not the issue order); P . V of the first 64 keys of a tile starts while the softmax works on the others.
+// P is hi + lo, both fp16, and both multiply V: with one fp16 value the result carried the rounding of every probability, where the
+// kernel before this one (64 rows a CTA, mma.sync) rounded to fp16 too, but relative to a maximum that followed the keys 32 at a time,
+// so that the largest of them stayed exact.  Error against 64 bits of fp32 results, scale 128^-1/2 / 1.0 (2000 tokens): before 1.5e-4 /
+// 3.3e-5; one value with this kernel's lagging reference 1.6e-4 / 5.0e-5; the exact maximum as reference, O rescaled with nearly every
+// key tile, 1.5e-4 / 3.5e-5; hi + lo 1.1e-6 / 0.9e-6.
+// What bounds it: per 128 keys and 256 rows 3072 clocks of MMAs, 2048 of ex2 (16 a clock) and the splitting beside them, and the chain
+// Q.K -> softmax -> P.V of one tile.  4000 causal tokens, 32 heads over 8, the call: 609 us before, 160 with one value, 176 with one
+// value and the exact maximum, 195 so: 672 TFLOP/s, each product counted once (6000 tokens: 418 while P . V waited for a tile's 128
+// keys, 392 now).
 // Causal: query token s (0-based among the S new ones) sees keys <= L - S + s; key tiles beyond a tile's last row are skipped.  An
-// additive mask [B][1|Hq][S][L] is honoured.  Softmax and accumulation in 32 bits; Q and P enter the MMAs as fp16.  P is kept relative
-// to a reference 2^8 below fp16's comfortable range (values up to 2^14, nothing above 2^-32 of the row's maximum is flushed), and the
-// reference follows the row's maximum only when that grew by more than 2^6: O is then rescaled in TMEM, which is rarely.
-// The denominator sums the same rounded P (2.5 us of the 164): summed from the unrounded values it left up to 10 % more error, most
-// where a row's softmax is peaked.
+// additive mask [B][1|Hq][S][L] is honoured.  Softmax and accumulation in 32 bits; Q enters the MMAs as fp16.  P is kept relative to a
+// reference 2^8 below fp16's comfortable range (values up to 2^14), and the reference follows the row's maximum only when that grew by
+// more than 2^6: O is then rescaled in TMEM, which is rarely.
 
 constexpr int SP_ROWS = 128, SP_KEYS = 128, SP_SLOTS = 4;
 constexpr int SP_TILE = 128 * 256;                                    // 128 rows x 128 fp16, as two swizzled halves of 64 columns
@@ -57,9 +62,15 @@ __device__ __forceinline__ void sp_umma_ts_w(uint32_t tmem_d, uint32_t tmem_a, u
         "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
         ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(leader) : "memory");
 }
-// a += the first, b += the second of a pair of fp16 values, in 32 bits
-__device__ __forceinline__ void sp_add2(float& a, float& b, uint32_t pair) {
-    asm("{\n\t.reg .b16 lo, hi;\n\tmov.b32 {lo, hi}, %2;\n\tadd.rn.f32.f16 %0, lo, %0;\n\tadd.rn.f32.f16 %1, hi, %1;\n\t}" : "+f"(a), "+f"(b) : "r"(pair));
+// two probabilities as two fp16 values each, hi + lo
+__device__ __forceinline__ void sp_split2(float a, float b, uint32_t& hi, uint32_t& lo) {
+    asm("{\n\t.reg .b16 p, q, m;\n\t.reg .f32 x, y;\n\t"
+        "cvt.rn.f16x2.f32 %0, %3, %2;\n\t"
+        "mov.b32 {p, q}, %0;\n\t"
+        "mov.b16 m, 0xbc00;\n\t"
+        "fma.rn.f32.f16 x, p, m, %2;\n\t"
+        "fma.rn.f32.f16 y, q, m, %3;\n\t"
+        "cvt.rn.f16x2.f32 %1, y, x;\n\t}" : "=&r"(hi), "=r"(lo) : "f"(a), "f"(b));
 }
 __device__ __forceinline__ void sp_sts128(uint32_t a, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
     asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
@@ -75,10 +86,10 @@ sdp_fp8_prompt_kernel(const SdpArgs A, int n_qt) {
     auto kv_full = [&](int s) { return bars + s * 8; };
     auto kv_empty = [&](int s) { return bars + 32 + s * 8; };
     auto s_full = [&](int t) { return bars + 64 + t * 8; };
-    auto p_full = [&](int t) { return bars + 80 + t * 8; };
-    auto pv_done = [&](int t) { return bars + 96 + t * 8; };
-    const uint32_t drained = bars + 112;                               // every MMA that was issued is done
-    const uint32_t tmem_slot = bars + 120;
+    auto p_full = [&](int t, int c) { return bars + 80 + (2 * t + c) * 8; };      // P of 64 keys
+    auto pv_done = [&](int t) { return bars + 112 + t * 8; };
+    const uint32_t drained = bars + 128;                               // every MMA that was issued is done
+    const uint32_t tmem_slot = bars + 136;
     constexpr uint32_t TMEM_COLS = NT * 256;                           // S_t at 128 t, O_t behind all S
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const int hq = blockIdx.x % A.Hq, b = blockIdx.x / A.Hq, hkv = hq / (A.Hq / A.Hkv);
@@ -135,7 +146,7 @@ sdp_fp8_prompt_kernel(const SdpArgs A, int n_qt) {
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < SP_SLOTS; s++) { mbar_init(kv_full(s), 4); mbar_init(kv_empty(s), 1); }
-        for (int t = 0; t < 2; t++) { mbar_init(s_full(t), 1); mbar_init(p_full(t), 4); mbar_init(pv_done(t), 1); }
+        for (int t = 0; t < 2; t++) { mbar_init(s_full(t), 1); mbar_init(p_full(t, 0), 4); mbar_init(p_full(t, 1), 4); mbar_init(pv_done(t), 1); }
         mbar_init(drained, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -216,30 +227,28 @@ sdp_fp8_prompt_kernel(const SdpArgs A, int n_qt) {
                 }
                 const float shift = 8.0f - (m_ref == -CUDART_INF_F ? 0.0f : m_ref);
                 float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f, a3 = 0.0f;
-                // P of keys 64 c .. 64 c + 63 goes to columns 32 c .. 32 c + 31, whose scores have been read
+                // P of keys 64 c .. 64 c + 63 goes where their scores were: the high parts to the first 32 columns, the low parts to the others
 #pragma unroll 1
                 for (int c = 0; c < 2; c++) {
                     float x[64];
                     load(c, x);
-                    uint32_t pk[32];
+                    uint32_t hi[32], lo[32];
 #pragma unroll
                     for (int i = 0; i < 32; i += 2) {
                         const float p0 = ex2_approx(fmaf(x[2 * i], mul, shift)), p1 = ex2_approx(fmaf(x[2 * i + 1], mul, shift));
                         const float p2 = ex2_approx(fmaf(x[2 * i + 2], mul, shift)), p3 = ex2_approx(fmaf(x[2 * i + 3], mul, shift));
-                        const __half2 h0 = __floats2half2_rn(p0, p1), h1 = __floats2half2_rn(p2, p3);
-                        pk[i] = *reinterpret_cast<const uint32_t*>(&h0);
-                        pk[i + 1] = *reinterpret_cast<const uint32_t*>(&h1);
-                        // the denominator from the same rounded values that P . V takes: their rounding then cancels in the quotient
-                        sp_add2(a0, a1, pk[i]);
-                        sp_add2(a2, a3, pk[i + 1]);
+                        a0 += p0; a1 += p1; a2 += p2; a3 += p3;
+                        sp_split2(p0, p1, hi[i], lo[i]);
+                        sp_split2(p2, p3, hi[i + 1], lo[i + 1]);
                     }
-                    sp_tmem_st32(st + 32 * c, pk);
+                    sp_tmem_st32(st + 64 * c, hi);
+                    sp_tmem_st32(st + 64 * c + 32, lo);
+                    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(p_full(t, c));
                 }
                 sum += (a0 + a1) + (a2 + a3);
-                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
-                asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-                __syncwarp();
-                if (lane == 0) mbar_arrive(p_full(t));
             }
             if (!mbar_wait_lim(pv_done(t), (uint32_t)((nkt - 1) & 1), A.waits)) goto done;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -312,13 +321,15 @@ sdp_fp8_prompt_kernel(const SdpArgs A, int n_qt) {
             }
             umma_commit_w(s_full(t), leader);
         };
-        auto values = [&](int t, int j) {
+        auto values = [&](int t, int j, int c) {             // 64 keys
             // V tile: element (d, key) at half(d / 64), row key: LBO = the next 64 d, SBO = the next 8 keys; 16 keys a step
             const uint64_t vd = (make_desc(ring + ((2 * j + 1) % SP_SLOTS) * SP_TILE) & ~((uint64_t)0x3fff << 16)) | ((uint64_t)((SP_TILE / 2) >> 4) << 16);
 #pragma unroll
-            for (int k = 0; k < 8; k++)
-                sp_umma_ts_w(tmem + (NT + t) * 128, tmem + t * 128 + k * 8, vd + (uint64_t)((k * 2048) >> 4), id_o, (j > 0 || k > 0) ? 1u : 0u, leader);
-            umma_commit_w(pv_done(t), leader);
+            for (int k = 0; k < 4; k++)
+#pragma unroll
+                for (int lo = 1; lo >= 0; lo--)              // the small parts first
+                    sp_umma_ts_w(tmem + (NT + t) * 128, tmem + t * 128 + c * 64 + lo * 32 + k * 8, vd + (uint64_t)(((4 * c + k) * 2048) >> 4), id_o,
+                                 (j > 0 || c > 0 || k > 0 || lo == 0) ? 1u : 0u, leader);
         };
         if (nk > 0) {
             if (!mbar_wait_lim(kv_full(0), 0u, A.waits)) goto done;
@@ -337,9 +348,12 @@ sdp_fp8_prompt_kernel(const SdpArgs A, int n_qt) {
             for (int t = 0; t < NT; t++) {
                 const int nkt = t == 0 ? nk0 : nk1;
                 if (j >= nkt) continue;
-                if (!mbar_wait_lim(p_full(t), (uint32_t)(j & 1), A.waits)) goto done;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                values(t, j);
+                for (int c = 0; c < 2; c++) {
+                    if (!mbar_wait_lim(p_full(t, c), (uint32_t)(j & 1), A.waits)) goto done;
+                    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                    values(t, j, c);
+                }
+                umma_commit_w(pv_done(t), leader);
                 if (t == last) umma_commit_w(kv_empty(vi % SP_SLOTS), leader);
                 if (j + 1 < nkt) {
                     if (!mbar_wait_lim(pv_done(t), (uint32_t)(j & 1), A.waits)) goto done;         // S and P share their columns

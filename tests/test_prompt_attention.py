@@ -86,13 +86,27 @@ def test_masks(kv, cuda_device, S, L, Hq, kind):
 
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
 @pytest.mark.parametrize("S,L,Hq", [(70, 300, 2), (300, 512, 80)])
-def test_the_rounding_of_the_probabilities_cancels(kv, native_lib, cuda_device, dtype, S, L, Hq):
-    """Values of one everywhere: an output is the sum of the rounded probabilities over the denominator, and one again when the
-    denominator sums the same rounded values.  What is left are 32-bit sums: L / 16 steps of the tensor cores, each dropping up to
-    2^-22 of the sum, and L / 4 additions of 2^-24.  Summed before their rounding, a few large probabilities leave 1e-4."""
+def test_the_denominator_fits_what_the_product_sums(kv, native_lib, cuda_device, dtype, S, L, Hq):
+    """Values of one everywhere: an output is the sum of the probabilities that the product takes over the denominator, and one again.
+    What is left are 32-bit sums: L / 8 steps of the tensor cores, each dropping up to 2^-22 of the sum, and L / 4 additions of 2^-24.
+    Probabilities that are rounded for the one and not for the other leave 1e-4."""
     q, k, v = inputs(cuda_device, 1, Hq, Hq, S, L, dtype)
     v = torch.ones(v.shape, device=cuda_device).to(torch.float8_e5m2).view(torch.uint8)
     out = torch.empty(1, Hq, S, 128, device=cuda_device)
     for scale in (128 ** -0.5, 0.3):
         native_lib.lowbit_sdp_fp8_prefill(q, k, v, None, True, scale, out, torch.cuda.current_stream().cuda_stream)
-        assert float((out - 1).abs().max()) <= L / 16 * 2.0 ** -22 + L / 4 * 2.0 ** -24
+        assert float((out - 1).abs().max()) <= L / 8 * 2.0 ** -22 + L / 4 * 2.0 ** -24
+
+
+@pytest.mark.parametrize("S,L,Hq,Hkv,causal", [(40, 200, 2, 1, True), (129, 129, 4, 2, True), (300, 1077, 8, 2, True), (700, 700, 80, 8, True), (260, 900, 2, 2, False)])
+@pytest.mark.parametrize("scale", [0.02, 128 ** -0.5, 0.3, 1.0])
+def test_the_probabilities_are_not_rounded_to_16_bits(kv, native_lib, cuda_device, S, L, Hq, Hkv, causal, scale):
+    """32-bit results: the sums' error, not fp16's 2^-12 of every probability (1e-4 here, with the largest one exact or not).  A score's
+    eight steps drop up to 2^-23 of it each, which is that much of its probability; so do the L / 8 steps of P . V of the result."""
+    q, k, v = inputs(cuda_device, 1, Hq, Hkv, S, L, torch.float16)
+    out = torch.empty(1, Hq, S, 128, device=cuda_device)
+    native_lib.lowbit_sdp_fp8_prefill(q, k, v, None, causal, scale, out, torch.cuda.current_stream().cuda_stream)
+    want = statement(q, k, v, None, causal, scale)
+    keys = k.contiguous().view(torch.float8_e5m2).double().repeat_interleave(Hq // Hkv, 1)
+    largest = float((q.double() @ keys.transpose(-1, -2)).abs().max()) * scale
+    assert float((out.double() - want).norm() / want.norm()) <= (8 * largest + L / 8 + 4) * 2.0 ** -23
