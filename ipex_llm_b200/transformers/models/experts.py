@@ -20,7 +20,7 @@ def first_matrix(expert):
 
 def address_tables(mlp, dtype, device):
     """(gate_up addresses, down addresses, sizes, largest size, shared expert included?) as device arrays, or None when the
-    experts are not plain matrices of ``dtype`` (converted to a low-bit format); rebuilt when the weights moved.  A shared
+    experts are not plain matrices of ``dtype`` (converted to a low-bit format); rebuilt when any of the weights moved.  A shared
     expert that is a plain matrix too becomes the tables' last entry (the kernel runs it for every token)."""
     def plain(mods):
         return all(type(m) is nn.Linear and m.weight.dtype == dtype and m.weight.device == device and m.weight.is_contiguous() for m in mods)
@@ -30,7 +30,7 @@ def address_tables(mlp, dtype, device):
     with_shared = getattr(mlp, "shared", None) is not None and plain([first_matrix(mlp.shared), mlp.shared.down])
     if with_shared:
         experts.append(mlp.shared)
-    key = (device, dtype, with_shared) + tuple(m.weight.data_ptr() for e in (experts[0], experts[-1]) for m in (first_matrix(e), e.down))
+    key = (device, dtype, with_shared, tuple(e.ff for e in experts)) + tuple(m.weight.data_ptr() for e in experts for m in (first_matrix(e), e.down))
     if mlp._tables is None or mlp._tables[0] != key:
         def table(ws):
             return torch.tensor([w.weight.data_ptr() for w in ws], dtype=torch.int64, device=device)

@@ -54,6 +54,24 @@ def test_the_address_tables_follow_every_expert(name, e):
         assert table.tolist() == [lin.weight.data_ptr() for lin in mods]
 
 
+@pytest.mark.parametrize("part", ["gate_up", "down"])
+@pytest.mark.parametrize("e", range(3))
+def test_the_address_tables_of_plain_matrices_follow_every_expert(part, e):
+    from ipex_llm_b200.transformers.models import experts
+
+    class One(torch.nn.Module):
+        def __init__(self):
+            super().__init__()
+            self.gate_up, self.down, self.ff = torch.nn.Linear(16, 16, bias=False), torch.nn.Linear(8, 16, bias=False), 8
+    mlp = torch.nn.Module()
+    mlp.experts, mlp.shared, mlp._tables, cpu = torch.nn.ModuleList([One() for _ in range(3)]), None, None, torch.device("cpu")
+    experts.address_tables(mlp, torch.float32, cpu)
+    held = getattr(mlp.experts[e], part).weight
+    getattr(mlp.experts[e], part).weight = torch.nn.Parameter(held.detach().clone())
+    first, down = experts.address_tables(mlp, torch.float32, cpu)[:2]
+    assert first.tolist() == [x.gate_up.weight.data_ptr() for x in mlp.experts] and down.tolist() == [x.down.weight.data_ptr() for x in mlp.experts]
+
+
 def routing(dev, rows, top_k=2, seed=1, experts=E):
     g = torch.Generator(device=dev).manual_seed(seed)
     w, idx = torch.softmax(torch.randn(rows, experts, generator=g, device=dev), -1).topk(top_k, dim=-1)
