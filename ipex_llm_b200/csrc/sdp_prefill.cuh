@@ -18,14 +18,14 @@
 // 3.3e-5; one value with this kernel's lagging reference 1.6e-4 / 5.0e-5; the exact maximum as reference, O rescaled with nearly every
 // key tile, 1.5e-4 / 3.5e-5; hi + lo 1.1e-6 / 0.9e-6.
 // What bounds it: the chain Q.K -> softmax -> P.V of one tile, beside 3072 clocks of MMAs and 2048 of ex2 (16 a clock) per 128 keys and
-// 256 rows (2000 tokens: tensor pipe 46 % busy, XU 31 %, issue slots 39 %).  4000 causal tokens, 32 heads over 8, the call: 609 us before, 160 with one value, 176 with one
-// value and the exact maximum, 195 so: 672 TFLOP/s, each product counted once (6000 tokens: 418 while P . V waited for a tile's 128
-// keys, 392 now).
+// 256 rows (2000 tokens: tensor pipe 46 % busy, XU 31 %, issue slots 39 %).  4000 causal tokens, 32 heads over 8, the call: 609 us
+// before, 160 with one value, 176 with one value and the exact maximum, 195 so: 672 TFLOP/s, each product counted once (6000 tokens:
+// 418 while P . V waited for a tile's 128 keys, 392 now).
 // Causal: query token s (0-based among the S new ones) sees keys <= L - S + s; key tiles beyond a tile's last row are skipped.  An
 // additive mask [B][1|Hq][S][L] is honoured.  A value row that is not finite reaches the rows of its key tile that do not see it, as 0
-// times it.  Softmax and accumulation in 32 bits; Q enters the MMAs as fp16.  P is kept relative to a
-// reference 2^8 below fp16's comfortable range (values up to 2^14), and the reference follows the row's maximum only when that grew by
-// more than 2^6: O is then rescaled in TMEM, which is rarely.
+// times it.  Softmax and accumulation in 32 bits; Q enters the MMAs as fp16.  P is kept relative to a reference 2^8 below fp16's
+// comfortable range (values up to 2^14), and the reference follows the row's maximum only when that grew by more than 2^6: O is then
+// rescaled in TMEM, which is rarely.
 
 constexpr int SP_ROWS = 128, SP_KEYS = 128, SP_SLOTS = 4;
 constexpr int SP_TILE = 128 * 256;                                    // 128 rows x 128 fp16, as two swizzled halves of 64 columns

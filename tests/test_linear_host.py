@@ -61,7 +61,7 @@ def test_both_give_the_same_bits(lbl, cuda_device, monkeypatch, rows, dtype):
 
 @pytest.mark.gpu
 def test_other_threads_run_while_a_launch_waits(lbl, cuda_device):
-    """more launches than the device's queue holds, behind half a second of a busy stream: the calls wait, other threads do not"""
+    """more launches than the device's queue holds, behind a second of a busy stream: the calls wait, other threads do not"""
     lin = lbl.LowBitLinear(128, 128, lbl.SYM_INT4, bias=False).to(cuda_device).eval()
     x = torch.randn(1, 128, device=cuda_device).half()
     longest, stop = [0.0], threading.Event()
@@ -75,7 +75,7 @@ def test_other_threads_run_while_a_launch_waits(lbl, cuda_device):
     with torch.no_grad():
         lin(x)
         torch.cuda.synchronize()
-        torch.cuda._sleep(1000000000)                                               # cycles
+        torch.cuda._sleep(2000000000)                                               # cycles
         ticking = threading.Thread(target=clock)
         ticking.start()
         try:
@@ -85,4 +85,4 @@ def test_other_threads_run_while_a_launch_waits(lbl, cuda_device):
         finally:
             stop.set()
             ticking.join()
-    assert longest[0] < 0.2
+    assert longest[0] < 0.5
