@@ -262,6 +262,13 @@ int lowbit_decode_attention_cuda(void* d_qkv, int dtype, int64_t batch_stride, i
 int lowbit_greedy_advance_cuda(const void* d_logits, int dtype, int64_t row_stride, int B, int V, int64_t* d_next_ids,
                                int64_t* d_tokens, int64_t tokens_row_stride, int tokens_capacity, int32_t* d_state,
                                const int64_t* d_suppress_ids, void* stream);
+/* The pick behind a prompt: the same choice from its logits, for a sequence whose cache holds `length` tokens.  d_state becomes
+ * {length, 1, 0, suppress_below, n_suppress, 0, 0, 0} and d_suppress_ids [8] the n_suppress (<= 8) ids in host memory, the rest -1:
+ * nothing has to be copied there first. */
+int lowbit_greedy_start_cuda(const void* d_logits, int dtype, int64_t row_stride, int B, int V, int64_t* d_next_ids,
+                             int64_t* d_tokens, int64_t tokens_row_stride, int tokens_capacity, int32_t* d_state,
+                             int64_t* d_suppress_ids, int length, int suppress_below, int n_suppress,
+                             const int64_t* suppress_ids, void* stream);
 
 /* canonical <-> device layout on device buffers (same byte size, src != dst).
  * to_device != 0: canonical -> tiled ; 0: tiled -> canonical. */

@@ -526,6 +526,8 @@ _lib.lowbit_sdp_fp8_devlen_cuda.restype = ctypes.c_int
 _lib.lowbit_greedy_advance_cuda.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_int64, ctypes.c_int, ctypes.c_int, ctypes.c_void_p,
                                             ctypes.c_void_p, ctypes.c_int64, ctypes.c_int, _I32P, ctypes.c_void_p, ctypes.c_void_p]
 _lib.lowbit_greedy_advance_cuda.restype = ctypes.c_int
+_lib.lowbit_greedy_start_cuda.argtypes = _lib.lowbit_greedy_advance_cuda.argtypes[:-1] + [ctypes.c_int] * 3 + [_I64P, ctypes.c_void_p]
+_lib.lowbit_greedy_start_cuda.restype = ctypes.c_int
 
 
 def lowbit_rms_norm(x_2d, weight, eps, out, stream):
@@ -564,6 +566,15 @@ def lowbit_greedy_advance(logits, next_ids, tokens, state, stream, suppress_ids=
                                            tokens.data_ptr(), tokens.stride(0), tokens.shape[1], state.data_ptr(),
                                            suppress_ids.data_ptr() if suppress_ids is not None else None, stream),
            "lowbit_greedy_advance_cuda")
+
+
+def lowbit_greedy_start(logits, next_ids, tokens, state, suppress_ids, length, suppress_below, ids, stream):
+    """the pick behind a prompt of ``length`` cached tokens: as lowbit_greedy_advance, state and suppress_ids set up by the same launch"""
+    B, V = logits.shape
+    _check(_lib.lowbit_greedy_start_cuda(logits.data_ptr(), _DT_OF[logits.dtype], logits.stride(0), B, V, next_ids.data_ptr(),
+                                         tokens.data_ptr(), tokens.stride(0), tokens.shape[1], state.data_ptr(), suppress_ids.data_ptr(),
+                                         int(length), int(suppress_below), len(ids), (ctypes.c_int64 * max(len(ids), 1))(*ids), stream),
+           "lowbit_greedy_start_cuda")
 
 
 _lib.lowbit_decode_attention_workspace_size.argtypes = [ctypes.c_int] * 5

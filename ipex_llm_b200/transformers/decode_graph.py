@@ -205,10 +205,8 @@ class DecodeGraph:
         """after the prefill: pick the first token from its logits [B, V] and point the step's state at the cache.
         ``eos`` ids cannot be picked among the first ``min_new`` tokens (transformers' min_new_tokens rule)."""
         eos = list(eos)[:8]
-        self.suppress_ids.copy_(torch.tensor(eos + [-1] * (8 - len(eos)), dtype=torch.int64))
-        self.state.copy_(torch.tensor([prompt_len - 1, 0, 0, min_new if eos else 0, len(eos), 0, 0, 0], dtype=torch.int32))
-        logits = first_logits.contiguous()
-        ggml.lowbit_greedy_advance(logits, self.next_ids, self.tokens, self.state, _stream(self.device), self.suppress_ids)
+        ggml.lowbit_greedy_start(first_logits.contiguous(), self.next_ids, self.tokens, self.state, self.suppress_ids, prompt_len,
+                                 min_new if eos else 0, eos, _stream(self.device))
 
     def replay(self, n=1):
         for _ in range(n):
