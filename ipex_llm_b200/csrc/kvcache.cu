@@ -511,6 +511,42 @@ extern "C" size_t lowbit_sdp_fp8_workspace_size(int B, int Hq, int Hkv, int S, i
     return a > m ? a : m;
 }
 
+// The kernels whose key splits (at most 8) form a cluster and meet in its first CTA's shared memory, one launch
+static size_t sdp_cluster_smem(int n_split, int rt) { return SDP_WARPS * 3 * 8192 + 16 + (size_t)(n_split - 1) * rt * (128 + 4) * sizeof(float); }
+static int sdp_launch_cluster(void (*kern)(const SdpArgs), const SdpArgs& A, int tiles, bool pdl, cudaStream_t st) {
+    static bool configured[64][2] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    bool& ready = configured[dev & 63][A.qkv ? 1 : 0];                // one kernel with the step's inputs, one without
+    if (!ready) {
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sdp_cluster_smem(8, SDP_MMA_ROWS)) != cudaSuccess) {
+            set_error(LB_ERR_CUDA, "decode attention: cannot reserve %zu bytes of shared memory", sdp_cluster_smem(8, SDP_MMA_ROWS));
+            return LB_ERR_CUDA;
+        }
+        ready = true;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)A.n_split, (unsigned)(A.B * A.Hkv), (unsigned)tiles);
+    cfg.blockDim = dim3(SDP_WARPS * 32); cfg.dynamicSmemBytes = sdp_cluster_smem(A.n_split, A.rt); cfg.stream = st;
+    cudaLaunchAttribute at[2];
+    int na = 0;
+    at[na].id = cudaLaunchAttributeClusterDimension;
+    at[na].val.clusterDim.x = (unsigned)A.n_split; at[na].val.clusterDim.y = 1; at[na].val.clusterDim.z = 1; na++;
+    if (pdl) {
+        at[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        at[na].val.programmaticStreamSerializationAllowed = 1; na++;
+    }
+    cfg.attrs = at; cfg.numAttrs = na;
+    if (cudaLaunchKernelEx(&cfg, kern, A) != cudaSuccess) return check_launch();
+    note_launch();
+    return check_launch();
+}
+// ... for plain attention where that costs no resident CTA: two per SM with what the first one receives beside the rings, or no more than
+// one per SM anyway.  More than 8 splits (few heads over many keys: 16000 keys of one head 8.5 us) meet in memory as before
+static bool sdp_merges_in_cluster(const SdpArgs& A, int64_t groups) {
+    return A.n_split <= 8 && (sdp_cluster_smem(A.n_split, A.rt) <= 113 * 1024 || groups * A.n_split <= sm_count());
+}
+
 static int sdp_launch(const void* d_q, int q_dtype, const int64_t* q_strides, const void* d_k,
                       const int64_t* k_strides, const void* d_v, const int64_t* v_strides, const void* d_mask,
                       int mask_dtype, const int64_t* mask_strides, int causal, float scale, int B, int Hq,
@@ -533,7 +569,7 @@ static int sdp_launch(const void* d_q, int q_dtype, const int64_t* q_strides, co
         set_error(LB_ERR_WORKSPACE, "lowbit_sdp_fp8_cuda: workspace too small (%zu < %zu bytes)", workspace_bytes, need);
         return LB_ERR_WORKSPACE;
     }
-    SdpArgs A;
+    SdpArgs A = {};
     A.q = d_q; A.q_dtype = q_dtype; A.q_sb = q_strides[0]; A.q_sh = q_strides[1]; A.q_ss = q_strides[2];
     A.k = (const uint8_t*)d_k; A.k_sb = k_strides[0]; A.k_sh = k_strides[1]; A.k_ss = k_strides[2];
     A.v = (const uint8_t*)d_v; A.v_sb = v_strides[0]; A.v_sh = v_strides[1]; A.v_ss = v_strides[2];
@@ -565,6 +601,10 @@ static int sdp_launch(const void* d_q, int q_dtype, const int64_t* q_strides, co
         static const int nst = [] { const char* e = getenv("LOWBIT_SDP_RING"); return e ? atoi(e) : 3; }();
         if (D == 64) sdp_fp8_decode_mma_kernel<64, 4, 0, 0><<<grid, SDP_WARPS * 32, 0, st>>>(A);
         else if (nst == 0) sdp_fp8_decode_mma_kernel<128, 2, 0, 0><<<grid, SDP_WARPS * 32, 0, st>>>(A);
+        else if (nst == 3 && sdp_merges_in_cluster(A, (int64_t)B * Hkv * tiles)) {
+            A.early = 0;
+            return sdp_launch_cluster(sdp_fp8_decode_mma_kernel<128, 2, 3, 2>, A, tiles, false, st);
+        }
         else {
             auto kern = nst == 2 ? sdp_fp8_decode_mma_kernel<128, 3, 2, 0> : (nst == 4 ? sdp_fp8_decode_mma_kernel<128, 1, 4, 0> : sdp_fp8_decode_mma_kernel<128, 2, 3, 0>);
             const int smem = SDP_WARPS * (nst == 2 ? 2 : (nst == 4 ? 4 : 3)) * 8192;
@@ -736,33 +776,7 @@ extern "C" int lowbit_decode_attention_cuda(void* d_qkv, int dtype, int64_t batc
         A.rt = sdp_rt(Hq, Hkv, 1, true);
         A.part = nullptr; A.out = d_out; A.out_dtype = out_dtype;
         const int tiles = sdp_tiles(Hq, Hkv, 1, true);
-        auto kern = sdp_fp8_decode_mma_kernel<128, 2, 3, 1>;
-        const int smem = SDP_WARPS * 3 * 8192 + 16 + (A.n_split - 1) * A.rt * (D + 2) * (int)sizeof(float);
-        static int configured[64] = {};
-        int dev = 0; cudaGetDevice(&dev);
-        if (dev >= 0 && dev < 64 && configured[dev] < smem) {
-            const int ask = SDP_WARPS * 3 * 8192 + 16 + 7 * SDP_MMA_ROWS * (128 + 2) * (int)sizeof(float);
-            if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, ask) != cudaSuccess) {
-                set_error(LB_ERR_CUDA, "lowbit_decode_attention_cuda: cannot reserve %d bytes of shared memory", ask);
-                return LB_ERR_CUDA;
-            }
-            configured[dev] = ask;
-        }
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3((unsigned)A.n_split, (unsigned)(B * Hkv), (unsigned)tiles);
-        cfg.blockDim = dim3(SDP_WARPS * 32); cfg.dynamicSmemBytes = (size_t)smem; cfg.stream = (cudaStream_t)stream;
-        cudaLaunchAttribute at[2];
-        int na = 0;
-        at[na].id = cudaLaunchAttributeClusterDimension;
-        at[na].val.clusterDim.x = (unsigned)A.n_split; at[na].val.clusterDim.y = 1; at[na].val.clusterDim.z = 1; na++;
-        if (gemv_get_pdl()) {
-            at[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-            at[na].val.programmaticStreamSerializationAllowed = 1; na++;
-        }
-        cfg.attrs = at; cfg.numAttrs = na;
-        if (cudaLaunchKernelEx(&cfg, kern, A) != cudaSuccess) return check_launch();
-        note_launch();
-        return check_launch();
+        return sdp_launch_cluster(sdp_fp8_decode_mma_kernel<128, 2, 3, 1>, A, tiles, gemv_get_pdl(), (cudaStream_t)stream);
     }
     // separate kernels: rotary + cache write, attention with the device-side length, merge
     int rc = lowbit_rope_kv_append_cuda(d_qkv, dtype, batch_stride, batch_stride, B, 1, Hq, Hkv, D, d_cos, d_sin, cs_dtype, cs_row_stride,

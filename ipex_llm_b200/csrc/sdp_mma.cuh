@@ -55,10 +55,14 @@ __device__ __forceinline__ uint32_t sdp_map_to_rank(uint32_t local_addr, uint32_
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(local_addr), "r"(rank));
     return remote;
 }
-// remote store whose 4 bytes are counted on the destination CTA's mbarrier: the sender needs no fence and may exit
-__device__ __forceinline__ void sdp_st_async_f32(uint32_t remote_addr, float v, uint32_t remote_bar) {
-    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];"
-                 ::"r"(remote_addr), "r"(__float_as_uint(v)), "r"(remote_bar) : "memory");
+// remote stores whose bytes are counted on the destination CTA's mbarrier: the sender needs no fence and may exit
+__device__ __forceinline__ void sdp_st_async_v4(uint32_t remote_addr, const float (&v)[4], uint32_t remote_bar) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];"
+                 ::"r"(remote_addr), "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])), "r"(__float_as_uint(v[3])), "r"(remote_bar) : "memory");
+}
+__device__ __forceinline__ void sdp_st_async_v2(uint32_t remote_addr, float a, float b, uint32_t remote_bar) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.b32 [%0], {%1, %2}, [%3];"
+                 ::"r"(remote_addr), "r"(__float_as_uint(a)), "r"(__float_as_uint(b)), "r"(remote_bar) : "memory");
 }
 __device__ __forceinline__ float sdp_round_to(float v, int dt) {
     if (dt == DT_F16) return __half2float(__float2half_rn(v));
@@ -74,15 +78,20 @@ __device__ __forceinline__ float sdp_round_to(float v, int dt) {
 // shared memory (st.async + mbarrier transaction count, as the GEMV's split-K reduction does); the leader merges in rank
 // order and writes the output.  Same arithmetic as the separate kernels (rope.cu, kv_quantize, this kernel + the merge
 // kernel): rotate -> round -> quantise, the same split-local softmax, the same merge formula.
+// FUSED = 2 is plain attention (queries, key / value views, mask as for FUSED = 0) with that merge: no partial results in memory, no
+// second launch.  Recorded calls in a row, caches from memory, with the second launch -> now: 8 sequences x 4000 keys, 32 heads over 8
+// (66 MB, 4 splits) 18.9 -> 16.8 us; 16 x 1000 keys 13.9 -> 11.7; 4 x 300 keys 6.5 -> 4.7; 1 x 577 keys, 32 heads 6.3 -> 4.8; 8 new tokens
+// x 500 keys 7.3 -> 5.8.  What is left is a launch's start and end, about 5 us (the smallest shapes), and the keys at 5.4 TB/s.
 template <int D, int OCC, int NST, int FUSED>
 __global__ void __launch_bounds__(SDP_WARPS * 32, OCC)
 sdp_fp8_decode_mma_kernel(const SdpArgs A) {
+    constexpr bool STEP = FUSED == 1, MERGE = FUSED != 0;
     constexpr int NC = D / 64;                       // 16-byte pieces of a key row per lane
     constexpr int BPL = D / 8;                       // bytes of a value row per lane = output column tiles
     constexpr int VW = BPL / 4;                      // ... as 32-bit words
     static_assert(D == 64 || D == 128, "head_dim 64 or 128");
     static_assert(NST == 0 || D == 128, "the staged variant is written for 128-byte rows");
-    static_assert(!FUSED || (NST > 0 && D == 128), "the fused decode step is written for head_dim 128 and staged chunks");
+    static_assert(!MERGE || (NST > 0 && D == 128), "the in-cluster merge is written for head_dim 128 and staged chunks");
     extern __shared__ __align__(128) uint8_t sdp_ring[];            // NST > 0: [warp][stage][K 4 KB | V 4 KB]
     __shared__ float red_m[SDP_WARPS][SDP_MMA_ROWS], red_l[SDP_WARPS][SDP_MMA_ROWS];
     constexpr int RO = SDP_MMA_ROWS * (D + 16);       // floats of one warp's staged accumulators (NST > 0: in its ring)
@@ -95,10 +104,10 @@ sdp_fp8_decode_mma_kernel(const SdpArgs A) {
     const int n_rows = min(A.rt, rows_total - row0);
 
     asm volatile("griddepcontrol.launch_dependents;");               // the merge kernel may be scheduled as CTAs here retire
-    // FUSED: leader's receive barrier; the cluster barrier that publishes it is split around the main loop (free)
+    // MERGE: leader's receive barrier; the cluster barrier that publishes it is split around the main loop (free)
     const uint32_t rbar = sdp_smem_u32(sdp_ring) + SDP_WARPS * NST * 8192;
     float* const recv = reinterpret_cast<float*>(sdp_ring + SDP_WARPS * NST * 8192 + 16);
-    if (FUSED) {
+    if (MERGE) {
         if (A.n_split > 1) {
             if (split == 0 && threadIdx.x == 0) {
                 sdp_mbar_init(rbar, 1);
@@ -109,11 +118,11 @@ sdp_fp8_decode_mma_kernel(const SdpArgs A) {
         // qkv comes from the previous kernel.  The cache length and the cached rows come from earlier steps: a caller that
         // knows them complete (A.early: an ordinarily launched kernel lies between their producers and this call) lets the
         // first chunks stream in while the previous kernel drains; otherwise nothing is read before the wait.
-        if (!A.early) asm volatile("griddepcontrol.wait;" ::: "memory");
+        if (STEP && !A.early) asm volatile("griddepcontrol.wait;" ::: "memory");
     }
     int L, keys_per_split;
     sdp_lengths(A, L, keys_per_split);
-    const int new_pos = L - 1;                        // FUSED: position of the token being decoded
+    const int new_pos = L - 1;                        // STEP: position of the token being decoded
     const int key_begin = split * keys_per_split;
     const int key_end = min(L, key_begin + keys_per_split);
     // NST > 0: every warp streams its chunks through a ring of NST stages filled by cp.async (16 bytes per lane and
@@ -152,7 +161,7 @@ sdp_fp8_decode_mma_kernel(const SdpArgs A) {
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    if (FUSED && A.early) {
+    if (STEP && A.early) {
 #pragma unroll
         for (int s = 0; s < NST - 1; s++) stage_chunk(key_begin + (warp + SDP_WARPS * s) * 32, s);
         asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -165,7 +174,7 @@ sdp_fp8_decode_mma_kernel(const SdpArgs A) {
 #pragma unroll
         for (int i = 0; i < 8; i++) qa[c][i] = 0u;
     int my_hq = 0, my_st = 0;                         // query head / token of this lane's row
-    if (FUSED) {
+    if (STEP) {
         if (g < n_rows) {
             my_hq = hkv * n_rep + row0 + g;
             const uint16_t* qrow = reinterpret_cast<const uint16_t*>(A.qkv) + b * A.qkv_sb + (int64_t)my_hq * D + 16 * t;
@@ -228,9 +237,9 @@ sdp_fp8_decode_mma_kernel(const SdpArgs A) {
         }
     }
 
-    // FUSED: the new row of this kv head -- lane l owns key elements l, l + 32, l + 64, l + 96 (two rotary pairs) and
+    // STEP: the new row of this kv head -- lane l owns key elements l, l + 32, l + 64, l + 96 (two rotary pairs) and
     // value elements 4l .. 4l + 3 -- for every CTA whose range holds the new position; tile 0 also writes it to the cache
-    const bool has_new = FUSED && new_pos >= key_begin && new_pos < key_end;
+    const bool has_new = STEP && new_pos >= key_begin && new_pos < key_end;
     uint32_t knew = 0, vnew = 0;
     if (has_new) {
         const int64_t kbase = b * A.qkv_sb + (int64_t)(A.Hq + hkv) * D, vbase = kbase + (int64_t)A.Hkv * D;
@@ -268,7 +277,7 @@ sdp_fp8_decode_mma_kernel(const SdpArgs A) {
 #pragma unroll
     for (int i = 0; i < 4; i++) z[i][0] = z[i][1] = 0.0f;
 
-    if (NST > 0 && !(FUSED && A.early)) {
+    if (NST > 0 && !(STEP && A.early)) {
 #pragma unroll
         for (int s = 0; s < NST - 1; s++) stage_chunk(key_begin + (warp + SDP_WARPS * s) * 32, s);
     }
@@ -431,57 +440,62 @@ sdp_fp8_decode_mma_kernel(const SdpArgs A) {
             *reinterpret_cast<float4*>(red_o(warp) + g * (D + 16) + BPL * (2 * t + i) + 4 * (D == 128 ? (q ^ t) : q)) =
                 make_float4(o[4 * q][i], o[4 * q + 1][i], o[4 * q + 2][i], o[4 * q + 3][i]);
     __syncthreads();
-    float* part = FUSED ? nullptr : A.part + ((((int64_t)b * A.Hkv + hkv) * gridDim.z + tile) * A.n_split + split) * (A.rt * (D + 2));
-    const int ps = A.rt * (D + 2);                                    // floats of one CTA's partial result
-    if (FUSED && A.n_split > 1) {
+    float* part = MERGE ? nullptr : A.part + ((((int64_t)b * A.Hkv + hkv) * gridDim.z + tile) * A.n_split + split) * (A.rt * (D + 2));
+    constexpr int RS = D + 4;                                         // floats of a received row: m, l, -, -, o
+    const int ps = A.rt * RS;
+    if (MERGE && A.n_split > 1) {
         asm volatile("barrier.cluster.wait.aligned;" ::: "memory");  // the leader's barrier init is visible
-        if (split == 0 && threadIdx.x == 0) sdp_mbar_expect_tx(rbar, (uint32_t)((A.n_split - 1) * ps * 4));
+        if (split == 0 && threadIdx.x == 0) sdp_mbar_expect_tx(rbar, (uint32_t)((A.n_split - 1) * A.rt * (D + 2) * 4));
     }
-    const uint32_t rb = FUSED ? sdp_map_to_rank(rbar, 0) : 0u;
-    for (int i = threadIdx.x; i < A.rt * D; i += blockDim.x) {
-        const int r = i / D, d = i % D;
+    const uint32_t rb = MERGE ? sdp_map_to_rank(rbar, 0) : 0u;
+    // four columns a thread: element by element, eight rows took eight dependent rounds of this (7 of an 11 us call)
+    for (int i = threadIdx.x; i < A.rt * (D / 4); i += blockDim.x) {
+        const int r = i / (D / 4), d = 4 * (i % (D / 4));
         const int pos = D == 128 ? ((d & ~12) | ((((d >> 2) ^ (d >> 5)) & 3) << 2)) : d;       // where column d was staged
         float M = red_m[0][r];
 #pragma unroll
         for (int w = 1; w < SDP_WARPS; w++) M = fmaxf(M, red_m[w][r]);
-        float acc = 0.0f, lsum = 0.0f;
+        float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f}, lsum = 0.0f;
 #pragma unroll
         for (int w = 0; w < SDP_WARPS; w++) {
             const float f = (red_m[w][r] == -CUDART_INF_F) ? 0.0f : exp2f(red_m[w][r] - M);
-            acc = fmaf(red_o(w)[r * (D + 16) + pos], f, acc);
+            const float4 v = *reinterpret_cast<const float4*>(red_o(w) + r * (D + 16) + pos);
+            acc[0] = fmaf(v.x, f, acc[0]); acc[1] = fmaf(v.y, f, acc[1]); acc[2] = fmaf(v.z, f, acc[2]); acc[3] = fmaf(v.w, f, acc[3]);
             lsum = fmaf(red_l[w][r], f, lsum);
         }
-        if (!FUSED) {
-            part[r * (D + 2) + 2 + d] = acc;
-            if (d == 0) { part[r * (D + 2)] = M; part[r * (D + 2) + 1] = lsum; }
+        if (!MERGE) {
+            *reinterpret_cast<float2*>(part + r * (D + 2) + 2 + d) = make_float2(acc[0], acc[1]);
+            *reinterpret_cast<float2*>(part + r * (D + 2) + 4 + d) = make_float2(acc[2], acc[3]);
+            if (d == 0) *reinterpret_cast<float2*>(part + r * (D + 2)) = make_float2(M, lsum);
         } else if (split != 0) {
             // a peer: push (m, l, o) of the row into the leader's receive area and be done
-            const uint32_t dst = sdp_smem_u32(recv + (split - 1) * ps + r * (D + 2));
-            sdp_st_async_f32(sdp_map_to_rank(dst + 4 * (2 + d), 0), acc, rb);
-            if (d == 0) {
-                sdp_st_async_f32(sdp_map_to_rank(dst, 0), M, rb);
-                sdp_st_async_f32(sdp_map_to_rank(dst + 4, 0), lsum, rb);
-            }
+            const uint32_t dst = sdp_smem_u32(recv + (split - 1) * ps + r * RS);
+            sdp_st_async_v4(sdp_map_to_rank(dst + 4 * (4 + d), 0), acc, rb);
+            if (d == 0) sdp_st_async_v2(sdp_map_to_rank(dst, 0), M, lsum, rb);
         } else {
             // the leader: merge the splits in rank order (the merge kernel's formula), normalise, store
             if (A.n_split > 1) sdp_mbar_wait(rbar, 0);
             float Mall = M;
-            for (int k = 1; k < A.n_split; k++) Mall = fmaxf(Mall, recv[(k - 1) * ps + r * (D + 2)]);
+            for (int k = 1; k < A.n_split; k++) Mall = fmaxf(Mall, recv[(k - 1) * ps + r * RS]);
             const float f0 = (M == -CUDART_INF_F) ? 0.0f : exp2f(M - Mall);
-            float o = acc * f0, l = lsum * f0;
+            float o[4] = {acc[0] * f0, acc[1] * f0, acc[2] * f0, acc[3] * f0}, l = lsum * f0;
             for (int k = 1; k < A.n_split; k++) {
-                const float* pk = recv + (k - 1) * ps + r * (D + 2);
+                const float* pk = recv + (k - 1) * ps + r * RS;
                 const float f = (pk[0] == -CUDART_INF_F) ? 0.0f : exp2f(pk[0] - Mall);
-                o = fmaf(pk[2 + d], f, o);
+                const float4 v = *reinterpret_cast<const float4*>(pk + 4 + d);
+                o[0] = fmaf(v.x, f, o[0]); o[1] = fmaf(v.y, f, o[1]); o[2] = fmaf(v.z, f, o[2]); o[3] = fmaf(v.w, f, o[3]);
                 l = fmaf(pk[1], f, l);
             }
             const int rr = row0 + r;
             if (rr < rows_total) {
-                const float y = l > 0.0f ? o / l : 0.0f;
-                const int64_t oi = ((int64_t)b * A.Hq + (hkv * n_rep + rr)) * D + d;          // S == 1
-                if (A.out_dtype == DT_F32) ((float*)A.out)[oi] = y;
-                else if (A.out_dtype == DT_F16) ((__half*)A.out)[oi] = __float2half_rn(y);
-                else ((__nv_bfloat16*)A.out)[oi] = __float2bfloat16_rn(y);
+                const int64_t oi = (((int64_t)b * A.Hq + hkv * n_rep) * A.S + rr) * D + d;           // rows of a group: [query head][token]
+#pragma unroll
+                for (int e = 0; e < 4; e++) {
+                    const float y = l > 0.0f ? o[e] / l : 0.0f;
+                    if (A.out_dtype == DT_F32) ((float*)A.out)[oi + e] = y;
+                    else if (A.out_dtype == DT_F16) ((__half*)A.out)[oi + e] = __float2half_rn(y);
+                    else ((__nv_bfloat16*)A.out)[oi + e] = __float2bfloat16_rn(y);
+                }
             }
         }
     }

@@ -194,3 +194,27 @@ def test_decode_attention_one_launch_equals_the_separate_kernels(native_lib, cud
         assert float((got.double() - exact).abs().max()) <= tol, P
         assert float((got.double() - want.double()).abs().max()) <= tol, P
     assert launches == {1}, launches                     # every case here fits the one-launch kernel
+
+
+@pytest.mark.parametrize("B,Hq,Hkv,S,L", [(1, 4, 4, 1, 1), (2, 8, 4, 1, 129), (8, 32, 8, 1, 4001), (1, 32, 32, 1, 577), (1, 16, 2, 1, 1025), (1, 8, 1, 1, 16000),
+                                          (1, 32, 8, 8, 500), (1, 32, 8, 2, 31), (2, 12, 4, 3, 1000), (1, 8, 8, 32, 260)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("masked", [False, True])
+def test_attention_whose_key_splits_meet_in_a_cluster(native_lib, cuda_device, B, Hq, Hkv, S, L, dtype, masked):
+    """one, two, four and eight rows a CTA, one to eight splits (and more, which meet in memory), splits that hold no visible key.  Bound: the
+    probabilities and the result rounded to 16 bits, as for the other decode kernels"""
+    from ipex_llm_b200.transformers import kv
+    gen = torch.Generator(device=cuda_device).manual_seed(L)
+    q = torch.randn(B, S, Hq, 128, device=cuda_device, generator=gen).to(dtype).transpose(1, 2)
+    k, v = (torch.randn(B, Hkv, L, 128, device=cuda_device, generator=gen).to(torch.float8_e5m2).view(torch.uint8) for _ in range(2))
+    see = torch.ones(S, L, dtype=torch.bool, device=cuda_device).tril(L - S)
+    mask = None
+    if masked:
+        see[:, L // 2:] &= torch.rand(S, L - L // 2, device=cuda_device, generator=gen) < 0.02
+        see[0, :] = L == 1                               # a row that sees nothing gives zeros
+        mask = torch.zeros(1, 1, S, L, dtype=dtype, device=cuda_device).masked_fill_(~see, float("-inf"))
+    out = kv.scaled_dot_product_attention(q, k, v, mask, not masked, 128 ** -0.5)
+    kd, vd = (t.view(torch.float8_e5m2).double().repeat_interleave(Hq // Hkv, 1) for t in (k, v))
+    p = torch.softmax((q.double() @ kd.transpose(-1, -2) * 128 ** -0.5).masked_fill(~see, float("-inf")), -1).nan_to_num(0.0)
+    want = p @ vd
+    assert float((out.double() - want).abs().max()) <= (1e-3 if dtype == torch.float16 else 8e-3) * float(want.abs().max())
