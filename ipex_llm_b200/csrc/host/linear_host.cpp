@@ -1,8 +1,9 @@
 // linear_host.cpp -- the host side of one LowBitLinear.forward (reference low_bit_linear.py:638-725) in one native call:
 // checks, output, scratch, stream and launch.  In Python (tensor views, a ctypes call of fourteen arguments, the scratch lookup) the
 // same took 20 us around a 4 us kernel.  A CPython module (b200_host); the kernels are reached through the addresses of
-// libb200lowbit.so's entry points, which the package hands over once.  Beside it, the look at a mixture's experts that every call of
-// theirs begins with (expert_addresses).
+// libb200lowbit.so's entry points, which the package hands over once.  Beside it, attention over the 8-bit cache (attention: the Python
+// statements took 24 us around kernels of 5 to 17 us) and the look at a mixture's experts that every call of theirs begins with
+// (expert_addresses).
 #include <vector>
 #include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
@@ -15,9 +16,19 @@ namespace {
 using MatmulFn = int (*)(const void*, int, int64_t, int64_t, const void*, int, int64_t, void*, int, const void*, int, void*, size_t, void*);
 using WorkspaceFn = size_t (*)(int64_t, int64_t, int64_t, int);
 using HintFn = void (*)(const void*, size_t);
+using SdpFn = int (*)(const void*, int, const int64_t*, const void*, const int64_t*, const void*, const int64_t*, const void*, int, const int64_t*, int, float,
+                      int, int, int, int, int, int, void*, int, void*, size_t, void*);
+using SdpSupportedFn = int (*)(int, int, int, int);
+using SdpWorkspaceFn = size_t (*)(int, int, int, int, int, int);
+using SdpPromptFn = int (*)(const void*, int, const int64_t*, const void*, const int64_t*, const void*, const int64_t*, const void*, int, const int64_t*, int,
+                            float, int, int, int, int, int, int, void*, int, const int64_t*, void*);
 MatmulFn g_matmul = nullptr;
 WorkspaceFn g_workspace = nullptr;
 HintFn g_hint = nullptr;
+SdpFn g_sdp = nullptr;
+SdpSupportedFn g_sdp_supported = nullptr, g_sdp_prompt_supported = nullptr;
+SdpWorkspaceFn g_sdp_workspace = nullptr;
+SdpPromptFn g_sdp_prompt = nullptr;
 
 // other threads run Python meanwhile: an allocation or a launch may have to wait for the device
 struct WithoutGil {
@@ -30,8 +41,13 @@ int dtype_code(c10::ScalarType t) {
 }
 
 PyObject* attach(PyObject*, PyObject* args) {
-    unsigned long long m, w, h;
-    if (!PyArg_ParseTuple(args, "KKK", &m, &w, &h)) return nullptr;
+    unsigned long long m, w, h, s, ss, sw, p, ps;
+    if (!PyArg_ParseTuple(args, "KKKKKKKK", &m, &w, &h, &s, &ss, &sw, &p, &ps)) return nullptr;
+    g_sdp = reinterpret_cast<SdpFn>(s);
+    g_sdp_supported = reinterpret_cast<SdpSupportedFn>(ss);
+    g_sdp_workspace = reinterpret_cast<SdpWorkspaceFn>(sw);
+    g_sdp_prompt = reinterpret_cast<SdpPromptFn>(p);
+    g_sdp_prompt_supported = reinterpret_cast<SdpSupportedFn>(ps);
     g_matmul = reinterpret_cast<MatmulFn>(m);
     g_workspace = reinterpret_cast<WorkspaceFn>(w);
     g_hint = reinterpret_cast<HintFn>(h);
@@ -94,6 +110,62 @@ PyObject* linear(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     }
     if (rc) return PyLong_FromLong(rc);
     return THPVariable_Wrap(std::move(y));
+    END_HANDLE_TH_ERRORS
+}
+
+// attention(query, key, value, causal, scale, prompts)
+//   -> the result; None when this is not the plain case (dense rows, no mask, shapes that a kernel takes; with `prompts` false only
+//      those of at most 32 new tokens): the caller's general path then serves or refuses it; an int: the native error code.
+PyObject* attention(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
+    HANDLE_TH_ERRORS
+    if (n_args != 6 || !g_sdp) {
+        PyErr_SetString(PyExc_TypeError, "b200_host.attention takes six arguments, after attach()");
+        return nullptr;
+    }
+    if (!THPVariable_CheckExact(a[0]) || !THPVariable_CheckExact(a[1]) || !THPVariable_CheckExact(a[2])) Py_RETURN_NONE;
+    const at::Tensor &q = THPVariable_Unpack(a[0]), &k = THPVariable_Unpack(a[1]), &v = THPVariable_Unpack(a[2]);
+    const int causal = PyObject_IsTrue(a[3]), prompts = PyObject_IsTrue(a[5]);
+    const float scale = (float)PyFloat_AsDouble(a[4]);
+    if (PyErr_Occurred()) return nullptr;
+    for (const at::Tensor* t : {&q, &k, &v})
+        if (!t->is_cuda() || !t->has_storage() || t->dim() != 4 || t->numel() == 0 || t->device() != q.device() || t->stride(3) != 1) Py_RETURN_NONE;
+    const int dt = dtype_code(q.scalar_type());
+    if (dt < 0 || k.scalar_type() != at::kByte || v.scalar_type() != at::kByte) Py_RETURN_NONE;
+    const int64_t B = q.size(0), Hq = q.size(1), S = q.size(2), D = q.size(3), Hkv = k.size(1), L = k.size(2);
+    if (k.size(0) != B || k.size(3) != D || v.sizes() != k.sizes()) Py_RETURN_NONE;
+    for (const int64_t n : {B, Hq, S, L, B * Hq * S}) if (n > 0x7fffffff) Py_RETURN_NONE;
+    const bool few = S <= 32 && g_sdp_supported((int)Hq, (int)Hkv, (int)S, (int)D);
+    const void *const qp = q.const_data_ptr(), *const kp = k.const_data_ptr(), *const vp = v.const_data_ptr();
+    const int64_t qs[3] = {q.stride(0), q.stride(1), q.stride(2)}, ks[3] = {k.stride(0), k.stride(1), k.stride(2)}, vs[3] = {v.stride(0), v.stride(1), v.stride(2)};
+    if (!few) {
+        const auto at16 = [](const void* p, const int64_t (&s)[3], int64_t unit) {
+            return ((reinterpret_cast<uintptr_t>(p) & 15) | (uintptr_t)((s[0] | s[1] | s[2]) & (unit - 1))) == 0;
+        };
+        if (!prompts || dt == 0 || L < S || !g_sdp_prompt_supported((int)Hq, (int)Hkv, (int)D, dt) || !at16(kp, ks, 16) || !at16(vp, vs, 16) || !at16(qp, qs, 8))
+            Py_RETURN_NONE;
+    }
+    at::Tensor out;
+    int rc;
+    {
+        const WithoutGil released;
+        const c10::cuda::CUDAGuard guard(q.device());
+        const auto options = q.options().requires_grad(false);
+        void* const stream = c10::cuda::getCurrentCUDAStream(q.device().index()).stream();
+        if (few) {
+            out = at::empty({B, Hq, S, D}, options);
+            const size_t need = g_sdp_workspace((int)B, (int)Hq, (int)Hkv, (int)S, (int)L, (int)D);
+            at::Tensor scratch = at::empty({(int64_t)need}, options.dtype(at::kByte));
+            rc = g_sdp(qp, dt, qs, kp, ks, vp, vs, nullptr, 0, nullptr, causal, scale, (int)B, (int)Hq, (int)Hkv, (int)S, (int)L, (int)D, out.mutable_data_ptr(), dt,
+                       scratch.mutable_data_ptr(), need, stream);
+        } else {
+            out = at::empty({B, S, Hq, D}, options).transpose(1, 2);
+            const int64_t os[3] = {out.stride(0), out.stride(1), out.stride(2)};
+            rc = g_sdp_prompt(qp, dt, qs, kp, ks, vp, vs, nullptr, 0, nullptr, causal, scale, (int)B, (int)Hq, (int)Hkv, (int)S, (int)L, (int)D,
+                              out.mutable_data_ptr(), dt, os, stream);
+        }
+    }
+    if (rc) return PyLong_FromLong(rc);
+    return THPVariable_Wrap(std::move(out));
     END_HANDLE_TH_ERRORS
 }
 
@@ -163,6 +235,7 @@ PyObject* expert_addresses(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
 }
 
 PyMethodDef methods[] = {{"attach", attach, METH_VARARGS, nullptr},
+                         {"attention", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(attention)), METH_FASTCALL, nullptr},
                          {"expert_addresses", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(expert_addresses)), METH_FASTCALL, nullptr},
                          {"linear", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(linear)), METH_FASTCALL, nullptr},
                          {nullptr, nullptr, 0, nullptr}};

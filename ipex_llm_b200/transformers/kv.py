@@ -16,6 +16,7 @@ from transformers.cache_utils import Cache, DynamicLayer
 from ipex_llm_b200.utils.common import invalidInputError, LazyModule
 
 ggml = LazyModule("ipex_llm_b200.ggml.model.llama.llama_cpp")      # only the FP8 cache and its attention call it
+linears = LazyModule("ipex_llm_b200.transformers.low_bit_linear")   # their native host side has attention's too
 
 FP8_KV_ALLOC_LENGTH = 512
 KV_ALLOC_BLOCK_LENGTH = int(os.environ.get("KV_CACHE_ALLOC_BLOCK_LENGTH", 256))
@@ -309,6 +310,13 @@ def scaled_dot_product_attention(query: torch.Tensor, key: torch.Tensor, value: 
     _, n_kv_heads, kv_length, _ = key.shape
     scale = 1 / math.sqrt(head_dim) if scale is None else scale
     if key.dtype == torch.uint8:
+        if mask is None and query.is_cuda:
+            # the plain case: one native call does what the statements below do, and returns None where they are needed
+            host = linears._host if linears._host is not None else linears._load_host()
+            if host:
+                out = host.attention(query, key, value, is_causal, scale, seq_length > 32 and os.environ.get("IPEX_LLM_B200_SDP_PREFILL", "1") != "0")
+                if out is not None:
+                    return out if type(out) is not int else ggml._check(out, "lowbit_sdp_fp8_cuda")
         if seq_length <= 32 and ggml.lowbit_sdp_fp8_supported(n_heads, n_kv_heads, seq_length, head_dim):
             mask = _additive_mask(mask, query.dtype if query.dtype != torch.bfloat16 else torch.float32)
             return sdp_fp8(query, key, value, mask, scale, is_causal and mask is None)

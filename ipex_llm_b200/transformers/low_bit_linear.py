@@ -57,10 +57,12 @@ def _load_host():
                 module = importlib.util.module_from_spec(importlib.util.spec_from_loader("b200_host", loader))
                 loader.exec_module(module)
                 module.attach(*(ctypes.cast(getattr(ggml._lib, f), ctypes.c_void_p).value
-                                for f in ("lowbit_matmul_cuda", "lowbit_matmul_workspace_size", "lowbit_hint_next_weights")))
+                                for f in ("lowbit_matmul_cuda", "lowbit_matmul_workspace_size", "lowbit_hint_next_weights", "lowbit_sdp_fp8_cuda",
+                                          "lowbit_sdp_fp8_supported", "lowbit_sdp_fp8_workspace_size", "lowbit_sdp_fp8_prefill_strided_cuda",
+                                          "lowbit_sdp_fp8_prefill_supported")))
                 _host = module
             except Exception as e:
-                warnings.warn(f"the native host side of LowBitLinear is not available, its Python statements run instead: {e}")
+                warnings.warn(f"the native host side of LowBitLinear and attention is not available, its Python statements run instead: {e}")
                 _host = False
     return _host
 

@@ -86,3 +86,57 @@ def test_other_threads_run_while_a_launch_waits(lbl, cuda_device):
             stop.set()
             ticking.join()
     assert longest[0] < 0.5
+
+
+def _views(device, B, Hq, Hkv, S, L, D, dtype, order="shd"):
+    """queries as the models hand them over (or laid out as named), keys and values as views of a longer cache"""
+    gen = torch.Generator(device=device).manual_seed(B * L + S)
+    q = torch.randn(B, S, Hq, D, device=device, generator=gen).to(dtype).transpose(1, 2)
+    if order == "hsd":
+        q = q.contiguous()
+    elif order == "dense last dimension elsewhere":
+        q = q.transpose(2, 3).contiguous().transpose(2, 3)
+    elif order == "part of a wider row":
+        q = torch.cat([q, q], -1)[..., :D]
+    k, v = (torch.randn(B, Hkv, L + 40, D, device=device, generator=gen).to(torch.float8_e5m2).view(torch.uint8)[:, :, :L] for _ in range(2))
+    return q, k, v
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("shape", [(1, 4, 4, 1, 1, 128), (3, 8, 2, 1, 130, 128), (8, 32, 8, 1, 700, 128), (1, 8, 1, 1, 9000, 128), (2, 8, 8, 3, 257, 128),
+                                   (1, 32, 8, 8, 500, 128), (1, 12, 2, 32, 96, 128), (2, 8, 2, 1, 300, 64), (1, 4, 2, 5, 70, 96), (1, 4, 4, 33, 33, 128),
+                                   (2, 8, 2, 200, 301, 128), (1, 4, 2, 40, 60, 64), (1, 4, 4, 50, 50, 80)])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("order", ["shd", "hsd", "dense last dimension elsewhere", "part of a wider row"])
+def test_attention_gives_the_same_bits_and_layout_either_way(lbl, cuda_device, monkeypatch, shape, dtype, order):
+    """one native call, or the Python statements that it stands for (which serve the shapes it leaves to them)"""
+    from ipex_llm_b200.transformers import kv
+    B, Hq, Hkv, S, L, D = shape
+    q, k, v = _views(cuda_device, *shape, dtype, order)
+    for causal in (False, True):
+        for scale in (None, 0.5):
+            native = kv.scaled_dot_product_attention(q, k, v, None, causal, scale)
+            assert lbl._host
+            with monkeypatch.context() as m:
+                m.setattr(lbl, "_host", False)
+                want = kv.scaled_dot_product_attention(q, k, v, None, causal, scale)
+            assert native.dtype == want.dtype and native.stride() == want.stride() and torch.equal(native, want)
+
+
+@pytest.mark.gpu
+def test_attention_refuses_and_leaves_alone_what_it_did(lbl, cuda_device, monkeypatch):
+    """misaligned keys of a few tokens: the kernel's error either way; a batch, type or device that does not fit is not the native call's"""
+    from ipex_llm_b200.transformers import kv
+    q, k, v = _views(cuda_device, 1, 4, 2, 1, 64, 128, torch.float16)
+    odd = torch.zeros(k.numel() + 1, dtype=torch.uint8, device=cuda_device)[1:].view(1, 2, 64, 128)
+    host = lbl._load_host()
+    assert host
+    for serving in (host, False):
+        monkeypatch.setattr(lbl, "_host", serving)
+        with pytest.raises(RuntimeError):
+            kv.scaled_dot_product_attention(q, odd, v, None, False)
+    assert host.attention(q.double(), k, v, False, 1.0, True) is None
+    assert host.attention(q, k[:, :, :63], v, False, 1.0, True) is None
+    assert host.attention(torch.cat([q, q]), k, v, False, 1.0, True) is None
+    assert host.attention(q, k.cpu(), v, False, 1.0, True) is None
+    assert host.attention(q.expand(1, 4, 40, 128), torch.cat([k, k], 2), torch.cat([v, v], 2), True, 1.0, False) is None      # prompts switched off
