@@ -7,31 +7,38 @@
 // after 12 steps and is multiplied by the block's scale and added in 32-bit floats.  Formats whose value is not code x scale (asym_int4's
 // minima, nf4's table) stay on the GEMV.
 //
-// Layout of the work as in gemm_pair.cu: a cluster of two CTAs computes 256 features x up to 64 tokens with tcgen05.mma.cta_group::2, codes
-// expanded to bf16 = A operand, the token planes = B, each CTA staging half of the tokens (three boxes of 32 rows per k-block).  Every
-// k-block has a TMEM buffer of its own (eight of 64 columns); eight epilogue warps drain it: lane = feature, so a block's scale is one
-// value per lane, and a thread keeps 32 tokens' sums in registers over the unit's K range.
-//   warp 0 token planes (TMA), warp 1 MMAs / relay, warp 2 packed weights, warp 3 TMEM, warps 4-15 three expansion groups, 16-23 epilogue.
-// What it replaces ran chunks of 32 rows on the GEMV's mma.sync path, every chunk reading the weights again.  sym_int4, before -> now:
-// 4096 x 4096 at 33 rows 33.8 -> 17.4 us, 64 rows 50.4 -> 18.0, 200 rows 161 -> 37.7, 512 rows 400 -> 67.6; 11008 x 4096 at 512 rows
-// 938 -> 153; 1024 x 1024 at 33 rows 18.2 -> 12.4 (the smallest shape that reaches this kernel also gains).  Error against 64 bits,
-// relative to the result's norm: 4.8e-7 -> 1.5e-7 (sym_int4, 4096 x 4096), 2.5e-7 -> 1.6e-7 (e4m3).  A k-block costs 0.28 us at one unit
-// per pair: bound by the latency of staging and expansion, as in gemm_pair.cu; 12 MMA steps instead of 4 fit under it.
+// Layout of the work as in gemm_pair.cu: a cluster of two CTAs computes 256 features x up to 128 tokens with tcgen05.mma.cta_group::2,
+// codes expanded to bf16 = A operand, the token planes = B, each CTA staging half of the tokens (boxes of 32 rows, three planes per
+// k-block).  Every k-block has a TMEM buffer of its own; eight epilogue warps drain it: lane = feature, so a block's scale is one value
+// per lane, and a thread keeps half of the tile's tokens' sums in registers over the unit's K range.
+//   warp 0 token planes (TMA), warp 1 MMAs / relay, warp 2 packed weights, warp 3 TMEM, then two or three expansion groups of four
+//   warps, then eight warps of epilogue.
+// Tiles of 64 tokens alone (the first form) read A from shared memory for every 32 clocks of MMAs (N = 64 of twelve steps) and took 900
+// clocks a k-block: 500 of them four barrier tests one after the other (asked together and ahead now), then the MMAs themselves; at 128
+// tokens a step's math covers its operands.  All three planes in one step of N = 192 halved the MMA time but made the epilogue read
+// three times as much TMEM: 600 clocks a k-block, slower than either.  The kernel starts while split3_kernel runs and waits only in
+// front of the planes.  sym_int4, GEMV passes of 32 rows -> 64-token tiles -> now: 4096 x 4096 at 33 rows 33.8 -> 17.7 -> 15.6 us, 64 rows
+// 50.4 -> 18.1 -> 15.6, 200 rows 161 -> 38.0 -> 26.8, 512 rows 400 -> 69.9 -> 40.4; 11008 x 4096 at 512 rows 938 -> 160 -> 105; 1024 x 1024
+// at 33 rows 18.2 -> 12.5 -> 10.9.  Error against 64 bits, relative to the result's norm: the GEMV 4.8e-7, here 1.2e-7 to 1.5e-7
+// (sym_int4, 4096 x 4096).  At 512 rows the MMAs' twelve steps are 3/4 of the time; below 100 rows it is the three launches' ends.
 #include "tc_pair.cuh"
 
 namespace lowbit {
 namespace gemmtc {
 
-constexpr int kExThreads = 32 * 24, kExTok = 64, kExBufs = 8, kExGroups = 3;
-constexpr int kExDeq0 = 4, kExEpi0 = 16;
+constexpr int kExTok = 128, kExDeq0 = 4;     // most tokens of a tile; first expanding warp
 
-template <int QT> struct ExSmem {
+// TOK: 64 tokens or 128.  A thread of the epilogue keeps half of them, so the larger tile leaves registers for two expansion groups only;
+// its MMAs take that long.
+template <int QT, int TOK> struct ExShape {
+    static constexpr int kGroups = TOK == 64 ? 3 : 2, kEpi0 = kExDeq0 + 4 * kGroups, kThreads = 32 * (kEpi0 + 8);
+    static constexpr int kBufs = 512 / TOK;                            // TMEM: one for every k-block in flight
     static constexpr int kGroup = PackedBlock<QT>::kGroup, kPacked = 2 * kGroup;
-    static constexpr int kA = kExGroups, kP = 2 * kExGroups, kX = 6;
-    static constexpr int kXSlot = 3 * 4096;                            // three planes x 32 rows x 128 bytes
+    static constexpr int kA = TOK == 64 ? 3 : 4, kP = 6, kX = TOK == 64 ? 6 : 4;
+    static constexpr int kXPlane = TOK * 64, kXSlot = 3 * kXPlane;     // half of the tokens' rows of 128 bytes
     static constexpr int kTotal = 1024 + 512 + kA * kTileBytesAB + kP * kPacked + kX * kXSlot;
     static_assert(kTotal <= 232448, "shared memory");
-    static_assert((3 * kX + 2 * kP + 2 * kA + 2 * kExBufs + 1) * 8 + 8 <= 512, "barrier region");
+    static_assert(kP % kGroups == 0 && (3 * kX + 2 * kP + 2 * kA + 2 * kBufs + 1) * 8 + 8 <= 512, "barrier region");
 };
 
 struct ExactArgs {
@@ -43,12 +50,12 @@ struct ExactArgs {
     Waits waits;
 };
 
-template <int QT>
-__global__ void __launch_bounds__(kExThreads, 1)
+template <int QT, int TOK>
+__global__ void __launch_bounds__(ExShape<QT, TOK>::kThreads, 1)
 exact_kernel(const __grid_constant__ CUtensorMap xmap, const ExactArgs A) {
     using E = Expand<QT>;
-    using SM = ExSmem<QT>;
-    constexpr int KX = SM::kX, KP = SM::kP, KA = SM::kA;
+    using SM = ExShape<QT, TOK>;
+    constexpr int KX = SM::kX, KP = SM::kP, KA = SM::kA, GROUPS = SM::kGroups, BUFS = SM::kBufs;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t xring = base, aring = base + KX * SM::kXSlot, pring = aring + KA * kTileBytesAB, bars = pring + KP * SM::kPacked;
@@ -60,8 +67,8 @@ exact_kernel(const __grid_constant__ CUtensorMap xmap, const ExactArgs A) {
     auto a_full = [&](int s) { return bars + (3 * KX + 2 * KP + s) * 8; };             // CTA 0: both CTAs' tiles are expanded
     auto a_empty = [&](int s) { return bars + (3 * KX + 2 * KP + KA + s) * 8; };
     auto t_full = [&](int b) { return bars + (3 * KX + 2 * KP + 2 * KA + b) * 8; };
-    auto t_empty = [&](int b) { return bars + (3 * KX + 2 * KP + 2 * KA + kExBufs + b) * 8; };   // CTA 0: both epilogues have read it
-    const uint32_t drained = bars + (3 * KX + 2 * KP + 2 * KA + 2 * kExBufs) * 8;      // every MMA that was issued is done
+    auto t_empty = [&](int b) { return bars + (3 * KX + 2 * KP + 2 * KA + BUFS + b) * 8; };   // CTA 0: both epilogues have read it
+    const uint32_t drained = bars + (3 * KX + 2 * KP + 2 * KA + 2 * BUFS) * 8;      // every MMA that was issued is done
     const uint32_t tmem_slot = drained + 8;
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31, rank = (int)(blockIdx.x & 1);
     const int nb = (int)A.G.nb;
@@ -69,7 +76,7 @@ exact_kernel(const __grid_constant__ CUtensorMap xmap, const ExactArgs A) {
         for (int s = 0; s < KX; s++) { mbar_init(x_full(s), 1); mbar_init(x_empty(s), 1); mbar_init(xp_full(s), 1); }
         for (int s = 0; s < KP; s++) { mbar_init(p_full(s), 1); mbar_init(p_empty(s), 4); }
         for (int s = 0; s < KA; s++) { mbar_init(a_full(s), 8); mbar_init(a_empty(s), 1); }
-        for (int b = 0; b < kExBufs; b++) { mbar_init(t_full(b), 1); mbar_init(t_empty(b), 16); }
+        for (int b = 0; b < BUFS; b++) { mbar_init(t_full(b), 1); mbar_init(t_empty(b), 16); }
         mbar_init(drained, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
@@ -102,14 +109,16 @@ exact_kernel(const __grid_constant__ CUtensorMap xmap, const ExactArgs A) {
 
     if (warp == 0) {
         // ================= token planes: this CTA's half of the tile's tokens =================
+        asm volatile("griddepcontrol.wait;" ::: "memory");     // split3_kernel's; the weights' copies and expansion have begun meanwhile
         for (int unit = blockIdx.x >> 1; unit < n_units; unit += stride) {
             decode(unit, U);
-            const int row0 = U.m0 + rank * (U.n_tok >> 1);
+            const int row0 = U.m0 + rank * (U.n_tok >> 1), boxes = ((U.n_tok >> 1) + 31) >> 5;
             for (int kb = U.kb0; kb < U.kb1; kb++) {
                 if (!mbar_wait_lim(x_empty(s), (uint32_t)((round & 1) ^ 1), A.waits)) goto done;
-                mbar_expect_tx_w(x_full(s), SM::kXSlot, leader);
+                mbar_expect_tx_w(x_full(s), 3 * boxes * 4096, leader);
                 // rows of a plane beyond the last token belong to the next plane (or read zero): columns that nothing stores
-                for (int p = 0; p < 3; p++) tma_load_2d_w(xring + s * SM::kXSlot + p * 4096, &xmap, kb * 64, p * A.M + row0, x_full(s), leader);
+                for (int p = 0; p < 3; p++)
+                    for (int i = 0; i < boxes; i++) tma_load_2d_w(xring + s * SM::kXSlot + p * SM::kXPlane + i * 4096, &xmap, kb * 64, p * A.M + row0 + 32 * i, x_full(s), leader);
                 if (++s == KX) { s = 0; round++; }
             }
         }
@@ -117,28 +126,29 @@ exact_kernel(const __grid_constant__ CUtensorMap xmap, const ExactArgs A) {
         if (rank == 0) {
             // ================= MMA issuer: 3 planes x 4 steps per k-block, into the k-block's own TMEM buffer =================
             int sx = 0, rx = 0, sa = 0, ra = 0, tb = 0, rt = 0;
+            bool ready = false;
             for (int unit = blockIdx.x >> 1; unit < n_units; unit += stride) {
                 decode(unit, U);
                 const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (((uint32_t)U.n_tok >> 3) << 17) | ((256u >> 4) << 24);
                 for (int kb = U.kb0; kb < U.kb1; kb++) {
-                    if (!mbar_wait_lim(t_empty(tb), (uint32_t)((rt & 1) ^ 1), A.waits)) goto done;
-                    if (!mbar_wait_lim(x_full(sx), (uint32_t)(rx & 1), A.waits)) goto done;
-                    if (!mbar_wait_lim(xp_full(sx), (uint32_t)(rx & 1), A.waits)) goto done;
-                    if (!mbar_wait_lim(a_full(sa), (uint32_t)(ra & 1), A.waits)) goto done;
+                    if (!mbar_wait4_lim(ready, t_empty(tb), (uint32_t)((rt & 1) ^ 1), x_full(sx), (uint32_t)(rx & 1), xp_full(sx), (uint32_t)(rx & 1), a_full(sa),
+                                        (uint32_t)(ra & 1), A.waits)) goto done;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     const uint64_t ad = make_desc(aring + sa * kTileBytesAB), xd = make_desc(xring + sx * SM::kXSlot);
 #pragma unroll
                     for (int p = 2; p >= 0; p--)             // the small planes first
 #pragma unroll
                         for (int k4 = 0; k4 < 4; k4++)
-                            umma2_f16_w(tmem_base + tb * kExTok, ad + (uint64_t)((k4 * 32) >> 4), xd + (uint64_t)((p * 4096 + k4 * 32) >> 4), idesc,
+                            umma2_f16_w(tmem_base + tb * TOK, ad + (uint64_t)((k4 * 32) >> 4), xd + (uint64_t)((p * SM::kXPlane + k4 * 32) >> 4), idesc,
                                         (p < 2 || k4 > 0) ? 1u : 0u, leader);
                     umma2_commit_w(a_empty(sa), leader);
                     umma2_commit_w(x_empty(sx), leader);
                     umma2_commit_w(t_full(tb), leader);
                     if (++sx == KX) { sx = 0; rx++; }
                     if (++sa == KA) { sa = 0; ra++; }
-                    if (++tb == kExBufs) { tb = 0; rt++; }
+                    if (++tb == BUFS) { tb = 0; rt++; }
+                    // asked here, answered while the MMAs above are being issued
+                    ready = mbar_test4(t_empty(tb), (uint32_t)((rt & 1) ^ 1), x_full(sx), (uint32_t)(rx & 1), xp_full(sx), (uint32_t)(rx & 1), a_full(sa), (uint32_t)(ra & 1));
                 }
             }
         } else {
@@ -171,17 +181,17 @@ exact_kernel(const __grid_constant__ CUtensorMap xmap, const ExactArgs A) {
             }
             if (kb_end < U.kb1) goto done;
         }
-    } else if (warp >= kExDeq0 && warp < kExEpi0) {
-        // ================= expansion: group (warp - 4) / 4 takes every third k-block =================
+    } else if (warp >= kExDeq0 && warp < SM::kEpi0) {
+        // ================= expansion: group (warp - 4) / 4 takes every second (third) k-block =================
         const int grp = (warp - kExDeq0) >> 2, dw = (warp - kExDeq0) & 3, g = lane >> 2, t = lane & 3;
-        const uint32_t row0 = aring + grp * kTileBytesAB + 4 * dw * 1024 + g * 128;        // rows interleaved by 16 as in gemm_pair.cu
-        const __half2 one = __floats2half2_rn(1.0f, 1.0f), zero = __floats2half2_rn(0.0f, 0.0f);
-        int it = 0, turn = 0, sp = 0, rp = 0, ra = 0;
+        int end = 0, it = grp, sp = grp, rp = 0;
         for (int unit = blockIdx.x >> 1; unit < n_units; unit += stride) {
             decode(unit, U);
-            for (int kb = U.kb0; kb < U.kb1; kb++, it++, (++turn == kExGroups ? turn = 0 : 0), (++sp == KP ? (sp = 0, rp++) : 0)) {
-                if (turn != grp) continue;
-                // at its last k-block this group waited for the MMAs of k-block it - 6 = it - KP: the packed slot's earlier trips are over
+            end += U.kb1 - U.kb0;
+            for (; it < end; it += GROUPS, ((sp += GROUPS) >= KP ? (sp -= KP, rp++) : 0)) {
+                const int sa = it % KA;
+                const uint32_t row0 = aring + sa * kTileBytesAB + 4 * dw * 1024 + g * 128;     // rows interleaved by 16 as in gemm_pair.cu
+                // the slot's earlier trip (k-block it - KP) was this group's own
                 if (!mbar_wait_lim(p_full(sp), (uint32_t)(rp & 1), A.waits)) goto done;
                 typename E::Codes cw[2];
 #pragma unroll
@@ -192,12 +202,11 @@ exact_kernel(const __grid_constant__ CUtensorMap xmap, const ExactArgs A) {
 #pragma unroll
                     for (int k4 = 0; k4 < 4; k4++) {
                         uint32_t a[4];
-                        E::run(cw[gi], k4, one, one, zero, zero, 0u, a);                  // the codes' values, exact in fp16 and in bf16
-                        lo[gi][2 * k4] = h2_to_bf2(a[0]); lo[gi][2 * k4 + 1] = h2_to_bf2(a[2]);
-                        hi[gi][2 * k4] = h2_to_bf2(a[1]); hi[gi][2 * k4 + 1] = h2_to_bf2(a[3]);
+                        E::bf16(cw[gi], k4, a);
+                        lo[gi][2 * k4] = a[0]; lo[gi][2 * k4 + 1] = a[2];
+                        hi[gi][2 * k4] = a[1]; hi[gi][2 * k4 + 1] = a[3];
                     }
-                if (!mbar_wait_lim(a_empty(grp), (uint32_t)((ra & 1) ^ 1), A.waits)) goto done;
-                ra++;
+                if (!mbar_wait_lim(a_empty(sa), (uint32_t)(((it / KA) & 1) ^ 1), A.waits)) goto done;
 #pragma unroll
                 for (int gi = 0; gi < 2; gi++)
 #pragma unroll
@@ -208,12 +217,12 @@ exact_kernel(const __grid_constant__ CUtensorMap xmap, const ExactArgs A) {
                     }
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 __syncwarp();
-                if (lane == 0) { mbar_arrive(p_empty(sp)); mbar_arrive_at(a_full(grp), 0); }      // behind the stores: the codes have been used
+                if (lane == 0) { mbar_arrive(p_empty(sp)); mbar_arrive_at(a_full(sa), 0); }      // behind the stores: the codes have been used
             }
         }
-    } else if (warp >= kExEpi0) {
-        // ================= epilogue: TMEM lanes 32 * (warp % 4) .., tokens 32 * part .. + 31 =================
-        const int quarter = warp & 3, part = (warp - kExEpi0) >> 2, half = lane >> 4;
+    } else if (warp >= SM::kEpi0) {
+        // ================= epilogue: TMEM lanes 32 * (warp % 4) .., half `part` of the tile's tokens =================
+        const int quarter = warp & 3, part = (warp - SM::kEpi0) >> 2, half = lane >> 4;
         const int64_t N = A.G.rows;
         int tb = 0, rt = 0;
         for (int unit = blockIdx.x >> 1; unit < n_units; unit += stride) {
@@ -223,10 +232,11 @@ exact_kernel(const __grid_constant__ CUtensorMap xmap, const ExactArgs A) {
             // the lane's scales: row 16 quarter + (lane & 15) of 64-row group 2 ft + half, one fp16 per k-block, 128 bytes apart
             const int64_t rg = valid ? 2 * U.ft + half : 0;
             const __half* sp = reinterpret_cast<const __half*>(A.w + A.G.off_s + (rg * nb) * 128) + (lane & 7) * 8 + quarter * 2 + ((lane >> 3) & 1);
-            const int t0 = 32 * part;
-            float acc[32];
+            constexpr int TOKS = TOK / 2;
+            const int t0 = TOKS * part;
+            float acc[TOKS];
 #pragma unroll
-            for (int i = 0; i < 32; i++) acc[i] = 0.0f;
+            for (int i = 0; i < TOKS; i++) acc[i] = 0.0f;
             float next[4];
 #pragma unroll
             for (int i = 0; i < 4; i++) next[i] = U.kb0 + i < U.kb1 ? __half2float(sp[(int64_t)(U.kb0 + i) * 64]) : 0.0f;
@@ -242,17 +252,17 @@ exact_kernel(const __grid_constant__ CUtensorMap xmap, const ExactArgs A) {
                     if (!mbar_wait_lim(t_full(tb), (uint32_t)(rt & 1), A.waits)) goto done;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
-                    for (int c = 0; c < 32; c += 16) {
+                    for (int c = 0; c < TOKS; c += 16) {
                         if (t0 + c >= U.rows) break;
                         float v[16];
-                        tmem_ld16(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(tb * kExTok + t0 + c), v);
+                        tmem_ld16(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(tb * TOK + t0 + c), v);
 #pragma unroll
                         for (int j = 0; j < 16; j++) acc[c + j] = fmaf(d[i], v[j], acc[c + j]);
                     }
                     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                     __syncwarp();
                     if (lane == 0) mbar_arrive_at(t_empty(tb), 0);
-                    if (++tb == kExBufs) { tb = 0; rt++; }
+                    if (++tb == BUFS) { tb = 0; rt++; }
                 }
             }
             if (valid && t0 < U.rows) {
@@ -260,7 +270,7 @@ exact_kernel(const __grid_constant__ CUtensorMap xmap, const ExactArgs A) {
                 const float b = A.bias && A.ksplit == 1 ? A.bias[n] : 0.0f;
                 float* const dst = A.ksplit > 1 ? A.part + (int64_t)U.ks * A.M * N + at : A.y + at;
 #pragma unroll
-                for (int c = 0; c < 32; c += 16) {
+                for (int c = 0; c < TOKS; c += 16) {
                     float v[16];
 #pragma unroll
                     for (int j = 0; j < 16; j++) v[j] = acc[c + j];
@@ -289,6 +299,7 @@ done:
 
 // fp32 activations -> three bf16 planes whose sum reproduces them to 2^-24, four elements a thread
 __global__ void __launch_bounds__(256) split3_kernel(const float4* __restrict__ x, uint2* __restrict__ out, int64_t n4) {
+    asm volatile("griddepcontrol.launch_dependents;");
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n4; i += (int64_t)gridDim.x * blockDim.x) {
         const float4 q = x[i];
         float r[4] = {q.x, q.y, q.z, q.w};
@@ -306,45 +317,56 @@ __global__ void __launch_bounds__(256) split3_kernel(const float4* __restrict__ 
     }
 }
 
-template <int QT> static int exact_launch_one(const CUtensorMap& map, const ExactArgs& A, int64_t units, cudaStream_t st) {
-    constexpr int SMEM = ExSmem<QT>::kTotal;
+template <int QT, int TOK> static int exact_launch_tile(const CUtensorMap& map, const ExactArgs& A, int64_t units, cudaStream_t st) {
+    constexpr int SMEM = ExShape<QT, TOK>::kTotal;
     static int cached[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
     int& clusters = cached[dev & 63];
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(sm_count() & ~1)); cfg.blockDim = dim3(kExThreads); cfg.dynamicSmemBytes = SMEM; cfg.stream = st;
-    cudaLaunchAttribute at[1];
+    cfg.gridDim = dim3((unsigned)(sm_count() & ~1)); cfg.blockDim = dim3(ExShape<QT, TOK>::kThreads); cfg.dynamicSmemBytes = SMEM; cfg.stream = st;
+    cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
     cfg.attrs = at; cfg.numAttrs = 1;
     if (!clusters) {
         int c = 0;
-        if (cudaFuncSetAttribute(exact_kernel<QT>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess) {
+        if (cudaFuncSetAttribute(exact_kernel<QT, TOK>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess) {
             cudaGetLastError();
             set_error(LB_ERR_CUDA, "the two-SM fp32 matmul cannot be configured on this device");
             return LB_ERR_CUDA;
         }
-        if (cudaOccupancyMaxActiveClusters(&c, exact_kernel<QT>, &cfg) != cudaSuccess || c <= 0) { cudaGetLastError(); c = sm_count() / 2; }
+        if (cudaOccupancyMaxActiveClusters(&c, exact_kernel<QT, TOK>, &cfg) != cudaSuccess || c <= 0) { cudaGetLastError(); c = sm_count() / 2; }
         clusters = c;
     }
     cfg.gridDim = dim3(2u * (unsigned)(units < clusters ? units : clusters));
-    cudaLaunchKernelEx(&cfg, exact_kernel<QT>, map, A);
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.numAttrs = 2;
+    cudaLaunchKernelEx(&cfg, exact_kernel<QT, TOK>, map, A);
     note_launch();
     return LB_OK;
 }
+template <int QT> static int exact_launch_one(const CUtensorMap& map, const ExactArgs& A, int64_t units, cudaStream_t st) {
+    return A.tt <= 64 ? exact_launch_tile<QT, 64>(map, A, units, st) : exact_launch_tile<QT, 128>(map, A, units, st);
+}
 
-// K splits: rounds of the resident clusters x k-blocks per unit at 0.33 us, + the partial sums' round trip and its launch
+// Token tile and K splits: rounds of the resident clusters x k-blocks per unit + a unit's start and end, + the partial sums' round trip
+// and its launch.  A k-block: twelve MMA steps of half a clock per token (0.0031 us a token), 0.33 us of staging at least
 struct ExactPlan { int tt, ks; };
 static ExactPlan exact_plan(int64_t n_rows, int64_t nb, int64_t m) {
-    const int64_t clusters = sm_count() / 2, n_fp = (n_rows / 128 + 1) / 2, nt = (m + kExTok - 1) / kExTok;
-    ExactPlan best = {(int)(((m + nt - 1) / nt + 15) & ~int64_t(15)), 1};
+    const int64_t clusters = sm_count() / 2, n_fp = (n_rows / 128 + 1) / 2, nt0 = (m + kExTok - 1) / kExTok;
+    ExactPlan best = {kExTok, 1};
     double best_cost = 1e30;
-    for (int64_t ks = 1; ks == 1 || (ks <= 8 && nb / ks >= 8); ks++) {
-        const int64_t rounds = (n_fp * nt * ks + clusters - 1) / clusters;
-        double cost = (double)rounds * ((double)((nb + ks - 1) / ks) * 0.33 + 1.0);
-        if (ks > 1) cost += (double)ks * (double)m * (double)n_rows * 8.0 / 4.0e6 + 2.0;
-        if (cost < best_cost - 1e-9) { best_cost = cost; best.ks = (int)ks; }
+    for (int64_t nt = nt0; nt <= nt0 + 4 && nt <= (m + 31) / 32; nt++) {
+        const int64_t tt = ((m + nt - 1) / nt + 15) & ~int64_t(15);
+        const double mma = 0.0031 * (double)tt, per_kb = mma > 0.33 ? mma : 0.33;
+        for (int64_t ks = 1; ks == 1 || (ks <= 8 && nb / ks >= 8); ks++) {
+            const int64_t rounds = (n_fp * nt * ks + clusters - 1) / clusters;
+            double cost = (double)rounds * ((double)((nb + ks - 1) / ks) * per_kb + 1.5);
+            if (ks > 1) cost += (double)ks * (double)m * (double)n_rows * 8.0 / 4.0e6 + 2.0;
+            if (cost < best_cost - 1e-9) { best_cost = cost; best = {(int)tt, (int)ks}; }
+        }
     }
     return best;
 }

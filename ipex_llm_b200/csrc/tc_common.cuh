@@ -110,6 +110,26 @@ __device__ __forceinline__ bool mbar_wait3_lim(bool ready, uint32_t b0, uint32_t
         if (wait_over(t0, W)) return false;
     return true;
 }
+// the same for four
+__device__ __forceinline__ bool mbar_test4(uint32_t b0, uint32_t p0, uint32_t b1, uint32_t p1, uint32_t b2, uint32_t p2, uint32_t b3, uint32_t p3) {
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p, q, r, s;\n\t"
+                 "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+                 "mbarrier.test_wait.parity.shared::cta.b64 q, [%3], %4;\n\t"
+                 "mbarrier.test_wait.parity.shared::cta.b64 r, [%5], %6;\n\t"
+                 "mbarrier.test_wait.parity.shared::cta.b64 s, [%7], %8;\n\t"
+                 "and.pred p, p, q;\n\tand.pred r, r, s;\n\tand.pred p, p, r;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok) : "r"(b0), "r"(p0), "r"(b1), "r"(p1), "r"(b2), "r"(p2), "r"(b3), "r"(p3) : "memory");
+    return ok != 0;
+}
+__device__ __forceinline__ bool mbar_wait4_lim(bool ready, uint32_t b0, uint32_t p0, uint32_t b1, uint32_t p1, uint32_t b2, uint32_t p2, uint32_t b3, uint32_t p3,
+                                               const Waits& W) {
+    if (__all_sync(0xffffffffu, ready)) return true;
+    const long long t0 = clock64();
+    while (!__all_sync(0xffffffffu, mbar_test4(b0, p0, b1, p1, b2, p2, b3, p3)))
+        if (wait_over(t0, W)) return false;
+    return true;
+}
 // the phases of the last `n` of `issued` trips around a ring of n slots are complete: this warp's copies have landed
 template <typename Full> __device__ __forceinline__ void drain_ring(int issued, int n, Full full, const Waits& W) {
     const Waits late = {W.word, kWaitCycles};
@@ -160,6 +180,15 @@ __device__ __forceinline__ uint32_t and_or(uint32_t a, uint32_t b, uint32_t c) {
 // register order as the mma.sync fragments of the GEMV kernel (the tile layout is shared).
 template <int QT> struct Expand;
 
+// The same order of codes in bf16 pairs, exact and unscaled, for formats whose value is code x scale (bf16(), gemm_exact.cu): 4-bit codes
+// under the magic number 128, 8- and 6-bit floats as the upper halves of their 32-bit values.  A way that ends in cvt.rn.bf16x2.f32
+// (7 clocks of a quarter of an SM) took twice the clocks.
+__device__ __forceinline__ __nv_bfloat162 u2bf(uint32_t u) { return *reinterpret_cast<__nv_bfloat162*>(&u); }
+__device__ __forceinline__ uint32_t bf2u(__nv_bfloat162 v) { return *reinterpret_cast<uint32_t*>(&v); }
+__device__ __forceinline__ uint32_t h2_to_bf2_exact(uint32_t h) {            // at most 8 bits of significand
+    const float2 f = __half22float2(u2h(h));
+    return __byte_perm(__float_as_uint(f.x), __float_as_uint(f.y), 0x7632u);
+}
 template <int OFFSET> struct Expand4 {          // sym_int4 (OFFSET 1) / asym_int4 (OFFSET 2)
     static constexpr int kTileBytes = 512;
     static constexpr bool kHasMin = OFFSET == 2;
@@ -167,6 +196,11 @@ template <int OFFSET> struct Expand4 {          // sym_int4 (OFFSET 1) / asym_in
     // the lane's 16 bytes of the tile in one conflict-free LDS.128 (four LDS.32 at a 16-byte lane stride cost 4 wavefronts each)
     struct Codes { uint4 q; };
     __device__ static __forceinline__ void load(uint32_t codes, int lane, Codes& c) { c.q = lds128(codes + lane * 16); }
+    __device__ static __forceinline__ void bf16(const Codes& c, int s, uint32_t (&out)[4]) {
+        const uint32_t w = s == 0 ? c.q.x : s == 1 ? c.q.y : s == 2 ? c.q.z : c.q.w;
+#pragma unroll
+        for (int i = 0; i < 4; i++) out[i] = bf2u(__hsub2(u2bf(and_or(w >> (4 * i), 0x000f000fu, 0x43004300u)), u2bf(0x43084308u)));      // 128 + n - 136
+    }
     __device__ static __forceinline__ void run(const Codes& c, int s, __half2 dlo, __half2 dhi, __half2 mlo,
                                                __half2 mhi, uint32_t, uint32_t (&out)[4]) {
         const uint32_t w = s == 0 ? c.q.x : s == 1 ? c.q.y : s == 2 ? c.q.z : c.q.w;
@@ -210,6 +244,11 @@ template <int QT> struct Expand8 {
     }
     static constexpr int kLutBytes = 0;
     struct Codes { uint4 q0, q1; };
+    __device__ static __forceinline__ void bf16(const Codes& c, int s, uint32_t (&out)[4]) {
+        const uint32_t w[2] = {s == 0 ? c.q0.x : s == 1 ? c.q0.y : s == 2 ? c.q0.z : c.q0.w, s == 0 ? c.q1.x : s == 1 ? c.q1.y : s == 2 ? c.q1.z : c.q1.w};
+#pragma unroll
+        for (int i = 0; i < 4; i++) out[i] = h2_to_bf2_exact(pair(w[i & 1], i >> 1));
+    }
     __device__ static __forceinline__ void load(uint32_t codes, int lane, Codes& c) {
         c.q0 = lds128(codes + lane * 16); c.q1 = lds128(codes + 512 + lane * 16);
     }
@@ -234,6 +273,16 @@ template <> struct Expand<QT_FP6> {
     }
     static constexpr int kLutBytes = 0;
     struct Codes { uint4 lo; uint2 hi; };
+    __device__ static __forceinline__ void bf16(const Codes& c, int s, uint32_t (&out)[4]) {
+        const int u = s >> 1;
+        const uint32_t sh = (s & 1) ? 4u : 0u;
+        const uint32_t l[2] = {u ? c.lo.y : c.lo.x, u ? c.lo.w : c.lo.z}, h[2] = {c.hi.x, c.hi.y};
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            const uint32_t e = ((l[i & 1] >> sh) & 0x0f0f0f0fu) | (((h[i & 1] >> (2 * s)) & 0x03030303u) << 4);
+            out[i] = h2_to_bf2_exact(cvt2((unsigned short)(i >> 1 ? e >> 16 : e & 0xffffu)));
+        }
+    }
     __device__ static __forceinline__ void load(uint32_t codes, int lane, Codes& c) {
         c.lo = lds128(codes + lane * 16);
         asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(c.hi.x), "=r"(c.hi.y) : "r"(codes + 512 + lane * 8));
