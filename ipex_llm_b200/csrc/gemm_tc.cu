@@ -90,7 +90,6 @@ skinny_kernel(const __grid_constant__ CUtensorMap xmap, const SkinnyArgs A) {
 
     // the warp index through a shuffle: the compiler then treats everything derived from it as warp-uniform
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
-    if (A.pdl) asm volatile("griddepcontrol.launch_dependents;");
     const uint32_t lut = bars + 512 + 4 * lane;
     if constexpr (E::kLutBytes > 0) E::fill_lut(smem_raw + (bars + 512 - smem_u32(smem_raw)), threadIdx.x, kSkThreads);
     const int nb = (int)A.G.nb, np = nb >> 1;                // k-blocks / pairs of k-blocks per tile (nb is even)
@@ -261,6 +260,10 @@ skinny_kernel(const __grid_constant__ CUtensorMap xmap, const SkinnyArgs A) {
         for (int seg = 0; seg < n_seg; seg++) {
             mbar_wait(tmem_full(seg & 1), (uint32_t)((seg >> 1) & 1));
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            // the reduction may be scheduled while the last tiles are stored: it waits for this grid's end.  Calls in a row, launched
+            // behind the grid -> so: 40 rows, 11008 x 4096 21.5 -> 20.6 us, 17 rows, 1024 x 1024 16.5 -> 12.4, an MLP of 60 rows, 4096 /
+            // 14336, 74.4 -> 68.0.  (From the kernel's start the waiting blocks cost the recorded MLP 2 %.)
+            if (seg + 1 == n_seg) asm volatile("griddepcontrol.launch_dependents;");
             float* dst = A.part + ((int64_t)blockIdx.x * A.max_seg + seg) * (NTOK * 128) + quarter * 32 + lane;
             constexpr int CH = NTOK < 32 ? 16 : 32;
 #pragma unroll 1
@@ -291,10 +294,8 @@ struct SkReduceArgs {
     int mlp_act, n_ft1;      // mlp_act != 0: y = act(tile ft) * (tile ft + n_ft1), the fused MLP's two matrices (1 SiLU, 2 GELU)
 };
 __global__ void __launch_bounds__(128) skinny_reduce_kernel(const SkReduceArgs A) {
-    if (A.pdl) {
-        asm volatile("griddepcontrol.launch_dependents;");
-        asm volatile("griddepcontrol.wait;" ::: "memory");
-    }
+    if (A.pdl) asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const int ft = blockIdx.x, f = threadIdx.x;
     // CTA of item i = the largest c with c * total / grid <= i
     auto cta_of = [&](int64_t i) { return (int)(((i + 1) * A.grid + A.total - 1) / A.total - 1); };
@@ -441,7 +442,7 @@ static int skinny_launch_impl(const void* w, const void* w2, int mlp_act, int qt
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at; cfg.numAttrs = pdl ? 1 : 0;
+    cfg.attrs = at; cfg.numAttrs = 1;                         // whatever the switch for the launches around this one says
     if (!(A.dbg & 8)) cudaLaunchKernelEx(&cfg, skinny_reduce_kernel, R);
     note_launch();
     return check_launch();
