@@ -27,6 +27,7 @@
 // arrival) a k-block took 0.75 us instead of 0.25; what they order is shared memory, written behind a proxy fence and read by the
 // tensor cores of the SM that wrote it.
 // Every wait is bounded: see tc_common.cuh.
+#include <type_traits>
 #include "tc_pair.cuh"
 
 namespace lowbit {
@@ -341,30 +342,55 @@ pair_kernel(const __grid_constant__ CUtensorMap xmap, const PairArgs A) {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t acc = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * kPairTok);
             if (wide) {
+                // 32-bit results leave from the lanes: a warp stores a token's 32 features.  Conditions outside, as below
+                auto unit_out = [&](auto gated, auto split) {
+                    constexpr bool ACT = decltype(gated)::value, SPLIT = decltype(split)::value;
+                    // partial sums: [K split][token][features], behind gate and up [gate features | up features]
+                    const int64_t stride = ACT && SPLIT ? 2 * N : N;
+                    float* const out = SPLIT ? A.part + ((int64_t)U.ks * A.M + U.m0) * stride + (ACT ? half * N : 0) + n : (float*)A.y + (int64_t)U.m0 * N + n;
 #pragma unroll 1
-                for (int c = 0; c < rows; c += 16) {
-                    float v[16];
-                    tmem_ld16(acc + c, v);
-                    const int64_t at = (int64_t)(U.m0 + c) * N + n;
-                    if (A.act && A.ksplit > 1) {                     // [K split][token][gate features | up features]
-                        if (valid) store_feature(A.part + ((int64_t)U.ks * A.M + U.m0 + c) * 2 * N + half * N + n, 2 * N, v, rows - c, 0.0f, false);
-                    } else if (A.act) {
-                        float o[8];
-                        gate_up(v, A.act, half, o);
+                    for (int c = 0; c < rows; c += 32) {
+                        float v[32];
+                        tmem_ld32(acc + c, v);
+                        if (!valid) continue;
+                        float* p = out + c * stride;
+                        if (ACT && !SPLIT) {
 #pragma unroll
-                        for (int i = 0; i < 8; i++)
-                            if (valid && c + 2 * i + half < rows) ((float*)A.y)[at + (2 * i + half) * N] = o[i];
-                    } else if (valid) {
-                        if (A.ksplit > 1) store_feature(A.part + (int64_t)U.ks * A.M * N + at, N, v, rows - c, 0.0f, false);
-                        else store_feature((float*)A.y + at, N, v, rows - c, b, A.accumulate != 0);
+                            for (int h = 0; h < 2; h++) {
+                                float x[16], o[8];
+#pragma unroll
+                                for (int j = 0; j < 16; j++) x[j] = v[16 * h + j];
+                                gate_up(x, A.act, half, o);
+#pragma unroll
+                                for (int i = 0; i < 8; i++)
+                                    if (c + 16 * h + 2 * i + half < rows) p[(16 * h + 2 * i + half) * N] = o[i];
+                            }
+                        } else if (!SPLIT && A.accumulate) {
+#pragma unroll
+                            for (int j = 0; j < 32; j++, p += stride) if (c + j < rows) *p += v[j] + b;
+                        } else if (c + 32 <= rows) {
+#pragma unroll
+                            for (int j = 0; j < 32; j++, p += stride) *p = SPLIT ? v[j] : v[j] + b;
+                        } else {
+#pragma unroll
+                            for (int j = 0; j < 32; j++, p += stride) if (c + j < rows) *p = SPLIT ? v[j] : v[j] + b;
+                        }
                     }
-                    __syncwarp();
-                }
+                };
+                const std::true_type yes;
+                const std::false_type no;
+                if (!A.act) { if (A.ksplit > 1) unit_out(no, yes); else unit_out(no, no); }
+                else if (A.ksplit > 1) unit_out(yes, yes);
+                else unit_out(yes, no);
             } else {
-                // 16-bit results: 32 tokens at a time through shared memory, so that a token's 128 (64 behind the activation)
-                // features leave as one run of 16-byte stores.  Straight from the lanes (2-byte stores, runs of 32 bytes) a tile of
-                // 256 tokens took 8 us, 60 clocks per token and warp.  The two runs of 16 features that a warp holds sit in different
-                // halves of the banks (the chunk's pieces are permuted, and put back by the copy).
+                // 16-bit results: 32 tokens at a time through shared memory, so that a token's 128 (64 behind the activation) features
+                // leave as one run of 16-byte stores.  The accumulators are read in the fragment shape (a thread: two tokens of features
+                // g and g + 8 of 16), so that pairs of tokens are 8 x 8 matrices that stmatrix turns on their way, and gate and up of one
+                // feature are registers of one thread.  When every lane stored its feature's 32 tokens in 2 bytes each, with the kinds of results
+                // as conditions inside the loop (both sides computed for every value), 32 tokens took 1500 clocks beside the main loop and
+                // behind it (400 so), 32-bit results of a unit of 256 tokens 12 us (3.5 so), which nothing hides behind a cluster's last
+                // unit.  512 rows, 4096 x 11008, bf16 (K in two splits) 49.1 -> 40.6 us, fp16 44.8 -> 42.6, an MLP of 1000 rows, 4096 / 14336,
+                // bf16 323 -> 271, of 4000 rows 1198 -> 1099 (fewer clocks a k-block, too: 531 -> 478 beside an epilogue).
                 const bool f16 = A.y_dtype == DT_F16, y_vec = (reinterpret_cast<uintptr_t>(A.y) & 15) == 0;
                 auto put = [&](uint16_t* dst, const uint4& q) {
                     if (y_vec) { *reinterpret_cast<uint4*>(dst) = q; return; }
@@ -373,55 +399,79 @@ pair_kernel(const __grid_constant__ CUtensorMap xmap, const PairArgs A) {
                     for (int i = 0; i < 8; i++) dst[i] = (uint16_t)(w[i >> 1] >> (16 * (i & 1)));
                 };
                 uint16_t* const yb = (uint16_t*)A.y + (int64_t)U.m0 * N + f0;
+                // 16 TMEM lanes are 16 features: which ones of the tile's
+                const int first[2] = {16 * quarter, 64 + 16 * quarter};
+                // the lane's row address in four matrices: tokens 8 (lane / 16) + lane % 8 of 16, eight features of 16
+                const int tok = 8 * (lane >> 4) + (lane & 7), fh8 = (lane >> 3) & 1;
+                // type and activation known to the compiler: as conditions inside, both sides of them were computed for every value
+                auto unit_out = [&](auto half_type, auto gated) {
+                    constexpr bool F16 = decltype(half_type)::value, ACT = decltype(gated)::value;
+                    constexpr int LINE = ACT ? 128 : 256, LG = ACT ? 3 : 4;                  // bytes of a token's features, its 16-byte pieces
+                    auto pack = [](float x, float y) { return pack2<!F16>(x, y); };
+                    float bias[2][2] = {};                            // [16 lanes][g, g + 8]
+                    if (!ACT && A.bias && valid) {
+#pragma unroll
+                        for (int hh = 0; hh < 2; hh++)
+#pragma unroll
+                            for (int fh = 0; fh < 2; fh++) {
+                                const int64_t f = f0 + first[hh] + 8 * fh + (lane >> 2);
+                                bias[hh][fh] = F16 ? __half2float(((const __half*)A.bias)[f]) : __bfloat162float(((const __nv_bfloat16*)A.bias)[f]);
+                            }
+                    }
 #pragma unroll 1
-                for (int c = 0; c < rows; c += 32, chunk ^= 1u) {
-                    const uint32_t ob = obuf + chunk * 8192;
+                    for (int c = 0; c < rows; c += 32, chunk ^= 1u) {
+                        const uint32_t ob = obuf + chunk * 8192;
+                        float v[2][16];
+                        tmem_ld_frag32(acc + c, v[0]);
+                        tmem_ld_frag32(acc + ((uint32_t)16 << 16) + c, v[1]);
+                        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                        if (!ACT && A.accumulate && valid) {
 #pragma unroll
-                    for (int h = 0; h < 2; h++) {
-                        float v[16];
-                        tmem_ld16(acc + c + 16 * h, v);
-                        if (A.act) {
-                            float o[8];
-                            gate_up(v, A.act, half, o);
-                            const uint32_t at = ob + (uint32_t)((16 * h + half) * 128 + (((16 * quarter + (lane & 15)) * 2) ^ (half << 6)));
+                            for (int hh = 0; hh < 2; hh++)
 #pragma unroll
-                            for (int i = 0; i < 8; i++) {
-                                const uint16_t bits = f16 ? __half_as_ushort(__float2half_rn(o[i])) : __bfloat16_as_ushort(__float2bfloat16_rn(o[i]));
-                                asm volatile("st.shared.u16 [%0], %1;" ::"r"(at + i * 256), "h"(bits) : "memory");
+                                for (int i = 0; i < 16; i++) {
+                                    const int t = c + 8 * (i >> 2) + 2 * (lane & 3) + (i & 1);
+                                    const uint16_t* yp = yb + (int64_t)t * N + first[hh] + 8 * ((i >> 1) & 1) + (lane >> 2);
+                                    if (t < rows) v[hh][i] += F16 ? __half2float(__ushort_as_half(*yp)) : __bfloat162float(__ushort_as_bfloat16(*yp));
+                                }
+                        }
+#pragma unroll
+                        for (int hh = 0; hh < (ACT ? 1 : 2); hh++)
+#pragma unroll
+                            for (int p = 0; p < 2; p++) {             // 16 tokens
+                                uint32_t m[4];
+#pragma unroll
+                                for (int j = 0; j < 4; j++) {         // tokens 8 (j / 2) of them, features 8 (j % 2) of 16
+                                    const int i = 8 * p + 4 * (j >> 1) + 2 * (j & 1);
+                                    m[j] = ACT ? pack(apply_act(v[0][i], A.act) * v[1][i], apply_act(v[0][i + 1], A.act) * v[1][i + 1])
+                                               : pack(v[hh][i] + bias[hh][j & 1], v[hh][i + 1] + bias[hh][j & 1]);
+                                }
+                                const int r = 16 * p + tok, piece = (first[hh] >> 3) + fh8;
+                                stmatrix4_trans(ob + (uint32_t)(r * LINE + ((piece ^ (r & 7)) << 4)), m);
                             }
-                        } else {
-                            if (A.accumulate) {
-                                const uint16_t* yp = (const uint16_t*)A.y + (int64_t)(U.m0 + c + 16 * h) * N + n;
+                        asm volatile("barrier.cta.sync 1, 128;" ::: "memory");
+                        // the other buffer is written next: everybody passes the next barrier only after this copy
+                        const int n_rows = min(32, rows - c);
+                        const int r0 = e_tid >> LG, p = e_tid & ((1 << LG) - 1);             // piece p: 8 features from 8 p
+                        uint16_t* const to = yb + (int64_t)(c + r0) * N + p * 8;
+                        constexpr int STEP = 128 >> LG;                                      // rows between a thread's pieces: 8 or 16
+                        const uint32_t from = ob + (uint32_t)(r0 * LINE + ((p ^ (r0 & 7)) << 4));
+                        if (valid && n_rows == 32 && y_vec) {
+                            uint4 q[32 / STEP];
 #pragma unroll
-                                for (int j = 0; j < 16; j++)
-                                    if (valid && c + 16 * h + j < rows)
-                                        v[j] += f16 ? __half2float(__ushort_as_half(yp[j * N])) : __bfloat162float(__ushort_as_bfloat16(yp[j * N]));
-                            }
-                            const uint32_t at = ob + (uint32_t)(16 * h * 256 + quarter * 64 + half * 32 + (lane & 15) * 2);
+                            for (int i = 0; i < 32 / STEP; i++) q[i] = lds128(from + i * STEP * LINE);
 #pragma unroll
-                            for (int j = 0; j < 16; j++) {
-                                const uint16_t bits = f16 ? __half_as_ushort(__float2half_rn(v[j] + b)) : __bfloat16_as_ushort(__float2bfloat16_rn(v[j] + b));
-                                asm volatile("st.shared.u16 [%0], %1;" ::"r"(at + j * 256), "h"(bits) : "memory");
-                            }
+                            for (int i = 0; i < 32 / STEP; i++) *reinterpret_cast<uint4*>(to + (int64_t)i * STEP * N) = q[i];
+                        } else if (valid) {
+                            for (int i = 0; r0 + i * STEP < n_rows; i++) put(to + (int64_t)i * STEP * N, lds128(from + i * STEP * LINE));
                         }
                     }
-                    asm volatile("barrier.cta.sync 1, 128;" ::: "memory");
-                    // the other buffer is written next: everybody passes the next barrier only after this copy
-                    const int n_rows = min(32, rows - c);
-                    if (valid) {
-                        if (A.act) {
-                            for (int i = e_tid; i < n_rows * 8; i += 128) {
-                                const int r = i >> 3, p = i & 7;
-                                put(yb + (int64_t)(c + r) * N + p * 8, lds128(ob + r * 128 + (uint32_t)((p ^ ((r & 1) << 2)) * 16)));
-                            }
-                        } else {
-                            for (int i = e_tid; i < n_rows * 16; i += 128) {
-                                const int r = i >> 4, p = i & 15;              // piece p: 8 features from 8 p
-                                put(yb + (int64_t)(c + r) * N + p * 8, lds128(ob + r * 256 + (uint32_t)((((p >> 1) & 3) * 4 + (p >> 3) * 2 + (p & 1)) * 16)));
-                            }
-                        }
-                    }
-                }
+                };
+                const std::true_type yes;
+                const std::false_type no;
+                if (!A.act) { if (f16) unit_out(yes, no); else unit_out(no, no); }
+                else if (f16) unit_out(yes, yes);
+                else unit_out(no, yes);
             }
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();

@@ -332,6 +332,11 @@ template <> struct Expand<QT_NF4> {
     }
 };
 
+template <bool BF> __device__ __forceinline__ uint32_t pack2(float a, float b) {
+    if (BF) return bf2u(__floats2bfloat162_rn(a, b));
+    return h2u(__floats2half2_rn(a, b));
+}
+
 // bytes of one 64-row group x one k-block as the kernels stage it: codes, fp16 scales [, minima]
 template <int QT> struct PackedBlock {
     static constexpr int kSuper = RG_TILES * Expand<QT>::kTileBytes;

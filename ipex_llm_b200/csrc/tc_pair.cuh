@@ -27,6 +27,21 @@ __device__ __forceinline__ void umma2_commit_w(uint32_t bar, uint32_t leader) {
         "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %2;\n\t}"
         ::"r"(bar), "r"(leader), "h"((uint16_t)3) : "memory");
 }
+// 16 TMEM lanes x 32 columns as mma fragments: v[4 i + ..] = (lane g, columns 8 i + 2 t, + 1), (lane g + 8, the same) for thread 4 g + t.
+// No wait
+__device__ __forceinline__ void tmem_ld_frag32(uint32_t taddr, float (&v)[16]) {
+    uint32_t* r = reinterpret_cast<uint32_t*>(v);
+    asm volatile(
+        "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+        : "r"(taddr));
+}
+// four 8 x 8 matrices of 16-bit elements, each stored turned: lane 8 j + i gives the address of row i (a column of the fragment) of matrix j
+__device__ __forceinline__ void stmatrix4_trans(uint32_t addr, const uint32_t (&m)[4]) {
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(m[0]), "r"(m[1]), "r"(m[2]), "r"(m[3]) : "memory");
+}
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
     uint32_t r[16];
     asm volatile(
