@@ -557,13 +557,14 @@ static int pair_launch(int qt, bool bf, const CUtensorMap& map, const PairArgs& 
     return LB_ERR_ARG;
 }
 
-// Token tile and K splits of a matmul: the pair that minimises rounds of the resident clusters x k-blocks per unit x time per
-// k-block + the start and end of a unit and, when K is split, the partial sums' round trip through memory at ~4 TB/s and the second
-// launch.  Time per k-block, measured at 4096 x 11008 and 4096 x 4096: 0.0011 us per token once the MMAs set the pace (0.282 at 256),
-// below that the expansion and the chain around it: 0.19 us for sym_int4 with fp16 activations, 0.24 with bf16, 0.29 for nf4's table;
-// the other formats were not measured and take sym_int4's figures.  What the line between (128 tokens, K whole) and (256, two splits) is worth at 512 tokens, 4096 x 11008:
-// sym_int4 fp16 43.4 against 48.2 us, bf16 50.3 against 48.8, nf4 58.1 against 50.1.
-constexpr double kPaces[3] = {0.19, 0.24, 0.29};
+// Token tile and K splits of a matmul: the pair that minimises rounds of the resident clusters x (k-blocks per unit x time per k-block
+// + the start and end of a unit) and, when K is split, the partial sums' round trip through memory and the second launch.  Times as the
+// power cap leaves them (1.6 to 1.75 GHz), sym_int4 but for nf4's table (the other formats take sym_int4's): a k-block 0.0012 us per token
+// once the MMAs set the pace, below that 0.215 us for the expansion and the chain around it with fp16 activations, 0.275 with bf16, 0.35
+// for nf4; a unit 1.2 us and 6 ns per token of its results.  Where the line lies, whole K against the split one at 512 rows, 4096 x
+// 11008: fp16 43.9 (128-token tiles) / 41.9 us (256, two splits), bf16 47.8 / 41.8; at 512 rows, 4096 x 4096: fp16 22.1 / 24.7, bf16
+// 24.0 / 24.4, nf4 28.4 / 26.1; at 200 rows fp16 20.1 / 17.2 (208 tokens, four splits).
+constexpr double kPaces[3] = {0.215, 0.275, 0.35};
 static double pair_pace(int qt, bool bf) { return kPaces[qt == QT_NF4 ? 2 : bf ? 1 : 0]; }
 struct PairPlan { int tt, ks; };
 static PairPlan pair_plan(double pace, int64_t n_fp, int64_t nb, int64_t m, int64_t n_out, bool may_split) {
@@ -572,12 +573,12 @@ static PairPlan pair_plan(double pace, int64_t n_fp, int64_t nb, int64_t m, int6
     double best_cost = 1e30;
     for (int64_t nt = nt0; nt <= nt0 + 8 && nt <= (m + 31) / 32; nt++) {
         const int64_t tt = ((m + nt - 1) / nt + 15) & ~int64_t(15);
-        const double mma = 0.0011 * (double)tt, per_kb = mma > pace ? mma : pace;
+        const double mma = 0.0012 * (double)tt, per_kb = mma > pace ? mma : pace;
         const int64_t max_ks = may_split ? (nb / 8 < 8 ? nb / 8 : 8) : 1;
         for (int64_t ks = 1; ks == 1 || ks <= max_ks; ks++) {
             const int64_t rounds = (n_fp * nt * ks + clusters - 1) / clusters;
-            double cost = (double)rounds * ((double)((nb + ks - 1) / ks) * per_kb + 1.0);
-            if (ks > 1) cost += (double)ks * (double)m * (double)n_out * 8.0 / 4.0e6 + 3.0;
+            double cost = (double)rounds * ((double)((nb + ks - 1) / ks) * per_kb + 1.2 + 0.006 * (double)tt);
+            if (ks > 1) cost += (double)ks * (double)m * (double)n_out * 8.0 / 8.0e6 + 2.5;
             if (cost < best_cost - 1e-9) { best_cost = cost; best = {(int)tt, (int)ks}; }
         }
     }
