@@ -271,6 +271,18 @@ int lowbit_matmul_cuda(const void* d_w, int qtype, int64_t n_rows, int64_t k, co
     return rc;
 }
 
+int lowbit_matmul_grad_supported(int qtype, int64_t n_rows, int64_t k) { return gemm_tc_grad_supported(qtype, n_rows, k) ? 1 : 0; }
+size_t lowbit_matmul_grad_workspace_size(int64_t n_rows, int64_t k, int64_t m) { return gemm_tc_grad_workspace_size(n_rows, k, m); }
+int lowbit_matmul_grad_cuda(const void* d_w, int qtype, int64_t n_rows, int64_t k, const void* d_grad, int dtype, int64_t m, void* d_out,
+                            void* workspace, size_t workspace_bytes, void* stream) {
+    t_launches = 0;
+    if (m == 0) return LB_OK;
+    const int rc = !d_w || !d_grad || !d_out || m < 0 || m > 0x7fffffff ? LB_ERR_ARG
+                 : gemm_tc_grad_launch(d_w, qtype, n_rows, k, d_grad, dtype, m, d_out, workspace, workspace_bytes, (cudaStream_t)stream);
+    if (rc == LB_ERR_ARG) set_error(rc, "lowbit_matmul_grad_cuda: bad argument (qtype %d, N %lld, K %lld, M %lld)", qtype, (long long)n_rows, (long long)k, (long long)m);
+    return rc;
+}
+
 size_t lowbit_mlp_workspace_size(int64_t n_rows, int64_t k, int64_t m, int x_dtype) {
     if (use_skinny(B200_QT_SYM_INT4, n_rows, k, m, x_dtype)) return gemm_skinny_mlp_workspace_size(n_rows, k, m);
     if (use_gemm(B200_QT_SYM_INT4, n_rows, k, m, x_dtype)) return gemm_tc_mlp_workspace_size(n_rows, k, m);

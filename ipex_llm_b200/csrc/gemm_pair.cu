@@ -82,7 +82,13 @@ __device__ __forceinline__ void gate_up(const float (&v)[16], int act, int half,
     }
 }
 
-template <int QT, bool BF>
+// GRAD: the product with the transposed weights, dx[M][K] = g[M][N] . dequant(W[N][K]), in the same loop: a k-block is 64 rows of W, a
+// feature tile 128 of its columns (two k-blocks of the packed layout, side by side in memory).  The expanded tile is the same image in
+// shared memory -- 64 elements of one weight row to a 128-byte line -- read as an MN-major operand, so nothing is transposed (K-major in
+// its place takes the same time).  Weights are rounded once from their 32-bit value (expand_once).  What it replaces wrote the
+// dequantised matrix to memory for a library product: forward and backward of 1024 rows, 11008 x 4096, nf4 bf16 167 -> 158 us, sym_int4
+// fp16 160 -> 139, of 3000 rows, 8192 x 8192, 668 -> 593, of 20 rows, 14336 x 14336, nf4 263 -> 140.
+template <int QT, bool BF, bool GRAD>
 __global__ void __launch_bounds__(kPairThreads, 1)
 pair_kernel(const __grid_constant__ CUtensorMap xmap, const PairArgs A) {
     using E = Expand<QT>;
@@ -110,9 +116,12 @@ pair_kernel(const __grid_constant__ CUtensorMap xmap, const PairArgs A) {
     // the warp index through a shuffle: the compiler then treats everything derived from it as warp-uniform
     const int warp = __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const int rank = (int)(blockIdx.x & 1);
-    const uint32_t lut = lut0 + 4 * lane;
-    if constexpr (E::kLutBytes > 0) E::fill_lut(smem_raw + (lut0 - smem_u32(smem_raw)), threadIdx.x, kPairThreads);
-    const int nb = (int)A.G.nb;
+    const uint32_t lut = lut0 + (GRAD ? 8 * (lane & 15) : 4 * lane);
+    if constexpr (E::kLutBytes > 0) {
+        if (GRAD) fill_nf4_pairs(smem_raw + (lut0 - smem_u32(smem_raw)), threadIdx.x, kPairThreads);
+        else E::fill_lut(smem_raw + (lut0 - smem_u32(smem_raw)), threadIdx.x, kPairThreads);
+    }
+    const int nb = GRAD ? (int)(A.G.rows >> 6) : (int)A.G.nb;          // k-blocks of the product
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < KX; s++) { mbar_init(x_full(s), 1); mbar_init(x_empty(s), 1); mbar_init(xp_full(s), 1); }
@@ -198,8 +207,8 @@ pair_kernel(const __grid_constant__ CUtensorMap xmap, const PairArgs A) {
             bool ready = false;
             for (int unit = blockIdx.x >> 1; unit < n_units; unit += stride, ti++) {
                 decode(unit, U);
-                // c F32 (1<<4), a/b format (0 f16, 1 bf16), both K-major, N (>>3 at bit 17), M = 256 (>>4 at bit 24)
-                const uint32_t idesc = (1u << 4) | ((BF ? 1u : 0u) << 7) | ((BF ? 1u : 0u) << 10) | (((uint32_t)U.n_tok >> 3) << 17) | ((256u >> 4) << 24);
+                // c F32 (1<<4), a/b format (0 f16, 1 bf16), both K-major (GRAD: A MN-major), N (>>3 at bit 17), M = 256 (>>4 at bit 24)
+                const uint32_t idesc = (GRAD ? 1u << 15 : 0u) | (1u << 4) | ((BF ? 1u : 0u) << 7) | ((BF ? 1u : 0u) << 10) | (((uint32_t)U.n_tok >> 3) << 17) | ((256u >> 4) << 24);
                 const int buf = ti & 1;
                 if (!mbar_wait_lim(tmem_empty(buf), (uint32_t)(((ti >> 1) & 1) ^ 1), A.waits)) goto done;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -208,10 +217,13 @@ pair_kernel(const __grid_constant__ CUtensorMap xmap, const PairArgs A) {
                     const int sa = it & 3;
                     if (!mbar_wait3_lim(ready, x_full(sx), (uint32_t)(rx & 1), xp_full(sx), (uint32_t)(rx & 1), a_full(sa), (uint32_t)((it >> 2) & 1), A.waits)) goto done;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint64_t ad = make_desc(aring + sa * kTileBytesAB), xd = make_desc(xring + sx * kTileBytesAB);
+                    uint64_t ad = make_desc(aring + sa * kTileBytesAB);
+                    const uint64_t xd = make_desc(xring + sx * kTileBytesAB);
+                    // MN-major: LBO = the next 64 features (8 KB), SBO = the next eight lines; a step of 16 lines
+                    if (GRAD) ad = (ad & ~((uint64_t)0x3fff << 16)) | ((uint64_t)(8192 >> 4) << 16);
 #pragma unroll
                     for (int k4 = 0; k4 < 4; k4++)           // the address field counts 16-byte units
-                        umma2_f16_w(acc, ad + (uint64_t)((k4 * 32) >> 4), xd + (uint64_t)((k4 * 32) >> 4), idesc, (kb > U.kb0 || k4 > 0) ? 1u : 0u, leader);
+                        umma2_f16_w(acc, ad + (uint64_t)((GRAD ? k4 * 2048 : k4 * 32) >> 4), xd + (uint64_t)((k4 * 32) >> 4), idesc, (kb > U.kb0 || k4 > 0) ? 1u : 0u, leader);
                     umma2_commit_w(a_empty(sa), leader);
                     umma2_commit_w(x_empty(sx), leader);
                     if (++sx == KX) { sx = 0; rx++; }
@@ -249,7 +261,8 @@ pair_kernel(const __grid_constant__ CUtensorMap xmap, const PairArgs A) {
 #pragma unroll
                 for (int gi = 0; gi < 2; gi++) {
                     const uint8_t* wb = gi ? w1 : w0;
-                    const int64_t u = (gi ? rg1 : rg0) * nb + kb;
+                    // GRAD: row group kb, the tile's two blocks of 64 columns
+                    const int64_t u = GRAD ? (int64_t)kb * A.G.nb + min(2 * (int64_t)U.ft + gi, A.G.nb - 1) : (gi ? rg1 : rg0) * nb + kb;
                     const uint32_t dst = pring + s * SM::kPacked + gi * SM::kGroup;
                     bulk_g2s_w(dst, wb + u * PackedBlock<QT>::kSuper, PackedBlock<QT>::kSuper, p_full(s), leader);
                     bulk_g2s_w(dst + PackedBlock<QT>::kSuper, wb + A.G.off_s + u * 128, 128, p_full(s), leader);
@@ -263,7 +276,8 @@ pair_kernel(const __grid_constant__ CUtensorMap xmap, const PairArgs A) {
         // ================= dequant: group (warp - 4) / 4 takes every fourth k-block; a warp expands 16 rows of either row group =================
         const int grp = (warp - kPairDeq0) >> 2, dw = (warp - kPairDeq0) & 3;
         const int g = lane >> 2, t = lane & 3;
-        const uint32_t row0 = aring + grp * kTileBytesAB + 4 * dw * 1024 + g * 128;        // rows 32 dw + g, + 8; + 16, + 24 for the second group
+        // rows 32 dw + g, + 8; + 16, + 24 for the second group.  GRAD: lines 16 dw + g, + 8 of either block
+        const uint32_t row0 = aring + grp * kTileBytesAB + (GRAD ? 2 : 4) * dw * 1024 + g * 128, row_step = GRAD ? 8192 : 2048;
         // k-blocks are numbered over all units of the cluster: `end` behind the unit's last, `it` this group's next
         int end = 0, it = grp;
         for (int unit = blockIdx.x >> 1; unit < n_units; unit += stride) {
@@ -287,6 +301,7 @@ pair_kernel(const __grid_constant__ CUtensorMap xmap, const PairArgs A) {
                 uint32_t lo[2][8], hi[2][8];
 #pragma unroll
                 for (int gi = 0; gi < 2; gi++) {
+                    if constexpr (GRAD) { expand_once<QT, BF>(cw[gi], dq[gi], mq[gi], lut, lo[gi], hi[gi]); continue; }
                     const __half2 d2 = u2h(dq[gi]), m2 = u2h(mq[gi]);
                     const __half2 dlo = __low2half2(d2), dhi = __high2half2(d2);
                     const __half2 mlo = __low2half2(m2), mhi = __high2half2(m2);
@@ -307,7 +322,7 @@ pair_kernel(const __grid_constant__ CUtensorMap xmap, const PairArgs A) {
                 for (int gi = 0; gi < 2; gi++)
 #pragma unroll
                     for (int q = 0; q < 2; q++) {               // k-steps 2q, 2q+1 -> one 16-byte chunk per row; 128B swizzle: chunk ^ (row & 7)
-                        const uint32_t at = row0 + gi * 2048 + (uint32_t)((2 * t + q) ^ g) * 16;
+                        const uint32_t at = row0 + gi * row_step + (uint32_t)((2 * t + q) ^ g) * 16;
                         asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(lo[gi][4 * q]), "r"(lo[gi][4 * q + 1]), "r"(lo[gi][4 * q + 2]), "r"(lo[gi][4 * q + 3]) : "memory");
                         asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(at + 1024), "r"(hi[gi][4 * q]), "r"(hi[gi][4 * q + 1]), "r"(hi[gi][4 * q + 2]), "r"(hi[gi][4 * q + 3]) : "memory");
                     }
@@ -321,7 +336,7 @@ pair_kernel(const __grid_constant__ CUtensorMap xmap, const PairArgs A) {
     } else if (warp >= kPairEpi0) {
         // ================= epilogue: TMEM lanes 32 * (warp % 4) .. + 31 =================
         const int quarter = warp & 3, half = lane >> 4, e_tid = threadIdx.x - 32 * kPairEpi0;
-        const int64_t N = A.G.rows;
+        const int64_t N = GRAD ? A.G.k : A.G.rows;
         const bool wide = A.ksplit > 1 || A.y_dtype == DT_F32;        // 32-bit results go straight to memory
         uint32_t chunk = 0;
         int ti = 0;
@@ -329,7 +344,7 @@ pair_kernel(const __grid_constant__ CUtensorMap xmap, const PairArgs A) {
             decode(unit, U);
             const int buf = ti & 1, rows = U.m_end - U.m0;
             const int64_t f0 = (int64_t)U.ft * (A.act ? 64 : 128);
-            const int64_t n = f0 + (A.act ? 0 : 64 * half) + 16 * quarter + (lane & 15);
+            const int64_t n = GRAD ? f0 + 32 * quarter + lane : f0 + (A.act ? 0 : 64 * half) + 16 * quarter + (lane & 15);
             const bool valid = f0 < N;                                // the last pair's second tile may not exist
             float b = 0.0f;
             if (A.bias && valid && A.ksplit == 1)
@@ -379,7 +394,7 @@ pair_kernel(const __grid_constant__ CUtensorMap xmap, const PairArgs A) {
                 };
                 const std::true_type yes;
                 const std::false_type no;
-                if (!A.act) { if (A.ksplit > 1) unit_out(no, yes); else unit_out(no, no); }
+                if (GRAD || !A.act) { if (A.ksplit > 1) unit_out(no, yes); else unit_out(no, no); }
                 else if (A.ksplit > 1) unit_out(yes, yes);
                 else unit_out(yes, no);
             } else {
@@ -400,7 +415,7 @@ pair_kernel(const __grid_constant__ CUtensorMap xmap, const PairArgs A) {
                 };
                 uint16_t* const yb = (uint16_t*)A.y + (int64_t)U.m0 * N + f0;
                 // 16 TMEM lanes are 16 features: which ones of the tile's
-                const int first[2] = {16 * quarter, 64 + 16 * quarter};
+                const int first[2] = {GRAD ? 32 * quarter : 16 * quarter, GRAD ? 32 * quarter + 16 : 64 + 16 * quarter};
                 // the lane's row address in four matrices: tokens 8 (lane / 16) + lane % 8 of 16, eight features of 16
                 const int tok = 8 * (lane >> 4) + (lane & 7), fh8 = (lane >> 3) & 1;
                 // type and activation known to the compiler: as conditions inside, both sides of them were computed for every value
@@ -469,7 +484,7 @@ pair_kernel(const __grid_constant__ CUtensorMap xmap, const PairArgs A) {
                 };
                 const std::true_type yes;
                 const std::false_type no;
-                if (!A.act) { if (f16) unit_out(yes, no); else unit_out(no, no); }
+                if (GRAD || !A.act) { if (f16) unit_out(yes, no); else unit_out(no, no); }
                 else if (f16) unit_out(yes, yes);
                 else unit_out(no, yes);
             }
@@ -514,7 +529,7 @@ __global__ void __launch_bounds__(256) reduce_gated_kernel(const float* __restri
 }
 
 // clusters of two that can be resident at once (one CTA per SM; an SM without a partner in its group stays idle)
-template <int QT, bool BF>
+template <int QT, bool BF, bool GRAD>
 static int pair_clusters() {
     static int cached[64] = {};
     int dev = 0;
@@ -522,7 +537,7 @@ static int pair_clusters() {
     int& n = cached[dev & 63];
     if (n) return n;
     constexpr int SMEM = PairSmem<QT>::kTotal;
-    if (cudaFuncSetAttribute(pair_kernel<QT, BF>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess) { cudaGetLastError(); return 0; }
+    if (cudaFuncSetAttribute(pair_kernel<QT, BF, GRAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM) != cudaSuccess) { cudaGetLastError(); return 0; }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(sm_count() & ~1)); cfg.blockDim = dim3(kPairThreads); cfg.dynamicSmemBytes = SMEM;
     cudaLaunchAttribute at[1];
@@ -530,14 +545,14 @@ static int pair_clusters() {
     at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
     cfg.attrs = at; cfg.numAttrs = 1;
     int c = 0;
-    if (cudaOccupancyMaxActiveClusters(&c, pair_kernel<QT, BF>, &cfg) != cudaSuccess || c <= 0) { cudaGetLastError(); c = sm_count() / 2; }
+    if (cudaOccupancyMaxActiveClusters(&c, pair_kernel<QT, BF, GRAD>, &cfg) != cudaSuccess || c <= 0) { cudaGetLastError(); c = sm_count() / 2; }
     n = c;
     return n;
 }
 
-template <int QT, bool BF>
+template <int QT, bool BF, bool GRAD>
 static int pair_launch_one(const CUtensorMap& map, const PairArgs& A, int64_t units, cudaStream_t st) {
-    const int clusters = pair_clusters<QT, BF>();
+    const int clusters = pair_clusters<QT, BF, GRAD>();
     if (clusters <= 0) { set_error(LB_ERR_CUDA, "the two-SM matmul kernel cannot be configured on this device"); return LB_ERR_CUDA; }
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2u * (unsigned)(units < clusters ? units : clusters)); cfg.blockDim = dim3(kPairThreads);
@@ -546,12 +561,13 @@ static int pair_launch_one(const CUtensorMap& map, const PairArgs& A, int64_t un
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
     cfg.attrs = at; cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, pair_kernel<QT, BF>, map, A);
+    cudaLaunchKernelEx(&cfg, pair_kernel<QT, BF, GRAD>, map, A);
     note_launch();
     return LB_OK;
 }
+template <bool GRAD = false>
 static int pair_launch(int qt, bool bf, const CUtensorMap& map, const PairArgs& A, int64_t units, cudaStream_t st) {
-#define PAIR_CASE(Q) case Q: return bf ? pair_launch_one<Q, true>(map, A, units, st) : pair_launch_one<Q, false>(map, A, units, st);
+#define PAIR_CASE(Q) case Q: return bf ? pair_launch_one<Q, true, GRAD>(map, A, units, st) : pair_launch_one<Q, false, GRAD>(map, A, units, st);
     switch (qt) { PAIR_CASE(QT_SYM_INT4) PAIR_CASE(QT_ASYM_INT4) PAIR_CASE(QT_NF4) PAIR_CASE(QT_FP8_E4M3) PAIR_CASE(QT_FP8_E5M2) PAIR_CASE(QT_FP6) }
 #undef PAIR_CASE
     return LB_ERR_ARG;
@@ -628,11 +644,43 @@ int gemm_tc_launch(const void* w, int qt, int64_t n_rows, int64_t k, const void*
     if (p.ks > 1 && !holds_partials(workspace, workspace_bytes, (size_t)p.ks * m * n_rows)) p = pair_plan(pair_pace(qt, bf), A.n_fp, k / 64, m, n_rows, false);
     A.tt = p.tt; A.ksplit = p.ks; A.part = (float*)workspace;
     const int64_t units = (int64_t)A.n_fp * ((m + p.tt - 1) / p.tt) * p.ks;
-    if (const int rc = pair_launch(qt, bf, map, A, units, st)) return rc;
+    if (const int rc = pair_launch<>(qt, bf, map, A, units, st)) return rc;
     if (p.ks > 1) {
         const int64_t mn = m * n_rows;
         int rg = (int)((mn / 4 + 255) / 256); if (rg > sm_count() * 8) rg = sm_count() * 8;
         reduce_partials_kernel<<<rg, 256, 0, st>>>(A.part, p.ks, mn, n_rows, y, y_dtype, bias, accumulate);
+        note_launch();
+    }
+    return check_launch();
+}
+
+// dx[m][k] = g[m][n_rows] . dequant(W): what a training step takes back through a frozen projection.  Whole 64-row groups (the rows behind
+// the last one lie in another layout) and tiles of 128 columns
+bool gemm_tc_grad_supported(int qt, int64_t n_rows, int64_t k) { return gemm_tc_supported(qt, 128, k) && n_rows >= 64 && n_rows % 64 == 0 && k % 128 == 0; }
+size_t gemm_tc_grad_workspace_size(int64_t n_rows, int64_t k, int64_t m) {
+    using namespace gemmtc;
+    const int ks = most_splits((k / 128 + 1) / 2, n_rows / 64, m, k);
+    return ks > 1 ? (size_t)ks * m * k * sizeof(float) : 0;
+}
+int gemm_tc_grad_launch(const void* w, int qt, int64_t n_rows, int64_t k, const void* g, int dtype, int64_t m, void* dx, void* workspace,
+                        size_t workspace_bytes, cudaStream_t st) {
+    using namespace gemmtc;
+    qt = canon_qtype(qt);
+    if (!gemm_tc_grad_supported(qt, n_rows, k) || (dtype != DT_F16 && dtype != DT_BF16) || (((uintptr_t)g | (uintptr_t)w) & 15)) return LB_ERR_ARG;
+    const bool bf = dtype == DT_BF16;
+    CUtensorMap map;
+    if (const int rc = encode_rows(&map, g, bf, m, n_rows, 32)) return rc;
+    PairArgs A = {};
+    if (const int rc = make_waits(&A.waits, kWaitCycles)) return rc;
+    A.w = (const uint8_t*)w; A.G = make_geom(n_rows, k, qt); A.M = (int)m; A.y = dx; A.y_dtype = dtype;
+    A.n_fp = (int)((k / 128 + 1) / 2);
+    PairPlan p = pair_plan(pair_pace(qt, bf), A.n_fp, n_rows / 64, m, k, true);
+    if (p.ks > 1 && !holds_partials(workspace, workspace_bytes, (size_t)p.ks * m * k)) p = pair_plan(pair_pace(qt, bf), A.n_fp, n_rows / 64, m, k, false);
+    A.tt = p.tt; A.ksplit = p.ks; A.part = (float*)workspace;
+    if (const int rc = pair_launch<true>(qt, bf, map, A, (int64_t)A.n_fp * ((m + p.tt - 1) / p.tt) * p.ks, st)) return rc;
+    if (p.ks > 1) {
+        int rg = (int)((m * k / 4 + 255) / 256); if (rg > sm_count() * 8) rg = sm_count() * 8;
+        reduce_partials_kernel<<<rg, 256, 0, st>>>(A.part, p.ks, m * k, k, dx, dtype, nullptr, 0);
         note_launch();
     }
     return check_launch();
@@ -656,7 +704,7 @@ int gemm_tc_mlp_launch(const void* w_gate, const void* w_up, int act, int qt, in
     PairPlan p = pair_plan(pair_pace(qt, bf), A.n_fp, k / 64, m, 2 * n_rows, true);
     if (p.ks > 1 && !holds_partials(workspace, workspace_bytes, (size_t)p.ks * m * 2 * n_rows)) p = pair_plan(pair_pace(qt, bf), A.n_fp, k / 64, m, 2 * n_rows, false);
     A.tt = p.tt; A.ksplit = p.ks; A.part = (float*)workspace;
-    if (const int rc = pair_launch(qt, bf, map, A, (int64_t)A.n_fp * ((m + A.tt - 1) / A.tt) * p.ks, st)) return rc;
+    if (const int rc = pair_launch<>(qt, bf, map, A, (int64_t)A.n_fp * ((m + A.tt - 1) / A.tt) * p.ks, st)) return rc;
     if (p.ks > 1) {
         int rg = (int)((m * n_rows / 4 + 255) / 256); if (rg > sm_count() * 8) rg = sm_count() * 8;
         reduce_gated_kernel<<<rg, 256, 0, st>>>(A.part, p.ks, m, n_rows, y, y_dtype, act);
@@ -687,7 +735,7 @@ int gemm_tc_experts_launch(const unsigned long long* tab, const unsigned long lo
     A.G = make_geom(n_rows, k, qt); A.M = (int)rows; A.y = y; A.y_dtype = y_dtype; A.ksplit = 1; A.tt = kPairTok;
     A.n_fp = (int)((n_rows / (tab2 ? 64 : 128) + 1) / 2);
     const int64_t most = (rows < n_experts ? rows : n_experts) + rows / kPairTok;        // tiles: one per used expert and one per 256 rows
-    if (const int rc = pair_launch(qt, bf, map, A, most * A.n_fp, st)) return rc;
+    if (const int rc = pair_launch<>(qt, bf, map, A, most * A.n_fp, st)) return rc;
     return check_launch();
 }
 

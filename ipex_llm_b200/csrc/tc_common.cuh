@@ -337,6 +337,64 @@ template <bool BF> __device__ __forceinline__ uint32_t pack2(float a, float b) {
     return h2u(__floats2half2_rn(a, b));
 }
 
+// The same order of weights rounded ONCE to the activation type from their 32-bit value, the bits that dequantising (layout.cu) gives, for
+// the product with the transposed weights.  code x scale: the product of an fp16 code and an fp16 scale is rounded once as it is; to bf16
+// with the scale in two parts, d = hi + lo, exact, as the code times lo is (at most 4 + 3 bits): fma(code, hi, code * lo).  Minima and
+// table: in 32 bits.
+struct ScaleBf { __nv_bfloat162 hi, lo; };
+__device__ __forceinline__ ScaleBf split_scale(__half d) {
+    const float f = __half2float(d);
+    const __nv_bfloat16 hi = __float2bfloat16_rn(f);
+    ScaleBf s;
+    s.hi = __bfloat162bfloat162(hi);
+    s.lo = __bfloat162bfloat162(__float2bfloat16_rn(fabsf(f) <= 65504.0f ? f - __bfloat162float(hi) : 0.0f));      // none of an infinite scale
+    return s;
+}
+__device__ __forceinline__ uint32_t scaled_bf(uint32_t code, const ScaleBf& d) { return bf2u(__hfma2(u2bf(code), d.hi, __hmul2(u2bf(code), d.lo))); }
+// rows g (lo) and g + 8 (hi) of one 16 x 64 tile; registers 2 k4, 2 k4 + 1 of either row are k-step k4
+template <int QT, bool BF>
+__device__ __forceinline__ void expand_once(const typename Expand<QT>::Codes& c, uint32_t dq, uint32_t mq, uint32_t lut, uint32_t (&lo)[8], uint32_t (&hi)[8]) {
+    using E = Expand<QT>;
+    const __half2 d2 = u2h(dq), m2 = u2h(mq);
+    ScaleBf sl, sh;
+    if constexpr (BF && QT != QT_NF4 && QT != QT_ASYM_INT4) { sl = split_scale(__low2half(d2)); sh = split_scale(__high2half(d2)); }
+    const float f[2] = {__low2float(d2), __high2float(d2)}, b[2] = {__low2float(m2), __high2float(m2)};
+#pragma unroll
+    for (int k4 = 0; k4 < 4; k4++) {
+        uint32_t a[4];
+        if constexpr (QT == QT_NF4) {
+            const uint32_t w = k4 == 0 ? c.q.x : k4 == 1 ? c.q.y : k4 == 2 ? c.q.z : c.q.w;
+#pragma unroll
+            for (int i = 0; i < 4; i++) {
+                float x, y;
+                asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(x), "=f"(y) : "r"(lut + __byte_perm(w, 0u, 0x4440u + i) * 128u));
+                a[i] = pack2<BF>(x * f[i & 1], y * f[i & 1]);
+            }
+        } else if constexpr (QT == QT_ASYM_INT4 && BF) {
+            const __half2 one = __floats2half2_rn(1.0f, 1.0f), zero = __floats2half2_rn(0.0f, 0.0f);
+            E::run(c, k4, one, one, zero, zero, 0u, a);              // the codes
+#pragma unroll
+            for (int i = 0; i < 4; i++) { const float2 n = __half22float2(u2h(a[i])); a[i] = pack2<BF>(fmaf(n.x, f[i & 1], b[i & 1]), fmaf(n.y, f[i & 1], b[i & 1])); }
+        } else if constexpr (BF) {
+            E::bf16(c, k4, a);
+#pragma unroll
+            for (int i = 0; i < 4; i++) a[i] = scaled_bf(a[i], i & 1 ? sh : sl);
+        } else {
+            E::run(c, k4, __low2half2(d2), __high2half2(d2), __low2half2(m2), __high2half2(m2), lut, a);
+        }
+        lo[2 * k4] = a[0]; lo[2 * k4 + 1] = a[2]; hi[2 * k4] = a[1]; hi[2 * k4 + 1] = a[3];
+    }
+}
+// nf4's table for it: entry b = the two 32-bit values of code byte b, in 16 slots (a 64-bit load is served half a warp at a time)
+__device__ __forceinline__ void fill_nf4_pairs(uint8_t* lut, int tid, int nthreads) {
+    for (int e = tid; e < 256; e += nthreads) {
+        const float4 v = make_float4(kNF4Table[e & 15], kNF4Table[e >> 4], kNF4Table[e & 15], kNF4Table[e >> 4]);
+        float4* dst = reinterpret_cast<float4*>(lut + e * 128);
+#pragma unroll
+        for (int c = 0; c < 8; c++) dst[c] = v;
+    }
+}
+
 // bytes of one 64-row group x one k-block as the kernels stage it: codes, fp16 scales [, minima]
 template <int QT> struct PackedBlock {
     static constexpr int kSuper = RG_TILES * Expand<QT>::kTileBytes;
@@ -367,9 +425,16 @@ static int encode_rows(CUtensorMap* map, const void* x, bool bf, int64_t rows, i
     const cuuint64_t gstride[1] = {(cuuint64_t)k * 2};
     const cuuint32_t box[2] = {64, (cuuint32_t)box_rows};
     const cuuint32_t estr[2] = {1, 1};
-    const CUresult r = enc(map, bf ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(x), gdim,
+    auto encode = [&] { return enc(map, bf ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(x), gdim,
                            gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                           CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                           CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE); };
+    CUresult r = encode();
+    if (r == CUDA_ERROR_INVALID_CONTEXT) {                // a thread (autograd's, say) before its first runtime call: bind its device's context
+        int dev = 0;
+        cudaGetDevice(&dev);
+        cudaSetDevice(dev);
+        r = encode();
+    }
     if (r != CUDA_SUCCESS) { set_error(LB_ERR_CUDA, "cuTensorMapEncodeTiled failed (%d)", (int)r); return LB_ERR_CUDA; }
     return LB_OK;
 }

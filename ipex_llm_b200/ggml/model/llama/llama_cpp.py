@@ -197,6 +197,27 @@ def lowbit_matmul_cuda(d_w, qtype, n_rows, k, d_x, x_dtype, m, d_y, y_dtype, d_b
            "lowbit_matmul_cuda")
 
 
+_lib.lowbit_matmul_grad_supported.argtypes = [ctypes.c_int, ctypes.c_int64, ctypes.c_int64]
+_lib.lowbit_matmul_grad_supported.restype = ctypes.c_int
+_lib.lowbit_matmul_grad_workspace_size.argtypes = [ctypes.c_int64] * 3
+_lib.lowbit_matmul_grad_workspace_size.restype = ctypes.c_size_t
+_lib.lowbit_matmul_grad_cuda.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_int64, ctypes.c_int64, ctypes.c_void_p, ctypes.c_int, ctypes.c_int64,
+                                         ctypes.c_void_p, ctypes.c_void_p, ctypes.c_size_t, ctypes.c_void_p]
+_lib.lowbit_matmul_grad_cuda.restype = ctypes.c_int
+
+
+def lowbit_matmul_grad_supported(qtype, n_rows, k):
+    return bool(_lib.lowbit_matmul_grad_supported(qtype, n_rows, k))
+
+
+def lowbit_matmul_grad_workspace_size(n_rows, k, m):
+    return _lib.lowbit_matmul_grad_workspace_size(n_rows, k, m)
+
+
+def lowbit_matmul_grad_cuda(d_w, qtype, n_rows, k, d_grad, dtype, m, d_out, workspace, workspace_bytes, stream):
+    _check(_lib.lowbit_matmul_grad_cuda(d_w, qtype, n_rows, k, d_grad, dtype, m, d_out, workspace, workspace_bytes, stream), "lowbit_matmul_grad_cuda")
+
+
 _lib.lowbit_dequantize_rows_cuda.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_int64, ctypes.c_int64, ctypes.c_void_p,
                                              ctypes.c_int, ctypes.c_int64, ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p]
 _lib.lowbit_dequantize_rows_cuda.restype = ctypes.c_int

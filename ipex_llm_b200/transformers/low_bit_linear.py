@@ -494,10 +494,48 @@ def ggml_matmul_src1_x_src0_t(src0: torch.Tensor, src1: torch.Tensor, src0_shape
     return result_t
 
 
+@functools.lru_cache(maxsize=4096)
+def _grad_plan(qtype, N, K, M):
+    """bytes of scratch for the gradient's product; None: the shape is not the kernel's.  Looking nf4's table up takes longer than the MMAs of
+    a tile, so that with many rows the dequantised matrix wins (forward and backward, 1024 rows, 11008 x 4096: 158 against 167 us; 2000
+    rows, 2048 x 8192: 135 against 127)"""
+    if qtype == NF4 and M > 1280:
+        return None
+    return ggml.lowbit_matmul_grad_workspace_size(N, K, M) if ggml.lowbit_matmul_grad_supported(qtype, N, K) else None
+
+
+def _plain_gradient(grad, weight, shape, qtype):
+    """whether one launch can form grad @ dequant(weight): a half-precision tensor with storage on the weight's device, nothing recorded for
+    another derivative, a shape that the kernel takes"""
+    return (type(grad) is torch.Tensor and grad.dtype in (torch.float16, torch.bfloat16) and grad.device == weight.device and weight.is_cuda
+            and grad.numel() > 0 and not (torch.is_grad_enabled() and grad.requires_grad) and torch._C._has_storage(grad)
+            and weight.is_contiguous() and weight.data_ptr() % 16 == 0 and _grad_plan(qtype, *shape, grad.numel() // shape[0]) is not None)
+
+
+def lowbit_matmul_grad(grad_2d, weight, weight_shape, qtype):
+    """grad [M, N] (fp16 / bf16) @ dequant(W [N, K], tiled device layout) -> [M, K]"""
+    N, K = weight_shape
+    if not grad_2d.is_contiguous():
+        grad_2d = grad_2d.contiguous()
+    elif grad_2d.data_ptr() % 16:
+        grad_2d = grad_2d.clone()
+    M, dev = grad_2d.shape[0], grad_2d.device
+    need = _grad_plan(qtype, N, K, M)
+    invalidInputError(need is not None, f"unsupported gradient shape ({N}, {K})")
+    out = torch.empty((M, K), dtype=grad_2d.dtype, device=dev)
+    ws = _scratch(dev, need, out)
+    w = weight.view(torch.uint8) if weight.dtype != torch.uint8 else weight
+    with _on_device(dev):
+        ggml.lowbit_matmul_grad_cuda(w.data_ptr(), qtype, N, K, grad_2d.data_ptr(), _TORCH_TO_DT[grad_2d.dtype], M, out.data_ptr(), ws.data_ptr(), need,
+                                     _raw_stream(dev))
+    return out
+
+
 class MatMulLowBit(torch.autograd.Function):
     """LBL:532-577, the autograd wrapper of the device matmul (QLoRA-style training freezes the packed
     weight: only the activation gets a gradient).  forward = the dequant-GEMV / GEMM kernels,
-    backward = grad_output @ dequant(W) with W dequantised by the tiled-layout kernel."""
+    backward = grad_output @ dequant(W) in one launch, or, where that does not serve (32-bit gradients, a derivative of
+    the gradient, batched gradients, other shapes), with W dequantised by the tiled-layout kernel."""
 
     @staticmethod
     def forward(ctx, A, weight, output_size):
@@ -513,8 +551,12 @@ class MatMulLowBit(torch.autograd.Function):
         A, weight = ctx.tensors
         grad_A = None
         if ctx.needs_input_grad[0]:
-            dequant_weight = dequantize_device_layout(weight.data, tuple(weight._shape), weight.qtype, dtype=grad_output.dtype)
-            grad_A = torch.matmul(grad_output, dequant_weight)
+            shape = tuple(weight._shape)
+            if _plain_gradient(grad_output, weight.data, shape, weight.qtype):
+                grad_A = lowbit_matmul_grad(grad_output.reshape(-1, shape[0]), weight.data, shape, weight.qtype).view(grad_output.shape[:-1] + (shape[1],))
+            else:
+                dequant_weight = dequantize_device_layout(weight.data, shape, weight.qtype, dtype=grad_output.dtype)
+                grad_A = torch.matmul(grad_output, dequant_weight)
         return grad_A, None, None
 
 
