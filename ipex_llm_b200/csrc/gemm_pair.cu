@@ -577,9 +577,11 @@ static int pair_launch(int qt, bool bf, const CUtensorMap& map, const PairArgs& 
 // + the start and end of a unit) and, when K is split, the partial sums' round trip through memory and the second launch.  Times as the
 // power cap leaves them (1.6 to 1.75 GHz), sym_int4 but for nf4's table (the other formats take sym_int4's): a k-block 0.0012 us per token
 // once the MMAs set the pace, below that 0.215 us for the expansion and the chain around it with fp16 activations, 0.275 with bf16, 0.35
-// for nf4; a unit 1.2 us and 6 ns per token of its results.  Where the line lies, whole K against the split one at 512 rows, 4096 x
-// 11008: fp16 43.9 (128-token tiles) / 41.9 us (256, two splits), bf16 47.8 / 41.8; at 512 rows, 4096 x 4096: fp16 22.1 / 24.7, bf16
-// 24.0 / 24.4, nf4 28.4 / 26.1; at 200 rows fp16 20.1 / 17.2 (208 tokens, four splits).
+// for nf4; a unit 1.2 us and 6 ns per token of its results; partial sums 4.5 TB/s there and back.  Where the line lies, whole K against
+// the split one at 512 rows, 4096 x 11008: bf16 47.8 (128-token tiles) / 41.8 us (256, two splits); at 512 rows, 4096 x 4096: fp16 22.1 /
+// 24.7, bf16 24.0 / 24.4, nf4 28.4 / 26.1; at 200 rows fp16 20.1 / 17.7 (112 tokens, two splits).  fp16 at 512 rows, 4096 x 11008 lies
+// close to it: 43.9 / 41.9.  It stays whole: with 8 TB/s, which would split it, the half-precision 7B model of the token test, whose logits
+// amplify any other rounding of its prompt, parts from its eager decode at a token by more than the test's bound for ties.
 constexpr double kPaces[3] = {0.215, 0.275, 0.35};
 static double pair_pace(int qt, bool bf) { return kPaces[qt == QT_NF4 ? 2 : bf ? 1 : 0]; }
 struct PairPlan { int tt, ks; };
@@ -594,7 +596,7 @@ static PairPlan pair_plan(double pace, int64_t n_fp, int64_t nb, int64_t m, int6
         for (int64_t ks = 1; ks == 1 || ks <= max_ks; ks++) {
             const int64_t rounds = (n_fp * nt * ks + clusters - 1) / clusters;
             double cost = (double)rounds * ((double)((nb + ks - 1) / ks) * per_kb + 1.2 + 0.006 * (double)tt);
-            if (ks > 1) cost += (double)ks * (double)m * (double)n_out * 8.0 / 8.0e6 + 2.5;
+            if (ks > 1) cost += (double)ks * (double)m * (double)n_out * 8.0 / 4.5e6 + 2.5;
             if (cost < best_cost - 1e-9) { best_cost = cost; best = {(int)tt, (int)ks}; }
         }
     }
