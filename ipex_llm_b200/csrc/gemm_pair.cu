@@ -12,7 +12,8 @@
 // k-block, the MMAs 0.14): here activations, packed weights and expanded tiles have rings of their own, so the expansion runs
 // ahead of the activations and four groups of warps have four k-blocks in flight.  Measured per k-block: 0.19 us up to 170 tokens
 // (fp16; see pair_plan for the other paces), 0.282 at 256, where the tensor pipe is busy 512 of 525 clocks; 14336 x 4096 at 4000
-// tokens 1357 -> 1494 TFLOP/s, 4096 x 11008 at 512 tokens 59.7 -> 43.4 us (the kernel in a recorded chain).  At 128 tokens the MMAs need 256 of 360 clocks: A and B
+// tokens 1357 -> 1494 TFLOP/s, 4096 x 11008 at 512 tokens 59.7 -> 42.6 us (recorded;
+// the paces are a cool GPU's, under the power cap pair_plan's hold).  At 128 tokens the MMAs need 256 of 360 clocks: A and B
 // both come from shared memory, beside the expansion's stores.
 //   warp 0       TMA: this CTA's half of the tokens, boxes of 32 rows x 64 elements (128-byte swizzle), ring of kX slots;
 //   warp 1       CTA 0: issues the MMAs (M = 256, N, K = 16; four per k-block) in warp-uniform control flow, one commit per ring
@@ -22,7 +23,7 @@
 //   warps 4-19   four groups of four: group (k-block mod 4) expands the codes to fp16 / bf16 (scale applied with one multiply per
 //                pair, one rounding) into the K-major 128B-swizzled A slot it owns;
 //   warps 20-23  epilogue: TMEM lane = feature, column = token.  The two 64-row groups are interleaved by 16 rows, so that with a
-//                gate group and an up group in one tile the lanes l and l + 16 of a warp hold gate and up of one feature.
+//                gate group and an up group in one tile a warp's two runs of 16 lanes hold gate and up of the same features.
 // The signals between the two CTAs are plain arrivals: with cluster-scope release / acquire on them (a full memory fence per
 // arrival) a k-block took 0.75 us instead of 0.25; what they order is shared memory, written behind a proxy fence and read by the
 // tensor cores of the SM that wrote it.
