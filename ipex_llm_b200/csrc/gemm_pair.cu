@@ -13,7 +13,7 @@
 // ahead of the activations and four groups of warps have four k-blocks in flight.  Measured per k-block: 0.19 us up to 170 tokens
 // (fp16; see pair_plan for the other paces), 0.282 at 256, where the tensor pipe is busy 512 of 525 clocks; 14336 x 4096 at 4000
 // tokens 1357 -> 1494 TFLOP/s, 4096 x 11008 at 512 tokens 59.7 -> 42.6 us (recorded;
-// the paces are a cool GPU's, under the power cap pair_plan's hold).  At 128 tokens the MMAs need 256 of 360 clocks: A and B
+// the paces are a cool GPU's).  At 128 tokens the MMAs need 256 of 360 clocks: A and B
 // both come from shared memory, beside the expansion's stores.
 //   warp 0       TMA: this CTA's half of the tokens, boxes of 32 rows x 64 elements (128-byte swizzle), ring of kX slots;
 //   warp 1       CTA 0: issues the MMAs (M = 256, N, K = 16; four per k-block) in warp-uniform control flow, one commit per ring
@@ -574,16 +574,18 @@ static int pair_launch(int qt, bool bf, const CUtensorMap& map, const PairArgs& 
     return LB_ERR_ARG;
 }
 
-// Token tile and K splits of a matmul: the pair that minimises rounds of the resident clusters x (k-blocks per unit x time per k-block
-// + the start and end of a unit) and, when K is split, the partial sums' round trip through memory and the second launch.  Times as the
-// power cap leaves them (1.6 to 1.75 GHz), sym_int4 but for nf4's table (the other formats take sym_int4's): a k-block 0.0012 us per token
-// once the MMAs set the pace, below that 0.215 us for the expansion and the chain around it with fp16 activations, 0.275 with bf16, 0.35
-// for nf4; a unit 1.2 us and 6 ns per token of its results; partial sums 4.5 TB/s there and back.  Where the line lies, whole K against
-// the split one at 512 rows, 4096 x 11008: bf16 47.8 (128-token tiles) / 41.8 us (256, two splits); at 512 rows, 4096 x 4096: fp16 22.1 /
-// 24.7, bf16 24.0 / 24.4, nf4 28.4 / 26.1; at 200 rows fp16 20.1 / 17.7 (112 tokens, two splits).  fp16 at 512 rows, 4096 x 11008 lies
-// close to it: 43.9 / 41.9.  It stays whole: with 8 TB/s, which would split it, the half-precision 7B model of the token test, whose logits
-// amplify any other rounding of its prompt, parts from its eager decode at a token by more than the test's bound for ties.
-constexpr double kPaces[3] = {0.215, 0.275, 0.35};
+// Token tile and K splits of a matmul: the pair that minimises rounds of the resident clusters x k-blocks per unit x time per
+// k-block + the start and end of a unit and, when K is split, the partial sums' round trip through memory at ~4 TB/s and the second
+// launch.  Time per k-block on a cool GPU, measured at 4096 x 11008 and 4096 x 4096: 0.0011 us per token once the MMAs set the pace
+// (0.282 at 256), below that the expansion and the chain around it: 0.19 us for sym_int4 with fp16 activations, 0.24 with bf16, 0.29 for
+// nf4's table; the other formats were not measured and take sym_int4's figures.  Both sides of the line under the power cap, 128-token
+// tiles of the whole K against 256-token tiles of two splits, 4096 x 11008: 512 rows sym_int4 fp16 48.5 / 48.1 us, bf16 52.1 / 41.7, nf4
+// 64.1 / 42.8, 500 rows fp16 49.4 / 41.0.  Over 357 shapes and formats (65 to 1500 rows, 1024 to 11008 features, K 2048 to 14336) the 332
+// choices that were timed lie 1.6 % over the best tile and split, 12 of them more than 10 %, most of these because partial sums that stay
+// in L2 cost less than is charged here (a fit over all times: 27 TB/s and 3.5 us).  Charging less moves which prompts are split, and so the
+// order of their 32-bit sums: with 4.5 TB/s and slower k-blocks the choices were 1.1 % over the best, and the logits of a decode step
+// behind some prompts moved by 7e-3 (the e5m2 cache takes a low bit a long way).  That was taken back: 0.5 % do not pay for other results.
+constexpr double kPaces[3] = {0.19, 0.24, 0.29};
 static double pair_pace(int qt, bool bf) { return kPaces[qt == QT_NF4 ? 2 : bf ? 1 : 0]; }
 struct PairPlan { int tt, ks; };
 static PairPlan pair_plan(double pace, int64_t n_fp, int64_t nb, int64_t m, int64_t n_out, bool may_split) {
@@ -592,12 +594,12 @@ static PairPlan pair_plan(double pace, int64_t n_fp, int64_t nb, int64_t m, int6
     double best_cost = 1e30;
     for (int64_t nt = nt0; nt <= nt0 + 8 && nt <= (m + 31) / 32; nt++) {
         const int64_t tt = ((m + nt - 1) / nt + 15) & ~int64_t(15);
-        const double mma = 0.0012 * (double)tt, per_kb = mma > pace ? mma : pace;
+        const double mma = 0.0011 * (double)tt, per_kb = mma > pace ? mma : pace;
         const int64_t max_ks = may_split ? (nb / 8 < 8 ? nb / 8 : 8) : 1;
         for (int64_t ks = 1; ks == 1 || ks <= max_ks; ks++) {
             const int64_t rounds = (n_fp * nt * ks + clusters - 1) / clusters;
-            double cost = (double)rounds * ((double)((nb + ks - 1) / ks) * per_kb + 1.2 + 0.006 * (double)tt);
-            if (ks > 1) cost += (double)ks * (double)m * (double)n_out * 8.0 / 4.5e6 + 2.5;
+            double cost = (double)rounds * ((double)((nb + ks - 1) / ks) * per_kb + 1.0);
+            if (ks > 1) cost += (double)ks * (double)m * (double)n_out * 8.0 / 4.0e6 + 3.0;
             if (cost < best_cost - 1e-9) { best_cost = cost; best = {(int)tt, (int)ks}; }
         }
     }

@@ -187,6 +187,22 @@ def test_prompt_matmul_fp32_tiles(lbl, native_lib, cuda_device, qtype, m, n, k):
     test_prompt_matmul_fp32_keeps_its_contract(lbl, native_lib, cuda_device, qtype, m, n, k)
 
 
+@pytest.mark.parametrize("qtype,dtype,m,n,k", [("sym_int4", torch.float16, 200, 4096, 4096), ("sym_int4", torch.float16, 500, 4096, 11008),
+                                               ("sym_int4", torch.float16, 512, 4096, 11008), ("fp8_e4m3", torch.float16, 256, 4096, 4096),
+                                               ("sym_int4", torch.bfloat16, 1500, 1024, 4096), ("nf4", torch.bfloat16, 512, 4096, 4096)])
+def test_prompts_whose_k_range_stays_whole(lbl, native_lib, cuda_device, qtype, dtype, m, n, k):
+    """a split is another order of the sums, which decode steps behind a prompt show: the same bits with and without room for partial sums"""
+    p = lbl.FP4Params(torch.randn(n, k, device=cuda_device, generator=torch.Generator(device=cuda_device).manual_seed(k)) * 0.02,
+                      qtype=lbl.ggml_tensor_qtype[qtype]).to(cuda_device)
+    x = torch.randn(m, k, device=cuda_device, generator=torch.Generator(device=cuda_device).manual_seed(m)).to(dtype)
+    room, dt = torch.empty(8 * m * n * 4, dtype=torch.uint8, device=cuda_device), lbl._TORCH_TO_DT[dtype]
+    y = [torch.empty(m, n, dtype=dtype, device=cuda_device) for _ in range(2)]
+    for out, size in zip(y, (room.numel(), 0)):
+        native_lib.lowbit_matmul_cuda(p.data.data_ptr(), p.qtype, n, k, x.data_ptr(), dt, m, out.data_ptr(), dt, None, 0, room.data_ptr(), size,
+                                      torch.cuda.current_stream().cuda_stream)
+    assert torch.equal(*y)
+
+
 @pytest.mark.parametrize("offset", [4, 8])
 def test_scratch_off_a_16_byte_boundary(lbl, native_lib, cuda_device, offset):
     """shapes that would split K run it whole, within the same bounds; 32-bit activations, whose planes lie there, are refused"""
