@@ -505,10 +505,12 @@ def _grad_plan(qtype, N, K, M):
 
 
 def _plain_gradient(grad, weight, shape, qtype):
-    """whether one launch can form grad @ dequant(weight): a half-precision tensor with storage on the weight's device, nothing recorded for
-    another derivative, a shape that the kernel takes"""
+    """whether one launch can form grad @ dequant(weight): a half-precision tensor whose storage holds its values, on the weight's device,
+    nothing recorded for another derivative (backward or forward), no autocast to another type, a shape that the kernel takes"""
     return (type(grad) is torch.Tensor and grad.dtype in (torch.float16, torch.bfloat16) and grad.device == weight.device and weight.is_cuda
             and grad.numel() > 0 and not (torch.is_grad_enabled() and grad.requires_grad) and torch._C._has_storage(grad)
+            and not grad.is_neg() and not grad._is_zerotensor() and torch.autograd.forward_ad.unpack_dual(grad).tangent is None
+            and (not torch.is_autocast_enabled("cuda") or torch.get_autocast_dtype("cuda") == grad.dtype)
             and weight.is_contiguous() and weight.data_ptr() % 16 == 0 and _grad_plan(qtype, *shape, grad.numel() // shape[0]) is not None)
 
 

@@ -3,6 +3,7 @@ import threading
 
 import pytest
 import torch
+import torch.autograd.forward_ad as fw
 
 pytestmark = pytest.mark.gpu
 QTYPES = ["sym_int4", "asym_int4", "nf4", "fp8_e4m3", "fp8_e5m2", "fp6"]
@@ -57,8 +58,8 @@ def test_gradient_edges(lbl, native_lib, cuda_device, qtype, dtype, m, n, k):
 
 
 def test_backward_takes_it_or_the_general_path(lbl, cuda_device, monkeypatch):
-    """expanded and 3-dimensional half gradients in one launch; 32-bit ones, a derivative of the gradient, batched ones and other shapes by
-    dequantising, with the same values"""
+    """expanded and 3-dimensional half gradients in one launch; 32-bit ones, a derivative of the gradient in either direction, batched, negated
+    and zero ones, those under an autocast to another type and other shapes by dequantising, with the same values"""
     calls = []
     real = lbl.lowbit_matmul_grad
     monkeypatch.setattr(lbl, "lowbit_matmul_grad", lambda *a: calls.append(1) or real(*a))
@@ -80,6 +81,23 @@ def test_backward_takes_it_or_the_general_path(lbl, cuda_device, monkeypatch):
     assert not calls and torch.allclose(gg.double(), wd[torch.float16].sum(1).expand_as(gg), rtol=2e-3, atol=2e-3)
     (batched,) = torch.autograd.grad(y, x, torch.stack([g.detach(), 2 * g.detach()]), is_grads_batched=True)
     assert not calls and torch.allclose(batched[0].double(), g.detach().double() @ wd[torch.float16], rtol=2e-3, atol=2e-3)
+    tangent = torch.randn(5, 256, device=cuda_device).half()
+    with fw.dual_level():                                               # a tangent of the gradient is carried on
+        (gd,) = torch.autograd.grad(y, x, fw.make_dual(g.detach(), tangent), retain_graph=True)
+        primal, moved = fw.unpack_dual(gd)
+        assert not calls and moved is not None
+        assert torch.allclose(primal.double(), g.detach().double() @ wd[torch.float16], rtol=2e-3, atol=2e-3)
+        assert torch.allclose(moved.double(), tangent.double() @ wd[torch.float16], rtol=2e-3, atol=2e-3)
+    for lazy, want in ((torch._neg_view(g.detach()), -g.detach().double()),       # the sign and the zeros are not in memory
+                       (torch._efficientzerotensor((5, 256), dtype=torch.float16, device=cuda_device), torch.zeros(5, 256, device=cuda_device).double())):
+        (gl,) = torch.autograd.grad(y, x, lazy, retain_graph=True)
+        assert not calls and torch.allclose(gl.double(), want @ wd[torch.float16], rtol=2e-3, atol=2e-3)
+    with torch.autocast("cuda", dtype=torch.bfloat16):                  # the product in bf16, as autocast has matmul do it
+        (ga,) = torch.autograd.grad(y, x, g.detach(), retain_graph=True)
+        assert not calls and torch.equal(ga, torch.matmul(g.detach(), wd[torch.float16].half()).half())
+    (gp,) = torch.autograd.grad(y, x, g.detach(), retain_graph=True)    # ... and a plain one is the kernel's again
+    assert len(calls) == 1 and torch.allclose(gp.double(), g.detach().double() @ wd[torch.float16], rtol=2e-3, atol=2e-3)
+    calls.clear()
     q = weight(lbl, cuda_device, 100, 192, "sym_int4")                  # rows behind the last 64, columns no multiple of 128
     x = torch.randn(70, 192, device=cuda_device).half().requires_grad_(True)
     lbl.MatMulLowBit.apply(x, q, 100).sum().backward()
