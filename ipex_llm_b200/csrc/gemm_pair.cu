@@ -574,36 +574,45 @@ static int pair_launch(int qt, bool bf, const CUtensorMap& map, const PairArgs& 
     return LB_ERR_ARG;
 }
 
-// Token tile and K splits of a matmul: the pair that minimises rounds of the resident clusters x k-blocks per unit x time per
-// k-block + the start and end of a unit and, when K is split, the partial sums' round trip through memory at ~4 TB/s and the second
-// launch.  Time per k-block on a cool GPU, measured at 4096 x 11008 and 4096 x 4096: 0.0011 us per token once the MMAs set the pace
-// (0.282 at 256), below that the expansion and the chain around it: 0.19 us for sym_int4 with fp16 activations, 0.24 with bf16, 0.29 for
-// nf4's table; the other formats were not measured and take sym_int4's figures.  Both sides of the line under the power cap, 128-token
-// tiles of the whole K against 256-token tiles of two splits, 4096 x 11008: 512 rows sym_int4 fp16 48.5 / 48.1 us, bf16 52.1 / 41.7, nf4
-// 64.1 / 42.8, 500 rows fp16 49.4 / 41.0.  Over 357 shapes and formats (65 to 1500 rows, 1024 to 11008 features, K 2048 to 14336) the 332
-// choices that were timed lie 1.6 % over the best tile and split, 12 of them more than 10 %, most of these because partial sums that stay
-// in L2 cost less than is charged here (a fit over all times: 27 TB/s and 3.5 us).  Charging less moves which prompts are split, and so the
-// order of their 32-bit sums: with 4.5 TB/s and slower k-blocks the choices were 1.1 % over the best, and the logits of a decode step
-// behind some prompts moved by 7e-3 (the e5m2 cache takes a low bit a long way).  That was taken back: 0.5 % do not pay for other results.
-constexpr double kPaces[3] = {0.19, 0.24, 0.29};
-static double pair_pace(int qt, bool bf) { return kPaces[qt == QT_NF4 ? 2 : bf ? 1 : 0]; }
+// Token tile and K splits of a matmul, each the one that minimises rounds of the resident clusters x (k-blocks per unit x time per k-block
+// + the start and end of a unit) and, when K is split, the partial sums' round trip through memory and the second launch.  A k-block takes
+// a time per token once the MMAs set the pace, below that the expansion and the chain around it; sym_int4 with fp16 activations, with
+// bf16, and nf4's table were measured, the other formats take sym_int4's figures.
+//
+// The tile changes no bit of a result.  It goes by the times under the power cap (1.6 to 1.75 GHz): 4000 rows, 4096 x 14336, with the tile
+// of the split's figures / with this one: fp8_e5m2 fp16 424 (176 tokens) / 369 us (224), fp8_e4m3 412 / 386, nf4 bf16 410 (256) / 378
+// (224), sym_int4 fp16 323 / 329.
+//
+// The split is the order of a result's 32-bit sums.  It goes by a cool GPU's times (4096 x 11008 and 4096 x 4096; partial sums at ~4 TB/s).
+// Both sides of its line under the power cap, 128-token tiles of the whole K against 256-token tiles of two splits, 4096 x 11008: 512 rows
+// sym_int4 fp16 48.5 / 48.1 us, bf16 52.1 / 41.7, nf4 64.1 / 42.8, 500 rows fp16 49.4 / 41.0.  Over 332 shapes and formats (65 to 1500
+// rows, 1024 to 11008 features, K 2048 to 14336) the choices lie 1.6 % over the best tile and split, 12 of them more than 10 %, most of
+// these because partial sums that stay in L2 cost less than is charged here (a fit over all times: 27 TB/s and 3.5 us).  Charging less moves
+// which prompts are split: with the tile's figures and 4.5 TB/s the choices were 1.1 % over the best, and the logits of a decode step behind
+// some prompts moved by 7e-3 (the e5m2 cache takes a low bit a long way).  0.5 % do not pay for other results.
+struct PairTimes { double token, pace[3], unit, unit_token; };       // us: a k-block per token, at least (fp16, bf16, nf4); a unit, per token
+constexpr PairTimes kSplitTimes = {0.0011, {0.19, 0.24, 0.29}, 1.0, 0.0}, kTileTimes = {0.0012, {0.215, 0.275, 0.35}, 1.2, 0.006};
+static int pair_kind(int qt, bool bf) { return qt == QT_NF4 ? 2 : bf ? 1 : 0; }
 struct PairPlan { int tt, ks; };
-static PairPlan pair_plan(double pace, int64_t n_fp, int64_t nb, int64_t m, int64_t n_out, bool may_split) {
+static PairPlan pair_plan(int kind, int64_t n_fp, int64_t nb, int64_t m, int64_t n_out, bool may_split) {
     const int64_t clusters = sm_count() / 2, nt0 = (m + kPairTok - 1) / kPairTok;
-    PairPlan best = {256, 1};
-    double best_cost = 1e30;
-    for (int64_t nt = nt0; nt <= nt0 + 8 && nt <= (m + 31) / 32; nt++) {
-        const int64_t tt = ((m + nt - 1) / nt + 15) & ~int64_t(15);
-        const double mma = 0.0011 * (double)tt, per_kb = mma > pace ? mma : pace;
-        const int64_t max_ks = may_split ? (nb / 8 < 8 ? nb / 8 : 8) : 1;
-        for (int64_t ks = 1; ks == 1 || ks <= max_ks; ks++) {
-            const int64_t rounds = (n_fp * nt * ks + clusters - 1) / clusters;
-            double cost = (double)rounds * ((double)((nb + ks - 1) / ks) * per_kb + 1.0);
-            if (ks > 1) cost += (double)ks * (double)m * (double)n_out * 8.0 / 4.0e6 + 3.0;
-            if (cost < best_cost - 1e-9) { best_cost = cost; best = {(int)tt, (int)ks}; }
+    auto best_of = [&](const PairTimes& T, int64_t ks0, int64_t ks1) {
+        PairPlan best = {256, (int)ks0};
+        double best_cost = 1e30;
+        for (int64_t nt = nt0; nt <= nt0 + 8 && nt <= (m + 31) / 32; nt++) {
+            const int64_t tt = ((m + nt - 1) / nt + 15) & ~int64_t(15);
+            const double mma = T.token * (double)tt, per_kb = mma > T.pace[kind] ? mma : T.pace[kind];
+            for (int64_t ks = ks0; ks <= ks1; ks++) {
+                const int64_t rounds = (n_fp * nt * ks + clusters - 1) / clusters;
+                double cost = (double)rounds * ((double)((nb + ks - 1) / ks) * per_kb + T.unit + T.unit_token * (double)tt);
+                if (ks > 1) cost += (double)ks * (double)m * (double)n_out * 8.0 / 4.0e6 + 3.0;
+                if (cost < best_cost - 1e-9) { best_cost = cost; best = {(int)tt, (int)ks}; }
+            }
         }
-    }
-    return best;
+        return best;
+    };
+    const int64_t most = may_split && nb >= 16 ? (nb / 8 < 8 ? nb / 8 : 8) : 1, ks = best_of(kSplitTimes, 1, most).ks;
+    return best_of(kTileTimes, ks, ks);
 }
 static bool holds_partials(const void* workspace, size_t bytes, size_t count) {
     return workspace && ((uintptr_t)workspace & 15) == 0 && bytes >= count * sizeof(float);
@@ -611,8 +620,8 @@ static bool holds_partials(const void* workspace, size_t bytes, size_t count) {
 // splits that a workspace has to hold, whatever the format and type
 static int most_splits(int64_t n_fp, int64_t nb, int64_t m, int64_t n_out) {
     int ks = 1;
-    for (const double pace : kPaces) {
-        const PairPlan p = pair_plan(pace, n_fp, nb, m, n_out, true);
+    for (int kind = 0; kind < 3; kind++) {
+        const PairPlan p = pair_plan(kind, n_fp, nb, m, n_out, true);
         if (p.ks > ks) ks = p.ks;
     }
     return ks;
@@ -644,9 +653,9 @@ int gemm_tc_launch(const void* w, int qt, int64_t n_rows, int64_t k, const void*
     if (const int rc = make_waits(&A.waits, kWaitCycles)) return rc;
     A.w = (const uint8_t*)w; A.G = make_geom(n_rows, k, qt); A.M = (int)m; A.y = y; A.y_dtype = y_dtype; A.bias = bias; A.accumulate = accumulate;
     A.n_fp = (int)((n_rows / 128 + 1) / 2);
-    PairPlan p = pair_plan(pair_pace(qt, bf), A.n_fp, k / 64, m, n_rows, true);
+    PairPlan p = pair_plan(pair_kind(qt, bf), A.n_fp, k / 64, m, n_rows, true);
     // a caller's workspace without room for partial sums, or not aligned for their 16-byte loads: the whole K range per unit
-    if (p.ks > 1 && !holds_partials(workspace, workspace_bytes, (size_t)p.ks * m * n_rows)) p = pair_plan(pair_pace(qt, bf), A.n_fp, k / 64, m, n_rows, false);
+    if (p.ks > 1 && !holds_partials(workspace, workspace_bytes, (size_t)p.ks * m * n_rows)) p = pair_plan(pair_kind(qt, bf), A.n_fp, k / 64, m, n_rows, false);
     A.tt = p.tt; A.ksplit = p.ks; A.part = (float*)workspace;
     const int64_t units = (int64_t)A.n_fp * ((m + p.tt - 1) / p.tt) * p.ks;
     if (const int rc = pair_launch<>(qt, bf, map, A, units, st)) return rc;
@@ -679,8 +688,8 @@ int gemm_tc_grad_launch(const void* w, int qt, int64_t n_rows, int64_t k, const 
     if (const int rc = make_waits(&A.waits, kWaitCycles)) return rc;
     A.w = (const uint8_t*)w; A.G = make_geom(n_rows, k, qt); A.M = (int)m; A.y = dx; A.y_dtype = dtype;
     A.n_fp = (int)((k / 128 + 1) / 2);
-    PairPlan p = pair_plan(pair_pace(qt, bf), A.n_fp, n_rows / 64, m, k, true);
-    if (p.ks > 1 && !holds_partials(workspace, workspace_bytes, (size_t)p.ks * m * k)) p = pair_plan(pair_pace(qt, bf), A.n_fp, n_rows / 64, m, k, false);
+    PairPlan p = pair_plan(pair_kind(qt, bf), A.n_fp, n_rows / 64, m, k, true);
+    if (p.ks > 1 && !holds_partials(workspace, workspace_bytes, (size_t)p.ks * m * k)) p = pair_plan(pair_kind(qt, bf), A.n_fp, n_rows / 64, m, k, false);
     A.tt = p.tt; A.ksplit = p.ks; A.part = (float*)workspace;
     if (const int rc = pair_launch<true>(qt, bf, map, A, (int64_t)A.n_fp * ((m + p.tt - 1) / p.tt) * p.ks, st)) return rc;
     if (p.ks > 1) {
@@ -706,8 +715,8 @@ int gemm_tc_mlp_launch(const void* w_gate, const void* w_up, int act, int qt, in
     if (const int rc = make_waits(&A.waits, kWaitCycles)) return rc;
     A.w = (const uint8_t*)w_gate; A.w2 = (const uint8_t*)w_up; A.act = act; A.G = make_geom(n_rows, k, qt); A.M = (int)m; A.y = y; A.y_dtype = y_dtype;
     A.n_fp = (int)((n_rows / 64 + 1) / 2);
-    PairPlan p = pair_plan(pair_pace(qt, bf), A.n_fp, k / 64, m, 2 * n_rows, true);
-    if (p.ks > 1 && !holds_partials(workspace, workspace_bytes, (size_t)p.ks * m * 2 * n_rows)) p = pair_plan(pair_pace(qt, bf), A.n_fp, k / 64, m, 2 * n_rows, false);
+    PairPlan p = pair_plan(pair_kind(qt, bf), A.n_fp, k / 64, m, 2 * n_rows, true);
+    if (p.ks > 1 && !holds_partials(workspace, workspace_bytes, (size_t)p.ks * m * 2 * n_rows)) p = pair_plan(pair_kind(qt, bf), A.n_fp, k / 64, m, 2 * n_rows, false);
     A.tt = p.tt; A.ksplit = p.ks; A.part = (float*)workspace;
     if (const int rc = pair_launch<>(qt, bf, map, A, (int64_t)A.n_fp * ((m + A.tt - 1) / A.tt) * p.ks, st)) return rc;
     if (p.ks > 1) {

@@ -203,6 +203,23 @@ def test_prompts_whose_k_range_stays_whole(lbl, native_lib, cuda_device, qtype, 
     assert torch.equal(*y)
 
 
+@pytest.mark.parametrize("qtype,dtype", [("sym_int4", torch.float16), ("nf4", torch.bfloat16), ("fp8_e4m3", torch.float16)])
+@pytest.mark.parametrize("n,k", [(1280, 1024), (14336, 384)])
+def test_the_token_tile_changes_no_bit(lbl, native_lib, cuda_device, qtype, dtype, n, k):
+    """a prompt's rows computed with those of longer prompts, in other tiles, K whole (no room for partial sums)"""
+    p = lbl.FP4Params(torch.randn(n, k, device=cuda_device, generator=torch.Generator(device=cuda_device).manual_seed(k)) * 0.02,
+                      qtype=lbl.ggml_tensor_qtype[qtype]).to(cuda_device)
+    x = torch.randn(4000, k, device=cuda_device, generator=torch.Generator(device=cuda_device).manual_seed(n)).to(dtype)
+    dt, st = lbl._TORCH_TO_DT[dtype], torch.cuda.current_stream().cuda_stream
+    def rows(m):
+        y, none = torch.empty(m, n, dtype=dtype, device=cuda_device), torch.empty(16, dtype=torch.uint8, device=cuda_device)
+        native_lib.lowbit_matmul_cuda(p.data.data_ptr(), p.qtype, n, k, x.data_ptr(), dt, m, y.data_ptr(), dt, None, 0, none.data_ptr(), 0, st)
+        return y
+    longest = rows(4000)
+    for m in (65, 70, 200, 512, 1000, 3999):
+        assert torch.equal(rows(m), longest[:m]), m
+
+
 @pytest.mark.parametrize("offset", [4, 8])
 def test_scratch_off_a_16_byte_boundary(lbl, native_lib, cuda_device, offset):
     """shapes that would split K run it whole, within the same bounds; 32-bit activations, whose planes lie there, are refused"""
