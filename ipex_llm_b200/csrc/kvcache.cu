@@ -569,6 +569,10 @@ static int sdp_launch(const void* d_q, int q_dtype, const int64_t* q_strides, co
         set_error(LB_ERR_WORKSPACE, "lowbit_sdp_fp8_cuda: workspace too small (%zu < %zu bytes)", workspace_bytes, need);
         return LB_ERR_WORKSPACE;
     }
+    if ((uintptr_t)workspace & 3) {
+        set_error(LB_ERR_ARG, "lowbit_sdp_fp8_cuda: the workspace must be 4-byte aligned");
+        return LB_ERR_ARG;
+    }
     SdpArgs A = {};
     A.q = d_q; A.q_dtype = q_dtype; A.q_sb = q_strides[0]; A.q_sh = q_strides[1]; A.q_ss = q_strides[2];
     A.k = (const uint8_t*)d_k; A.k_sb = k_strides[0]; A.k_sh = k_strides[1]; A.k_ss = k_strides[2];

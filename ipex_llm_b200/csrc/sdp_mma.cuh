@@ -441,6 +441,7 @@ sdp_fp8_decode_mma_kernel(const SdpArgs A) {
                 make_float4(o[4 * q][i], o[4 * q + 1][i], o[4 * q + 2][i], o[4 * q + 3][i]);
     __syncthreads();
     float* part = MERGE ? nullptr : A.part + ((((int64_t)b * A.Hkv + hkv) * gridDim.z + tile) * A.n_split + split) * (A.rt * (D + 2));
+    const bool pairs = (reinterpret_cast<uintptr_t>(A.part) & 7) == 0;  // a caller's workspace may lie on 4 bytes; every row is an even number of floats
     constexpr int RS = D + 4;                                         // floats of a received row: m, l, -, -, o
     const int ps = A.rt * RS;
     if (MERGE && A.n_split > 1) {
@@ -464,9 +465,16 @@ sdp_fp8_decode_mma_kernel(const SdpArgs A) {
             lsum = fmaf(red_l[w][r], f, lsum);
         }
         if (!MERGE) {
-            *reinterpret_cast<float2*>(part + r * (D + 2) + 2 + d) = make_float2(acc[0], acc[1]);
-            *reinterpret_cast<float2*>(part + r * (D + 2) + 4 + d) = make_float2(acc[2], acc[3]);
-            if (d == 0) *reinterpret_cast<float2*>(part + r * (D + 2)) = make_float2(M, lsum);
+            float* const row = part + r * (D + 2);
+            if (pairs) {
+                *reinterpret_cast<float2*>(row + 2 + d) = make_float2(acc[0], acc[1]);
+                *reinterpret_cast<float2*>(row + 4 + d) = make_float2(acc[2], acc[3]);
+                if (d == 0) *reinterpret_cast<float2*>(row) = make_float2(M, lsum);
+            } else {
+#pragma unroll
+                for (int e = 0; e < 4; e++) row[2 + d + e] = acc[e];
+                if (d == 0) { row[0] = M; row[1] = lsum; }
+            }
         } else if (split != 0) {
             // a peer: push (m, l, o) of the row into the leader's receive area and be done
             const uint32_t dst = sdp_smem_u32(recv + (split - 1) * ps + r * RS);

@@ -190,6 +190,25 @@ def test_sdp_fp8_strided_and_misaligned_caches(kv, cuda_device):
     assert torch.equal(kv.sdp_fp8(q_t, k_u8, v_u8, None, scale, True), dense)
 
 
+@pytest.mark.parametrize("B,Hq,Hkv,S,L,D", [(2, 8, 2, 1, 700, 64), (1, 8, 1, 3, 9000, 128), (1, 4, 2, 5, 300, 96), (1, 8, 8, 1, 200, 128)])
+def test_sdp_fp8_workspace_on_four_bytes(kv, native_lib, cuda_device, B, Hq, Hkv, S, L, D):
+    """a workspace needs a float's alignment: the same bits off an 8-byte boundary (key splits that meet in memory, in a cluster, and the
+    CUDA-core kernel), an error off a 4-byte one"""
+    gen = torch.Generator(device=cuda_device).manual_seed(L)
+    q = torch.randn(B, Hq, S, D, device=cuda_device, generator=gen).half()
+    k, v = (torch.randn(B, Hkv, L, D, device=cuda_device, generator=gen).to(torch.float8_e5m2).view(torch.uint8) for _ in range(2))
+    want = kv.sdp_fp8(q, k, v, None, D ** -0.5, True)
+    size, st = native_lib.lowbit_sdp_fp8_workspace_size(B, Hq, Hkv, S, L, D), torch.cuda.current_stream().cuda_stream
+    room, length = torch.empty(size + 16, dtype=torch.uint8, device=cuda_device), torch.tensor([L], dtype=torch.int32, device=cuda_device)
+    for offset in (4, 12):
+        out, later = torch.empty_like(want), torch.empty_like(want)
+        native_lib.lowbit_sdp_fp8(q, k, v, None, True, D ** -0.5, out, room[offset:], st)
+        native_lib.lowbit_sdp_fp8_devlen(q, k, v, True, D ** -0.5, length, 0, later, room[offset:], st)
+        assert torch.equal(out, want) and torch.equal(later, want)
+    with pytest.raises(RuntimeError):
+        native_lib.lowbit_sdp_fp8(q, k, v, None, True, D ** -0.5, torch.empty_like(want), room[2:], st)
+
+
 @pytest.mark.parametrize("B,Hq,Hkv,S,L,dtype,causal", [
     (1, 32, 32, 512, 512, torch.float16, True),        # Llama-2-7B prefill, 512-token prompt
     (2, 8, 2, 100, 300, torch.bfloat16, True),         # GQA, a chunked prefill behind 200 cached tokens, ragged tiles
