@@ -495,13 +495,14 @@ def ggml_matmul_src1_x_src0_t(src0: torch.Tensor, src1: torch.Tensor, src0_shape
 
 
 @functools.lru_cache(maxsize=4096)
-def _grad_plan(qtype, N, K, M):
-    """bytes of scratch for the gradient's product; None: the shape is not the kernel's.  Looking nf4's table up takes longer than the MMAs of
-    a tile, so that with many rows the dequantised matrix wins (forward and backward, 1024 rows, 11008 x 4096: 158 against 167 us; 2000
-    rows, 2048 x 8192: 135 against 127)"""
+def _grad_plan(device, qtype, N, K, M):
+    """bytes of scratch for the gradient's product on ``device`` (its number of SMs decides the splits); None: the shape is not the kernel's.
+    Looking nf4's table up takes longer than the MMAs of a tile, so that with many rows the dequantised matrix wins (forward and backward,
+    1024 rows, 11008 x 4096: 158 against 167 us; 2000 rows, 2048 x 8192: 135 against 127)"""
     if qtype == NF4 and M > 1280:
         return None
-    return ggml.lowbit_matmul_grad_workspace_size(N, K, M) if ggml.lowbit_matmul_grad_supported(qtype, N, K) else None
+    with _on_device(device):
+        return ggml.lowbit_matmul_grad_workspace_size(N, K, M) if ggml.lowbit_matmul_grad_supported(qtype, N, K) else None
 
 
 def _plain_gradient(grad, weight, shape, qtype):
@@ -511,7 +512,7 @@ def _plain_gradient(grad, weight, shape, qtype):
             and grad.numel() > 0 and not (torch.is_grad_enabled() and grad.requires_grad) and torch._C._has_storage(grad)
             and not grad.is_neg() and not grad._is_zerotensor() and torch.autograd.forward_ad.unpack_dual(grad).tangent is None
             and (not torch.is_autocast_enabled("cuda") or torch.get_autocast_dtype("cuda") == grad.dtype)
-            and weight.is_contiguous() and weight.data_ptr() % 16 == 0 and _grad_plan(qtype, *shape, grad.numel() // shape[0]) is not None)
+            and weight.is_contiguous() and weight.data_ptr() % 16 == 0 and _grad_plan(weight.device, qtype, *shape, grad.numel() // shape[0]) is not None)
 
 
 def lowbit_matmul_grad(grad_2d, weight, weight_shape, qtype):
@@ -522,7 +523,7 @@ def lowbit_matmul_grad(grad_2d, weight, weight_shape, qtype):
     elif grad_2d.data_ptr() % 16:
         grad_2d = grad_2d.clone()
     M, dev = grad_2d.shape[0], grad_2d.device
-    need = _grad_plan(qtype, N, K, M)
+    need = _grad_plan(dev, qtype, N, K, M)
     invalidInputError(need is not None, f"unsupported gradient shape ({N}, {K})")
     out = torch.empty((M, K), dtype=grad_2d.dtype, device=dev)
     ws = _scratch(dev, need, out)

@@ -27,6 +27,31 @@ def test_importing_the_package_neither_builds_nor_loads_it():
     subprocess.run([sys.executable, "-c", code], cwd=ROOT, check=True)
 
 
+def test_the_gradients_scratch_is_asked_for_on_the_weights_device(lbl, monkeypatch):
+    """the number of SMs decides the splits: each device its own answer, whichever device is the current one"""
+    current = [0]
+
+    class Guard:
+        def __init__(self, device):
+            self.device = device.index
+
+        def __enter__(self):
+            self.before, current[0] = current[0], self.device
+
+        def __exit__(self, *exc):
+            current[0] = self.before
+
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: current[0])
+    monkeypatch.setattr(torch.cuda, "device", Guard)
+    monkeypatch.setattr(lbl.ggml, "lowbit_matmul_grad_workspace_size", lambda n, k, m: 1000 + current[0])
+    lbl._grad_plan.cache_clear()
+    try:
+        sizes = [lbl._grad_plan(torch.device("cuda", i), lbl.SYM_INT4, 4096, 4096, 100) for i in (0, 1, 0)]
+    finally:
+        lbl._grad_plan.cache_clear()
+    assert sizes == [1000, 1001, 1000] and current == [0]
+
+
 def test_the_file_is_named_by_what_it_is_bound_to():
     from ipex_llm_b200 import build_native
     name = os.path.basename(build_native.build_host())
