@@ -307,8 +307,10 @@ int lowbit_matmul_cuda(const void* d_w, int qtype, int64_t n_rows, int64_t k,
 /* grad_in[m][k] = grad[m][n_rows] . dequant(W): the gradient that MatMulLowBit's backward (reference low_bit_linear.py:545-559) takes back
  * through a packed weight in the tiled layout, the weights rounded once to dtype (fp16 / bf16), 32-bit sums.  n_rows a multiple of 64, k
  * of 128 (lowbit_matmul_grad_supported); weight and gradient 16-byte aligned.  workspace: lowbit_matmul_grad_workspace_size() bytes for the
- * partial sums of a split row range, or less, or NULL: then the rows are not split. */
+ * partial sums of a split row range, or less, or NULL: then the rows are not split.  lowbit_matmul_grad_faster: whether it takes less time
+ * for m rows than dequantising the weight and a library product (nf4 with many rows may not). */
 int lowbit_matmul_grad_supported(int qtype, int64_t n_rows, int64_t k);
+int lowbit_matmul_grad_faster(int qtype, int64_t n_rows, int64_t k, int64_t m);
 size_t lowbit_matmul_grad_workspace_size(int64_t n_rows, int64_t k, int64_t m);
 int lowbit_matmul_grad_cuda(const void* d_w, int qtype, int64_t n_rows, int64_t k, const void* d_grad, int dtype, int64_t m,
                             void* d_out, void* workspace, size_t workspace_bytes, void* stream);

@@ -272,6 +272,9 @@ int lowbit_matmul_cuda(const void* d_w, int qtype, int64_t n_rows, int64_t k, co
 }
 
 int lowbit_matmul_grad_supported(int qtype, int64_t n_rows, int64_t k) { return gemm_tc_grad_supported(qtype, n_rows, k) ? 1 : 0; }
+int lowbit_matmul_grad_faster(int qtype, int64_t n_rows, int64_t k, int64_t m) {
+    return gemm_tc_grad_supported(qtype, n_rows, k) && m > 0 && gemm_tc_grad_faster(qtype, n_rows, k, m) ? 1 : 0;
+}
 size_t lowbit_matmul_grad_workspace_size(int64_t n_rows, int64_t k, int64_t m) { return gemm_tc_grad_workspace_size(n_rows, k, m); }
 int lowbit_matmul_grad_cuda(const void* d_w, int qtype, int64_t n_rows, int64_t k, const void* d_grad, int dtype, int64_t m, void* d_out,
                             void* workspace, size_t workspace_bytes, void* stream) {

@@ -676,6 +676,26 @@ size_t gemm_tc_grad_workspace_size(int64_t n_rows, int64_t k, int64_t m) {
     const int ks = most_splits((k / 128 + 1) / 2, n_rows / 64, m, k);
     return ks > 1 ? (size_t)ks * m * k * sizeof(float) : 0;
 }
+// Whether it is the better way than dequantising for a library product.  Formats but nf4: always (2000 to 6000 rows, six matrices of 4096 to
+// 14336: fp8 0.88 to 1.02 of its time, the 4-bit ones 0.77 to 0.95; fewer rows or smaller matrices: less device time but for matrices under
+// 5 M weights, whose 6 to 12 us no pass waits for).  nf4's table sets a pace of 0.38 us a k-block, so there it goes by cost: rounds of the plan's
+// units against the matrix's way through memory (0.70 us per million weights) and the product (1590 TFLOP/s), all us, fitted to 542 times
+// of 21 matrices, 16 to 4000 rows; this launch / the other way, bf16: 11008 x 4096 at 512 rows 52 / 63, 1024 rows 94 / 92 (taken), 1280
+// rows 159 / 117 (not); 8192 x 8192 at 1024 rows 116 / 133 (taken), 3000 rows 393 / 332 (not); 2048 x 8192 at 2000 rows 70 / 60 (not);
+// 4096 x 11008 at 1280 rows 93 / 101 (taken).  Over all of them 0.925 of the other way's time, the better of the two each time 0.916.  Below
+// 40 us the pass waits for the host, which one call holds up less than two: forward and backward of 1024 rows, 4096 x 4096, 110 / 120 us
+// though the GPU takes 38 / 34.
+bool gemm_tc_grad_faster(int qt, int64_t n_rows, int64_t k, int64_t m) {
+    using namespace gemmtc;
+    if (canon_qtype(qt) != QT_NF4) return true;
+    const int64_t n_fp = (k / 128 + 1) / 2, nb = n_rows / 64, clusters = sm_count() / 2;
+    const PairPlan p = pair_plan(pair_kind(QT_NF4, false), n_fp, nb, m, k, true);
+    const int64_t rounds = (n_fp * ((m + p.tt - 1) / p.tt) * p.ks + clusters - 1) / clusters;
+    const double per_kb = 0.0019 * p.tt > 0.38 ? 0.0019 * p.tt : 0.38;
+    const double here = (double)rounds * ((double)((nb + p.ks - 1) / p.ks) * per_kb + 1.5) + 8.0 + (p.ks > 1 ? 2.7 : 0.0);
+    const double there = 5.5 + (double)n_rows * (double)k * (0.70e-6 + 2.0 * (double)m / 1590e6);
+    return here < there || there < 40.0;
+}
 int gemm_tc_grad_launch(const void* w, int qt, int64_t n_rows, int64_t k, const void* g, int dtype, int64_t m, void* dx, void* workspace,
                         size_t workspace_bytes, cudaStream_t st) {
     using namespace gemmtc;

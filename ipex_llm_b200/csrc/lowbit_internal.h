@@ -95,6 +95,7 @@ int gemm_tc_launch(const void* w, int qt, int64_t n_rows, int64_t k, const void*
                    int y_dtype, const void* bias, int accumulate, void* workspace, size_t workspace_bytes, cudaStream_t st);
 bool gemm_tc_grad_supported(int qt, int64_t n_rows, int64_t k);
 size_t gemm_tc_grad_workspace_size(int64_t n_rows, int64_t k, int64_t m);
+bool gemm_tc_grad_faster(int qt, int64_t n_rows, int64_t k, int64_t m);
 int gemm_tc_grad_launch(const void* w, int qt, int64_t n_rows, int64_t k, const void* g, int dtype, int64_t m, void* dx, void* workspace,
                         size_t workspace_bytes, cudaStream_t st);
 int gemm_tc_mlp_launch(const void* w_gate, const void* w_up, int act, int qt, int64_t n_rows, int64_t k, const void* x, int x_dtype,

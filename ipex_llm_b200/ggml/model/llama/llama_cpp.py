@@ -199,6 +199,8 @@ def lowbit_matmul_cuda(d_w, qtype, n_rows, k, d_x, x_dtype, m, d_y, y_dtype, d_b
 
 _lib.lowbit_matmul_grad_supported.argtypes = [ctypes.c_int, ctypes.c_int64, ctypes.c_int64]
 _lib.lowbit_matmul_grad_supported.restype = ctypes.c_int
+_lib.lowbit_matmul_grad_faster.argtypes = [ctypes.c_int] + [ctypes.c_int64] * 3
+_lib.lowbit_matmul_grad_faster.restype = ctypes.c_int
 _lib.lowbit_matmul_grad_workspace_size.argtypes = [ctypes.c_int64] * 3
 _lib.lowbit_matmul_grad_workspace_size.restype = ctypes.c_size_t
 _lib.lowbit_matmul_grad_cuda.argtypes = [ctypes.c_void_p, ctypes.c_int, ctypes.c_int64, ctypes.c_int64, ctypes.c_void_p, ctypes.c_int, ctypes.c_int64,
@@ -208,6 +210,10 @@ _lib.lowbit_matmul_grad_cuda.restype = ctypes.c_int
 
 def lowbit_matmul_grad_supported(qtype, n_rows, k):
     return bool(_lib.lowbit_matmul_grad_supported(qtype, n_rows, k))
+
+
+def lowbit_matmul_grad_faster(qtype, n_rows, k, m):
+    return bool(_lib.lowbit_matmul_grad_faster(qtype, n_rows, k, m))
 
 
 def lowbit_matmul_grad_workspace_size(n_rows, k, m):

@@ -496,13 +496,16 @@ def ggml_matmul_src1_x_src0_t(src0: torch.Tensor, src1: torch.Tensor, src0_shape
 
 @functools.lru_cache(maxsize=4096)
 def _grad_plan(device, qtype, N, K, M):
-    """bytes of scratch for the gradient's product on ``device`` (its number of SMs decides the splits); None: the shape is not the kernel's.
-    Looking nf4's table up takes longer than the MMAs of a tile, so that with many rows the dequantised matrix wins (forward and backward,
-    1024 rows, 11008 x 4096: 158 against 167 us; 2000 rows, 2048 x 8192: 135 against 127)"""
-    if qtype == NF4 and M > 1280:
-        return None
+    """bytes of scratch for the gradient's product on ``device`` (its number of SMs decides the splits); None: the shape is not the kernel's"""
     with _on_device(device):
         return ggml.lowbit_matmul_grad_workspace_size(N, K, M) if ggml.lowbit_matmul_grad_supported(qtype, N, K) else None
+
+
+@functools.lru_cache(maxsize=4096)
+def _grad_faster(device, qtype, N, K, M):
+    """whether MatMulLowBit's backward of M rows takes that product: the kernel's shape, and quicker than the dequantised matrix"""
+    with _on_device(device):
+        return ggml.lowbit_matmul_grad_faster(qtype, N, K, M)
 
 
 def _plain_gradient(grad, weight, shape, qtype):
@@ -512,7 +515,7 @@ def _plain_gradient(grad, weight, shape, qtype):
             and grad.numel() > 0 and not (torch.is_grad_enabled() and grad.requires_grad) and torch._C._has_storage(grad)
             and not grad.is_neg() and not grad._is_zerotensor() and torch.autograd.forward_ad.unpack_dual(grad).tangent is None
             and (not torch.is_autocast_enabled("cuda") or torch.get_autocast_dtype("cuda") == grad.dtype)
-            and weight.is_contiguous() and weight.data_ptr() % 16 == 0 and _grad_plan(weight.device, qtype, *shape, grad.numel() // shape[0]) is not None)
+            and weight.is_contiguous() and weight.data_ptr() % 16 == 0 and _grad_faster(weight.device, qtype, *shape, grad.numel() // shape[0]))
 
 
 def lowbit_matmul_grad(grad_2d, weight, weight_shape, qtype):

@@ -52,6 +52,17 @@ def test_the_gradients_scratch_is_asked_for_on_the_weights_device(lbl, monkeypat
     assert sizes == [1000, 1001, 1000] and current == [0]
 
 
+@pytest.mark.parametrize("n,k,taken,left", [(11008, 4096, (16, 512, 1024), (1280, 4000)), (8192, 8192, (16, 512, 1024), (3000, 4000)),
+                                            (4096, 11008, (16, 512, 1280), (4000,)), (2048, 8192, (16, 512), (2000, 3000)),
+                                            (1024, 1024, (1, 1024), ()), (14336, 14336, (16, 1024), (3000,))])
+def test_nf4_gradients_are_taken_where_that_is_quicker(lbl, n, k, taken, left):
+    """both sides of the line for matrices whose times stand at the rule (148 SMs); the other formats always, shapes it has no kernel for never"""
+    faster = lbl.ggml.lowbit_matmul_grad_faster
+    assert [m for m in taken if not faster(lbl.NF4, n, k, m)] == [] and [m for m in left if faster(lbl.NF4, n, k, m)] == []
+    assert all(faster(q, n, k, m) for q in (lbl.SYM_INT4, lbl.ASYM_INT4, lbl.ggml_tensor_qtype["fp6"], lbl.ggml_tensor_qtype["fp8_e4m3"]) for m in taken + left)
+    assert not any(faster(q, a, b, 64) for q in (lbl.SYM_INT4, lbl.NF4) for a, b in ((n + 32, k), (n, k + 64))) and not faster(lbl.NF4, n, k, 0)
+
+
 def test_the_file_is_named_by_what_it_is_bound_to():
     from ipex_llm_b200 import build_native
     name = os.path.basename(build_native.build_host())
