@@ -57,6 +57,16 @@ def test_gradient_edges(lbl, native_lib, cuda_device, qtype, dtype, m, n, k):
     assert bool(((whole.double() - want).abs() <= bound).all())
 
 
+@pytest.mark.parametrize("m,n,k", [(1100, 576, 8320), (1500, 576, 8320), (2500, 320, 4224)])
+@pytest.mark.parametrize("qtype,dtype", [("sym_int4", torch.float16), ("nf4", torch.bfloat16), ("fp8_e4m3", torch.bfloat16), ("asym_int4", torch.float16)])
+def test_gradient_over_several_units_a_cluster(lbl, native_lib, cuda_device, qtype, dtype, m, n, k):
+    """rings, parities and the second accumulator carried from unit to unit, an epilogue beside the next unit's products, tiles of 192 to 256
+    tokens with a ragged last one"""
+    units = (k // 128 + 1) // 2 * -(-m // 256)                         # at least: no tile holds more than 256 tokens
+    assert units > 2 * (torch.cuda.get_device_properties(cuda_device).multi_processor_count // 2)
+    test_gradient_edges(lbl, native_lib, cuda_device, qtype, dtype, m, n, k)
+
+
 def test_backward_takes_it_or_the_general_path(lbl, cuda_device, monkeypatch):
     """expanded and 3-dimensional half gradients in one launch; 32-bit ones, a derivative of the gradient in either direction, batched, negated
     and zero ones, those under an autocast to another type and other shapes by dequantising, with the same values"""
