@@ -351,8 +351,12 @@ template <int QT> static int exact_launch_one(const CUtensorMap& map, const Exac
     return A.tt <= 64 ? exact_launch_tile<QT, 64>(map, A, units, st) : exact_launch_tile<QT, 128>(map, A, units, st);
 }
 
-// Token tile and K splits: rounds of the resident clusters x k-blocks per unit + a unit's start and end, + the partial sums' round trip
-// and its launch.  A k-block: twelve MMA steps of half a clock per token (0.0031 us a token), 0.33 us of staging at least
+// Token tile and K splits: rounds of the resident clusters x (k-blocks per unit + a unit's start and end), + the partial sums' round trip and
+// its launch.  Fitted to 918 times (33 to 512 rows, 1024 to 11008 features, K 2048 to 11008, sym_int4 and fp8): a k-block 0.40 us in tiles of
+// up to 64 tokens, 0.52 above (its MMAs, 0.0031 us a token, are 3/4 of that at 128), a unit 1.2 us and 0.014 a token, partial sums 6.6 TB/s
+// and 2.7 us.  Over 120 shapes the choice lies 0.4 % over the best tile and split; with 0.33 us for either tile it was 1.6 %.  sym_int4, its
+// tile then / now: 65 rows, 2048 x 2048 14.2 us (80 tokens) / 12.6 (48), 512 rows 24.0 (96) / 20.5 (64); 48 rows, 11008 x 4096 33.1 (K
+// whole) / 30.4 (three splits); at 128 rows, 4096 x 11008, tiles of 64 take 47.5, of 128 37.2, as then
 struct ExactPlan { int tt, ks; };
 static ExactPlan exact_plan(int64_t n_rows, int64_t nb, int64_t m) {
     const int64_t clusters = sm_count() / 2, n_fp = (n_rows / 128 + 1) / 2, nt0 = (m + kExTok - 1) / kExTok;
@@ -360,11 +364,11 @@ static ExactPlan exact_plan(int64_t n_rows, int64_t nb, int64_t m) {
     double best_cost = 1e30;
     for (int64_t nt = nt0; nt <= nt0 + 4 && nt <= (m + 31) / 32; nt++) {
         const int64_t tt = ((m + nt - 1) / nt + 15) & ~int64_t(15);
-        const double mma = 0.0031 * (double)tt, per_kb = mma > 0.33 ? mma : 0.33;
+        const double per_kb = tt <= 64 ? 0.40 : 0.52;
         for (int64_t ks = 1; ks == 1 || (ks <= 8 && nb / ks >= 8); ks++) {
             const int64_t rounds = (n_fp * nt * ks + clusters - 1) / clusters;
-            double cost = (double)rounds * ((double)((nb + ks - 1) / ks) * per_kb + 1.5);
-            if (ks > 1) cost += (double)ks * (double)m * (double)n_rows * 8.0 / 4.0e6 + 2.0;
+            double cost = (double)rounds * ((double)((nb + ks - 1) / ks) * per_kb + 1.2 + 0.014 * (double)tt);
+            if (ks > 1) cost += (double)ks * (double)m * (double)n_rows * 8.0 / 6.6e6 + 2.7;
             if (cost < best_cost - 1e-9) { best_cost = cost; best = {(int)tt, (int)ks}; }
         }
     }
