@@ -600,7 +600,7 @@ def lowbit_greedy_start(logits, next_ids, tokens, state, suppress_ids, length, s
     B, V = logits.shape
     _check(_lib.lowbit_greedy_start_cuda(logits.data_ptr(), _DT_OF[logits.dtype], logits.stride(0), B, V, next_ids.data_ptr(),
                                          tokens.data_ptr(), tokens.stride(0), tokens.shape[1], state.data_ptr(), suppress_ids.data_ptr(),
-                                         int(length), int(suppress_below), len(ids), (ctypes.c_int64 * max(len(ids), 1))(*ids), stream),
+                                         int(length), int(suppress_below), len(ids), (ctypes.c_int64 * max(len(ids), 1))(*map(int, ids)), stream),
            "lowbit_greedy_start_cuda")
 
 

@@ -136,13 +136,13 @@ def test_greedy_advance_min_new_tokens_rule(native_lib, cuda_device):
     assert tokens[0, :3].tolist() == [3, 3, 7]
 
 
-@pytest.mark.parametrize("B,V,below,ids", [(1, 1000, 0, []), (3, 32000, 2, [7]), (2, 33, 1, [0, 5, 32, 8, 1, 2, 3, 4]), (5, 4097, 0, [3, 4])])
+@pytest.mark.parametrize("B,V,below,ids", [(1, 1000, 0, []), (3, 32000, 2, [7]), (2, 33, 1, [0, 5, 32, 8, 1, 2, 3, 4]), (5, 4097, 0, [3, 4]), (1, 50, 1, [7.0])])
 def test_greedy_start_equals_set_up_state_and_a_pick(native_lib, cuda_device, B, V, below, ids):
     """the pick behind a prompt sets the step's state up itself: the same tokens and state as both copied there first"""
     ggml, dev = native_lib, cuda_device
     logits = torch.randn(B, V, device=dev, generator=torch.Generator(device=dev).manual_seed(V)).half()
     for i in ids[:1]:
-        logits[:, i] = 9.0                              # would be picked
+        logits[:, int(i)] = 9.0                         # would be picked
     got, want = ({"next_ids": torch.full((B,), -5, dtype=torch.int64, device=dev), "tokens": torch.full((B, 4), -7, dtype=torch.int64, device=dev),
                   "state": torch.full((8,), 99, dtype=torch.int32, device=dev), "sup": torch.full((8,), 99, dtype=torch.int64, device=dev)} for _ in range(2))
     want["state"].copy_(torch.tensor([39, 0, 0, below, len(ids), 0, 0, 0]))
