@@ -166,7 +166,8 @@ int lowbit_rotary_inplaced_cuda(void* d_q, const int64_t* q_strides, int Hq, voi
  * (models/common.py:279-283: key.dtype == uint8, seq_length <= 32).  q [B][Hq][S][D] (q_dtype), k / v uint8
  * [B][Hkv][L][D] (GQA: Hq a multiple of Hkv), mask NULL or additive [B][1|Hq][S][L] (mask_strides[1] = 0
  * broadcasts over heads), causal != 0: query token s sees keys <= L - S + s.  out [B][Hq][S][D] contiguous.
- * Softmax and accumulation in fp32; split over the key axis with a deterministic merge (two launches).
+ * Softmax and accumulation in fp32; split over the key axis with a deterministic merge: on the tensor cores with D = 128 up to eight
+ * splits meet in a thread-block cluster (one launch; the workspace is not written), others in the workspace (two launches).
  * Key cache pointer and strides 16-byte aligned, value cache and workspace 4-byte.  D in {64, 96, 128, 192, 256}, S <= 32.
  * fp16 / bf16 queries with D = 64 or 128, a positive scale, a 16-byte aligned value cache (pointer and strides) and
  * 16-byte aligned query rows run on the tensor cores (q.k and p.v as mma.m16n8k16 from the fp8 bytes, P and Q as
@@ -183,8 +184,8 @@ int lowbit_sdp_fp8_cuda(const void* d_q, int q_dtype, const int64_t* q_strides, 
  * scale) (models/common.py:264-286: the prefill, and any call with more than 32 query tokens).  Arguments as
  * lowbit_sdp_fp8_cuda (causal != 0: query token s sees keys <= L - S + s; additive mask optional), any S >= 1, no
  * workspace.  fp16 / bf16 queries with head_dim 128 (lowbit_sdp_fp8_prefill_supported); 16-byte aligned caches, query rows
- * and output.  One CTA per 64 query rows of a query head; the 32-key chunks are staged once per CTA through a cp.async ring
- * and both products run on the tensor cores from the e5m2 bytes (csrc/sdp_prefill.cuh).  Same tolerance as the decode kernel. */
+ * and output.  One CTA per 128 or 256 query rows of a query head; keys and values are expanded to fp16 in shared memory 128 at a time
+ * and both products are tcgen05 MMAs, the probabilities as two fp16 values each in TMEM (csrc/sdp_prefill.cuh). */
 int lowbit_sdp_fp8_prefill_supported(int Hq, int Hkv, int D, int q_dtype);
 int lowbit_sdp_fp8_prefill_cuda(const void* d_q, int q_dtype, const int64_t* q_strides, const void* d_k,
                                 const int64_t* k_strides, const void* d_v, const int64_t* v_strides, const void* d_mask,

@@ -12,9 +12,9 @@
 // k-block, the MMAs 0.14): here activations, packed weights and expanded tiles have rings of their own, so the expansion runs
 // ahead of the activations and four groups of warps have four k-blocks in flight.  Measured per k-block: 0.19 us up to 170 tokens
 // (fp16; see pair_plan for the other paces), 0.282 at 256, where the tensor pipe is busy 512 of 525 clocks; 14336 x 4096 at 4000
-// tokens 1357 -> 1494 TFLOP/s, 4096 x 11008 at 512 tokens 59.7 -> 42.6 us (recorded;
-// the paces are a cool GPU's).  At 128 tokens the MMAs need 256 of 360 clocks: A and B
-// both come from shared memory, beside the expansion's stores.
+// tokens 1357 -> 1494 TFLOP/s, 4096 x 11008 at 512 tokens in fp16 59.7 -> 42.6 us.  All of a cool GPU in short recorded chains; in a
+// long stream of calls, under the power cap, the latter takes 51.  At 128 tokens the MMAs need 256 of 360 clocks: A and B both come from
+// shared memory, beside the expansion's stores.
 //   warp 0       TMA: this CTA's half of the tokens, boxes of 32 rows x 64 elements (128-byte swizzle), ring of kX slots;
 //   warp 1       CTA 0: issues the MMAs (M = 256, N, K = 16; four per k-block) in warp-uniform control flow, one commit per ring
 //                (multicast to both CTAs); CTA 1: relays "my half has landed" to CTA 0's barrier;
@@ -87,8 +87,8 @@ __device__ __forceinline__ void gate_up(const float (&v)[16], int act, int half,
 // feature tile 128 of its columns (two k-blocks of the packed layout, side by side in memory).  The expanded tile is the same image in
 // shared memory -- 64 elements of one weight row to a 128-byte line -- read as an MN-major operand, so nothing is transposed (K-major in
 // its place takes the same time).  Weights are rounded once from their 32-bit value (expand_once).  What it replaces wrote the
-// dequantised matrix to memory for a library product: forward and backward of 1024 rows, 11008 x 4096, nf4 bf16 167 -> 158 us, sym_int4
-// fp16 160 -> 139, of 3000 rows, 8192 x 8192, 668 -> 593, of 20 rows, 14336 x 14336, nf4 263 -> 140.
+// dequantised matrix to memory for a library product: forward and backward of 1024 rows, 11008 x 4096, through MatMulLowBit, nf4 bf16
+// 193 -> 181 us, sym_int4 186 -> 159, of 20 rows, 14336 x 14336, nf4 259 -> 136; recorded, of 3000 rows, 8192 x 8192, sym_int4, 668 -> 593.
 template <int QT, bool BF, bool GRAD>
 __global__ void __launch_bounds__(kPairThreads, 1)
 pair_kernel(const __grid_constant__ CUtensorMap xmap, const PairArgs A) {
@@ -405,8 +405,9 @@ pair_kernel(const __grid_constant__ CUtensorMap xmap, const PairArgs A) {
                 // feature are registers of one thread.  When every lane stored its feature's 32 tokens in 2 bytes each, with the kinds of results
                 // as conditions inside the loop (both sides computed for every value), 32 tokens took 1500 clocks beside the main loop and
                 // behind it (400 so), 32-bit results of a unit of 256 tokens 12 us (3.5 so), which nothing hides behind a cluster's last
-                // unit.  512 rows, 4096 x 11008, bf16 (K in two splits) 49.1 -> 40.6 us, fp16 44.8 -> 42.6, an MLP of 1000 rows, 4096 / 14336,
-                // bf16 323 -> 271, of 4000 rows 1198 -> 1099 (fewer clocks a k-block, too: 531 -> 478 beside an epilogue).
+                // unit.  Recorded, short chains: 512 rows, 4096 x 11008, bf16 (K in two splits) 49.1 -> 40.6 us, fp16 44.8 -> 42.6, an MLP of 1000
+                // rows, 4096 / 14336, bf16 323 -> 271, of 4000 rows 1198 -> 1099 (fewer clocks a k-block, too: 531 -> 478 beside an epilogue);
+                // a stream of calls under the power cap: the MLP of 4000 rows 1263 -> 1171, 512 rows in fp16 52.7 -> 51.2.
                 const bool f16 = A.y_dtype == DT_F16, y_vec = (reinterpret_cast<uintptr_t>(A.y) & 15) == 0;
                 auto put = [&](uint16_t* dst, const uint4& q) {
                     if (y_vec) { *reinterpret_cast<uint4*>(dst) = q; return; }

@@ -261,7 +261,7 @@ skinny_kernel(const __grid_constant__ CUtensorMap xmap, const SkinnyArgs A) {
             mbar_wait(tmem_full(seg & 1), (uint32_t)((seg >> 1) & 1));
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             // the reduction may be scheduled while the last tiles are stored: it waits for this grid's end.  Calls in a row, launched
-            // behind the grid -> so: 40 rows, 11008 x 4096 21.5 -> 20.6 us, 17 rows, 1024 x 1024 16.5 -> 12.4, an MLP of 60 rows, 4096 /
+            // behind the grid -> so: 40 rows, 11008 x 4096 20.5 -> 18.6 us, 17 rows, 1024 x 1024 16.5 -> 12.4, an MLP of 60 rows, 4096 /
             // 14336, 74.4 -> 68.0.  (From the kernel's start the waiting blocks cost the recorded MLP 2 %.)
             if (seg + 1 == n_seg) asm volatile("griddepcontrol.launch_dependents;");
             float* dst = A.part + ((int64_t)blockIdx.x * A.max_seg + seg) * (NTOK * 128) + quarter * 32 + lane;

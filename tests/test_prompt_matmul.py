@@ -180,10 +180,11 @@ def test_prompt_matmul_fp32_keeps_its_contract(lbl, native_lib, cuda_device, qty
     assert bool(((half.double() - want).abs() <= tol * mag + 2.0 ** -11 * want.abs() + 2.0 ** -25).all())
 
 
-@pytest.mark.parametrize("m,n,k", [(48, 19200, 384), (64, 9600, 832), (65, 128, 64), (128, 2176, 1088), (129, 9600, 256), (385, 4736, 448)])
+@pytest.mark.parametrize("m,n,k", [(48, 19200, 384), (64, 9600, 832), (65, 128, 64), (128, 2176, 1088), (129, 9600, 256), (385, 4736, 448), (257, 9728, 832),
+                                   (512, 9728, 640)])
 @pytest.mark.parametrize("qtype", ["sym_int4", "fp8_e4m3", "fp8_e5m2", "fp6"])
 def test_prompt_matmul_fp32_tiles(lbl, native_lib, cuda_device, qtype, m, n, k):
-    """tiles of 64 and of 128 tokens: the line between them, several rounds of units through the rings, k-blocks no multiple of the rings"""
+    """tiles of 64 and of 128 tokens: the line between them, several rounds of units of either through the rings, k-blocks no multiple of the rings"""
     test_prompt_matmul_fp32_keeps_its_contract(lbl, native_lib, cuda_device, qtype, m, n, k)
 
 
