@@ -481,25 +481,55 @@ sdp_fp8_decode_mma_kernel(const SdpArgs A) {
             sdp_st_async_v4(sdp_map_to_rank(dst + 4 * (4 + d), 0), acc, rb);
             if (d == 0) sdp_st_async_v2(sdp_map_to_rank(dst, 0), M, lsum, rb);
         } else {
-            // the leader: merge the splits in rank order (the merge kernel's formula), normalise, store
+            // the leader: merge the splits, normalise, store
             if (A.n_split > 1) sdp_mbar_wait(rbar, 0);
             float Mall = M;
             for (int k = 1; k < A.n_split; k++) Mall = fmaxf(Mall, recv[(k - 1) * ps + r * RS]);
-            const float f0 = (M == -CUDART_INF_F) ? 0.0f : exp2f(M - Mall);
-            float o[4] = {acc[0] * f0, acc[1] * f0, acc[2] * f0, acc[3] * f0}, l = lsum * f0;
-            for (int k = 1; k < A.n_split; k++) {
-                const float* pk = recv + (k - 1) * ps + r * RS;
-                const float f = (pk[0] == -CUDART_INF_F) ? 0.0f : exp2f(pk[0] - Mall);
-                const float4 v = *reinterpret_cast<const float4*>(pk + 4 + d);
-                o[0] = fmaf(v.x, f, o[0]); o[1] = fmaf(v.y, f, o[1]); o[2] = fmaf(v.z, f, o[2]); o[3] = fmaf(v.w, f, o[3]);
-                l = fmaf(pk[1], f, l);
+            float o[4], l;
+            if constexpr (STEP) {                                     // in rank order
+                const float f0 = (M == -CUDART_INF_F) ? 0.0f : exp2f(M - Mall);
+#pragma unroll
+                for (int e = 0; e < 4; e++) o[e] = acc[e] * f0;
+                l = lsum * f0;
+                for (int k = 1; k < A.n_split; k++) {
+                    const float* pk = recv + (k - 1) * ps + r * RS;
+                    const float f = (pk[0] == -CUDART_INF_F) ? 0.0f : exp2f(pk[0] - Mall);
+                    const float4 v = *reinterpret_cast<const float4*>(pk + 4 + d);
+                    o[0] = fmaf(v.x, f, o[0]); o[1] = fmaf(v.y, f, o[1]); o[2] = fmaf(v.z, f, o[2]); o[3] = fmaf(v.w, f, o[3]);
+                    l = fmaf(pk[1], f, l);
+                }
+            } else {
+                // in the merge kernel's order, so that a result has the same bits wherever its splits meet: a warp of its four takes every
+                // fourth split, the denominators fold over lanes 4, 2 and 1 apart, and the quotient is a product with 1 / l
+                float f[8], t[8];
+#pragma unroll
+                for (int k = 0; k < 8; k++) {
+                    const float* pk = recv + (k - 1) * ps + r * RS;
+                    const float m = k == 0 ? M : k < A.n_split ? pk[0] : -CUDART_INF_F;
+                    f[k] = m == -CUDART_INF_F ? 0.0f : exp2f(m - Mall);
+                    t[k] = __fmul_rn(k == 0 ? lsum : k < A.n_split ? pk[1] : 0.0f, f[k]);
+                }
+                l = ((t[0] + t[4]) + (t[2] + t[6])) + ((t[1] + t[5]) + (t[3] + t[7]));
+#pragma unroll
+                for (int w = 0; w < 4; w++) {
+                    float a[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+                    for (int k = w; k < 8; k += 4) {
+                        if (k >= A.n_split) continue;
+                        const float4 v = k == 0 ? make_float4(acc[0], acc[1], acc[2], acc[3]) : *reinterpret_cast<const float4*>(recv + (k - 1) * ps + r * RS + 4 + d);
+                        a[0] = fmaf(v.x, f[k], a[0]); a[1] = fmaf(v.y, f[k], a[1]); a[2] = fmaf(v.z, f[k], a[2]); a[3] = fmaf(v.w, f[k], a[3]);
+                    }
+#pragma unroll
+                    for (int e = 0; e < 4; e++) o[e] = w == 0 ? a[e] : o[e] + a[e];
+                }
             }
+            const float inv = l > 0.0f ? 1.0f / l : 0.0f;
             const int rr = row0 + r;
             if (rr < rows_total) {
                 const int64_t oi = (((int64_t)b * A.Hq + hkv * n_rep) * A.S + rr) * D + d;           // rows of a group: [query head][token]
 #pragma unroll
                 for (int e = 0; e < 4; e++) {
-                    const float y = l > 0.0f ? o[e] / l : 0.0f;
+                    const float y = !STEP ? o[e] * inv : l > 0.0f ? o[e] / l : 0.0f;
                     if (A.out_dtype == DT_F32) ((float*)A.out)[oi + e] = y;
                     else if (A.out_dtype == DT_F16) ((__half*)A.out)[oi + e] = __float2half_rn(y);
                     else ((__nv_bfloat16*)A.out)[oi + e] = __float2bfloat16_rn(y);

@@ -2,6 +2,9 @@
 C ABI, against the statements they restate: transformers' RMSNorm, the separate rotary + cache-quantise kernels,
 the host-length decode attention, torch.argmax."""
 import math
+import os
+import subprocess
+import sys
 
 import pytest
 import torch
@@ -194,6 +197,32 @@ def test_decode_attention_one_launch_equals_the_separate_kernels(native_lib, cud
         assert float((got.double() - exact).abs().max()) <= tol, P
         assert float((got.double() - want.double()).abs().max()) <= tol, P
     assert launches == {1}, launches                     # every case here fits the one-launch kernel
+
+
+_SPLIT_SHAPES = [(1, 4, 4, 1, 1), (2, 16, 8, 21, 21), (5, 32, 16, 24, 24), (2, 8, 4, 1, 129), (10, 32, 32, 1, 700), (1, 32, 32, 1, 577), (1, 16, 2, 1, 1025),
+                 (4, 4, 1, 1, 285), (4, 32, 8, 3, 780), (1, 32, 8, 8, 500), (8, 32, 8, 1, 4001)]
+
+
+def _attention_of_all_shapes(device):
+    from ipex_llm_b200.transformers import kv
+    out = []
+    for B, Hq, Hkv, S, L in _SPLIT_SHAPES:
+        gen = torch.Generator(device=device).manual_seed(B * L + S)
+        q = torch.randn(B, S, Hq, 128, device=device, generator=gen).half().transpose(1, 2)
+        k, v = (torch.randn(B, Hkv, L, 128, device=device, generator=gen).to(torch.float8_e5m2).view(torch.uint8) for _ in range(2))
+        out.append(kv.scaled_dot_product_attention(q, k, v, None, True, 128 ** -0.5).cpu())
+    return out
+
+
+def test_key_splits_give_the_same_bits_in_a_cluster_and_in_memory(native_lib, cuda_device, tmp_path):
+    """one to eight splits: the cluster's first CTA sums in the merge kernel's order.  A fourth stage of the ring (read once a process) sends
+    every shape to the merge kernel"""
+    path, tests = str(tmp_path / "out.pt"), os.path.dirname(os.path.abspath(__file__))
+    code = (f"import sys, torch; sys.path.insert(0, {tests!r}); import test_decode_ops as t\n"
+            f"torch.save(t._attention_of_all_shapes(torch.device('cuda', 0)), {path!r})")
+    subprocess.run([sys.executable, "-c", code], check=True, cwd=os.path.dirname(tests), env=dict(os.environ, LOWBIT_SDP_RING="4"))
+    for shape, here, there in zip(_SPLIT_SHAPES, _attention_of_all_shapes(cuda_device), torch.load(path)):
+        assert torch.equal(here, there), shape
 
 
 @pytest.mark.parametrize("B,Hq,Hkv,S,L", [(1, 4, 4, 1, 1), (2, 8, 4, 1, 129), (8, 32, 8, 1, 4001), (1, 32, 32, 1, 577), (1, 16, 2, 1, 1025), (1, 8, 1, 1, 16000),
