@@ -78,10 +78,11 @@ __device__ __forceinline__ float sdp_round_to(float v, int dt) {
 // shared memory (st.async + mbarrier transaction count, as the GEMV's split-K reduction does); the leader merges in rank
 // order and writes the output.  Same arithmetic as the separate kernels (rope.cu, kv_quantize, this kernel + the merge
 // kernel): rotate -> round -> quantise, the same split-local softmax, the same merge formula.
-// FUSED = 2 is plain attention (queries, key / value views, mask as for FUSED = 0) with that merge: no partial results in memory, no
-// second launch.  Recorded calls in a row, caches from memory, with the second launch -> now: 8 sequences x 4000 keys, 32 heads over 8
-// (66 MB, 4 splits) 18.9 -> 16.8 us; 16 x 1000 keys 13.9 -> 11.7; 4 x 300 keys 6.5 -> 4.7; 1 x 577 keys, 32 heads 6.3 -> 4.8; 8 new tokens
-// x 500 keys 7.3 -> 5.8.  What is left is a launch's start and end, about 5 us (the smallest shapes), and the keys at 5.4 TB/s.
+// FUSED = 2 is plain attention (queries, key / value views, mask as for FUSED = 0) with that merge, summed in the merge kernel's order: no
+// partial results in memory, no second launch.  Recorded calls in a row, caches from memory, with the second launch -> now: 8 sequences x
+// 4000 keys, 32 heads over 8 (66 MB, 4 splits) 18.7 -> 16.5 us; 16 x 1000 keys 13.7 -> 11.6; 4 x 300 keys 6.9 -> 5.1; 1 x 577 keys, 32
+// heads 6.8 -> 5.9; 8 new tokens x 500 keys 7.0 -> 5.8; a prompt of 24 tokens 8.4 -> 4.8.  What is left is a launch's start and end, about
+// 5 us (the smallest shapes), and the keys at 5.4 TB/s.
 template <int D, int OCC, int NST, int FUSED>
 __global__ void __launch_bounds__(SDP_WARPS * 32, OCC)
 sdp_fp8_decode_mma_kernel(const SdpArgs A) {
