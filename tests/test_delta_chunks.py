@@ -113,3 +113,42 @@ def test_a_prompt_in_portions_of_its_scratch(ops, cuda_device):
     o = ops.gated_delta_rule(conv, G, H, D, V, proj, 1, 1 + H, a_log, bias, state, 0, pad)
     assert float((o.double() - want_o).abs().max()) <= 2e-6 * max(1.0, float(want_o.abs().max()))
     assert float((state.double() - want_s).abs().max()) <= 2e-6 * max(1.0, float(want_s.abs().max()))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("bad", [float("nan"), float("-inf")])
+@pytest.mark.parametrize("what", ["query", "key", "value"])
+def test_nothing_of_a_later_token_reaches_an_earlier_one(ops, cuda_device, dtype, bad, what):
+    """a query, a key, a value that is no number, as a chunk's first token and inside one: the tokens before it come out bit for bit as
+    without it; a query stays with its own token, a key reaches every column behind it"""
+    B, S, G, H, D, V = 1, 100, 1, 5, 128, 40
+    conv, proj, a_log, bias, state = inputs(cuda_device, B, S, G, H, D, V, dtype)
+    pad = torch.zeros(B, dtype=torch.int32, device=cuda_device)
+    o = ops.gated_delta_rule(conv, G, H, D, V, proj, 1, 1 + H, a_log, bias, state.clone(), 0, pad)
+    for at in (32, 45):
+        c = conv.clone()
+        c[0, at, {"query": 5, "key": D + 5, "value": 2 * D + 2 * V + 7}[what]] = bad
+        got = ops.gated_delta_rule(c, G, H, D, V, proj, 1, 1 + H, a_log, bias, state.clone(), 0, pad)
+        assert torch.equal(got[:, :at], o[:, :at])
+        if what == "query":
+            assert not bool(got[:, at].isfinite().any()) and torch.equal(got[:, at + 1:], o[:, at + 1:])
+        elif what == "key":
+            assert not bool(got[:, at:].isfinite().any())
+        else:
+            assert not bool(got[:, at:, 2, 7].isfinite().any())
+            got[:, at:, 2, 7] = o[:, at:, 2, 7]
+            assert torch.equal(got, o)
+
+
+@pytest.mark.parametrize("dtype,power", [(torch.float32, 55), (torch.float32, -55), (torch.bfloat16, 40), (torch.bfloat16, -40), (torch.float16, -6), (torch.float16, 11)])
+def test_keys_and_queries_of_any_size(ops, cuda_device, dtype, power):
+    """the unit vectors' factors are powers of two and a rest: keys and queries far from one, and tokens without any"""
+    B, S, G, H, D, V = 1, 96, 2, 2, 96, 24
+    conv, proj, a_log, bias, state = inputs(cuda_device, B, S, G, H, D, V, dtype)
+    conv[..., :2 * G * D] *= 2.0 ** power
+    conv[:, 40, :2 * G * D] = 0
+    pad = torch.zeros(B, dtype=torch.int32, device=cuda_device)
+    want_o, want_s = statement(conv, proj, a_log, bias, state, G, H, D, V, 0, pad)
+    o = ops.gated_delta_rule(conv, G, H, D, V, proj, 1, 1 + H, a_log, bias, state, 0, pad)
+    assert float((o.double() - want_o).abs().max()) <= 2e-6 * max(1.0, float(want_o.abs().max()))
+    assert float((state.double() - want_s).abs().max()) <= 2e-6 * max(1.0, float(want_s.abs().max()))
