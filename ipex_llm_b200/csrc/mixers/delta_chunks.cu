@@ -672,7 +672,6 @@ __global__ void __launch_bounds__(64 * DW, 1) delta_walk_kernel(const ChunkArgs 
 #pragma unroll
                 for (int e = 0; e < 4; ++e) odd |= !(fabsf(u[tt][e]) <= 1e38f);
             odd = __any_sync(0xffffffffu, odd);
-            if (!odd && lane == 0) arrive(empty + 8 * slot);         // (the one by one way reads A again)
             float f[4][4];
 #pragma unroll
             for (int tt = 0; tt < 4; ++tt)
@@ -689,6 +688,10 @@ __global__ void __launch_bounds__(64 * DW, 1) delta_walk_kernel(const ChunkArgs 
                 }
 #pragma unroll
             for (int e = 0; e < 4; ++e) r[e] += (x[0][e] + x[1][e]) + x[2][e];
+            if (!odd) {                                 // all that was read has been used (an arrival behind loads under way may be overtaken)
+                __syncwarp();
+                if (lane == 0) arrive(empty + 8 * slot);
+            }
             if (odd)
 #pragma unroll 1
                 for (int j = 0; j < 8 * w + 8; ++j) {
@@ -854,7 +857,7 @@ __global__ void __launch_bounds__(64 * DW, 1) delta_walk_kernel(const ChunkArgs 
 #pragma unroll
         for (int tt = 0; tt < 4; ++tt) op[(tt * DW + warp) * 32 + lane] = make_float4(oa[tt][0], oa[tt][1], oa[tt][2], oa[tt][3]);
         __syncwarp();
-        if (lane == 0) { arrive(ready + 8 * slot); arrive(empty + 8 * slot); }
+        if (lane == 0) arrive(ready + 8 * slot);
         if constexpr (STAGES == 2) next_w();
         const float2 dd = make_float2(decay, decay);
 #pragma unroll
@@ -869,6 +872,8 @@ __global__ void __launch_bounds__(64 * DW, 1) delta_walk_kernel(const ChunkArgs 
                 }
             split_pair(m[2 * kt], m[2 * kt + 1], mp[kt]);
         }
+        __syncwarp();
+        if (lane == 0) arrive(empty + 8 * slot);        // all that was read has been used
     }
 #pragma unroll
     for (int dt = 0; dt < DTL; ++dt)
