@@ -544,6 +544,22 @@ def test_gemm_skinny_random_shapes(lbl, cuda_device):
         assert bool((err <= bound + 1e-6 * want.abs()).all()), (trial, qtype, N, K, M, float((err / bound).max()))
 
 
+@pytest.mark.parametrize("qtype", ["sym_int4", "asym_int4", "nf4", "fp8_e4m3", "fp6"])
+@pytest.mark.parametrize("xdt,tol,M", [(torch.float16, 1e-3, 17), (torch.bfloat16, 8e-3, 32), (torch.float16, 1e-3, 33), (torch.bfloat16, 8e-3, 64)])
+def test_gemm_skinny_rings_go_round(lbl, cuda_device, qtype, xdt, tol, M):
+    """32 items per block: every ring (2 to 12 stages of weights, odd ones too, 2 to 4 of activations, 4 expanded tiles) goes round at least
+    twice.  A stage read a round early or late would give another block's weights; ten launches without a pause, bit for bit the same"""
+    N, K = 9472, 8192                                                # 74 tiles x 64 pairs over 148 blocks
+    g = torch.Generator(device=cuda_device).manual_seed(1290 + M)
+    tiled = lbl.FP4Params(torch.randn(N, K, generator=g, device=cuda_device) * 0.02, qtype=qid(qtype)).to(cuda_device).data
+    x = torch.randn(M, K, generator=g, device=cuda_device).to(xdt)
+    ys = [lbl.lowbit_matmul(x, tiled, (N, K), qid(qtype), out_dtype=torch.float32) for _ in range(10)]
+    assert lbl.ggml.last_launch_count() == 2 and all(torch.equal(y, ys[0]) for y in ys[1:])
+    wd = lbl.dequantize_device_layout(tiled, (N, K), qid(qtype)).double()
+    bound = tol * (x.double().abs() @ wd.abs().T) + 1e-30
+    assert bool(((ys[0].double() - x.double() @ wd.T).abs() <= bound).all())
+
+
 def test_gemm_skinny_epilogue_window_and_determinism(lbl, cuda_device):
     rng = np.random.default_rng(1260)
     N, K, M = 1024, 2048, 40
