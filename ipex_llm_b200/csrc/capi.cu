@@ -235,7 +235,7 @@ static int matmul_dispatch(const void* d_w, int qtype, int64_t n_rows, int64_t k
                            cudaStream_t st) {
     if (use_skinny(qtype, n_rows, k, m, x_dtype))
         return gemm_skinny_launch(d_w, qtype, n_rows, k, d_x, x_dtype, m, d_y, y_dtype, d_bias, accumulate, workspace,
-                                  workspace_bytes, st, gemv_get_pdl());
+                                  workspace_bytes, st, launch_overlaps(st) ? 2 : gemv_get_pdl());
     if (use_gemm(qtype, n_rows, k, m, x_dtype))
         return gemm_tc_launch(d_w, qtype, n_rows, k, d_x, x_dtype, m, d_y, y_dtype, d_bias, accumulate, workspace, workspace_bytes, st);
     // a caller's scratch of the GEMV's size still runs its chunks of 32 rows
@@ -326,7 +326,7 @@ int lowbit_mlp_cuda(const void* d_w_gate, const void* d_w_up, int qtype, int64_t
     } else if (use_skinny(qtype, n_rows, k, m, x_dtype)) {
         // 17..64 half-precision rows: both matrices in one pass of the skinny tensor-core kernel, act * up in its reduction launch
         rc = gemm_skinny_mlp_launch(d_w_gate, d_w_up, act + 1, qtype, n_rows, k, d_x, x_dtype, m, d_y, y_dtype, workspace, workspace_bytes,
-                                    st, gemv_get_pdl());
+                                    st, launch_overlaps(st) ? 2 : gemv_get_pdl());
     } else if (use_gemm(qtype, n_rows, k, m, x_dtype)) {
         rc = gemm_tc_mlp_launch(d_w_gate, d_w_up, act + 1, qtype, n_rows, k, d_x, x_dtype, m, d_y, y_dtype, workspace, workspace_bytes, st);
     } else {

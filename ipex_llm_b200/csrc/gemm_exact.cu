@@ -112,6 +112,7 @@ exact_kernel(const __grid_constant__ CUtensorMap xmap, const ExactArgs A) {
         asm volatile("griddepcontrol.wait;" ::: "memory");     // split3_kernel's; the weights' copies and expansion have begun meanwhile
         for (int unit = blockIdx.x >> 1; unit < n_units; unit += stride) {
             decode(unit, U);
+            if (unit + stride >= n_units) asm volatile("griddepcontrol.launch_dependents;");     // the cluster's last unit
             const int row0 = U.m0 + rank * (U.n_tok >> 1), boxes = ((U.n_tok >> 1) + 31) >> 5;
             for (int kb = U.kb0; kb < U.kb1; kb++) {
                 if (!mbar_wait_lim(x_empty(s), (uint32_t)((round & 1) ^ 1), A.waits)) goto done;
@@ -299,7 +300,8 @@ done:
 
 // fp32 activations -> three bf16 planes whose sum reproduces them to 2^-24, four elements a thread
 __global__ void __launch_bounds__(256) split3_kernel(const float4* __restrict__ x, uint2* __restrict__ out, int64_t n4) {
-    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;");     // not before the wait: the matmul reads its weights ahead of its own
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n4; i += (int64_t)gridDim.x * blockDim.x) {
         const float4 q = x[i];
         float r[4] = {q.x, q.y, q.z, q.w};
@@ -394,7 +396,7 @@ int gemm_exact_launch(const void* w, int qt, int64_t n_rows, int64_t k, const vo
     if (!workspace || workspace_bytes < gemm_exact_workspace_size(n_rows, k, m)) return LB_ERR_WORKSPACE;
     const int64_t n4 = m * k / 4;                                       // k is a multiple of 64
     int sg = (int)((n4 + 255) / 256); if (sg > sm_count() * 8) sg = sm_count() * 8;
-    split3_kernel<<<sg, 256, 0, st>>>((const float4*)x, (uint2*)workspace, n4);
+    launch_behind(split3_kernel, dim3((unsigned)sg), 256, 0, st, launch_overlaps(st), (const float4*)x, (uint2*)workspace, n4);
     note_launch();
     CUtensorMap map;
     if (const int rc = encode_rows(&map, workspace, true, 3 * m, k, 32)) return rc;
@@ -415,7 +417,7 @@ int gemm_exact_launch(const void* w, int qt, int64_t n_rows, int64_t k, const vo
     if (p.ks > 1) {
         const int64_t mn = m * n_rows;
         int rg = (int)((mn / 4 + 255) / 256); if (rg > sm_count() * 8) rg = sm_count() * 8;
-        reduce_partials_kernel<<<rg, 256, 0, st>>>(A.part, p.ks, mn, n_rows, y, DT_F32, bias, accumulate);
+        launch_behind(reduce_partials_kernel, dim3((unsigned)rg), 256, 0, st, launch_overlaps(st), A.part, p.ks, mn, n_rows, y, DT_F32, bias, accumulate);
         note_launch();
     }
     return check_launch();

@@ -134,6 +134,7 @@ pair_kernel(const __grid_constant__ CUtensorMap xmap, const PairArgs A) {
     }
     // an expert's rows in tiles of at most 256 tokens, evenly cut; few rows are another kernel's
     auto tiles_of = [](int rows) { return rows > (int)kExactRows ? (rows + kPairTok - 1) / kPairTok : 0; };
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     if (warp == 2 && A.offs) {
         int before = 0;
         for (int e0 = 0; e0 < A.n_experts; e0 += 32) {
@@ -192,6 +193,7 @@ pair_kernel(const __grid_constant__ CUtensorMap xmap, const PairArgs A) {
         // ================= activations: this CTA's half of the tile's tokens =================
         for (int unit = blockIdx.x >> 1; unit < n_units; unit += stride) {
             decode(unit, U);
+            if (unit + stride >= n_units) asm volatile("griddepcontrol.launch_dependents;");     // the cluster's last unit
             const int half = U.n_tok >> 1, boxes = (half + 31) >> 5, row0 = U.m0 + rank * half;
             for (int kb = U.kb0; kb < U.kb1; kb++) {
                 if (!mbar_wait_lim(x_empty(s), (uint32_t)((round & 1) ^ 1), A.waits)) goto done;
@@ -514,6 +516,8 @@ done:
 
 // the same behind a split MLP: y[token][n] = act(sum of the gate partials) * (sum of the up partials)
 __global__ void __launch_bounds__(256) reduce_gated_kernel(const float* __restrict__ part, int ksplit, int64_t m, int64_t n, void* y, int y_dtype, int act) {
+    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const int64_t mn = m * n, n4 = n / 4;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < mn / 4; i += (int64_t)gridDim.x * blockDim.x) {
         const int64_t token = i / n4, col = (i - token * n4) * 4;
@@ -559,10 +563,10 @@ static int pair_launch_one(const CUtensorMap& map, const PairArgs& A, int64_t un
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2u * (unsigned)(units < clusters ? units : clusters)); cfg.blockDim = dim3(kPairThreads);
     cfg.dynamicSmemBytes = PairSmem<QT>::kTotal; cfg.stream = st;
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-    cfg.attrs = at; cfg.numAttrs = 1;
+    cfg.attrs = at; cfg.numAttrs = add_overlap(at, 1, launch_overlaps(st));
     cudaLaunchKernelEx(&cfg, pair_kernel<QT, BF, GRAD>, map, A);
     note_launch();
     return LB_OK;
@@ -663,7 +667,7 @@ int gemm_tc_launch(const void* w, int qt, int64_t n_rows, int64_t k, const void*
     if (p.ks > 1) {
         const int64_t mn = m * n_rows;
         int rg = (int)((mn / 4 + 255) / 256); if (rg > sm_count() * 8) rg = sm_count() * 8;
-        reduce_partials_kernel<<<rg, 256, 0, st>>>(A.part, p.ks, mn, n_rows, y, y_dtype, bias, accumulate);
+        launch_behind(reduce_partials_kernel, dim3((unsigned)rg), 256, 0, st, launch_overlaps(st), A.part, p.ks, mn, n_rows, y, y_dtype, bias, accumulate);
         note_launch();
     }
     return check_launch();
@@ -715,7 +719,7 @@ int gemm_tc_grad_launch(const void* w, int qt, int64_t n_rows, int64_t k, const 
     if (const int rc = pair_launch<true>(qt, bf, map, A, (int64_t)A.n_fp * ((m + p.tt - 1) / p.tt) * p.ks, st)) return rc;
     if (p.ks > 1) {
         int rg = (int)((m * k / 4 + 255) / 256); if (rg > sm_count() * 8) rg = sm_count() * 8;
-        reduce_partials_kernel<<<rg, 256, 0, st>>>(A.part, p.ks, m * k, k, dx, dtype, nullptr, 0);
+        launch_behind(reduce_partials_kernel, dim3((unsigned)rg), 256, 0, st, launch_overlaps(st), A.part, p.ks, m * k, k, dx, dtype, nullptr, 0);
         note_launch();
     }
     return check_launch();
@@ -742,7 +746,7 @@ int gemm_tc_mlp_launch(const void* w_gate, const void* w_up, int act, int qt, in
     if (const int rc = pair_launch<>(qt, bf, map, A, (int64_t)A.n_fp * ((m + A.tt - 1) / A.tt) * p.ks, st)) return rc;
     if (p.ks > 1) {
         int rg = (int)((m * n_rows / 4 + 255) / 256); if (rg > sm_count() * 8) rg = sm_count() * 8;
-        reduce_gated_kernel<<<rg, 256, 0, st>>>(A.part, p.ks, m, n_rows, y, y_dtype, act);
+        launch_behind(reduce_gated_kernel, dim3((unsigned)rg), 256, 0, st, launch_overlaps(st), A.part, p.ks, m, n_rows, y, y_dtype, act);
         note_launch();
     }
     return check_launch();

@@ -41,7 +41,7 @@ struct SkinnyArgs {
     int M;
     float* part;             // [gridDim.x * max_seg][NTOK][128] fp32 partial tiles
     int max_seg;
-    int pdl;
+    int pdl;                 // launched as a programmatic dependent: 1 in a recorded step (the weights are complete), 2 outside one
 };
 
 template <int QT, int NTOK> struct SkSmem {
@@ -135,6 +135,7 @@ skinny_kernel(const __grid_constant__ CUtensorMap xmap, const SkinnyArgs A) {
         // ================= packed weights: the whole warp runs the loop, one elected lane issues the copies.  The first round does not
         // depend on the previous kernel and is not held up by it
         const uint32_t leader = elect_leader();
+        if (A.pdl == 2) asm volatile("griddepcontrol.wait;" ::: "memory");
         for (int it = 0; it < n_items; it++) {
             const int s = it % NS;
             if (it >= NS) mbar_wait(free_bar(s), (uint32_t)((it / NS - 1) & 1));

@@ -165,7 +165,7 @@ int gemv_launch_ex(const void* w, const void* w2, int act, int qt, int64_t n_row
             A.w = (const uint8_t*)w; A.w2 = (const uint8_t*)w2; A.act = act; A.G = G; A.M = (int)mc;
             A.y = yc; A.y_dtype = y_dtype; A.bias = bias; A.accumulate = accumulate;
             A.plane_stride = mc * k;
-            A.pdl = g_pdl; A.ts = g_ts;
+            A.pdl = launch_overlaps(st) && push.world == 0 ? 2 : g_pdl; A.ts = g_ts;
             A.next_w = t_next_w; A.next_bytes = t_next_bytes;
             t_next_w = nullptr; t_next_bytes = 0;            // one-shot hint
             A.push_world = push.world; A.push_rank = push.rank; A.push_slot_bytes = push.slot_bytes; A.push_epochs = push.epochs;

@@ -32,7 +32,7 @@ struct GemvArgs {
     void* y; int y_dtype;     // [M][rows]
     const void* bias;         // NULL or [rows] of y_dtype
     int accumulate;
-    int pdl;                  // launched with programmatic stream serialization
+    int pdl;                  // launched with programmatic stream serialization: 1 in a recorded step (the weights are complete), 2 outside one
     const uint8_t* next_w;    // hint: weights of the NEXT matmul on this stream, prefetched into L2 (or NULL)
     unsigned long long next_bytes;
     unsigned long long* ts;   // development: per-warp phase timestamps (8 per warp) or NULL

@@ -398,7 +398,7 @@ gemv_kernel(const GemvArgs A) {
     const int nbt = (MODE == 2) ? nb * A.n_seg : nb;   // k-blocks along the (concatenated) K axis
     if (A.pdl) asm volatile("griddepcontrol.launch_dependents;");
     // the routed expert ids come from the previous kernel: nothing can be fetched before it is done
-    if (MODE != 0 && A.pdl) asm volatile("griddepcontrol.wait;" ::: "memory");
+    if ((MODE != 0 && A.pdl) || A.pdl == 2) asm volatile("griddepcontrol.wait;" ::: "memory");
 
     auto expert_of = [&](int z, bool& ok) -> int {
         const long long e = A.sel_i64 ? reinterpret_cast<const long long*>(A.sel)[z]

@@ -607,7 +607,7 @@ static int sdp_launch(const void* d_q, int q_dtype, const int64_t* q_strides, co
         else if (nst == 0) sdp_fp8_decode_mma_kernel<128, 2, 0, 0><<<grid, SDP_WARPS * 32, 0, st>>>(A);
         else if (nst == 3 && sdp_merges_in_cluster(A, (int64_t)B * Hkv * tiles)) {
             A.early = 0;
-            return sdp_launch_cluster(sdp_fp8_decode_mma_kernel<128, 2, 3, 2>, A, tiles, false, st);
+            return sdp_launch_cluster(sdp_fp8_decode_mma_kernel<128, 2, 3, 2>, A, tiles, launch_overlaps(st), st);
         }
         else {
             auto kern = nst == 2 ? sdp_fp8_decode_mma_kernel<128, 3, 2, 0> : (nst == 4 ? sdp_fp8_decode_mma_kernel<128, 1, 4, 0> : sdp_fp8_decode_mma_kernel<128, 2, 3, 0>);

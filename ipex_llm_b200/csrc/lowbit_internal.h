@@ -39,6 +39,30 @@ int quantize_launch(const float* src, void* dst, int qt, size_t n, int k, int64_
 // gemv.cu
 void gemv_set_pdl(int on);
 int gemv_get_pdl();
+// Launches outside a recorded step overlap their starts: a kernel is launched as a programmatic dependent of the one in front and waits
+// (griddepcontrol.wait) before it touches global memory, so that what it reads and overwrites is ordered as without; its scheduling, its
+// barriers and its TMEM are off the chain, 1 to 2 us a call behind a kernel that releases its dependents early.  In a recorded step (the
+// switch on) the launches of these kernels stay ordinary: kernels there read inputs ahead of their wait because an ordinary launch lies in
+// front of them; and in a stream that is being captured the graph's edges are left as they were.
+inline bool launch_overlaps(cudaStream_t st) {
+    if (gemv_get_pdl()) return false;
+    cudaStreamCaptureStatus state = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(st, &state) == cudaSuccess && state == cudaStreamCaptureStatusNone;
+}
+inline int add_overlap(cudaLaunchAttribute* at, int n, bool on) {
+    if (!on) return n;
+    at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[n].val.programmaticStreamSerializationAllowed = 1;
+    return n + 1;
+}
+template <typename... P, typename... Q>
+inline void launch_behind(void (*kern)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, bool overlap, Q... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid; cfg.blockDim = dim3((unsigned)threads); cfg.dynamicSmemBytes = smem; cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    cfg.attrs = at; cfg.numAttrs = add_overlap(at, 0, overlap);
+    cudaLaunchKernelEx(&cfg, kern, P(args)...);
+}
 struct GemvPush;
 void gemv_set_push(const GemvPush* p);   // the next gemv_launch_ex on this thread pushes its result to the peers (comm.cu)
 void gemv_set_next_weights(const void* w, size_t bytes);

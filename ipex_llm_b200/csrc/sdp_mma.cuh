@@ -120,6 +120,8 @@ sdp_fp8_decode_mma_kernel(const SdpArgs A) {
         // knows them complete (A.early: an ordinarily launched kernel lies between their producers and this call) lets the
         // first chunks stream in while the previous kernel drains; otherwise nothing is read before the wait.
         if (STEP && !A.early) asm volatile("griddepcontrol.wait;" ::: "memory");
+        // plain attention is scheduled while the kernel in front of it drains, and reads nothing of it before its end
+        if (!STEP) asm volatile("griddepcontrol.wait;" ::: "memory");
     }
     int L, keys_per_split;
     sdp_lengths(A, L, keys_per_split);

@@ -106,6 +106,8 @@ sdp_fp8_prompt_kernel(const SdpArgs A, int n_qt) {
     };
     int nk = tiles_of(0);
     if (NT == 2) nk = max(nk, tiles_of(1));
+    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
 
     // ---- before the barriers exist: the queries into their tiles, the first keys on their way
     if (warp < 4 * NT) {
@@ -389,7 +391,7 @@ template <int NT, bool MASK> int sdp_prompt_launch_nt(const SdpArgs& A, cudaStre
         configured_dev[dev & 63] = true;
     }
     const int n_qt = (A.S + NT * SP_ROWS - 1) / (NT * SP_ROWS);
-    sdp_fp8_prompt_kernel<NT, MASK><<<dim3((unsigned)(A.B * A.Hq), (unsigned)n_qt), sp_threads(NT), sp_smem(NT), st>>>(A, n_qt);
+    launch_behind(sdp_fp8_prompt_kernel<NT, MASK>, dim3((unsigned)(A.B * A.Hq), (unsigned)n_qt), sp_threads(NT), sp_smem(NT), st, launch_overlaps(st), A, n_qt);
     note_launch();
     return check_launch();
 }

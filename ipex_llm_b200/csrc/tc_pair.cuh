@@ -67,6 +67,8 @@ __device__ __forceinline__ void store_feature(float* p, int64_t stride, const fl
 // K split: y[token][n] = sum over splits (in split order) of the fp32 partials, + bias, + y when accumulating
 static __global__ void __launch_bounds__(256) reduce_partials_kernel(const float* __restrict__ part, int ksplit, int64_t mn, int64_t n_cols,
                                                               void* y, int y_dtype, const void* bias, int accumulate) {
+    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     for (int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) * 4; i < mn; i += (int64_t)gridDim.x * blockDim.x * 4) {
         float4 a = *reinterpret_cast<const float4*>(part + i);
         for (int ks = 1; ks < ksplit; ks++) {
