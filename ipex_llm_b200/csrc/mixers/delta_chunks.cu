@@ -164,6 +164,8 @@ __global__ void __launch_bounds__(DT, 2) delta_gram_kernel(const ChunkArgs a) {
     uint4* const tp = reinterpret_cast<uint4*>(qs);
     const int c = blockIdx.x, g = blockIdx.y / a.parts, part = blockIdx.y % a.parts, b = blockIdx.z;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, gq = lane >> 2, tq = lane & 3;
+    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const int t0 = first_token(a, b) + c * DC, nt = min(DC, a.S - t0);
     if (nt <= 0) return;
     const int ld = 2 * a.kv_heads * a.dim + a.heads * a.vdim;
@@ -586,10 +588,6 @@ __global__ void __launch_bounds__(64 * DW, 1) delta_walk_kernel(const ChunkArgs 
     const uint32_t full = (uint32_t)__cvta_generic_to_shared(up_sh + 2 * 2 * 3 * 64), ready = full + 8 * STAGES, empty = ready + 8 * STAGES;
     const int col0 = blockIdx.x * DV, h = blockIdx.y, b = blockIdx.z, g = h / (a.heads / a.kv_heads);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, gq = lane >> 2, tq = lane & 3;
-    const int first = first_token(a, b), n = (a.S - first + DC - 1) / DC;
-    const int cols = min(DV, a.vdim - col0);
-    const long o_ld = (long)a.heads * a.vdim;
-    float* const ob = a.o + (((long)b * a.seq) * a.heads + h) * a.vdim + col0;
     if (threadIdx.x == 0) {
 #pragma unroll
         for (int i = 0; i < STAGES; ++i) {
@@ -599,6 +597,12 @@ __global__ void __launch_bounds__(64 * DW, 1) delta_walk_kernel(const ChunkArgs 
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    const int first = first_token(a, b), n = (a.S - first + DC - 1) / DC;
+    const int cols = min(DV, a.vdim - col0);
+    const long o_ld = (long)a.heads * a.vdim;
+    float* const ob = a.o + (((long)b * a.seq) * a.heads + h) * a.vdim + col0;
     __syncthreads();
 
     if (warp >= DW) {                                   // outputs: C_t Q M0 + A U, eight tokens per warp
@@ -899,8 +903,18 @@ template <typename T, int D> int launch_chunks(ChunkArgs a, cudaStream_t st) {
     }
     a.parts = 1;                                        // until every SM has a block (a part forms the Gram matrices again, a fifth of a head's work)
     while (a.parts * 2 <= a.heads / a.kv_heads && (long)a.n_chunks * a.kv_heads * a.B * a.parts < 148 && a.kv_heads * a.parts * 2 <= 65535) a.parts *= 2;
-    delta_gram_kernel<T, D><<<dim3(a.n_chunks, a.kv_heads * a.parts, a.B), DT, gram, st>>>(a);
-    delta_walk_kernel<T, D><<<dim3((a.vdim + DV - 1) / DV, a.heads, a.B), 64 * DW, walk, st>>>(a);
+    // Both start while the kernel in front drains and wait for its end before they touch memory; in a captured stream the graph's edges stay plain
+    cudaStreamCaptureStatus state = cudaStreamCaptureStatusNone;
+    const bool overlap = cudaStreamIsCapturing(st, &state) == cudaSuccess && state == cudaStreamCaptureStatusNone;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.stream = st; cfg.attrs = at; cfg.numAttrs = overlap ? 1 : 0;
+    cfg.gridDim = dim3(a.n_chunks, a.kv_heads * a.parts, a.B); cfg.blockDim = dim3(DT); cfg.dynamicSmemBytes = gram;
+    cudaLaunchKernelEx(&cfg, delta_gram_kernel<T, D>, (const ChunkArgs)a);
+    cfg.gridDim = dim3((a.vdim + DV - 1) / DV, a.heads, a.B); cfg.blockDim = dim3(64 * DW); cfg.dynamicSmemBytes = walk;
+    cudaLaunchKernelEx(&cfg, delta_walk_kernel<T, D>, (const ChunkArgs)a);
     return mixers_status();
 }
 
