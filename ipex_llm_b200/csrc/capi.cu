@@ -204,7 +204,7 @@ static bool use_gemm(int qtype, int64_t n_rows, int64_t k, int64_t m, int x_dtyp
     return x_dtype != DT_F32 && m > max_m && gemm_tc_supported(qtype, n_rows, k);
 }
 
-// fp32 rows beyond one pass of the GEMV, fp32 results: the same arithmetic on pairs of SMs (gemm_exact.cu), where code x scale is the value.
+// fp32 rows beyond one pass of the GEMV, fp32 results: the same arithmetic on pairs of SMs (gemm_exact.cu), where the value is code x scale or that plus a minimum.
 // The line lies at the GEMV's 32 rows: at 33 rows, two passes against one launch, 33.8 -> 17.4 us at 4096 x 4096, 18.2 -> 12.4 at 1024 x 1024
 static bool use_exact(int qtype, int64_t n_rows, int64_t k, int64_t m, int x_dtype, int y_dtype) {
     return x_dtype == DT_F32 && y_dtype == DT_F32 && m > kGemvMaxM && gemm_exact_supported(qtype, n_rows, k, m);
@@ -226,7 +226,7 @@ size_t lowbit_matmul_workspace_size(int64_t n_rows, int64_t k, int64_t m, int x_
     if (use_gemm(B200_QT_SYM_INT4, n_rows, k, m, x_dtype)) return gemm_tc_workspace_size(n_rows, k, m);
     const size_t gemv = gemv_workspace_size(n_rows, k, m, x_dtype);
     if (!use_exact(B200_QT_SYM_INT4, n_rows, k, m, x_dtype, DT_F32)) return gemv;
-    const size_t exact = gemm_exact_workspace_size(n_rows, k, m);          // the size is asked without the format: enough for either
+    const size_t exact = gemm_exact_workspace_size(B200_QT_ASYM_INT4, n_rows, k, m);     // the size is asked without the format: enough for each
     return exact > gemv ? exact : gemv;
 }
 
@@ -239,7 +239,7 @@ static int matmul_dispatch(const void* d_w, int qtype, int64_t n_rows, int64_t k
     if (use_gemm(qtype, n_rows, k, m, x_dtype))
         return gemm_tc_launch(d_w, qtype, n_rows, k, d_x, x_dtype, m, d_y, y_dtype, d_bias, accumulate, workspace, workspace_bytes, st);
     // a caller's scratch of the GEMV's size still runs its chunks of 32 rows
-    if (use_exact(qtype, n_rows, k, m, x_dtype, y_dtype) && workspace && workspace_bytes >= gemm_exact_workspace_size(n_rows, k, m) &&
+    if (use_exact(qtype, n_rows, k, m, x_dtype, y_dtype) && workspace && workspace_bytes >= gemm_exact_workspace_size(qtype, n_rows, k, m) &&
         !(((uintptr_t)d_x | (uintptr_t)d_w | (uintptr_t)workspace) & 15))
         return gemm_exact_launch(d_w, qtype, n_rows, k, d_x, m, d_y, d_bias, accumulate, workspace, workspace_bytes, st);
     return gemv_launch(d_w, qtype, n_rows, k, d_x, x_dtype, m, d_y, y_dtype, d_bias, accumulate, workspace, workspace_bytes, st);

@@ -4,8 +4,8 @@
 //
 // The arithmetic is the exact GEMV's (gemv_kernel.cuh): the CODES (4-bit offsets, e4m3 / e5m2 / e3m2 values) are exact in bf16, an
 // activation is the sum of three bf16 planes, so every product is exact in 32 bits; a 64-element block's sum leaves the tensor cores
-// after 12 steps and is multiplied by the block's scale and added in 32-bit floats.  Formats whose value is not code x scale (asym_int4's
-// minima, nf4's table) stay on the GEMV.
+// after 12 steps and is multiplied by the block's scale and added in 32-bit floats.  asym_int4's minima multiply the
+// activations' sums per block, which split3_kernel leaves; nf4, whose value is not a code times a scale, stays on the GEMV.
 //
 // Layout of the work as in gemm_pair.cu: a cluster of two CTAs computes 256 features x up to 128 tokens with tcgen05.mma.cta_group::2,
 // codes expanded to bf16 = A operand, the token planes = B, each CTA staging half of the tokens (boxes of 32 rows, three planes per
@@ -19,7 +19,8 @@
 // three times as much TMEM: 600 clocks a k-block, slower than either.  The kernel starts while split3_kernel runs and waits only in
 // front of the planes.  sym_int4, GEMV passes of 32 rows -> 64-token tiles -> now: 4096 x 4096 at 33 rows 33.8 -> 17.7 -> 15.6 us, 64 rows
 // 50.4 -> 18.1 -> 15.6, 200 rows 161 -> 38.0 -> 26.8, 512 rows 400 -> 69.9 -> 40.4; 11008 x 4096 at 512 rows 938 -> 160 -> 105; 1024 x 1024
-// at 33 rows 18.2 -> 12.5 -> 10.9.  Error against 64 bits, relative to the result's norm: the GEMV 4.8e-7, here 1.2e-7 to 1.5e-7
+// at 33 rows 18.2 -> 12.5 -> 10.9.  asym_int4 (passes -> now): 4096 x 4096 at 33 rows 46.1 -> 25.6, 200 rows 198 -> 44.0, 1000 rows 915 ->
+// 128, 31232 x 9280 at 506 rows 3812 -> 804; the minima's loads straight from L2, two blocks under way, took 1422 there.  Error against 64 bits, relative to the result's norm: the GEMV 4.8e-7, here 1.2e-7 to 1.5e-7
 // (sym_int4, 4096 x 4096).  At 512 rows the MMAs' twelve steps are 3/4 of the time; below 100 rows it is the three launches' ends.
 #include "tc_pair.cuh"
 
@@ -36,7 +37,7 @@ template <int QT, int TOK> struct ExShape {
     static constexpr int kGroup = PackedBlock<QT>::kGroup, kPacked = 2 * kGroup;
     static constexpr int kA = TOK == 64 ? 3 : 4, kP = 6, kX = TOK == 64 ? 6 : 4;
     static constexpr int kXPlane = TOK * 64, kXSlot = 3 * kXPlane;     // half of the tokens' rows of 128 bytes
-    static constexpr int kTotal = 1024 + 512 + kA * kTileBytesAB + kP * kPacked + kX * kXSlot;
+    static constexpr int kTotal = 1024 + 512 + kA * kTileBytesAB + kP * kPacked + kX * kXSlot + (Expand<QT>::kHasMin ? 8 * TOK * 4 : 0);
     static_assert(kTotal <= 232448, "shared memory");
     static_assert(kP % kGroups == 0 && (3 * kX + 2 * kP + 2 * kA + 2 * kBufs + 1) * 8 + 8 <= 512, "barrier region");
 };
@@ -47,6 +48,7 @@ struct ExactArgs {
     int M, tt, n_fp, ksplit;
     float* y; const float* bias; int accumulate;
     float* part;
+    const float* sums; int sum_rows;        // minima: [k-block][sum_rows] the activations' sums, tokens padded to whole 16
     Waits waits;
 };
 
@@ -58,7 +60,7 @@ exact_kernel(const __grid_constant__ CUtensorMap xmap, const ExactArgs A) {
     constexpr int KX = SM::kX, KP = SM::kP, KA = SM::kA, GROUPS = SM::kGroups, BUFS = SM::kBufs;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    const uint32_t xring = base, aring = base + KX * SM::kXSlot, pring = aring + KA * kTileBytesAB, bars = pring + KP * SM::kPacked;
+    const uint32_t xring = base, aring = base + KX * SM::kXSlot, pring = aring + KA * kTileBytesAB, bars = base + SM::kTotal - 1536;
     auto x_full = [&](int s) { return bars + s * 8; };
     auto x_empty = [&](int s) { return bars + (KX + s) * 8; };
     auto xp_full = [&](int s) { return bars + (2 * KX + s) * 8; };                     // CTA 0: the other half has landed
@@ -238,18 +240,64 @@ exact_kernel(const __grid_constant__ CUtensorMap xmap, const ExactArgs A) {
             float acc[TOKS];
 #pragma unroll
             for (int i = 0; i < TOKS; i++) acc[i] = 0.0f;
-            float next[4];
+            // value = (code - 8) d + (min + 8 d) with minima: the second part times the block's activations' sums, in the time that a wait for
+            // the block's MMAs takes; a block's scale and minimum are kept as they are stored
+            if (E::kHasMin && unit == (int)(blockIdx.x >> 1)) asm volatile("griddepcontrol.wait;" ::: "memory");
+            auto block = [&](int kb) {
+                __half2 h = __half2half2(__ushort_as_half(0));
+                if (kb < U.kb1) {
+                    h.x = sp[(int64_t)kb * 64];
+                    if constexpr (E::kHasMin) h.y = sp[(int64_t)kb * 64 + (A.G.off_m - A.G.off_s) / 2];
+                }
+                return h;
+            };
+            // the warp's tokens' sums of a block, loaded one block ahead and handed round through shared memory
+            const uint32_t sums_at = pring + KP * SM::kPacked + (uint32_t)(warp - SM::kEpi0) * (2 * TOKS * 4);
+            auto sums = [&](int kb) {
+                constexpr int kEach = TOKS / 32;
+                float2 v = make_float2(0.0f, 0.0f);
+                if (E::kHasMin && kb < U.kb1 && t0 + kEach * lane < U.rows) {
+                    const float* const at = A.sums + (int64_t)kb * A.sum_rows + U.m0 + t0 + kEach * lane;
+                    if constexpr (kEach == 2) v = *reinterpret_cast<const float2*>(at);
+                    else v.x = *at;
+                }
+                return v;
+            };
+            float2 ahead = sums(U.kb0);
+            __syncwarp();                                        // the last unit's reads lie before the first writes
+            constexpr int kAhead = E::kHasMin ? 2 : 4;           // blocks' scales loaded ahead; with sums the registers are full
+            __half2 next[kAhead];
 #pragma unroll
-            for (int i = 0; i < 4; i++) next[i] = U.kb0 + i < U.kb1 ? __half2float(sp[(int64_t)(U.kb0 + i) * 64]) : 0.0f;
-            for (int kb = U.kb0; kb < U.kb1; kb += 4) {
-                float d[4];
+            for (int i = 0; i < kAhead; i++) next[i] = block(U.kb0 + i);
+            for (int kb = U.kb0; kb < U.kb1; kb += kAhead) {
+                __half2 now[kAhead];
 #pragma unroll
-                for (int i = 0; i < 4; i++) d[i] = next[i];
+                for (int i = 0; i < kAhead; i++) now[i] = next[i];
 #pragma unroll
-                for (int i = 0; i < 4; i++) next[i] = kb + 4 + i < U.kb1 ? __half2float(sp[(int64_t)(kb + 4 + i) * 64]) : 0.0f;
+                for (int i = 0; i < kAhead; i++) next[i] = block(kb + kAhead + i);
 #pragma unroll
-                for (int i = 0; i < 4; i++) {
+                for (int i = 0; i < kAhead; i++) {
                     if (kb + i >= U.kb1) break;
+                    const float d = __low2float(now[i]);
+                    if constexpr (E::kHasMin) {
+                        const float least = fmaf(8.0f, d, __high2float(now[i]));
+                        const uint32_t held = sums_at + (uint32_t)((kb + i) & 1) * (TOKS * 4);
+                        if constexpr (TOKS == 64) asm volatile("st.shared.v2.f32 [%0], {%1, %2};" ::"r"(held + lane * 8), "f"(ahead.x), "f"(ahead.y) : "memory");
+                        else asm volatile("st.shared.f32 [%0], %1;" ::"r"(held + lane * 4), "f"(ahead.x) : "memory");
+                        __syncwarp();                            // the one of the next block lies between these reads and the next writes here
+                        ahead = sums(kb + i + 1);
+#pragma unroll
+                        for (int c = 0; c < TOKS; c += 16) {
+                            if (t0 + c >= U.rows) break;
+#pragma unroll
+                            for (int j = 0; j < 16; j += 4) {
+                                float4 v;
+                                asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(held + (c + j) * 4) : "memory");
+                                acc[c + j] = fmaf(least, v.x, acc[c + j]); acc[c + j + 1] = fmaf(least, v.y, acc[c + j + 1]);
+                                acc[c + j + 2] = fmaf(least, v.z, acc[c + j + 2]); acc[c + j + 3] = fmaf(least, v.w, acc[c + j + 3]);
+                            }
+                        }
+                    }
                     if (!mbar_wait_lim(t_full(tb), (uint32_t)(rt & 1), A.waits)) goto done;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
@@ -258,7 +306,7 @@ exact_kernel(const __grid_constant__ CUtensorMap xmap, const ExactArgs A) {
                         float v[16];
                         tmem_ld16(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(tb * TOK + t0 + c), v);
 #pragma unroll
-                        for (int j = 0; j < 16; j++) acc[c + j] = fmaf(d[i], v[j], acc[c + j]);
+                        for (int j = 0; j < 16; j++) acc[c + j] = fmaf(d, v[j], acc[c + j]);
                     }
                     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                     __syncwarp();
@@ -298,13 +346,20 @@ done:
     }
 }
 
-// fp32 activations -> three bf16 planes whose sum reproduces them to 2^-24, four elements a thread
-__global__ void __launch_bounds__(256) split3_kernel(const float4* __restrict__ x, uint2* __restrict__ out, int64_t n4) {
+// fp32 activations -> three bf16 planes whose sum reproduces them to 2^-24, four elements a thread; `sums`: those of 64 elements, for minima
+__global__ void __launch_bounds__(256) split3_kernel(const float4* __restrict__ x, uint2* __restrict__ out, int64_t n4, float* __restrict__ sums, int k4, int sum_rows) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;");     // not before the wait: the matmul reads its weights ahead of its own
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n4; i += (int64_t)gridDim.x * blockDim.x) {
         const float4 q = x[i];
         float r[4] = {q.x, q.y, q.z, q.w};
+        if (sums) {                                        // 16 lanes hold a block of 64, and all of them are here
+            float v = (q.x + q.y) + (q.z + q.w);
+#pragma unroll
+            for (int d = 1; d < 16; d <<= 1) v += __shfl_xor_sync(0xffffu << (threadIdx.x & 16), v, d);
+            const int64_t token = i / k4;
+            if ((threadIdx.x & 15) == 0) sums[((i - token * k4) >> 4) * sum_rows + token] = v;
+        }
 #pragma unroll
         for (int p = 0; p < 3; p++) {
             uint32_t b[4];
@@ -377,26 +432,30 @@ static ExactPlan exact_plan(int64_t n_rows, int64_t nb, int64_t m) {
     return best;
 }
 static size_t exact_planes_bytes(int64_t k, int64_t m) { return ((size_t)3 * m * k * 2 + 255) / 256 * 256; }
+static int64_t exact_sum_rows(int64_t m) { return (m + 15) / 16 * 16; }
+static size_t exact_sums_bytes(int64_t k, int64_t m) { return ((size_t)(k / 64) * exact_sum_rows(m) * 4 + 255) / 256 * 256; }
 }  // namespace gemmtc
 
 bool gemm_exact_supported(int qt, int64_t n_rows, int64_t k, int64_t m) {
     qt = canon_qtype(qt);
-    return (qt == QT_SYM_INT4 || qt == QT_FP8_E4M3 || qt == QT_FP8_E5M2 || qt == QT_FP6) && gemm_tc_supported(qt, n_rows, k) && 3 * m < 0x7fffffff;
+    return (qt == QT_SYM_INT4 || qt == QT_ASYM_INT4 || qt == QT_FP8_E4M3 || qt == QT_FP8_E5M2 || qt == QT_FP6) && gemm_tc_supported(qt, n_rows, k) && 3 * m < 0x7fffffff;
 }
-size_t gemm_exact_workspace_size(int64_t n_rows, int64_t k, int64_t m) {
+size_t gemm_exact_workspace_size(int qt, int64_t n_rows, int64_t k, int64_t m) {
     using namespace gemmtc;
     const ExactPlan p = exact_plan(n_rows, k / 64, m);
-    return exact_planes_bytes(k, m) + (p.ks > 1 ? (size_t)p.ks * m * n_rows * sizeof(float) : 0);
+    return exact_planes_bytes(k, m) + (canon_qtype(qt) == QT_ASYM_INT4 ? exact_sums_bytes(k, m) : 0) +
+           (p.ks > 1 ? (size_t)p.ks * m * n_rows * sizeof(float) : 0);
 }
 int gemm_exact_launch(const void* w, int qt, int64_t n_rows, int64_t k, const void* x, int64_t m, void* y, const void* bias, int accumulate,
                       void* workspace, size_t workspace_bytes, cudaStream_t st) {
     using namespace gemmtc;
     qt = canon_qtype(qt);
     if (!gemm_exact_supported(qt, n_rows, k, m) || (((uintptr_t)x | (uintptr_t)w | (uintptr_t)workspace) & 15)) return LB_ERR_ARG;
-    if (!workspace || workspace_bytes < gemm_exact_workspace_size(n_rows, k, m)) return LB_ERR_WORKSPACE;
+    if (!workspace || workspace_bytes < gemm_exact_workspace_size(qt, n_rows, k, m)) return LB_ERR_WORKSPACE;
+    float* const sums = qt == QT_ASYM_INT4 ? (float*)((char*)workspace + exact_planes_bytes(k, m)) : nullptr;
     const int64_t n4 = m * k / 4;                                       // k is a multiple of 64
     int sg = (int)((n4 + 255) / 256); if (sg > sm_count() * 8) sg = sm_count() * 8;
-    launch_behind(split3_kernel, dim3((unsigned)sg), 256, 0, st, launch_overlaps(st), (const float4*)x, (uint2*)workspace, n4);
+    launch_behind(split3_kernel, dim3((unsigned)sg), 256, 0, st, launch_overlaps(st), (const float4*)x, (uint2*)workspace, n4, sums, (int)(k / 4), (int)exact_sum_rows(m));
     note_launch();
     CUtensorMap map;
     if (const int rc = encode_rows(&map, workspace, true, 3 * m, k, 32)) return rc;
@@ -404,11 +463,13 @@ int gemm_exact_launch(const void* w, int qt, int64_t n_rows, int64_t k, const vo
     ExactArgs A = {};
     if (const int rc = make_waits(&A.waits, kWaitCycles)) return rc;
     A.w = (const uint8_t*)w; A.G = make_geom(n_rows, k, qt); A.M = (int)m; A.tt = p.tt; A.n_fp = (int)((n_rows / 128 + 1) / 2); A.ksplit = p.ks;
-    A.y = (float*)y; A.bias = (const float*)bias; A.accumulate = accumulate; A.part = (float*)((char*)workspace + exact_planes_bytes(k, m));
+    A.y = (float*)y; A.bias = (const float*)bias; A.accumulate = accumulate; A.part = (float*)((char*)workspace + exact_planes_bytes(k, m) + (sums ? exact_sums_bytes(k, m) : 0));
+    A.sums = sums; A.sum_rows = (int)exact_sum_rows(m);
     const int64_t units = (int64_t)A.n_fp * ((m + p.tt - 1) / p.tt) * p.ks;
     int rc = LB_ERR_ARG;
     switch (qt) {
         case QT_SYM_INT4: rc = exact_launch_one<QT_SYM_INT4>(map, A, units, st); break;
+        case QT_ASYM_INT4: rc = exact_launch_one<QT_ASYM_INT4>(map, A, units, st); break;
         case QT_FP8_E4M3: rc = exact_launch_one<QT_FP8_E4M3>(map, A, units, st); break;
         case QT_FP8_E5M2: rc = exact_launch_one<QT_FP8_E5M2>(map, A, units, st); break;
         case QT_FP6:      rc = exact_launch_one<QT_FP6>(map, A, units, st); break;

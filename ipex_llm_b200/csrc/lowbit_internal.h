@@ -130,7 +130,7 @@ int gemm_tc_experts_launch(const unsigned long long* tab, const unsigned long lo
 
 // gemm_exact.cu (the fp32 prompt matmul: codes and activation planes exact on the tensor cores)
 bool gemm_exact_supported(int qt, int64_t n_rows, int64_t k, int64_t m);
-size_t gemm_exact_workspace_size(int64_t n_rows, int64_t k, int64_t m);
+size_t gemm_exact_workspace_size(int qt, int64_t n_rows, int64_t k, int64_t m);
 int gemm_exact_launch(const void* w, int qt, int64_t n_rows, int64_t k, const void* x, int64_t m, void* y, const void* bias, int accumulate,
                       void* workspace, size_t workspace_bytes, cudaStream_t st);
 

@@ -188,6 +188,25 @@ def test_prompt_matmul_fp32_tiles(lbl, native_lib, cuda_device, qtype, m, n, k):
     test_prompt_matmul_fp32_keeps_its_contract(lbl, native_lib, cuda_device, qtype, m, n, k)
 
 
+@pytest.mark.parametrize("m,n,k", [(33, 9600, 192), (48, 19200, 384), (65, 128, 64), (97, 4736, 1088), (129, 9600, 256), (385, 4736, 448), (512, 9728, 640)])
+def test_prompt_matmul_fp32_with_minima(lbl, native_lib, cuda_device, m, n, k):
+    """the activations' sums beside the codes: both tiles' remainders, more than one unit per cluster, K ranges of an odd number of blocks;
+    activations away from zero, where the minima are most of the result, to the same bound; a workspace without room for the sums"""
+    test_prompt_matmul_fp32_keeps_its_contract(lbl, native_lib, cuda_device, "asym_int4", m, n, k)
+    [(w, wd)], qt = weights(lbl, cuda_device, m + n, n, k, "asym_int4")
+    x = acts(cuda_device, k, m, k, torch.float32) + 3
+    want, mag = x.double() @ wd.T, x.double().abs() @ wd.abs().T
+    size = native_lib.lowbit_matmul_workspace_size(n, k, m, native_lib.DT_F32)
+    outs = []
+    for room in (size, 256 * ((3 * m * k * 2 + 255) // 256)):                  # the second holds the planes alone
+        ws, y = torch.full((room,), 255, dtype=torch.uint8, device=cuda_device), torch.empty(m, n, device=cuda_device)
+        native_lib.lowbit_matmul_cuda(w.data_ptr(), qt, n, k, x.data_ptr(), native_lib.DT_F32, m, y.data_ptr(), native_lib.DT_F32, None, False,
+                                      ws.data_ptr(), ws.numel(), torch.cuda.current_stream().cuda_stream)
+        outs.append((y.double() - want).abs())
+        assert bool((outs[-1] <= 2e-6 * mag).all())
+    assert float(outs[0].norm()) <= 1.05 * float(outs[1].norm())
+
+
 @pytest.mark.parametrize("qtype,dtype,m,n,k", [("sym_int4", torch.float16, 200, 4096, 4096), ("sym_int4", torch.float16, 500, 4096, 11008),
                                                ("sym_int4", torch.float16, 512, 4096, 11008), ("fp8_e4m3", torch.float16, 256, 4096, 4096),
                                                ("sym_int4", torch.bfloat16, 1500, 1024, 4096), ("nf4", torch.bfloat16, 512, 4096, 4096)])
