@@ -204,7 +204,7 @@ static bool use_gemm(int qtype, int64_t n_rows, int64_t k, int64_t m, int x_dtyp
     return x_dtype != DT_F32 && m > max_m && gemm_tc_supported(qtype, n_rows, k);
 }
 
-// fp32 rows beyond one pass of the GEMV, fp32 results: the same arithmetic on pairs of SMs (gemm_exact.cu), where the value is code x scale or that plus a minimum.
+// fp32 rows beyond one pass of the GEMV, fp32 results: the same arithmetic on pairs of SMs (gemm_exact.cu), in every format.
 // The line lies at the GEMV's 32 rows: at 33 rows, two passes against one launch, 33.8 -> 17.4 us at 4096 x 4096, 18.2 -> 12.4 at 1024 x 1024
 static bool use_exact(int qtype, int64_t n_rows, int64_t k, int64_t m, int x_dtype, int y_dtype) {
     return x_dtype == DT_F32 && y_dtype == DT_F32 && m > kGemvMaxM && gemm_exact_supported(qtype, n_rows, k, m);

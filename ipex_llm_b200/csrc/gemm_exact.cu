@@ -5,7 +5,7 @@
 // The arithmetic is the exact GEMV's (gemv_kernel.cuh): the CODES (4-bit offsets, e4m3 / e5m2 / e3m2 values) are exact in bf16, an
 // activation is the sum of three bf16 planes, so every product is exact in 32 bits; a 64-element block's sum leaves the tensor cores
 // after 12 steps and is multiplied by the block's scale and added in 32-bit floats.  asym_int4's minima multiply the
-// activations' sums per block, which split3_kernel leaves; nf4, whose value is not a code times a scale, stays on the GEMV.
+// activations' sums per block, which split3_kernel leaves; nf4's table is the sum of two bf16 planes (2^-17), as there.
 //
 // Layout of the work as in gemm_pair.cu: a cluster of two CTAs computes 256 features x up to 128 tokens with tcgen05.mma.cta_group::2,
 // codes expanded to bf16 = A operand, the token planes = B, each CTA staging half of the tokens (boxes of 32 rows, three planes per
@@ -20,7 +20,8 @@
 // front of the planes.  sym_int4, GEMV passes of 32 rows -> 64-token tiles -> now: 4096 x 4096 at 33 rows 33.8 -> 17.7 -> 15.6 us, 64 rows
 // 50.4 -> 18.1 -> 15.6, 200 rows 161 -> 38.0 -> 26.8, 512 rows 400 -> 69.9 -> 40.4; 11008 x 4096 at 512 rows 938 -> 160 -> 105; 1024 x 1024
 // at 33 rows 18.2 -> 12.5 -> 10.9.  asym_int4 (passes -> now): 4096 x 4096 at 33 rows 46.1 -> 25.6, 200 rows 198 -> 44.0, 1000 rows 915 ->
-// 128, 31232 x 9280 at 506 rows 3812 -> 804; the minima's loads straight from L2, two blocks under way, took 1422 there.  Error against 64 bits, relative to the result's norm: the GEMV 4.8e-7, here 1.2e-7 to 1.5e-7
+// 128, 31232 x 9280 at 506 rows 3812 -> 804; the minima's loads straight from L2, two blocks under way, took 1422 there.
+// nf4: 56.4 -> 29.7, 245 -> 48.1, 1166 -> 142, 5013 -> 1084.  Error against 64 bits, relative to the result's norm: the GEMV 4.8e-7, here 1.2e-7 to 1.5e-7
 // (sym_int4, 4096 x 4096).  At 512 rows the MMAs' twelve steps are 3/4 of the time; below 100 rows it is the three launches' ends.
 #include "tc_pair.cuh"
 
@@ -29,10 +30,48 @@ namespace gemmtc {
 
 constexpr int kExTok = 128, kExDeq0 = 4;     // most tokens of a tile; first expanding warp
 
+// nf4's table is held as two bf16 planes, the GEMV's: a k-block is two A tiles and 24 MMA steps into one TMEM buffer, on the same packed
+// weights and token planes.  A tile's values come out of registers, four codes to a byte permutation of the table's low and high halves (the
+// shared table that the 16-bit kernel reads costs 32 KB a plane, which the token planes' ring needs).
+template <int QT> struct ExWeights {
+    static constexpr int kPlanes = 1;
+    struct Table {};
+    __device__ static __forceinline__ void table(bool, Table&) {}
+};
+template <> struct ExWeights<QT_NF4> {
+    static constexpr int kPlanes = 2;
+    struct Table { uint32_t lo[4], hi[4]; };                           // low and high bytes of 16 bf16 values
+    __device__ static __forceinline__ void table(bool rest, Table& T) {
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            T.lo[i] = T.hi[i] = 0;
+#pragma unroll
+            for (int j = 0; j < 4; j++) {
+                const float v = kNF4Table[4 * i + j];
+                const __nv_bfloat16 h = __float2bfloat16_rn(v);
+                const uint32_t b = __bfloat16_as_ushort(rest ? __float2bfloat16_rn(v - __bfloat162float(h)) : h);
+                T.lo[i] |= (b & 0xffu) << (8 * j); T.hi[i] |= (b >> 8) << (8 * j);
+            }
+        }
+    }
+    // byte b of the lane's word is the code pair of out[b]
+    __device__ static __forceinline__ void expand(const Table& T, uint32_t w, uint32_t (&out)[4]) {
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const uint32_t c = w >> (16 * h), at = c & 0x7777u, upper = __byte_perm(0xff00u, 0u, (c >> 3) & 0x1111u);
+            const uint32_t lo = (__byte_perm(T.lo[0], T.lo[1], at) & ~upper) | (__byte_perm(T.lo[2], T.lo[3], at) & upper);
+            const uint32_t hi = (__byte_perm(T.hi[0], T.hi[1], at) & ~upper) | (__byte_perm(T.hi[2], T.hi[3], at) & upper);
+            out[2 * h] = __byte_perm(lo, hi, 0x5140u);
+            out[2 * h + 1] = __byte_perm(lo, hi, 0x7362u);
+        }
+    }
+};
+
 // TOK: 64 tokens or 128.  A thread of the epilogue keeps half of them, so the larger tile leaves registers for two expansion groups only;
 // its MMAs take that long.
 template <int QT, int TOK> struct ExShape {
     static constexpr int kGroups = TOK == 64 ? 3 : 2, kEpi0 = kExDeq0 + 4 * kGroups, kThreads = 32 * (kEpi0 + 8);
+    static constexpr int kSteps = ExWeights<QT>::kPlanes;              // A tiles of a k-block
     static constexpr int kBufs = 512 / TOK;                            // TMEM: one for every k-block in flight
     static constexpr int kGroup = PackedBlock<QT>::kGroup, kPacked = 2 * kGroup;
     static constexpr int kA = TOK == 64 ? 3 : 4, kP = 6, kX = TOK == 64 ? 6 : 4;
@@ -57,7 +96,7 @@ __global__ void __launch_bounds__(ExShape<QT, TOK>::kThreads, 1)
 exact_kernel(const __grid_constant__ CUtensorMap xmap, const ExactArgs A) {
     using E = Expand<QT>;
     using SM = ExShape<QT, TOK>;
-    constexpr int KX = SM::kX, KP = SM::kP, KA = SM::kA, GROUPS = SM::kGroups, BUFS = SM::kBufs;
+    constexpr int KX = SM::kX, KP = SM::kP, KA = SM::kA, GROUPS = SM::kGroups, BUFS = SM::kBufs, STEPS = SM::kSteps;
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t xring = base, aring = base + KX * SM::kXSlot, pring = aring + KA * kTileBytesAB, bars = base + SM::kTotal - 1536;
@@ -76,7 +115,7 @@ exact_kernel(const __grid_constant__ CUtensorMap xmap, const ExactArgs A) {
     const int nb = (int)A.G.nb;
     if (threadIdx.x == 0) {
         for (int s = 0; s < KX; s++) { mbar_init(x_full(s), 1); mbar_init(x_empty(s), 1); mbar_init(xp_full(s), 1); }
-        for (int s = 0; s < KP; s++) { mbar_init(p_full(s), 1); mbar_init(p_empty(s), 4); }
+        for (int s = 0; s < KP; s++) { mbar_init(p_full(s), 1); mbar_init(p_empty(s), 4 * STEPS); }
         for (int s = 0; s < KA; s++) { mbar_init(a_full(s), 8); mbar_init(a_empty(s), 1); }
         for (int b = 0; b < BUFS; b++) { mbar_init(t_full(b), 1); mbar_init(t_empty(b), 16); }
         mbar_init(drained, 1);
@@ -133,7 +172,7 @@ exact_kernel(const __grid_constant__ CUtensorMap xmap, const ExactArgs A) {
             for (int unit = blockIdx.x >> 1; unit < n_units; unit += stride) {
                 decode(unit, U);
                 const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | (((uint32_t)U.n_tok >> 3) << 17) | ((256u >> 4) << 24);
-                for (int kb = U.kb0; kb < U.kb1; kb++) {
+                for (int kb = STEPS * U.kb0; kb < STEPS * U.kb1; kb++) {
                     if (!mbar_wait4_lim(ready, t_empty(tb), (uint32_t)((rt & 1) ^ 1), x_full(sx), (uint32_t)(rx & 1), xp_full(sx), (uint32_t)(rx & 1), a_full(sa),
                                         (uint32_t)(ra & 1), A.waits)) goto done;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -143,13 +182,15 @@ exact_kernel(const __grid_constant__ CUtensorMap xmap, const ExactArgs A) {
 #pragma unroll
                         for (int k4 = 0; k4 < 4; k4++)
                             umma2_f16_w(tmem_base + tb * TOK, ad + (uint64_t)((k4 * 32) >> 4), xd + (uint64_t)((p * SM::kXPlane + k4 * 32) >> 4), idesc,
-                                        (p < 2 || k4 > 0) ? 1u : 0u, leader);
+                                        (p < 2 || k4 > 0 || kb % STEPS) ? 1u : 0u, leader);
                     umma2_commit_w(a_empty(sa), leader);
-                    umma2_commit_w(x_empty(sx), leader);
-                    umma2_commit_w(t_full(tb), leader);
-                    if (++sx == KX) { sx = 0; rx++; }
                     if (++sa == KA) { sa = 0; ra++; }
-                    if (++tb == BUFS) { tb = 0; rt++; }
+                    if (kb % STEPS == STEPS - 1) {
+                        umma2_commit_w(x_empty(sx), leader);
+                        umma2_commit_w(t_full(tb), leader);
+                        if (++sx == KX) { sx = 0; rx++; }
+                        if (++tb == BUFS) { tb = 0; rt++; }
+                    }
                     // asked here, answered while the MMAs above are being issued
                     ready = mbar_test4(t_empty(tb), (uint32_t)((rt & 1) ^ 1), x_full(sx), (uint32_t)(rx & 1), xp_full(sx), (uint32_t)(rx & 1), a_full(sa), (uint32_t)(ra & 1));
                 }
@@ -187,14 +228,17 @@ exact_kernel(const __grid_constant__ CUtensorMap xmap, const ExactArgs A) {
     } else if (warp >= kExDeq0 && warp < SM::kEpi0) {
         // ================= expansion: group (warp - 4) / 4 takes every second (third) k-block =================
         const int grp = (warp - kExDeq0) >> 2, dw = (warp - kExDeq0) & 3, g = lane >> 2, t = lane & 3;
-        int end = 0, it = grp, sp = grp, rp = 0;
+        int end = 0, it = grp, sp = grp / STEPS, rp = 0;      // `it` counts A tiles, STEPS to a k-block: the rest of a table's values first
+        typename ExWeights<QT>::Table values, others;
+        ExWeights<QT>::table(grp % 2 == 0, values);
+        ExWeights<QT>::table(grp % 2 == 1, others);
         for (int unit = blockIdx.x >> 1; unit < n_units; unit += stride) {
             decode(unit, U);
-            end += U.kb1 - U.kb0;
-            for (; it < end; it += GROUPS, ((sp += GROUPS) >= KP ? (sp -= KP, rp++) : 0)) {
+            end += STEPS * (U.kb1 - U.kb0);
+            for (; it < end; it += GROUPS) {
                 const int sa = it % KA;
                 const uint32_t row0 = aring + sa * kTileBytesAB + 4 * dw * 1024 + g * 128;     // rows interleaved by 16 as in gemm_pair.cu
-                // the slot's earlier trip (k-block it - KP) was this group's own
+                // the slot's earlier trip (KP k-blocks before) was this group's own too
                 if (!mbar_wait_lim(p_full(sp), (uint32_t)(rp & 1), A.waits)) goto done;
                 typename E::Codes cw[2];
 #pragma unroll
@@ -205,7 +249,12 @@ exact_kernel(const __grid_constant__ CUtensorMap xmap, const ExactArgs A) {
 #pragma unroll
                     for (int k4 = 0; k4 < 4; k4++) {
                         uint32_t a[4];
-                        E::bf16(cw[gi], k4, a);
+                        if constexpr (STEPS == 2) {
+                            const uint32_t w = k4 == 0 ? cw[gi].q.x : k4 == 1 ? cw[gi].q.y : k4 == 2 ? cw[gi].q.z : cw[gi].q.w;
+                            ExWeights<QT>::expand(values, w, a);
+                        } else {
+                            E::bf16(cw[gi], k4, a);
+                        }
                         lo[gi][2 * k4] = a[0]; lo[gi][2 * k4 + 1] = a[2];
                         hi[gi][2 * k4] = a[1]; hi[gi][2 * k4 + 1] = a[3];
                     }
@@ -221,6 +270,12 @@ exact_kernel(const __grid_constant__ CUtensorMap xmap, const ExactArgs A) {
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 __syncwarp();
                 if (lane == 0) { mbar_arrive(p_empty(sp)); mbar_arrive_at(a_full(sa), 0); }      // behind the stores: the codes have been used
+                if (STEPS == 1) {
+                    if ((sp += GROUPS) >= KP) { sp -= KP; rp++; }
+                } else {
+                    sp = (it + GROUPS) / STEPS % KP; rp = (it + GROUPS) / STEPS / KP;
+                    if (GROUPS % 2) { const auto t = values; values = others; others = t; }
+                }
             }
         }
     } else if (warp >= SM::kEpi0) {
@@ -438,7 +493,7 @@ static size_t exact_sums_bytes(int64_t k, int64_t m) { return ((size_t)(k / 64) 
 
 bool gemm_exact_supported(int qt, int64_t n_rows, int64_t k, int64_t m) {
     qt = canon_qtype(qt);
-    return (qt == QT_SYM_INT4 || qt == QT_ASYM_INT4 || qt == QT_FP8_E4M3 || qt == QT_FP8_E5M2 || qt == QT_FP6) && gemm_tc_supported(qt, n_rows, k) && 3 * m < 0x7fffffff;
+    return (qt == QT_SYM_INT4 || qt == QT_ASYM_INT4 || qt == QT_NF4 || qt == QT_FP8_E4M3 || qt == QT_FP8_E5M2 || qt == QT_FP6) && gemm_tc_supported(qt, n_rows, k) && 3 * m < 0x7fffffff;
 }
 size_t gemm_exact_workspace_size(int qt, int64_t n_rows, int64_t k, int64_t m) {
     using namespace gemmtc;
@@ -470,6 +525,7 @@ int gemm_exact_launch(const void* w, int qt, int64_t n_rows, int64_t k, const vo
     switch (qt) {
         case QT_SYM_INT4: rc = exact_launch_one<QT_SYM_INT4>(map, A, units, st); break;
         case QT_ASYM_INT4: rc = exact_launch_one<QT_ASYM_INT4>(map, A, units, st); break;
+        case QT_NF4:      rc = exact_launch_one<QT_NF4>(map, A, units, st); break;
         case QT_FP8_E4M3: rc = exact_launch_one<QT_FP8_E4M3>(map, A, units, st); break;
         case QT_FP8_E5M2: rc = exact_launch_one<QT_FP8_E5M2>(map, A, units, st); break;
         case QT_FP6:      rc = exact_launch_one<QT_FP6>(map, A, units, st); break;

@@ -207,6 +207,17 @@ def test_prompt_matmul_fp32_with_minima(lbl, native_lib, cuda_device, m, n, k):
     assert float(outs[0].norm()) <= 1.05 * float(outs[1].norm())
 
 
+@pytest.mark.parametrize("m,n,k", [(33, 9600, 192), (48, 19200, 832), (64, 1024, 8192), (65, 128, 64), (129, 9600, 256), (385, 4736, 448), (512, 9728, 1088)])
+def test_prompt_matmul_fp32_through_the_table(lbl, native_lib, cuda_device, m, n, k):
+    """nf4's two tiles per k-block: both tiles' remainders, rings that go round with two and with three expansion groups, the same bits each time"""
+    test_prompt_matmul_fp32_keeps_its_contract(lbl, native_lib, cuda_device, "nf4", m, n, k)
+    [(w, _)], qt = weights(lbl, cuda_device, 3, n, k, "nf4")
+    x = acts(cuda_device, 4, m, k, torch.float32)
+    first = lbl.lowbit_matmul(x, w, (n, k), qt)
+    for _ in range(8):
+        assert torch.equal(lbl.lowbit_matmul(x, w, (n, k), qt), first)
+
+
 @pytest.mark.parametrize("qtype,dtype,m,n,k", [("sym_int4", torch.float16, 200, 4096, 4096), ("sym_int4", torch.float16, 500, 4096, 11008),
                                                ("sym_int4", torch.float16, 512, 4096, 11008), ("fp8_e4m3", torch.float16, 256, 4096, 4096),
                                                ("sym_int4", torch.bfloat16, 1500, 1024, 4096), ("nf4", torch.bfloat16, 512, 4096, 4096)])
