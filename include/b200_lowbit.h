@@ -297,8 +297,8 @@ size_t lowbit_matmul_workspace_size(int64_t n_rows, int64_t k, int64_t m, int x_
  * weights as the 128-row operand, beyond that the prefill GEMM (activations and expanded weights enter the MMA as
  * fp16 / bf16, fp32 accumulation: about 1e-3 * sum|x w|); both may use a second, reduction launch.
  * fp32 activations: kept to 2^-24 -- the fp32-in / fp32-out contract of ggml_compute_forward_mul_mat_q_fp32 -- by the
- * GEMV, and beyond 32 rows with fp32 results by the tensor cores on three bf16 planes (formats whose value is code x scale;
- * the others, other result types and a workspace of 32 rows' size keep to the GEMV, 32 rows at a time); cast to fp16 first to trade that precision for the GEMM,
+ * GEMV, and beyond 32 rows with fp32 results by the tensor cores on three bf16 planes (n_rows a multiple of 128;
+ * other shapes, other result types and a workspace of 32 rows' size keep to the GEMV, 32 rows at a time); cast to fp16 first to trade that precision for the GEMM,
  * as the reference's XPU path does (LBL:700-705). */
 int lowbit_matmul_cuda(const void* d_w, int qtype, int64_t n_rows, int64_t k,
                        const void* d_x, int x_dtype, int64_t m,
