@@ -115,6 +115,8 @@ template <typename T> __device__ __forceinline__ T load_now(const T* p, bool the
     }
 }
 __device__ __forceinline__ bool finite(float v) { return fabsf(v) < INFINITY; }
+// enters the products of planes: no infinity, no NaN, and no value whose first plane rounds to infinity (from 3.3962e38 on)
+__device__ __forceinline__ bool splits(float v) { return fabsf(v) <= 1e38f; }
 // one copy of the code (the kernel is run through once per block, and its length is time), two at a time
 __device__ __noinline__ double2 exp_64(double x, double y) { return make_double2(exp(x), exp(y)); }
 // the gates of one token, lane = token; in double: a decay's error counts as often as there are tokens behind it.
@@ -402,8 +404,8 @@ __global__ void __launch_bounds__(DT, 2) delta_gram_kernel(const ChunkArgs a) {
             for (int p = 0; p < 3; ++p) to[32 * p] = make_uint4(pl[0][p], pl[1][p], pl[2][p], pl[3][p]);
         }
         __syncthreads();
-        // W = T K and U0 = T V, 32 columns per warp at a time.  Values that are no numbers leave the products (whose zeros would turn them into NaN
-        // for earlier tokens)
+        // W = T K and U0 = T V, 32 columns per warp at a time.  Values that do not split leave the products (whose zeros would turn them into NaN
+        // for earlier tokens) and are added one by one
         const int n_w = D / 32, n_v = (a.vdim + 31) / 32;
         const bool pairs = (a.vdim & 1) == 0 && ((uintptr_t)a.o & 7) == 0;               // the outputs' rows start on 8 bytes
         uint32_t y[4][2][2][NP];                        // [8 columns][16 tokens][half][plane]
@@ -459,8 +461,8 @@ __global__ void __launch_bounds__(DT, 2) delta_gram_kernel(const ChunkArgs a) {
                             own[n][e][0] = __uint_as_float(__byte_perm(lo, hi, 0x5410)); own[n][e][1] = __uint_as_float(__byte_perm(lo, hi, 0x7632));
                         }
                         float f0 = to_f(v[n][e][0]), f1 = to_f(v[n][e][1]);
-                        if (!finite(f0)) { f0 = 0.0f; odd = true; }
-                        if (!finite(f1)) { f1 = 0.0f; odd = true; }
+                        if (!splits(f0)) { f0 = 0.0f; odd = true; }
+                        if (!splits(f1)) { f1 = 0.0f; odd = true; }
                         split<NP>(f0, f1, y[n][e >> 1][e & 1]);
                     }
             }
@@ -527,7 +529,7 @@ __global__ void __launch_bounds__(DT, 2) delta_gram_kernel(const ChunkArgs a) {
                     if (c0 + lane < a.vdim)
                         for (int j = 0; j < nt; ++j) {
                             const float v = to_f(vp[(long)j * ld + lane - gq]);
-                            if (!finite(v))
+                            if (!splits(v))
                                 for (int t = j + 1; t < nt; ++t) ob[t * o_ld + lane] += inv[(hi * DC + t) * D_X + j] * diag[2 * hi * DC + j] * v;
                         }
                 }
@@ -668,19 +670,19 @@ __global__ void __launch_bounds__(64 * DW, 1) delta_walk_kernel(const ChunkArgs 
             }
             float r[4] = {ct0 * ((p0.x + p1.x) + (p2.x + p3.x)), ct1 * ((p0.y + p1.y) + (p2.y + p3.y)),
                           ct0 * ((p0.z + p1.z) + (p2.z + p3.z)), ct1 * ((p0.w + p1.w) + (p2.w + p3.w))};
-            // A token's sum must not meet what later tokens of the chunk hold if that is no number: such values leave the products (whose zeros
-            // would turn them into NaN) and enter one by one
+            // A token's sum must not meet what later tokens of the chunk hold if that does not split: such values leave the products (whose
+            // zeros would turn them into NaN) and enter one by one
             bool odd = false;
 #pragma unroll
             for (int tt = 0; tt < 4; ++tt)
 #pragma unroll
-                for (int e = 0; e < 4; ++e) odd |= !(fabsf(u[tt][e]) <= 1e38f);
+                for (int e = 0; e < 4; ++e) odd |= !splits(u[tt][e]);
             odd = __any_sync(0xffffffffu, odd);
             float f[4][4];
 #pragma unroll
             for (int tt = 0; tt < 4; ++tt)
 #pragma unroll
-                for (int e = 0; e < 4; ++e) f[tt][e] = fabsf(u[tt][e]) <= 1e38f ? u[tt][e] : 0.0f;
+                for (int e = 0; e < 4; ++e) f[tt][e] = splits(u[tt][e]) ? u[tt][e] : 0.0f;
             float x[3][4] = {};
 #pragma unroll
             for (int th = 0; th < 2; ++th)
@@ -702,7 +704,7 @@ __global__ void __launch_bounds__(64 * DW, 1) delta_walk_kernel(const ChunkArgs 
                     const float* const uj = reinterpret_cast<const float*>(us + (slot * 4 + (j >> 3)) * 32 + (lane & ~3) + ((j & 7) >> 1)) + (j & 1);
 #pragma unroll
                     for (int hf = 0; hf < 2; ++hf)
-                        if (const float v = uj[2 * hf]; !(fabsf(v) <= 1e38f))
+                        if (const float v = uj[2 * hf]; !splits(v))
 #pragma unroll
                             for (int s = 0; s < 2; ++s) {
                                 const int tl = 2 * tq + s;           // A [8 w + tl][j], of its planes

@@ -152,3 +152,27 @@ def test_keys_and_queries_of_any_size(ops, cuda_device, dtype, power):
     o = ops.gated_delta_rule(conv, G, H, D, V, proj, 1, 1 + H, a_log, bias, state, 0, pad)
     assert float((o.double() - want_o).abs().max()) <= 2e-6 * max(1.0, float(want_o.abs().max()))
     assert float((state.double() - want_s).abs().max()) <= 2e-6 * max(1.0, float(want_s.abs().max()))
+
+
+@pytest.mark.parametrize("dtype,value", [(torch.float32, torch.finfo(torch.float32).max), (torch.float32, torch.finfo(torch.float32).min), (torch.float32, 3.397e38),
+                                         (torch.float32, 1.1e38), (torch.bfloat16, torch.finfo(torch.bfloat16).min), (torch.bfloat16, torch.finfo(torch.bfloat16).max)])
+def test_the_largest_values_stay_behind_their_token(ops, cuda_device, dtype, value):
+    """values of the size of a mask's lowest, whose first bf16 plane may be an infinity: the tokens before one and the other columns come out
+    bit for bit as without it, the column behind it as float64 has it"""
+    B, S, G, H, D, V = 1, 100, 1, 5, 128, 40
+    conv, proj, a_log, bias, state = inputs(cuda_device, B, S, G, H, D, V, dtype)
+    pad = torch.zeros(B, dtype=torch.int32, device=cuda_device)
+    plain = state.clone()
+    o = ops.gated_delta_rule(conv, G, H, D, V, proj, 1, 1 + H, a_log, bias, plain, 0, pad)
+    for at in (32, 45):
+        c, s = conv.clone(), state.clone()
+        c[0, at, 2 * D + 2 * V + 7] = value
+        got = ops.gated_delta_rule(c, G, H, D, V, proj, 1, 1 + H, a_log, bias, s, 0, pad)
+        assert torch.equal(got[:, :at], o[:, :at])
+        want_o, want_s = statement(c, proj, a_log, bias, state, G, H, D, V, 0, pad)
+        for t, want, free in ((got[:, at:], want_o[:, at:], o[:, at:]), (s.movedim(2, 1), want_s.movedim(2, 1), plain.movedim(2, 1))):
+            column, w = t[:, :, 2, 7].double(), want[:, :, 2, 7]
+            assert float((column - w).abs().max()) <= 2e-6 * max(1.0, float(w.abs().max()))
+            t, free = t.clone(), free.clone()
+            t[:, :, 2, 7] = free[:, :, 2, 7] = 0
+            assert torch.equal(t, free)
