@@ -176,3 +176,19 @@ def test_the_largest_values_stay_behind_their_token(ops, cuda_device, dtype, val
             t, free = t.clone(), free.clone()
             t[:, :, 2, 7] = free[:, :, 2, 7] = 0
             assert torch.equal(t, free)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("at", [32, 63, 71])
+def test_the_largest_values_enter_the_state(ops, cuda_device, dtype, at):
+    """a gate that takes the largest value whole into the state, which forgets next to nothing: finite and right in the chunks behind it"""
+    B, S, G, H, D, V = 1, 200, 2, 4, 96, 24
+    conv, proj, a_log, bias, state = inputs(cuda_device, B, S, G, H, D, V, dtype)
+    a_log -= 8.0
+    conv[0, at, 2 * G * D:] = torch.finfo(dtype).min
+    proj[0, at, 1:1 + H] = 30.0
+    pad = torch.zeros(B, dtype=torch.int32, device=cuda_device)
+    want_o, want_s = statement(conv, proj, a_log, bias, state, G, H, D, V, 0, pad)
+    o = ops.gated_delta_rule(conv, G, H, D, V, proj, 1, 1 + H, a_log, bias, state, 0, pad)
+    assert float((o.double() - want_o).abs().max()) <= 2e-6 * float(want_o.abs().max())
+    assert float((state.double() - want_s).abs().max()) <= 2e-6 * float(want_s.abs().max())
