@@ -71,6 +71,10 @@ long mixers_gated_delta_chunks_workspace(int B, int S, int kv_heads, int heads, 
 int mixers_gated_delta_chunks(int dtype, const void* conv, int B, int S, int kv_heads, int heads, int dim, int vdim, const void* proj, int ld,
                               int off_b, int off_a, const void* A_log, const void* dt_bias, float* state, int slot0, const int32_t* pad,
                               float* o, float* workspace, mixers_stream_t stream);
+/* Its second launch bounds its waits, at about two seconds each.  One that runs out ends the kernel, and the launch's outputs and states
+ * are undefined: the next mixers_gated_delta_chunks on the device launches nothing and returns cudaErrorLaunchTimeout.  1 when a wait has run
+ * out on the current device and no call has reported it yet, 0 otherwise, -1 without a device.  Synchronises. */
+int mixers_wait_expired(void);
 
 /* Delta rule whose state decays per key channel.  conv as above; beta = sigmoid(proj[.., off_b + h]); z [B, S, heads * dim]: decay
  * logits, a = exp(-exp(A_log[h]) * softplus(z + dt_bias)) with dt_bias [heads * dim].  Per head:  M <- diag(a) M;

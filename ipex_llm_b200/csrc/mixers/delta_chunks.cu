@@ -15,7 +15,9 @@
 // are handed over.  Keys and queries stay as they were given, times a power of two near 1 / norm: a 16-bit input is then one (bf16) or two
 // (fp16) exact bf16 planes where a unit vector would need three; the rest of 1 / norm goes into the factors of a token.
 #include "mixers_common.cuh"
+#include <limits.h>
 #include <math.h>
+#include <stdlib.h>
 #include <string.h>
 #include <atomic>
 #include <mutex>
@@ -56,6 +58,7 @@ struct ChunkArgs {
     uint32_t* rows;                                     // [B][kv_heads][n_chunks][d_rows]
     uint32_t* side;                                     // [B][heads][n_chunks][d_side]
     unsigned int* late;                                 // in host memory: a wait ran out
+    long long limit; int most;                          // of a wait, in SM clocks; the chunks that come (tests: fewer than there are)
     float* state; float* o;                             // o holds U0 until the walk has read it
 };
 
@@ -546,17 +549,31 @@ __device__ __forceinline__ void bulk_copy(uint32_t dst, const void* src, uint32_
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
 __device__ __forceinline__ void arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
-// about two seconds; a wait that runs out raises the device's word in host memory, and the results are undefined
-__device__ __forceinline__ void wait_for(uint32_t bar, uint32_t parity, unsigned int* late) {
+// A wait that runs out raises the device's word in host memory and the block's in shared memory.  The block's waits end at once from then on, its
+// results are undefined, and the warp that brings the chunks in brings no more and stays until its copies have landed
+constexpr long long kWait = 4000000000ll;               // about two seconds
+__device__ __forceinline__ bool arrived(uint32_t bar, uint32_t parity) {
+    uint32_t there;
+    asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }" : "=r"(there) : "r"(bar), "r"(parity) : "memory");
+    return there != 0;
+}
+__device__ __forceinline__ bool wait_on(uint32_t bar, uint32_t parity, unsigned int* late, long long limit, volatile int* failed) {
     const long long t0 = clock64();
-    for (uint32_t there = 0; !there;) {
-        asm volatile("{ .reg .pred p; mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }" : "=r"(there) : "r"(bar), "r"(parity) : "memory");
-        if (!there && clock64() - t0 > 4000000000ll) {
+    while (!arrived(bar, parity))
+        if (clock64() - t0 > limit || (failed && *failed)) {
+            if (failed) *failed = 1;
             *(volatile unsigned int*)late = 1u;
             __threadfence_system();
-            return;
+            return false;
         }
-    }
+    return true;
+}
+__device__ __forceinline__ void wait_for(uint32_t bar, uint32_t parity, const ChunkArgs& a, volatile int* failed) {
+    if (!arrived(bar, parity)) wait_on(bar, parity, a.late, a.limit, failed);
+}
+// whole warp, the same answer in every lane
+__device__ __forceinline__ bool wait_warp(uint32_t bar, uint32_t parity, const ChunkArgs& a, volatile int* failed) {
+    return __all_sync(0xffffffffu, arrived(bar, parity)) || __all_sync(0xffffffffu, wait_on(bar, parity, a.late, a.limit, failed));
 }
 // two accumulator tiles side by side, [16 x 8] each, as planes of one [16 x 16] operand
 __device__ __forceinline__ void split_pair(const float (&l)[4], const float (&r)[4], uint32_t (&a)[3][4]) {
@@ -591,7 +608,9 @@ __global__ void __launch_bounds__(64 * DW, 1) delta_walk_kernel(const ChunkArgs 
     const uint32_t full = (uint32_t)__cvta_generic_to_shared(up_sh + 2 * 2 * 3 * 64), ready = full + 8 * STAGES, empty = ready + 8 * STAGES;
     const int col0 = blockIdx.x * DV, h = blockIdx.y, b = blockIdx.z, g = h / (a.heads / a.kv_heads);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, gq = lane >> 2, tq = lane & 3;
+    volatile int* const failed = reinterpret_cast<volatile int*>(up_sh + 2 * 2 * 3 * 64 + 3 * STAGES);
     if (threadIdx.x == 0) {
+        *failed = 0;
 #pragma unroll
         for (int i = 0; i < STAGES; ++i) {
             asm volatile("mbarrier.init.shared::cta.b64 [%0], 33;" ::"r"(full + 8 * i) : "memory");
@@ -615,10 +634,11 @@ __global__ void __launch_bounds__(64 * DW, 1) delta_walk_kernel(const ChunkArgs 
         const uint32_t* const side = a.side + ((long)b * a.heads + h) * a.n_chunks * d_side<D>();
         const uint32_t at0 = (uint32_t)__cvta_generic_to_shared(sh);
         const bool wide = (a.vdim & 3) == 0 && ((uintptr_t)a.o & 15) == 0;
+        const int come = min(n, a.most);
         auto bring = [&](int c) {
             const int slot = c % STAGES;
             const uint32_t at = at0 + slot * STAGE * 4, bar = full + 8 * slot;
-            if (c >= STAGES) wait_for(empty + 8 * slot, (c / STAGES - 1) & 1, a.late);
+            if (c >= STAGES && !wait_warp(empty + 8 * slot, (c / STAGES - 1) & 1, a, failed)) return false;
             if (lane == 0) {
                 asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "n"(4 * (d_rows<D, NP>() + d_side<D>())) : "memory");
                 bulk_copy(at + 4 * d_rows<D, NP>(), side + (long)c * d_side<D>(), 4 * d_side<D>(), bar);
@@ -642,18 +662,20 @@ __global__ void __launch_bounds__(64 * DW, 1) delta_walk_kernel(const ChunkArgs 
                 }
             }
             asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
+            return true;
         };
         if (w == 0)
 #pragma unroll 1
-            for (int c = 0; c < STAGES && c < n; ++c) bring(c);
+            for (int c = 0; c < STAGES && c < come; ++c) bring(c);
         for (int i = threadIdx.x - 32 * DW; i < first * DV; i += 32 * DW) if (i % DV < cols) ob[(i / DV) * o_ld + i % DV] = 0.0f;
+        int c = 0;
 #pragma unroll 1
-        for (int c = 0; c < n; ++c) {
+        for (; c < n; ++c) {
             const float* const stage = sh + (c % STAGES) * STAGE;
             constexpr Products<3, 3> pr;
             const int slot = c % STAGES;
-            wait_for(ready + 8 * slot, (c / STAGES) & 1, a.late);
-            wait_for(full + 8 * slot, (c / STAGES) & 1, a.late);     // (long over; A and the factors were written by copies)
+            wait_for(ready + 8 * slot, (c / STAGES) & 1, a, failed);
+            if (!wait_warp(full + 8 * slot, (c / STAGES) & 1, a, failed)) break;     // (long over; A and the factors were written by copies)
             const float4* const at = osum + (slot * 4 + w) * DW * 32 + lane;
             const float4 p0 = at[0], p1 = at[32], p2 = at[64], p3 = at[96];
             const float ct0 = stage[CD + 8 * w + 2 * tq], ct1 = stage[CD + 8 * w + 2 * tq + 1];
@@ -729,8 +751,10 @@ __global__ void __launch_bounds__(64 * DW, 1) delta_walk_kernel(const ChunkArgs 
                 const int t = first + c * DC + 8 * w + 2 * tq + (e & 1), col = gq + 8 * (e >> 1);
                 if (t < a.S && col < cols) ob[t * o_ld + col] = r[e];
             }
-            if (w == 0 && c + STAGES < n) bring(c + STAGES);         // (copies are waited for before their chunk is read, and every chunk is)
+            if (w == 0 && c + STAGES < come && !bring(c + STAGES)) break;            // (every chunk's copies are waited for before it is read)
         }
+        if (w == 0 && c < n)                            // a wait ran out: the copies under way
+            for (const int end = min(come, c + STAGES); c < end; ++c) wait_on(full + 8 * (c % STAGES), (c / STAGES) & 1, a.late, kWait, nullptr);
         return;
     }
 
@@ -757,7 +781,7 @@ __global__ void __launch_bounds__(64 * DW, 1) delta_walk_kernel(const ChunkArgs 
     uint32_t mp[KT][3][4];                              // the state's planes
 #pragma unroll
     for (int kt = 0; kt < KT; ++kt) split_pair(m[2 * kt], m[2 * kt + 1], mp[kt]);
-    if (n > 0) { wait_for(full, 0, a.late); load_w(0); }
+    if (n > 0) { wait_for(full, 0, a, failed); load_w(0); }
 #pragma unroll 1
     for (int c = 0; c < n; ++c) {
         const int slot = c % STAGES;
@@ -799,7 +823,7 @@ __global__ void __launch_bounds__(64 * DW, 1) delta_walk_kernel(const ChunkArgs 
 #pragma unroll
             for (int p = 0; p < NP; ++p) kf[dt][p] = kat[(dt * NP + p) * 32];
         auto next_w = [&] {
-            if (c + 1 < n) { wait_for(full + 8 * ((c + 1) % STAGES), ((c + 1) / STAGES) & 1, a.late); load_w(c + 1); }
+            if (c + 1 < n) { wait_for(full + 8 * ((c + 1) % STAGES), ((c + 1) / STAGES) & 1, a, failed); load_w(c + 1); }
         };
         if constexpr (STAGES > 2) next_w();             // (of two chunks the second comes while the first is used)
 #pragma unroll
@@ -894,7 +918,7 @@ __global__ void __launch_bounds__(64 * DW, 1) delta_walk_kernel(const ChunkArgs 
 template <typename T, int D> int launch_chunks(ChunkArgs a, cudaStream_t st) {
     constexpr int NP = d_planes<T>();
     constexpr int gram = (DC * (D + 8) + 2 * DC * D_G + 3 * DC + 2 * DH * DC + DH * DC * D_X + D_TP) * 4 + (2 + DH * 4) * DC * 8;
-    constexpr int walk = (d_stages<D, NP>() * d_stage<D, NP>() + (2 * DW + d_stages<D, NP>() * (DW + 1)) * 4 * 32 * 4 + 2 * 2 * 3 * 64 * 2) * 4 + 24 * d_stages<D, NP>();
+    constexpr int walk = (d_stages<D, NP>() * d_stage<D, NP>() + (2 * DW + d_stages<D, NP>() * (DW + 1)) * 4 * 32 * 4 + 2 * 2 * 3 * 64 * 2) * 4 + 24 * d_stages<D, NP>() + 8;
     static_assert(walk <= 232448, "shared memory");
     static bool configured_dev[64] = {};                // the attributes are per device context
     int dev = 0;
@@ -964,6 +988,9 @@ static unsigned int* late_word() {
     return cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64 ? words.load(std::memory_order_acquire) + 32 * dev : nullptr;
 }
 
+// the limit of the waits in this thread's launches, 0: the usual one
+static thread_local long long t_wait_limit = 0;
+
 template <typename T> static int run_portions(ChunkArgs a, cudaStream_t st) {
     const int S = a.S, slot0 = a.slot0, step = DC * (int)portion_chunks(a.B, S, a.kv_heads, a.heads, a.dim);
     const long ld = 2 * a.kv_heads * a.dim + a.heads * a.vdim;
@@ -991,7 +1018,7 @@ extern "C" int mixers_gated_delta_chunks(int dtype, const void* conv, int B, int
     a.B = B; a.S = S; a.kv_heads = kv_heads; a.heads = heads; a.dim = dim; a.vdim = vdim; a.ld_proj = ld; a.off_b = off_b; a.off_a = off_a;
     a.q_scale = 1.0 / sqrt((double)dim);
     a.slot0 = slot0; a.pad = pad; a.state = state; a.o = o; a.rows = reinterpret_cast<uint32_t*>(workspace);
-    a.late = late_word();
+    a.late = late_word(); a.limit = t_wait_limit ? llabs(t_wait_limit) : kWait; a.most = t_wait_limit < 0 ? 1 : INT_MAX;
     if (!a.late) return (int)cudaErrorMemoryAllocation;
     if (*(volatile unsigned int*)a.late) {              // a wait inside an earlier call ran out: its results are undefined
         *(volatile unsigned int*)a.late = 0;
@@ -1000,3 +1027,13 @@ extern "C" int mixers_gated_delta_chunks(int dtype, const void* conv, int B, int
     MIXERS_DISPATCH(dtype, return run_portions<T>(a, (cudaStream_t)stream));
     return 0;
 }
+
+extern "C" int mixers_wait_expired(void) {
+    if (cudaDeviceSynchronize() != cudaSuccess) { cudaGetLastError(); return -1; }
+    const unsigned int* const late = late_word();
+    return late ? *(const volatile unsigned int*)late != 0 : -1;
+}
+
+// development aid, not in the public header: the limit, in SM clocks, of the waits in this thread's launches (0: the usual one; below zero: a
+// block's first chunk alone comes, and the waits for the others run out after that many clocks)
+extern "C" void mixers_debug_set_wait_limit(long long clocks) { t_wait_limit = clocks; }

@@ -99,6 +99,8 @@ def lib():
             fn.argtypes, fn.restype = argtypes, _c_int
         loaded.mixers_gated_delta_chunks_workspace.argtypes = [_c_int] * 5
         loaded.mixers_gated_delta_chunks_workspace.restype = _c_long
+        loaded.mixers_wait_expired.argtypes, loaded.mixers_wait_expired.restype = [], _c_int
+        loaded.mixers_debug_set_wait_limit.argtypes, loaded.mixers_debug_set_wait_limit.restype = [ctypes.c_longlong], None
         loaded.mixers_softmax_attention_workspace.argtypes = [_c_int] * 7
         loaded.mixers_softmax_attention_workspace.restype = _c_long
         _lib, LIB_PATH = loaded, path

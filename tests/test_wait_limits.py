@@ -89,3 +89,45 @@ def test_wherever_a_wait_runs_out_the_next_call_is_right(native_lib, cuda_device
                 call()
             torch.cuda.synchronize()
         assert torch.equal(call(), want)
+
+
+@pytest.fixture
+def delta_limit(cuda_device):
+    """sets the limit of this thread's delta-rule launches; below zero only a block's first chunk comes"""
+    from ipex_llm_b200.ggml.model import mixers_cpp
+    yield mixers_cpp.lib().mixers_debug_set_wait_limit
+    mixers_cpp.lib().mixers_debug_set_wait_limit(0)
+
+
+def delta_call(dev, dtype, dim, tokens=300):
+    from ipex_llm_b200.transformers.models import mixer_ops as ops
+    B, G, H, V = 2, 2, 4, 40
+    conv, proj = rows(dev, B * tokens, 2 * G * dim + H * V, dtype).view(B, tokens, -1), rows(dev, B * tokens, 2 * H, dtype).view(B, tokens, -1)
+    a_log, bias, state = rows(dev, 1, H, dtype)[0], rows(dev, 2, H, dtype)[0], rows(dev, B * H * dim, V, torch.float32).view(B, H, dim, V)
+    pad = torch.tensor([0, 50], dtype=torch.int32, device=dev)
+
+    def call():
+        s = state.clone()
+        o = ops.gated_delta_rule(conv, G, H, dim, V, proj, 0, H, a_log, bias, s, 0, pad)
+        return torch.cat([o.flatten(), s.flatten()])
+    return call
+
+
+@pytest.mark.parametrize("clocks", [-20, -100000, 1, 300, 1500, 6000])
+@pytest.mark.parametrize("dtype,dim", [(torch.float32, 128), (torch.bfloat16, 128), (torch.float16, 64)])       # two chunks in shared memory, and three
+def test_a_delta_rule_wait_that_runs_out_is_reported_once(delta_limit, cuda_device, dtype, dim, clocks):
+    """chunks that never come, and limits of the order of the kernel's own waits (which run out in the middle of the work, or not at all)"""
+    from ipex_llm_b200.ggml.model import mixers_cpp
+    call, expired = delta_call(cuda_device, dtype, dim), mixers_cpp.lib().mixers_wait_expired
+    want = call()
+    assert expired() == 0
+    for _ in range(5):
+        delta_limit(clocks)
+        got = call()
+        delta_limit(0)
+        if expired():
+            with pytest.raises(mixers_cpp.MixersNativeError, match="702"):
+                call()
+        else:
+            assert clocks > 0 and torch.equal(got, want)
+        assert expired() == 0 and torch.equal(call(), want)
