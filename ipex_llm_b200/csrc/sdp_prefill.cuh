@@ -106,7 +106,6 @@ sdp_fp8_prompt_kernel(const SdpArgs A, int n_qt) {
     };
     int nk = tiles_of(0);
     if (NT == 2) nk = max(nk, tiles_of(1));
-    asm volatile("griddepcontrol.launch_dependents;");
     asm volatile("griddepcontrol.wait;" ::: "memory");
 
     // ---- before the barriers exist: the queries into their tiles, the first keys on their way
@@ -162,6 +161,8 @@ sdp_fp8_prompt_kernel(const SdpArgs A, int n_qt) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     uint32_t tmem;
     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem) : "r"(tmem_slot));
+    // not before every block holds its columns: a dependent that allocates in front of its wait must find nobody who still wants some
+    asm volatile("griddepcontrol.launch_dependents;");
 
     const uint32_t leader = elect_leader();
     if (warp < 4 * NT) {
