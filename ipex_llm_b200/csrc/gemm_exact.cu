@@ -402,7 +402,7 @@ done:
 }
 
 // fp32 activations -> three bf16 planes whose sum reproduces them to 2^-24, four elements a thread; `sums`: those of 64 elements, for minima
-__global__ void __launch_bounds__(256) split3_kernel(const float4* __restrict__ x, uint2* __restrict__ out, int64_t n4, float* __restrict__ sums, int k4, int sum_rows) {
+__global__ void __launch_bounds__(256) split3_kernel(const float4* x, uint2* out, int64_t n4, float* sums, int k4, int sum_rows) {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;");     // not before the wait: the matmul reads its weights ahead of its own
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n4; i += (int64_t)gridDim.x * blockDim.x) {

@@ -515,7 +515,7 @@ done:
 }
 
 // the same behind a split MLP: y[token][n] = act(sum of the gate partials) * (sum of the up partials)
-__global__ void __launch_bounds__(256) reduce_gated_kernel(const float* __restrict__ part, int ksplit, int64_t m, int64_t n, void* y, int y_dtype, int act) {
+__global__ void __launch_bounds__(256) reduce_gated_kernel(const float* part, int ksplit, int64_t m, int64_t n, void* y, int y_dtype, int act) {
     asm volatile("griddepcontrol.launch_dependents;");
     asm volatile("griddepcontrol.wait;" ::: "memory");
     const int64_t mn = m * n, n4 = n / 4;

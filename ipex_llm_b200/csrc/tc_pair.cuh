@@ -65,7 +65,7 @@ __device__ __forceinline__ void store_feature(float* p, int64_t stride, const fl
     for (int j = 0; j < 16; j++) if (j < cnt) p[j * stride] = accumulate ? v[j] + bias + p[j * stride] : v[j] + bias;
 }
 // K split: y[token][n] = sum over splits (in split order) of the fp32 partials, + bias, + y when accumulating
-static __global__ void __launch_bounds__(256) reduce_partials_kernel(const float* __restrict__ part, int ksplit, int64_t mn, int64_t n_cols,
+static __global__ void __launch_bounds__(256) reduce_partials_kernel(const float* part, int ksplit, int64_t mn, int64_t n_cols,
                                                               void* y, int y_dtype, const void* bias, int accumulate) {
     asm volatile("griddepcontrol.launch_dependents;");
     asm volatile("griddepcontrol.wait;" ::: "memory");

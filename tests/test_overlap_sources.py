@@ -49,3 +49,10 @@ def test_tensor_memory_is_held_before_dependents_may_start(params, body):
     one would wait for the other's columns and the other for the first one's end."""
     if "tcgen05.alloc" in body and "griddepcontrol.launch_dependents" in body:
         assert body.index("tcgen05.alloc") < body.index("griddepcontrol.launch_dependents")
+
+
+@pytest.mark.parametrize("params,body", KERNELS)
+def test_no_input_is_promised_to_be_constant(params, body):
+    """What the launch in front leaves is written while the kernel already runs.  const __restrict__ says that it is not, and lets the
+    compiler read it by the path for constants."""
+    assert "__restrict__" not in params
