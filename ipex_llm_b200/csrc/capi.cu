@@ -221,14 +221,16 @@ static bool use_skinny(int qtype, int64_t n_rows, int64_t k, int64_t m, int x_dt
     return m >= min_m && m <= max_m && gemm_skinny_supported(qtype, n_rows, k, m, x_dtype);
 }
 
-size_t lowbit_matmul_workspace_size(int64_t n_rows, int64_t k, int64_t m, int x_dtype) {
+static size_t matmul_workspace(int qtype, int64_t n_rows, int64_t k, int64_t m, int x_dtype) {
     if (use_skinny(B200_QT_SYM_INT4, n_rows, k, m, x_dtype)) return gemm_skinny_workspace_size(n_rows, k, m);
     if (use_gemm(B200_QT_SYM_INT4, n_rows, k, m, x_dtype)) return gemm_tc_workspace_size(n_rows, k, m);
     const size_t gemv = gemv_workspace_size(n_rows, k, m, x_dtype);
     if (!use_exact(B200_QT_SYM_INT4, n_rows, k, m, x_dtype, DT_F32)) return gemv;
-    const size_t exact = gemm_exact_workspace_size(B200_QT_ASYM_INT4, n_rows, k, m);     // the size is asked without the format: enough for each
+    const size_t exact = gemm_exact_workspace_size(qtype, n_rows, k, m);
     return exact > gemv ? exact : gemv;
 }
+// asked without the format: enough for each, asym_int4's sums of activations among them
+size_t lowbit_matmul_workspace_size(int64_t n_rows, int64_t k, int64_t m, int x_dtype) { return matmul_workspace(B200_QT_ASYM_INT4, n_rows, k, m, x_dtype); }
 
 static int matmul_dispatch(const void* d_w, int qtype, int64_t n_rows, int64_t k, const void* d_x, int x_dtype, int64_t m,
                            void* d_y, int y_dtype, const void* d_bias, int accumulate, void* workspace, size_t workspace_bytes,
@@ -301,16 +303,20 @@ int lowbit_mlp_cuda(const void* d_w_gate, const void* d_w_up, int qtype, int64_t
     if (act != 0 && act != 1) { set_error(LB_ERR_ARG, "lowbit_mlp_cuda: act must be 0 (SILU) or 1 (GELU), got %d", act); return LB_ERR_ARG; }
     if (!d_w_gate || !d_w_up || !d_x || !d_y || m < 0 || n_rows < 0) { set_error(LB_ERR_ARG, "lowbit_mlp_cuda: null pointer or negative size"); return LB_ERR_ARG; }
     const bool fused = gemv_mlp_fused_supported(qtype, n_rows, k, m, x_dtype);
-    const size_t base = (lowbit_matmul_workspace_size(n_rows, k, m, x_dtype) + 255) / 256 * 256;
-    const size_t need = fused ? base : lowbit_mlp_workspace_size(n_rows, k, m, x_dtype);
+    // 32-bit prompts: in every format a workspace without room for asym_int4's sums of activations is enough, and asym_int4 then runs as it
+    // does in lowbit_matmul_cuda without them
+    const size_t parts = 2 * (size_t)m * n_rows * sizeof(float), full = lowbit_mlp_workspace_size(n_rows, k, m, x_dtype);
+    size_t base = (matmul_workspace(qtype, n_rows, k, m, x_dtype) + 255) / 256 * 256;
+    const size_t least = (matmul_workspace(B200_QT_SYM_INT4, n_rows, k, m, x_dtype) + 255) / 256 * 256;
+    const size_t need = fused ? base : x_dtype == DT_F32 ? least + parts : full;
     std::unique_lock<std::mutex> lk(g_mu, std::defer_lock);
     if (!workspace) {
         lk.lock();
         DevState* S = dev_state();
         if (!S) { set_error(LB_ERR_NO_DEVICE, "lowbit_mlp_cuda: no CUDA device"); return LB_ERR_NO_DEVICE; }
-        if (need > S->ws.cap) {
+        if ((fused ? need : full) > S->ws.cap) {
             cudaDeviceSynchronize();
-            int rc = S->ws.ensure(need, true);
+            int rc = S->ws.ensure(fused ? need : full, true);
             if (rc) return rc;
         }
         workspace = S->ws.p; workspace_bytes = S->ws.cap;
@@ -331,6 +337,7 @@ int lowbit_mlp_cuda(const void* d_w_gate, const void* d_w_up, int qtype, int64_t
         rc = gemm_tc_mlp_launch(d_w_gate, d_w_up, act + 1, qtype, n_rows, k, d_x, x_dtype, m, d_y, y_dtype, workspace, workspace_bytes, st);
     } else {
         // behind the exact GEMV: the two intermediates in fp32
+        if (workspace_bytes < base + parts) base = least;
         float* tg = (float*)((char*)workspace + base);
         float* tu = tg + (size_t)m * n_rows;
         rc = matmul_dispatch(d_w_gate, qtype, n_rows, k, d_x, x_dtype, m, tg, DT_F32, nullptr, 0, workspace, base, st);

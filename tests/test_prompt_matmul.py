@@ -207,6 +207,32 @@ def test_prompt_matmul_fp32_with_minima(lbl, native_lib, cuda_device, m, n, k):
     assert float(outs[0].norm()) <= 1.05 * float(outs[1].norm())
 
 
+@pytest.mark.parametrize("qtype", ["sym_int4", "asym_int4", "nf4", "fp8_e4m3", "fp8_e5m2", "fp6"])
+@pytest.mark.parametrize("m,n,k", [(33, 256, 192), (100, 1024, 2048)])
+def test_mlp_fp32_in_a_workspace_without_sums(lbl, native_lib, cuda_device, qtype, m, n, k):
+    """only asym_int4's minima need the activations' sums, and without room for them it runs in passes; less than that is refused"""
+    [(gate, gd), (up, ud)], qt = weights(lbl, cuda_device, m, n, k, qtype, 2)
+    x = acts(cuda_device, m, m, k, torch.float32)
+    full = native_lib.lowbit_mlp_workspace_size(n, k, m, native_lib.DT_F32)
+    room = full - 256 * ((k // 64 * ((m + 15) // 16 * 16) * 4 + 255) // 256)
+    stream = torch.cuda.current_stream().cuda_stream
+
+    def call(size):
+        ws, y = torch.full((full,), 255, dtype=torch.uint8, device=cuda_device), torch.empty(m, n, device=cuda_device)
+        native_lib.lowbit_mlp_cuda(gate.data_ptr(), up.data_ptr(), qt, n, k, x.data_ptr(), native_lib.DT_F32, m, y.data_ptr(), native_lib.DT_F32, 0,
+                                   ws.data_ptr(), size, stream)
+        assert bool((ws[size:] == 255).all())
+        return y
+    want, got = call(full), call(room)
+    assert qtype == "asym_int4" or torch.equal(want, got)
+    a, b = x.double() @ gd.T, x.double() @ ud.T
+    mag = (x.double().abs() @ gd.abs().T) * b.abs() + (x.double().abs() @ ud.abs().T) * a.abs()
+    for y in (want, got):                         # each product to 2e-6 of its magnitude, silu's slope at most 1.1
+        assert bool(((y.double() - torch.nn.functional.silu(a) * b).abs() <= 3e-6 * mag + 1e-7).all())
+    with pytest.raises(native_lib.LowBitNativeError, match="workspace too small"):
+        call(room - 256)
+
+
 @pytest.mark.parametrize("m,n,k", [(33, 9600, 192), (48, 19200, 832), (64, 1024, 8192), (65, 128, 64), (129, 9600, 256), (385, 4736, 448), (512, 9728, 1088)])
 def test_prompt_matmul_fp32_through_the_table(lbl, native_lib, cuda_device, m, n, k):
     """nf4's two tiles per k-block: both tiles' remainders, rings that go round with two and with three expansion groups, the same bits each time"""
