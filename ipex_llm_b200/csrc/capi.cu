@@ -212,9 +212,11 @@ static bool use_exact(int qtype, int64_t n_rows, int64_t k, int64_t m, int x_dty
 
 // Batches between the GEMV's best range and a full 128-token tile take the tensor-core kernel with the operands swapped
 // (gemm_skinny_launch): weights rounded once to the activation dtype, the prefill kernel's precision contract.
-// Measured on 11008x4096 sym_int4: GEMV 12 us at M = 16 and 22 us at M = 32, this kernel 15.5 us for 9 <= M <= 32, 17-20 us
-// up to 64 (the split-K prefill kernel: 22-25 us), 29 us at 96-128 -- hence the window 17..64.
-// LOWBIT_SKINNY_MIN_M / LOWBIT_SKINNY_MAX_M (development) move the window; MIN_M above MAX_M switches the kernel off.
+// The window is 17..64 rows, in every format (fresh weights, back to back): 11008 x 4096 in sym_int4, this kernel against the GEMV 13.0 / 23.2 us at 17
+// rows and 13.3 / 24.3 at 32, against the prompt kernel 13.7 / 19.0 at 33, 15.3 / 19.0 at 64 and, in 128 columns, 21.7 / 19.8 at 65;
+// fp8_e4m3 15.4 / 20.9, 15.6 / 22.0, 15.9 / 18.7, 16.9 / 18.9, 20.7 / 19.8.  At 9 to 16 rows the GEMV takes 13.5 us against 12.8 there, 8.7 against 9.6
+// at 4096 x 4096 and 4.5 against 6.9 at 1024 x 1024.
+// LOWBIT_SKINNY_MIN_M / LOWBIT_SKINNY_MAX_M (development) move the window, up to 64 rows; MIN_M above MAX_M switches the kernel off.
 static bool use_skinny(int qtype, int64_t n_rows, int64_t k, int64_t m, int x_dtype) {
     static const int64_t min_m = [] { const char* e = getenv("LOWBIT_SKINNY_MIN_M"); return e ? (int64_t)atoi(e) : kExactRows + 1; }();
     static const int64_t max_m = [] { const char* e = getenv("LOWBIT_SKINNY_MAX_M"); return e ? (int64_t)atoi(e) : (int64_t)64; }();

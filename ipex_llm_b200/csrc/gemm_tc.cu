@@ -1,16 +1,17 @@
-// gemm_tc.cu -- kernel (c'): dequant-GEMM of small batches on the 5th-generation tensor cores (9 <= M <= 128 activation rows:
+// gemm_tc.cu -- kernel (c'): dequant-GEMM of small batches on the 5th-generation tensor cores (17 <= M <= 64 activation rows:
 // batched decode, short prefills).  The EXPANDED WEIGHTS are the 128-row A operand and the tokens are the N dimension
-// (16 / 32 / 48 / 64 / 128), so nothing is padded to a 128-token tile, an activation stage is NTOK x 256 bytes and the accumulator is NTOK TMEM columns.
+// (32 / 48 / 64), so nothing is padded to a 128-token tile, an activation stage is NTOK x 256 bytes and the accumulator is NTOK TMEM columns.
 //   * work = the linear sequence of (128-feature tile, PAIR of k-blocks) items, cut into gridDim.x contiguous ranges of
 //     equal length (stream-K): every SM expands the same number of blocks whatever the matrix shape; a range that crosses
 //     a tile boundary produces one partial result per tile it touches (fp32, in the workspace) and a second,
 //     programmatic-dependent launch adds a tile's partials in CTA order (deterministic) and applies bias / accumulate;
 //   * an item is 128 k: the barrier handshakes, the MMA thread's loop and the bulk copies are per item;
-//   * warp 0 streams PACKED weights through a ring of stages (the first round is requested before griddepcontrol.wait); a stage is free
-//     again when its codes have been expanded.  A warp of its own brings the activations' k-slices through a ring of two to four;
+//   * warp 0 streams PACKED weights through a ring of stages (in a recorded step, where they are complete, in front of
+//     griddepcontrol.wait); a stage is free again when its codes have been expanded.  A warp of its own brings the activations' k-slices
+//     through a ring of two to four;
 //   * 16 dequant warps in two groups take alternate items; a group fills 128 x 128 K-major 128B-swizzled A tiles (two 16 KB atoms each),
-//     two in turn (one for 65 to 128 tokens, where two do not fit), and every warp expands its 16 rows of both k-blocks: a group goes on
-//     while the MMAs of its last tile run, and its waits, LDS / STS latency and proxy fence overlap the other group's arithmetic;
+//     two in turn, and every warp expands its 16 rows of both k-blocks: a group goes on while the MMAs of its last tile run, and its
+//     waits, LDS / STS latency and proxy fence overlap the other group's arithmetic;
 //   * warp 1 issues tcgen05.mma M = 128, N = NTOK, K = 16 (8 per item) into one of two TMEM accumulators; ONE commit per
 //     item frees both the activations (for their warp) and the A tile;  4 epilogue warps read TMEM (lane = feature,
 //     column = token).
@@ -50,9 +51,9 @@ template <int QT, int NTOK> struct SkSmem {
     static constexpr int kGroup = 2 * kSuper + kAux;                            // one 64-row group, two k-blocks
     static constexpr int kX = NTOK * 256;                                       // two [NTOK][64] atoms
     static constexpr int kW = (2 * kGroup + 127) / 128 * 128;
-    static constexpr int kTiles = NTOK > 64 ? 2 : 4;                            // expanded tiles, two atoms each: two per group where they fit
+    static constexpr int kTiles = 4;                                            // expanded tiles, two atoms each: two per group
     static constexpr int kFree = 232448 - 1024 - 512 - kTiles * 2 * kTileBytesAB - Expand<QT>::kLutBytes;
-    static constexpr int kXStages = NTOK <= 32 ? 4 : NTOK <= 64 && kFree - 3 * kX >= 3 * kW ? 3 : 2;
+    static constexpr int kXStages = NTOK <= 32 ? 4 : kFree - 3 * kX >= 3 * kW ? 3 : 2;
     static constexpr int kFit = (kFree - kXStages * kX) / kW;
     static constexpr int kStages = kFit < kSkStagesMax ? kFit : kSkStagesMax;   // of packed weights
     static constexpr int kTotal = 1024 + 512 + kTiles * 2 * kTileBytesAB + kXStages * kX + kStages * kW + Expand<QT>::kLutBytes;
@@ -82,8 +83,10 @@ skinny_kernel(const __grid_constant__ CUtensorMap xmap, const SkinnyArgs A) {
     // A group waits for its own items only, and a barrier tells apart two rounds: with an odd ring of stages the rounds of a stage alternate
     // between the groups, so the barriers go round at twice its length
     constexpr int NF = (NS & 1) ? 2 * NS : NS;
-    static_assert(NS >= 2 && NX >= 2 && NX <= 4, "ring depth");
-    constexpr uint32_t ACC_COLS = NTOK, TMEM_COLS = NTOK <= 16 ? 32 : NTOK <= 32 ? 64 : NTOK <= 64 ? 128 : 256;   // a power of two
+    // an activation stage is waited for by the tile of the item NX before: not more stages than tiles, else that tile's barrier may be two
+    // rounds on; and a group's tiles are every second one
+    static_assert(NS >= 2 && NX >= 2 && NX <= 4 && NX <= NA && NA % 2 == 0, "ring depth");
+    constexpr uint32_t ACC_COLS = NTOK, TMEM_COLS = NTOK <= 32 ? 64 : 128;   // a power of two
     extern __shared__ uint8_t smem_raw[];
     const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t atiles = base, xring = atiles + NA * 2 * kTileBytesAB, ring = xring + NX * SM::kX, bars = ring + NS * SM::kW;
@@ -378,12 +381,13 @@ static int sk_launch_one(const CUtensorMap& map, const SkinnyArgs& A, int grid, 
 template <int QT>
 static int sk_launch_qt(bool bf, int ntok, const CUtensorMap& map, const SkinnyArgs& A, int grid, cudaStream_t st) {
 #define SK_CASE(N) case N: return bf ? sk_launch_one<QT, true, N>(map, A, grid, st) : sk_launch_one<QT, false, N>(map, A, grid, st);
-    switch (ntok) { SK_CASE(16) SK_CASE(32) SK_CASE(48) SK_CASE(64) SK_CASE(128) }
+    switch (ntok) { SK_CASE(32) SK_CASE(48) SK_CASE(64) }
 #undef SK_CASE
     return LB_ERR_ARG;
 }
-// 48: in 64 columns 33 to 48 rows moved a third more activations through shared memory (40 rows, 11008 x 4096, asym_int4: 13.3 -> 13.0 us a pass)
-static int sk_ntok(int64_t m) { return m <= 16 ? 16 : m <= 32 ? 32 : m <= 48 ? 48 : m <= 64 ? 64 : 128; }
+// 48 columns for 33 to 48 rows: 64 move a third more activations through shared memory.  48 rows against 49, 14336 x 4096: sym_int4 16.3 / 17.4 us,
+// asym_int4 16.3 / 16.8, nf4 19.8 / 21.0, fp8_e4m3 19.2 / 19.6, fp6 17.2 / 19.6
+static int sk_ntok(int64_t m) { return m <= 32 ? 32 : m <= 48 ? 48 : 64; }
 static int sk_grid(int64_t total) { const int sms = sm_count(); return (int)(total < sms ? total : sms); }
 static int sk_max_seg(int64_t total, int grid, int64_t np) { return (int)(((total + grid - 1) / grid + np - 1) / np + 1); }
 }  // namespace gemmtc
@@ -393,9 +397,9 @@ extern "C" int lowbit_debug_skinny_timestamps(unsigned long long* out) {
     return (int)cudaMemcpyFromSymbol(out, gemmtc::g_sk_ts, sizeof(gemmtc::g_sk_ts));
 }
 #endif
-// ---- skinny variant (9 <= m <= 128, fp16 / bf16 activations): see gemmtc::skinny_kernel
+// ---- skinny variant (at most 64 rows, fp16 / bf16 activations): see gemmtc::skinny_kernel
 bool gemm_skinny_supported(int qt, int64_t n_rows, int64_t k, int64_t m, int x_dtype) {
-    return (x_dtype == DT_F16 || x_dtype == DT_BF16) && m >= 1 && m <= 128 && gemm_tc_supported(qt, n_rows, k) && (n_rows % 128) == 0 &&
+    return (x_dtype == DT_F16 || x_dtype == DT_BF16) && m >= 1 && m <= 64 && gemm_tc_supported(qt, n_rows, k) && (n_rows % 128) == 0 &&
            (k % 128) == 0;                                 // an item is a pair of k-blocks
 }
 size_t gemm_skinny_workspace_size(int64_t n_rows, int64_t k, int64_t m) {

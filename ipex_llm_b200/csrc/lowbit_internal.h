@@ -136,7 +136,7 @@ int gemm_exact_launch(const void* w, int qt, int64_t n_rows, int64_t k, const vo
 
 // M above this goes to the tensor-core GEMM when the shape allows, else to chunks of the GEMV
 constexpr int64_t kGemvMaxM = 32;
-// the tensor-core GEMM with the operands swapped (weights = the 128-row operand, tokens = N): 9 <= m <= 128
+// the tensor-core GEMM with the operands swapped (weights = the 128-row operand, tokens = N): 17 <= m <= 64
 bool gemm_skinny_supported(int qt, int64_t n_rows, int64_t k, int64_t m, int x_dtype);
 size_t gemm_skinny_workspace_size(int64_t n_rows, int64_t k, int64_t m);
 size_t gemm_skinny_mlp_workspace_size(int64_t n_rows, int64_t k, int64_t m);
