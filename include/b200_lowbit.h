@@ -2,7 +2,7 @@
  * b200_lowbit.h -- C ABI of libb200lowbit.so: the B200 (sm_100a) replacement for the
  * low-bit linear entry points ipex-llm binds from its closed `libllama-api.so`.
  *
- * Reference paths are relative to /root/reference/python/llm/src/ipex_llm/ :
+ * Reference paths are relative to its python/llm/src/ipex_llm/ :
  *   LC = ggml/model/llama/llama_cpp.py      LBL = transformers/low_bit_linear.py
  *
  * Two families:

@@ -2,7 +2,7 @@
 // step can be recorded in a CUDA graph and replayed: every per-token quantity (cache length, position, the token
 // itself) is read from device memory, never baked into a launch.
 //
-// Reference call sites (closed xe_addons kernels; S = /root/reference/python/llm/src/ipex_llm/):
+// Reference call sites (closed xe_addons kernels; S = python/llm/src/ipex_llm/):
 //   rms_norm        xe_addons.rms_norm(weight, x_2d, eps)                 S/transformers/models/common.py:187-200
 //   rope + KV write xe_addons.rotary_half_with_cache_inplaced(q, k, cos, sin) followed by
 //                   DynamicFp8Cache.update -> xe_addons.quantize_key_value  S/transformers/models/llama.py:146-183,

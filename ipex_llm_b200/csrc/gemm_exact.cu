@@ -468,7 +468,8 @@ template <int QT> static int exact_launch_one(const CUtensorMap& map, const Exac
 // up to 64 tokens, 0.52 above (its MMAs, 0.0031 us a token, are 3/4 of that at 128), a unit 1.2 us and 0.014 a token, partial sums 6.6 TB/s
 // and 2.7 us.  Over 120 shapes the choice lies 0.4 % over the best tile and split; with 0.33 us for either tile it was 1.6 %.  sym_int4, its
 // tile then / now: 65 rows, 2048 x 2048 14.2 us (80 tokens) / 12.6 (48), 512 rows 24.0 (96) / 20.5 (64); 48 rows, 11008 x 4096 33.1 (K
-// whole) / 30.4 (three splits); at 128 rows, 4096 x 11008, tiles of 64 take 47.5, of 128 37.2, as then
+// whole) / 30.4 (three splits); at 128 rows, 4096 x 11008, tiles of 64 take 47.5, of 128 37.2, as then.  asym_int4 and nf4, whose k-blocks take
+// longer (another pass over the accumulators, 24 MMA steps for 12), are not among the fitted times: they take the plan of the others
 struct ExactPlan { int tt, ks; };
 static ExactPlan exact_plan(int64_t n_rows, int64_t nb, int64_t m) {
     const int64_t clusters = sm_count() / 2, n_fp = (n_rows / 128 + 1) / 2, nt0 = (m + kExTok - 1) / kExTok;

@@ -34,8 +34,9 @@
 //    "last arriver" fix-up cost 3-5 us of serial L2 round trips per launch -- more than the
 //    3.7 us the 24 MB of a gate_proj take at HBM speed.)  S is chosen so that groups x S fills
 //    the ~4 CTA slots of every SM.
-//  * griddepcontrol.wait sits between the first weight copies and the first read of x, so under
-//    programmatic dependent launch the weight stream of call i+1 overlaps the tail of call i.
+//  * in a recorded step griddepcontrol.wait sits between the first weight copies and the first read
+//    of x: the weights are complete, and their stream of call i+1 overlaps the tail of call i.
+//    Outside one the launch in front may be what writes the weights, and the wait comes first.
 #pragma once
 #include <cstdio>
 #include <cstdlib>
@@ -397,7 +398,7 @@ gemv_kernel(const GemvArgs A) {
     const int nb = (int)A.G.nb;
     const int nbt = (MODE == 2) ? nb * A.n_seg : nb;   // k-blocks along the (concatenated) K axis
     if (A.pdl) asm volatile("griddepcontrol.launch_dependents;");
-    // the routed expert ids come from the previous kernel: nothing can be fetched before it is done
+    // the routed expert ids come from the previous kernel, outside a recorded step the weights may: nothing can be fetched before it is done
     if ((MODE != 0 && A.pdl) || A.pdl == 2) asm volatile("griddepcontrol.wait;" ::: "memory");
 
     auto expert_of = [&](int z, bool& ok) -> int {
@@ -580,7 +581,7 @@ gemv_kernel(const GemvArgs A) {
                 }
         xrun += 128;
     };
-    // everything above is independent of the previous kernel's output: the wait sits right before the first
+    // in a recorded step everything above is independent of the previous kernel's output: the wait sits right before the first
     // read of x, so the set-up instructions of all resident warps run while the SM would be idle anyway
     if (MODE == 0 && A.pdl) asm volatile("griddepcontrol.wait;" ::: "memory");
     TS(2);

@@ -40,10 +40,14 @@ int quantize_launch(const float* src, void* dst, int qt, size_t n, int k, int64_
 void gemv_set_pdl(int on);
 int gemv_get_pdl();
 // Launches outside a recorded step overlap their starts: a kernel is launched as a programmatic dependent of the one in front and waits
-// (griddepcontrol.wait) before it touches global memory, so that what it reads and overwrites is ordered as without; its scheduling, its
-// barriers and its TMEM are off the chain, 1 to 2 us a call behind a kernel that releases its dependents early.  In a recorded step (the
-// switch on) the launches of these kernels stay ordinary: kernels there read inputs ahead of their wait because an ordinary launch lies in
-// front of them; and in a stream that is being captured the graph's edges are left as they were.
+// (griddepcontrol.wait) before it touches global memory, so that what it reads and overwrites is ordered as without.  That pays behind another
+// call of the library, 1 to 2 us; a kernel of torch or a copy releases nothing before it ends.  Off the chain are the scheduling of the blocks
+// and what stands in front of the wait: the barriers and TMEM of the kernel for 17 to 64 rows, nf4's table, barriers in the prompt matmul,
+// little or nothing in the GEMV, both attentions and the delta rule.  The GEMV, the decode attention, the reductions and the delta rule
+// release their dependents at their start, the prompt attention when it holds its TMEM, the others at their end or in their last unit.
+// Who releases early has his TMEM by then (a dependent may allocate in front of its wait), and no parameter is const __restrict__.
+// In a recorded step (the switch on) the launches of these kernels stay ordinary: kernels there read inputs ahead of their wait because an
+// ordinary launch lies in front of them; and in a stream that is being captured the graph's edges are left as they were.
 inline bool launch_overlaps(cudaStream_t st) {
     if (gemv_get_pdl()) return false;
     cudaStreamCaptureStatus state = cudaStreamCaptureStatusNone;

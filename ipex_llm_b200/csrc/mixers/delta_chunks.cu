@@ -10,9 +10,9 @@
 // The right side is linear in M0, so the system is solved before M0 is known: U = U0 - W M0 with T = (I + L)^-1 diag(beta), U0 = T V and
 // W = T (C o K).  delta_gram_kernel does that for all chunks at once; what stays serial is two products per chunk and block of 16 value
 // columns, W M0 and the state's update, with the outputs beside them (delta_walk_kernel).
-// Everything is 32-bit; the quotients C_t / C_j come from sums of logarithms held, and raised, in double precision (a quotient of 32-bit
-// products would carry the rounding of both), and so do the triangular inverse and the scalar factors, which are rounded once, as they
-// are handed over.  Keys and queries stay as they were given, times a power of two near 1 / norm: a 16-bit input is then one (bf16) or two
+// Everything is 32-bit, L, its inverse and T among it, but the gates, the norms, the quotients C_t / C_j and the scalar factors: they come from
+// sums of logarithms held, and raised, in double precision (a quotient of 32-bit products would carry the rounding of both) and are rounded
+// once, as they are handed over.  Keys and queries stay as they were given, times a power of two near 1 / norm: a 16-bit input is then one (bf16) or two
 // (fp16) exact bf16 planes where a unit vector would need three; the rest of 1 / norm goes into the factors of a token.
 #include "mixers_common.cuh"
 #include <limits.h>
@@ -921,15 +921,17 @@ template <typename T, int D> int launch_chunks(ChunkArgs a, cudaStream_t st) {
     constexpr int walk = (d_stages<D, NP>() * d_stage<D, NP>() + (2 * DW + d_stages<D, NP>() * (DW + 1)) * 4 * 32 * 4 + 2 * 2 * 3 * 64 * 2) * 4 + 24 * d_stages<D, NP>() + 8;
     static_assert(walk <= 232448, "shared memory");
     static bool configured_dev[64] = {};                // the attributes are per device context
+    static int sms_dev[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
     if (!configured_dev[dev & 63]) {
         cudaFuncSetAttribute(delta_gram_kernel<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, gram);
         cudaFuncSetAttribute(delta_walk_kernel<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, walk);
+        if (cudaDeviceGetAttribute(&sms_dev[dev & 63], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) { cudaGetLastError(); sms_dev[dev & 63] = 148; }
         configured_dev[dev & 63] = true;
     }
     a.parts = 1;                                        // until every SM has a block (a part forms the Gram matrices again, a fifth of a head's work)
-    while (a.parts * 2 <= a.heads / a.kv_heads && (long)a.n_chunks * a.kv_heads * a.B * a.parts < 148 && a.kv_heads * a.parts * 2 <= 65535) a.parts *= 2;
+    while (a.parts * 2 <= a.heads / a.kv_heads && (long)a.n_chunks * a.kv_heads * a.B * a.parts < sms_dev[dev & 63] && a.kv_heads * a.parts * 2 <= 65535) a.parts *= 2;
     // Both start while the kernel in front drains and wait for its end before they touch memory; in a captured stream the graph's edges stay plain
     cudaStreamCaptureStatus state = cudaStreamCaptureStatusNone;
     const bool overlap = cudaStreamIsCapturing(st, &state) == cudaSuccess && state == cudaStreamCaptureStatusNone;

@@ -3,7 +3,7 @@ replays it.
 
 Why it exists: at B200 speeds a decoded token of Llama-2-7B is about a millisecond of GPU work in ~300 kernels; issuing
 them from Python (the way the reference's XPU path runs its patched forwards,
-/root/reference/python/llm/src/ipex_llm/transformers/models/llama.py:129-205) costs ten times that.  The step below is
+python/llm/src/ipex_llm/transformers/models/llama.py:129-205) costs ten times that.  The step below is
 those same forwards -- qkv GEMV, rotary + FP8 cache write, fused decode attention, o_proj, fused gate/up MLP, down_proj,
 RMSNorm, lm_head, greedy pick -- written against static buffers, with every per-token quantity (cache length, position,
 token) in device memory, so that one graph launch per token replays it.  The residual stream is accumulated by the

@@ -4,7 +4,7 @@ transformers >= 5 keeps a layer's experts as two fused 3-D parameters (``gate_up
 [E, H, I]``) that ``is_linear_module`` never sees.  ``LowBitExperts`` replaces such a module: one ``LowBitLinear`` per
 expert and projection (the reference's layout -- ``expert.gate_proj / up_proj / down_proj`` -- which is what its fused
 decode path takes the weight addresses from), quantised exactly like any other linear.  Its forward follows the
-reference's MoE block forwards (/root/reference/python/llm/src/ipex_llm/transformers/models/qwen3_moe.py:70-132,
+reference's MoE block forwards (python/llm/src/ipex_llm/transformers/models/qwen3_moe.py:70-132,
 deepseek.py:280-330; the fork has no Mixtral forward of its own): one token -> ``moe_forward_vec`` over device tables of
 the experts' weight addresses behind the ``use_fuse_moe`` gate; more tokens in half precision -> ``moe_forward_tokens`` over the
 same tables (sorted on the device, one launch per projection over the experts of many rows); anything else -> per-expert ``LowBitLinear``

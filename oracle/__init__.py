@@ -6,7 +6,7 @@ ctypes wrapper over ``oracle/liblowbit_oracle.so`` (built from ``lowbit_oracle.c
 package ``ipex_llm_b200`` never does.
 
 Parity status: byte-level parity with the reference's closed binary is UNPINNED (the
-binary and any golden vectors are absent from /root/reference).  sym_int4/asym_int4 are
+binary and any golden vectors are absent from the reference's tree).  sym_int4/asym_int4 are
 pinned against gguf.quants and against vectors generated from the reference's own
 in-repo Python statements (tests/golden/make_golden.py); nf4/fp8/fp6 are build-defined.
 See the header of lowbit_oracle.c.

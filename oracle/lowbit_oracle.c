@@ -9,7 +9,7 @@
  * (ipex_llm_b200/csrc) never includes, links or calls anything from here.
  *
  * PARITY STATUS:
- *   - the reference's own binary for this path is NOT in /root/reference and the
+ *   - the reference's own binary for this path is NOT in its source tree and the
  *     reference has no golden vectors for it, so byte-level parity with the
  *     closed binary is UNPINNED;
  *   - sym_int4 / asym_int4 arithmetic follows public upstream ggml

@@ -8,7 +8,7 @@ CPU side of the check, run once in the build container:
 Every linear weight goes through the CPU oracle's quantise -> dequantise (oracle/lowbit_oracle.c: the bytes
 ggml_quantize_tensor produces and the values ggml_dequantize gives back), the fp32 model is run by transformers'
 stock forwards and generate loop -- i.e. the reference's "mode B" semantics, x . dequant(W)^T in fp32
-(/root/reference/python/llm/src/ipex_llm/transformers/low_bit_linear.py:581-583, 741-742) -- and the 128 tokens are
+(python/llm/src/ipex_llm/transformers/low_bit_linear.py:581-583, 741-742) -- and the 128 tokens are
 stored in tests/golden/llama7b_sym_int4_tokens.json together with the margin of every greedy choice (top-1 minus
 top-2 logit), so that a later mismatch can be told apart from a near tie.  tests/test_llama7b_tokens.py reproduces the
 tokens on the GPU through ipex_llm.transformers.AutoModelForCausalLM.from_model(...).generate().
