@@ -208,9 +208,10 @@ __global__ void __launch_bounds__(DT, 2) delta_gram_kernel(const ChunkArgs a) {
             const double r = (warp ? a.q_scale : 1.0) * rsqrt(norms[tid] + 1e-6);
             const bool plain = r > 0.0;                 // no infinity, no NaN among the sums; then it lies between 2^-65 and 2^10
             const int hi = __double2hiint(r);
-            // the rest lies in [1/4, 1/2): U C_last / C_t times it splits into planes whenever U is finite
-            scale[tid] = plain ? __int_as_float(((hi >> 20) - 1023 + 2 + 127) << 23) : (float)r;
-            norms[tid] = plain ? __hiloint2double((hi & 0xfffff) | 0x3fd00000, __double2loint(r)) : 1.0;
+            // a key's rest lies in [1/4, 1/2): U C_last / C_t times it splits into planes whenever U is finite; a query's in [1, 2): Q M0 before it
+            // is no larger than the output
+            scale[tid] = plain ? __int_as_float(((hi >> 20) - 1023 + (warp ? 0 : 2) + 127) << 23) : (float)r;
+            norms[tid] = plain ? __hiloint2double((hi & 0xfffff) | (warp ? 0x3ff00000 : 0x3fd00000), __double2loint(r)) : 1.0;
         }
         __syncthreads();
 #pragma unroll

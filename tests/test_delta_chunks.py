@@ -192,3 +192,19 @@ def test_the_largest_values_enter_the_state(ops, cuda_device, dtype, at):
     o = ops.gated_delta_rule(conv, G, H, D, V, proj, 1, 1 + H, a_log, bias, state, 0, pad)
     assert float((o.double() - want_o).abs().max()) <= 2e-6 * float(want_o.abs().max())
     assert float((state.double() - want_s).abs().max()) <= 2e-6 * float(want_s.abs().max())
+
+
+def test_the_largest_outputs(ops, cuda_device):
+    """a state near the end of the range that is read and hardly changed: every partial product stays in the range as the outputs do"""
+    B, S, G, H, D, V = 1, 96, 1, 2, 128, 24
+    conv, proj, a_log, bias, state = inputs(cuda_device, B, S, G, H, D, V, torch.float32)
+    conv[..., :D].abs_()
+    conv[..., D:2 * D] -= conv[..., D:2 * D].mean(-1, keepdim=True)                # keys at right angles to the state's columns
+    proj[..., 1:1 + H], a_log = -30.0, a_log - 8.0
+    state.fill_(2e38)
+    pad = torch.zeros(B, dtype=torch.int32, device=cuda_device)
+    want_o, want_s = statement(conv, proj, a_log, bias, state, G, H, D, V, 0, pad)
+    assert float(want_o.abs().max()) > 1.5e38
+    o = ops.gated_delta_rule(conv, G, H, D, V, proj, 1, 1 + H, a_log, bias, state, 0, pad)
+    assert float((o.double() - want_o).abs().max()) <= 2e-6 * float(want_o.abs().max())
+    assert float((state.double() - want_s).abs().max()) <= 2e-6 * float(want_s.abs().max())
