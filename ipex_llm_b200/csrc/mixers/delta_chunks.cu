@@ -147,7 +147,8 @@ __device__ __forceinline__ uint32_t turned(uint32_t v) {
 
 // grid (chunks, key/value heads x parts, batch).  Everything of a chunk that needs no state: unit vectors, Gram matrices, gates, L, A,
 // (I + L)^-1 per head, and its products with keys and values.  A block is a chain of short phases (gates in double 3400 clocks, the inverse
-// 3500, the products 10000 for four heads), two blocks a SM: bound by their latencies.  2048 tokens, 4 / 16 heads of 128, bf16: 27 us for
+// 3500, the products 10000 for four heads), two blocks a SM: bound by their latencies; at the 128 registers that this leaves 16 bytes (bf16, 64
+// dims) to 156 (fp32, 128) are spilled.  2048 tokens, 4 / 16 heads of 128, bf16: 27 us for
 // 45 MB written (19 us without the solved right sides, which the walk multiplied out itself).  The products by mma.sync: as scalar fmas
 // (a column per thread) the matrix's broadcast loads fill the shared-memory pipe, 84 us
 template <typename T, int D>
@@ -593,7 +594,8 @@ __device__ __forceinline__ void split_pair(const float (&l)[4], const float (&r)
 // chain two exchanges between the four warps: the slices' sums of W M0, then U as planes, each summed and split by one warp.  Q M0 fills
 // the tensor pipe while they wait; A U and the stores belong to the other four warps and may lag a chunk behind.
 // Measured, 2048 tokens, 16 heads, 128 x 128, bf16: 70 us, 1940 clocks a chunk, of which 960 in the tensor pipe (120 instructions a SM
-// quarter, 8 clocks each); the rest is the chain's latency (the splits, the exchanges).  When T (V - C o (K M0)) was formed inside the
+// quarter, 8 clocks each); the rest is the chain's latency (the splits, the exchanges).  68 us since the copying warp asks for its phases as
+// a whole warp.  When T (V - C o (K M0)) was formed inside the
 // walk, with eight partial sums and three barriers, and keys took three planes: 141 us, 4100 clocks.  Error of the outputs against 64 bits,
 // relative to their norm: 1.00e-7 (1.05e-7 then).
 template <typename T, int D>
