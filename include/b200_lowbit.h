@@ -243,7 +243,8 @@ int lowbit_rope_kv_append_cuda(void* d_qkv, int dtype, int64_t batch_stride, int
  * (lowbit_rope_kv_append_cuda, lowbit_sdp_fp8_devlen_cuda) and need the workspace.  Same results as the separate calls.
  * cache_complete != 0: the caller guarantees that *d_len and the cached rows below it were written by work that has
  * COMPLETED when this call's kernel starts -- under programmatic dependent launch that means an ordinarily launched
- * kernel (or a stream synchronisation) lies between their producers and this call, as between two decode steps; the
+ * kernel (or a stream synchronisation) lies between their producers and this call, as between two decode steps (a matmul,
+ * an attention or a delta rule of this library that was launched with the switch off is not ordinarily launched); the
  * kernel then stages its first chunks of the cache while the previous kernel (the qkv projection) still drains.  0 is
  * always safe. */
 size_t lowbit_decode_attention_workspace_size(int B, int Hq, int Hkv, int capacity, int D);
@@ -391,9 +392,10 @@ int lowbit_matmul_f32_noalloc_cuda(const void* d_w, int qtype, int64_t n_rows, i
                                    const float* d_x, int64_t m, void* d_y, int y_dtype,
                                    const void* d_bias, int accumulate, void* stream);
 
-/* on != 0: the matmul kernels are launched with programmatic stream serialization (PDL): a
- * kernel may start streaming its weights while the previous kernel on the stream drains; it
- * reads activations only after griddepcontrol.wait.  Process-wide switch, default off. */
+/* on != 0: for recorded steps: the matmul kernels are launched with programmatic stream serialization (PDL): a
+ * kernel may start streaming its weights while the previous kernel on the stream drains (they must be complete before
+ * that one starts); it reads activations only after griddepcontrol.wait.  Process-wide switch, default off: launches outside a
+ * capture then overlap their starts too, but read nothing, weights included, ahead of the wait. */
 void lowbit_set_programmatic_dependent_launch(int on);
 int lowbit_get_programmatic_dependent_launch(void);
 
